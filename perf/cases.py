@@ -294,3 +294,101 @@ def tolerance(case: Case) -> Any:
     if case["path"] == "ortho":
         return {"rel": 3e-2, "max": 0.3} if bf16_iteration else {"rel": 1e-2, "max": 6e-2}
     return {"rel": 3e-3, "max": 3e-2} if bf16_iteration else {"rel": 8e-4, "max": 1e-2}
+
+
+# ---------------------------------------------------------------------------
+# the same results in 64 bits
+# ---------------------------------------------------------------------------
+_S = 1.05   # safety factor the Gram iteration divides its coefficients by, to the first, third and fifth power
+_GRAM = [(8.28721201814563 / _S, -23.595886519098837 / _S**3, 17.300387312530933 / _S**5),
+         (4.107059111542203 / _S, -2.9478499167379106 / _S**3, 0.5448431082926601 / _S**5),
+         (3.9486908534822946 / _S, -2.908902115962949 / _S**3, 0.5518191394370137 / _S**5),
+         (3.3184196573706015 / _S, -2.488488024314874 / _S**3, 0.51004894012372 / _S**5),
+         (2.300652019954817 / _S, -1.6689039845747493 / _S**3, 0.4188073119525673 / _S**5)]
+_POLAR = [(8.156554524902461, -22.48329292557795, 15.878769915207462),
+          (4.042929935166739, -2.808917465908714, 0.5000178451051316),
+          (3.8916678022926607, -2.772484153217685, 0.5060648178503393),
+          (3.285753657755655, -2.3681294933425376, 0.46449024233003106),
+          (2.3465413258596377, -1.7097828382687081, 0.42323551169305323)]
+# kind -> the five steps' coefficients and the factor on the Frobenius norm
+_ITERATIONS = {"gram": (_GRAM, 1.0), "polar_express": (_POLAR, 1.02), "keller": ([(3.4445, -4.7750, 2.0315)] * 5, 1.0)}
+MAX_EXACT_FLOPS = 1e14   # a few seconds of 64-bit products
+
+
+def _polar(matrix: Tensor, kind: str, epsilon: float = 1e-8) -> Tensor:
+    """The five-step polynomial of one matrix."""
+    if matrix.shape[0] > matrix.shape[1]:
+        return _polar(matrix.T, kind, epsilon).T
+    table, norm_scale = _ITERATIONS[kind]
+    x = matrix.double()
+    x = x / (x.norm() * norm_scale + epsilon)
+    for a, b, c in table:
+        gram = x @ x.T
+        x = a * x + (b * gram + c * (gram @ gram)) @ x
+    return x
+
+
+def exact(case: Case, seed: int) -> Any:
+    """What ``run`` returns for ``prepare(case, seed)``, in 64 bits; None where that takes too long."""
+    if case["path"] == "ortho":
+        small, large = sorted((case["rows"], case["cols"]))
+        if case["count"] * 20.0 * (small * small * large + small**3 / 2) > MAX_EXACT_FLOPS:
+            return None
+        x = prepare(case, seed)["x"]
+        return torch.stack([_polar(matrix, case["kind"]) for matrix in x])
+    cost = sum(blocks * 20.0 * (min(k, cols) ** 2 * max(k, cols) + min(k, cols) ** 3 / 2)
+               for blocks, _, k, cols, _ in _matrices(case))
+    if cost > MAX_EXACT_FLOPS:
+        return None
+    state = prepare(case, seed)
+    optimizer, outputs = state["optimizer"], state["outputs"]
+    # every buffer that holds results, by its address, as a 64-bit copy the results are written to
+    copies = {}
+    for buffer in (outputs["weights"], *outputs["slabs"], outputs["exp_avg"], outputs["exp_avg_sq"], outputs["steps"]):
+        copies[buffer.untyped_storage().data_ptr()] = buffer.double()
+
+    def at(tensor: Tensor) -> Tensor:
+        copy = copies[tensor.untyped_storage().data_ptr()]
+        return copy.as_strided(tensor.shape, tensor.stride(), tensor.storage_offset())
+
+    settings = {id(p): group for group in optimizer.param_groups for p in group["params"]}
+    kind = {"dion3": "gram", "muon": "keller", "polar": "polar_express"}[case["update"]]
+    nesterov, normuon = case["update"] == "muon", case["update"] != "muon"
+    matrices = iter(_matrices(case))
+    names = [name for name, shape in _shapes(case)]
+    for name, parameter in zip(names, state["model"].order):
+        group, entry = settings[id(parameter)], optimizer.state[parameter]
+        lr, decay = group["lr"], group["weight_decay"]
+        weight, grad = at(parameter), parameter.grad.double()
+        weight *= 1.0 - lr * decay
+        if parameter.ndim < 2 or _is_table(name):
+            beta1, beta2 = group["betas"]
+            mean, square, step = at(entry["exp_avg"]), at(entry["exp_avg_sq"]), at(entry["adamw_step"])
+            step += 1.0
+            mean.mul_(beta1).add_(grad, alpha=1.0 - beta1)
+            square.mul_(beta2).add_(grad * grad, alpha=1.0 - beta2)
+            root = square.sqrt() / math.sqrt(1.0 - beta2 ** float(step)) + group["eps"]
+            weight -= lr / (1.0 - beta1 ** float(step)) * mean / root
+            continue
+        blocks, rows, k, cols, _ = next(matrices)
+        size = -lr * 0.2 * math.sqrt(max(rows, cols)) * math.sqrt(min(rows, cols) / min(k, cols))
+        momentum = at(entry["momentum"]).view(blocks, rows, cols)
+        variance = at(entry["variance"]).view(blocks, rows)
+        momentum += grad.view(blocks, rows, cols)
+        for m, v, w, g in zip(momentum, variance, weight.view(blocks, rows, cols), grad.view(blocks, rows, cols)):
+            chosen = m.abs().sum(1).topk(k).indices if k < rows else torch.arange(rows, device=DEVICE)
+            source = m[chosen]
+            m[chosen] = group["momentum"] * source
+            update = _polar(group["momentum"] * source + g if nesterov else source, kind)
+            if normuon:
+                squares = (update * update).sum(1)
+                v[chosen] = torch.lerp(v[chosen], squares / cols, 1.0 - group["muon_beta2"])
+                divisor = v[chosen].sqrt() + 1e-8
+                update = update / divisor[:, None] * (squares.sum().sqrt() / (squares / divisor**2).sum().sqrt())
+            w[chosen] += size * update
+    result: dict[str, Any] = {
+        "weights": at(outputs["weights"]), "slabs": [at(slab) for slab in outputs["slabs"]],
+        "exp_avg": at(outputs["exp_avg"]), "exp_avg_sq": at(outputs["exp_avg_sq"]), "steps": at(outputs["steps"])}
+    if case["ema"]:
+        result["shadows"] = [at(p).clone() for p in state["model"].order]   # the first update copies the weights
+    return result
