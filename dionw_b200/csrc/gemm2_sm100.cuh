@@ -240,7 +240,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   int* tile_ring = reinterpret_cast<int*>(tile_empty + kTileSlots);  // [kTileSlots]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tile_ring + kTileSlots);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint16_t* mirror_stage = reinterpret_cast<uint16_t*>(smem + size_t(kStages) * kStageBytes + 256);
+  uint8_t* mirror_stage = smem + size_t(kStages) * kStageBytes + 256;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -267,6 +267,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (threadIdx.x == 0) {
+    prefetch_map(&map_a);
+    prefetch_map(&map_b);
   }
   if (warp == 1) tmem_alloc2(tmem_slot, kTmemCols);
   tc_fence_before();
@@ -390,7 +394,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     const int ew = warp - 2;
     const int sub = warp & 3;
     const int first_chunk = (ew >> 2) * (kBN / 64);
-    uint16_t* stage = mirror_stage + ew * 32 * kMirrorPitch;
+    uint8_t* stage = mirror_stage + ew * 2 * kPieceBytes;
     const uint32_t leader_empty[2] = {peer_address(&acc_empty[0], 0), peer_address(&acc_empty[1], 0)};
     bool ok = true;
     for (uint32_t local = 0; ok; ++local) {

@@ -34,8 +34,8 @@ constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;        // 32 KB
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
 constexpr uint32_t kPanelBytes = 64 * kBK * 2;     // one 64-column panel of an MN-major B stage
-constexpr int kMirrorPitch = 34;                   // halves per staged row: 17 words, conflict-free both ways
-constexpr uint32_t kMirrorBytes = 8 * 32 * kMirrorPitch * 2;  // one 32 x 32 staging tile per epilogue warp
+constexpr uint32_t kPieceBytes = 32 * 32 * 2;      // one 32 x 32 piece of the output, 64 bytes a row
+constexpr uint32_t kMirrorBytes = 8 * 2 * kPieceBytes;  // per epilogue warp: a piece as it lies and its transpose
 constexpr size_t kSmemBytes =
     size_t(kStages) * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/ + kMirrorBytes;
 
@@ -140,6 +140,11 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// Brings a kernel argument's tensor map into the descriptor cache; touches no data of the operands.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols)
                : "memory");
@@ -171,18 +176,42 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-__device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
+// 16 accumulator rows x 32 columns in the layout of an mma.m16n8 result: register 4g + q of lane l is
+// row l / 4 + 8 * (q / 2), column 8g + 2 * (l % 4) + q % 2.  Valid after tmem_wait.
+__device__ __forceinline__ void tmem_load_16x32(uint32_t taddr, uint32_t* v) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr)
       : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The registers pass through the wait, so that no use of them can be moved in front of it.
+__device__ __forceinline__ void tmem_wait(uint32_t (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+        "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+        "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+        "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+      :
+      : "memory");
+}
+
+// Four 8 x 8 matrices of 2-byte elements between registers (mma layout) and shared memory; lane l gives
+// the address of row l % 8 of matrix l / 8.  The transposing store writes column l % 8 there instead.
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void stmatrix4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};"
+               ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void stmatrix4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+               ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 // Shared-memory matrix descriptor, 128-byte swizzle, version 1 (Blackwell).
@@ -262,208 +291,268 @@ __device__ __forceinline__ Tile sym_tile(int t, const Params& p) {
   return tile;
 }
 
-template <typename OutT>
-__device__ __forceinline__ OutT from_float(float v);
+// Two values as one word of the 2-byte type (the first in the low half), and back.
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(float a, float b);
 template <>
-__device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
+__device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
 template <>
-__device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <typename T>
+__device__ __forceinline__ float2 unpack2(uint32_t w);
+template <>
+__device__ __forceinline__ float2 unpack2<__half>(uint32_t w) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+template <>
+__device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
 
 // ----------------------------------------------------------------------------
 // epilogue of one accumulator: 128 rows (m_base ..) x 256 columns (n_base ..) of batch
 // ``batch``, read from TMEM at ``tmem_acc`` by the warp that owns sub-partition ``sub``;
 // this warp handles chunks first_chunk .. first_chunk+3 of the eight 32-column chunks.
 // Returns false when the bounded wait for the accumulator ran out.
+//
+// A warp works on 32 x 32 pieces.  The accumulator is read in the mma result layout, because
+// stmatrix turns that into rows of the piece and, with .trans, into rows of its mirror image at four
+// instructions each; global memory is read and written in "piece order" (lane l holds the 8
+// consecutive elements at row 8*it + l/4, column 8*(l%4), it = 0..3), so one instruction touches
+// 8 rows x 64 contiguous bytes.  The two staging tiles keep 16-byte units at unit ^ (row/2 & 3):
+// stmatrix, ldmatrix and the 16-byte accesses all go without bank conflicts.  Every class of piece
+// takes this one path: matrix edges only guard the final 16-byte accesses.
+//
+// What bounds it: in products of one or two waves (small matrices) nothing hides this chain, in
+// longer ones it runs under the next tile's main loop.  The first version read the accumulator row
+// by row, transposed with 2-byte gathers and sent diagonal pieces of B != A and all edge pieces
+// through per-element loops: a 256^3 mirrored product with Cin took 15.7 us in a chain of products,
+// this takes 8.1; 6 blocks of 517^3 17.8 us against 12.6.
 // ----------------------------------------------------------------------------
 template <typename InT, typename OutT, bool kSym>
 __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_base, int n_base, uint32_t tmem_acc,
                                               uint64_t* acc_full_bar, uint32_t acc_phase, volatile int* abort_flag,
-                                              uint16_t* stage, int sub, int lane, int first_chunk) {
-  const InT* cin = reinterpret_cast<const InT*>(p.cin);
-  OutT* out = reinterpret_cast<OutT*>(p.out);
-  OutT* out2 = reinterpret_cast<OutT*>(p.out2);
-  const int row_in_tile = sub * 32 + lane;
-  const int row = m_base + row_in_tile;
+                                              uint8_t* stage, int sub, int lane, int first_chunk) {
+  const uint16_t* cin = p.cin ? reinterpret_cast<const uint16_t*>(p.cin) + size_t(batch) * p.cin_batch : nullptr;
+  uint16_t* out = reinterpret_cast<uint16_t*>(p.out) + size_t(batch) * p.out_batch;
+  uint16_t* out2 = kSym && p.out2 ? reinterpret_cast<uint16_t*>(p.out2) + size_t(batch) * p.out_batch : nullptr;
   const int row0 = m_base + sub * 32;
-  const bool row_ok = row < p.m;
-  const InT* cin_row = cin ? cin + size_t(batch) * p.cin_batch + size_t(row) * p.ldc : nullptr;
-  OutT* out_b = out + size_t(batch) * p.out_batch;
-  OutT* out2_b = out2 ? out2 + size_t(batch) * p.out_batch : nullptr;
   // Class of the 32 x 32 piece at (row0, col0) under the symmetric schedule:
   // 0 stored as it is; 1 strictly below the diagonal: stored and stored transposed;
-  // 2 strictly above: skipped (its mirror image writes it); 3 on the diagonal of a
-  // product with B != A: lower triangle stored and mirrored element by element.
+  // 2 strictly above: skipped (its mirror image writes it); 3 on the diagonal of a product with
+  // B != A, which is symmetric only up to rounding: the lower triangle is stored and mirrored, so
+  // that the stored matrix is exactly symmetric.
   auto class_of = [&](int col0) -> int {
     if constexpr (!kSym) return 0;
     if (col0 + 32 <= row0) return 1;
     if (col0 >= row0 + 32) return 2;
     return p.mirror_diagonal != 0 ? 3 : 0;
   };
-  // Pieces wholly inside the matrix move between global memory and registers in
-  // "piece order": lane l holds 8 consecutive elements of row 8*it + l/4 at column
-  // 8*(l%4), it = 0..3, so one instruction touches 8 rows x 64 contiguous bytes.  The
-  // accumulator arrives in "row order" (lane = row); a 32 x 34 staging tile in shared
-  // memory converts between the two.
-  const bool aligned = (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(out_b) & 15u) == 0 &&
-                       (out2_b == nullptr || (reinterpret_cast<uintptr_t>(out2_b) & 15u) == 0) &&
-                       (cin == nullptr || ((p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(cin) & 15u) == 0 &&
-                                           (p.cin_batch & 7) == 0));
-  const bool rows_inside = row0 + 32 <= p.m;
-  const int piece_row = lane >> 2, piece_col = (lane & 3) * 8;
-  auto fast_piece = [&](int col0, int cls) { return aligned && rows_inside && col0 + 32 <= p.n && cls != 3; };
-  // The epilogue is a chain of dependent latencies; the Cin piece of the next chunk is
-  // requested before the current chunk is worked on.  (Requesting all four chunks of a
-  // tile up front was measured slower: 48 more live registers for no shorter chain.)
+  const bool out_aligned = (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 &&
+                           (reinterpret_cast<uintptr_t>(out2) & 15u) == 0;
+  const bool cin_aligned = (p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(cin) & 15u) == 0;
+  const int piece_row = lane >> 2, piece_unit = lane & 3, piece_col = piece_unit * 8;
+  // 16 bytes of Cin at (r, c): elements outside the matrix read as zero.
+  auto get = [&](int r, int c) -> uint4 {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (r >= p.m || c >= p.n) return v;
+    const uint16_t* at = cin + size_t(r) * p.ldc + c;
+    if (cin_aligned && c + 8 <= p.n) return *reinterpret_cast<const uint4*>(at);
+    uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (c + j < p.n) w[j >> 1] |= uint32_t(at[j]) << (16 * (j & 1));
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  };
+  auto put = [&](uint16_t* base, int r, int c, const uint4& v) {
+    if (r >= p.m || c >= p.n) return;
+    uint16_t* at = base + size_t(r) * p.ldo + c;
+    if (out_aligned && c + 8 <= p.n) {
+      *reinterpret_cast<uint4*>(at) = v;
+      return;
+    }
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (c + j < p.n) at[j] = uint16_t(w[j >> 1] >> (16 * (j & 1)));
+  };
+  auto unit_at = [](int row, int unit) -> uint32_t { return uint32_t(row * 64 + ((unit ^ ((row >> 1) & 3)) << 4)); };
+  uint8_t* mirror = stage + kPieceBytes;
+  const uint32_t stage_u32 = smem_u32(stage), mirror_u32 = smem_u32(mirror);
+  // This lane's row addresses for the four matrices of one ldmatrix / stmatrix: rows 16h + 8 * (i % 2),
+  // columns 16 * pair + 8 * (i / 2) of the piece, i = lane / 8.
+  auto matrix_at = [&](int h, int pair) { return unit_at(16 * h + ((lane >> 3) & 1) * 8 + (lane & 7), 2 * pair + (lane >> 4)); };
+  auto mirror_at = [&](int h, int pair) { return unit_at(16 * pair + (lane >> 4) * 8 + (lane & 7), 2 * h + ((lane >> 3) & 1)); };
+
+  // The Cin piece of the next chunk is requested before the current chunk is worked on.
   uint4 ahead[4];
   auto prefetch = [&](int chunk) {
     const int col0 = n_base + chunk * 32;
-    const int cls = class_of(col0);
-    if (cin == nullptr || cls == 2 || !fast_piece(col0, cls)) return;
-    const InT* base = cin + size_t(batch) * p.cin_batch + size_t(row0 + piece_row) * p.ldc + col0 + piece_col;
+    if (cin == nullptr || class_of(col0) == 2) return;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) ahead[it] = *reinterpret_cast<const uint4*>(base + size_t(8 * it) * p.ldc);
+    for (int it = 0; it < 4; ++it) ahead[it] = get(row0 + 8 * it + piece_row, col0 + piece_col);
   };
   prefetch(first_chunk);   // does not depend on the accumulator: overlaps the wait below
   if (!mbar_wait(acc_full_bar, acc_phase, abort_flag, p.status, p.wait_ns)) return false;
   tc_fence_after();
-  uint32_t* my_row = reinterpret_cast<uint32_t*>(stage + lane * kMirrorPitch);
-  // Sum of the squares of this row's rounded results over the warp's 128 columns, for NorMuon:
-  // the value is in registers here, so the row statistics need no second pass over the output.
-  // One partial per (row, 128 columns), added left to right: the order is fixed.
+  // Sums of the squares of the rounded results over the warp's 128 columns, for NorMuon: the values are
+  // in registers here, so the row statistics need no second pass over the output.  Lane l sums its
+  // columns of rows l/4 + 8i; the four lanes of a row are added at the end: the order is fixed.
   const bool want_sq = !kSym && p.rowsq != nullptr;
-  float sq = 0.0f;
+  float sq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
   for (int chunk = first_chunk; chunk < first_chunk + kBN / 64; ++chunk) {
     const int col0 = n_base + chunk * 32;
+    if (col0 >= p.n || row0 >= p.m) break;   // uniform over the warp
     const int cls = class_of(col0);
-    uint4 now[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) now[j] = ahead[j];
-    if (chunk + 1 < first_chunk + kBN / 64) prefetch(chunk + 1);
-    if (col0 >= p.n) break;       // uniform over the warp
-    if (cls == 2) continue;       // uniform over the warp
+    if (cls == 2) break;          // uniform over the warp; the chunks after it lie above the diagonal too
     uint32_t v[32];
     const uint32_t taddr = tmem_acc + (uint32_t(sub * 32) << 16) + uint32_t(chunk * 32);
-    tmem_load32(taddr, v);
-    if (fast_piece(col0, cls)) {
-      __align__(16) OutT r[32];
-      if (cin != nullptr) {
-        // Cin: piece order -> staging tile -> row order
+    tmem_load_16x32(taddr, v);
+    tmem_load_16x32(taddr + (16u << 16), v + 16);
+    uint32_t r[16];               // [half of the rows][column group of 8][row / 8 in the half]
+    if (cin != nullptr) {
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
-          uint32_t* dst = reinterpret_cast<uint32_t*>(stage + (8 * it + piece_row) * kMirrorPitch + piece_col);
-          dst[0] = now[it].x; dst[1] = now[it].y; dst[2] = now[it].z; dst[3] = now[it].w;
-        }
-        __syncwarp();
-        __align__(16) InT c[32];
-        uint32_t* cw = reinterpret_cast<uint32_t*>(c);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) cw[j] = my_row[j];
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          r[j] = from_float<OutT>(fmaf(p.beta, to_float<InT>(c[j]), p.alpha * __uint_as_float(v[j])));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = from_float<OutT>(p.alpha * __uint_as_float(v[j]));
-      }
-      if (want_sq) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float f = to_float<OutT>(r[j]);
-          sq = fmaf(f, f, sq);
-        }
-      }
-      // result: row order -> staging tile
-      const uint32_t* words = reinterpret_cast<const uint32_t*>(r);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) my_row[j] = words[j];
+      for (int it = 0; it < 4; ++it)
+        *reinterpret_cast<uint4*>(stage + unit_at(8 * it + piece_row, piece_unit)) = ahead[it];
+      if (chunk + 1 < first_chunk + kBN / 64) prefetch(chunk + 1);
       __syncwarp();
-      // stored as it is, in piece order
+      uint32_t c[16];
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
-        const int lr = 8 * it + piece_row;
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(stage + lr * kMirrorPitch + piece_col);
-        uint4 piece = make_uint4(src[0], src[1], src[2], src[3]);
-        const size_t at = size_t(row0 + lr) * p.ldo + col0 + piece_col;
-        *reinterpret_cast<uint4*>(out_b + at) = piece;
-        if constexpr (kSym) {
-          if (out2_b != nullptr) {
-            const int d = row0 + lr - (col0 + piece_col);  // position of the diagonal inside the 8 elements
-            if (d >= 0 && d < 8) {
-              OutT* e = reinterpret_cast<OutT*>(&piece);
-              e[d] = from_float<OutT>(to_float<OutT>(e[d]) + p.diag);
-            }
-            *reinterpret_cast<uint4*>(out2_b + at) = piece;
-          }
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int pair = 0; pair < 2; ++pair) {
+          uint32_t* f = c + 8 * h + 4 * pair;
+          ldmatrix4(stage_u32 + matrix_at(h, pair), f[0], f[1], f[2], f[3]);
         }
+      tmem_wait(v);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float2 cf = unpack2<InT>(c[j]);
+        r[j] = pack2<OutT>(fmaf(p.beta, cf.x, p.alpha * __uint_as_float(v[2 * j])),
+                           fmaf(p.beta, cf.y, p.alpha * __uint_as_float(v[2 * j + 1])));
       }
-      if constexpr (kSym) {
+      __syncwarp();               // every lane has its part of Cin: the staging tile is free
+    } else {
+      tmem_wait(v);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        r[j] = pack2<OutT>(p.alpha * __uint_as_float(v[2 * j]), p.alpha * __uint_as_float(v[2 * j + 1]));
+    }
+    if (want_sq) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int column = col0 + (j >> 1 & 3) * 8 + (lane & 3) * 2;
+        const float2 f = unpack2<OutT>(r[j]);
+        float& sum = sq[2 * (j >> 3) + (j & 1)];
+        if (column < p.n) sum = fmaf(f.x, f.x, sum);
+        if (column + 1 < p.n) sum = fmaf(f.y, f.y, sum);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int pair = 0; pair < 2; ++pair) {
+        const uint32_t* f = r + 8 * h + 4 * pair;
+        stmatrix4(stage_u32 + matrix_at(h, pair), f[0], f[1], f[2], f[3]);
+        if (kSym && cls != 0) stmatrix4_trans(mirror_u32 + mirror_at(h, pair), f[0], f[1], f[2], f[3]);
+      }
+    __syncwarp();
+    // Whole pieces, which are nearly all, go out with plain 16-byte stores, the four loads first.
+    const bool whole = out_aligned && row0 + 32 <= p.m && col0 + 32 <= p.n;   // uniform over the warp
+    uint4 piece[4];
+#pragma unroll
+    for (int it = 0; it < 4; ++it)
+      piece[it] = *reinterpret_cast<const uint4*>(stage + unit_at(8 * it + piece_row, piece_unit));
+    if constexpr (kSym) {
+      if (cls != 0) {
+        uint4 other[4];
+#pragma unroll
+        for (int it = 0; it < 4; ++it)
+          other[it] = *reinterpret_cast<const uint4*>(mirror + unit_at(8 * it + piece_row, piece_unit));
         if (cls == 1) {
-          // stored transposed: gather columns of the staging tile
-          const int seg = lane & 3;
+          if (whole) {
+            const size_t at = size_t(col0 + piece_row) * p.ldo + row0 + piece_col;
+#pragma unroll
+            for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out + at + size_t(8 * it) * p.ldo) = other[it];
+            if (out2 != nullptr) {
+#pragma unroll
+              for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out2 + at + size_t(8 * it) * p.ldo) = other[it];
+            }
+          } else {
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              put(out, col0 + 8 * it + piece_row, row0 + piece_col, other[it]);
+              if (out2 != nullptr) put(out2, col0 + 8 * it + piece_row, row0 + piece_col, other[it]);
+            }
+          }
+        } else {
+          // elements above the diagonal come from the mirror image; here row0 == col0
 #pragma unroll
           for (int it = 0; it < 4; ++it) {
-            const int cc = (lane >> 2) + 8 * it;  // source column = destination row
-            __align__(16) uint16_t gathered[8];
+            uint32_t* w = reinterpret_cast<uint32_t*>(&piece[it]);
+            const uint32_t o[4] = {other[it].x, other[it].y, other[it].z, other[it].w};
 #pragma unroll
-            for (int q = 0; q < 8; ++q) gathered[q] = stage[(seg * 8 + q) * kMirrorPitch + cc];
-            const size_t at = size_t(col0 + cc) * p.ldo + row0 + seg * 8;
-            *reinterpret_cast<uint4*>(out_b + at) = *reinterpret_cast<const uint4*>(gathered);
-            if (out2_b != nullptr)
-              *reinterpret_cast<uint4*>(out2_b + at) = *reinterpret_cast<const uint4*>(gathered);
+            for (int j = 0; j < 4; ++j) {
+              uint32_t mask = 0;
+              if (piece_col + 2 * j > 8 * it + piece_row) mask |= 0x0000FFFFu;
+              if (piece_col + 2 * j + 1 > 8 * it + piece_row) mask |= 0xFFFF0000u;
+              w[j] = (w[j] & ~mask) | (o[j] & mask);
+            }
           }
         }
       }
-      __syncwarp();
-      continue;
     }
-    // ---- pieces at the matrix edge, unaligned operands, symmetrised diagonal pieces: one row per lane
-    if (!row_ok) continue;
-    __align__(16) OutT r[32];
-    __align__(16) OutT r2[32];
+    const size_t at = size_t(row0 + piece_row) * p.ldo + col0 + piece_col;
+    if (whole) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      float x = p.alpha * __uint_as_float(v[j]);
-      if (cin_row != nullptr && col0 + j < p.n) x = fmaf(p.beta, to_float<InT>(cin_row[col0 + j]), x);
-      r[j] = from_float<OutT>(x);
-      if (want_sq && col0 + j < p.n) {
-        const float f = to_float<OutT>(r[j]);
-        sq = fmaf(f, f, sq);
-      }
-      if constexpr (kSym) r2[j] = (row == col0 + j) ? from_float<OutT>(to_float<OutT>(r[j]) + p.diag) : r[j];
+      for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out + at + size_t(8 * it) * p.ldo) = piece[it];
+    } else {
+#pragma unroll
+      for (int it = 0; it < 4; ++it) put(out, row0 + 8 * it + piece_row, col0 + piece_col, piece[it]);
     }
-    OutT* dst = out_b + size_t(row) * p.ldo + col0;
-    if (cls == 3) {
-      // A B^T with B != A is symmetric only up to rounding: keep the lower triangle of
-      // the diagonal piece and mirror it, so that the stored matrix is exactly symmetric.
-      for (int j = 0; j < 32; ++j) {
-        const int col = col0 + j;
-        if (col > row || col >= p.n) continue;
-        dst[j] = r[j];
-        if (out2_b != nullptr) out2_b[size_t(row) * p.ldo + col] = r2[j];
-        if (col < row) {
-          out_b[size_t(col) * p.ldo + row] = r[j];
-          if (out2_b != nullptr) out2_b[size_t(col) * p.ldo + row] = r[j];
+    if constexpr (kSym) {
+      if (out2 != nullptr) {
+        if (row0 == col0) {       // the piece on the diagonal: pieces and diagonal are both 32-aligned
+#pragma unroll
+          for (int it = 0; it < 4; ++it) {
+            uint32_t* w = reinterpret_cast<uint32_t*>(&piece[it]);
+            const int d = 8 * it + piece_row - piece_col;   // its position inside the 8 elements
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = unpack2<OutT>(w[j]);
+              if (d == 2 * j) w[j] = pack2<OutT>(f.x + p.diag, f.y);
+              if (d == 2 * j + 1) w[j] = pack2<OutT>(f.x, f.y + p.diag);
+            }
+          }
         }
-      }
-      continue;
-    }
-    for (int j = 0; j < 32; ++j) {
-      if (col0 + j >= p.n) break;
-      dst[j] = r[j];
-      if constexpr (kSym) {
-        if (out2_b != nullptr) out2_b[size_t(row) * p.ldo + col0 + j] = r2[j];
-        if (cls == 1) {
-          out_b[size_t(col0 + j) * p.ldo + row] = r[j];
-          if (out2_b != nullptr) out2_b[size_t(col0 + j) * p.ldo + row] = r[j];
+        if (whole) {
+#pragma unroll
+          for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out2 + at + size_t(8 * it) * p.ldo) = piece[it];
+        } else {
+#pragma unroll
+          for (int it = 0; it < 4; ++it) put(out2, row0 + 8 * it + piece_row, col0 + piece_col, piece[it]);
         }
       }
     }
+    __syncwarp();                 // the staging tiles are read: the next chunk may write them
   }
-  if (want_sq && row_ok) {
+  if (want_sq) {
     const int part = 2 * (n_base / kBN) + first_chunk / (kBN / 64);
-    p.rowsq[(size_t(batch) * p.m + row) * p.rowsq_parts + part] = sq;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float sum = sq[i];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      const int row = row0 + 8 * i + piece_row;
+      if (piece_unit == 0 && row < p.m) p.rowsq[(size_t(batch) * p.m + row) * p.rowsq_parts + part] = sum;
+    }
   }
   return true;
 }
@@ -482,7 +571,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   uint64_t* acc_empty = acc_full + 2;         // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint16_t* mirror_stage = reinterpret_cast<uint16_t*>(smem + size_t(kStages) * kStageBytes + 256);
+  uint8_t* mirror_stage = smem + size_t(kStages) * kStageBytes + 256;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -501,6 +590,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (threadIdx.x == 0) {
+    prefetch_map(&map_a);
+    prefetch_map(&map_b);
   }
   if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
   tc_fence_before();
@@ -578,7 +671,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int ew = warp - 2;                  // 0..7
     const int sub = warp & 3;                 // TMEM lanes 32*sub .. 32*sub+31
     const int first_chunk = (ew >> 2) * (kBN / 64);
-    uint16_t* stage = mirror_stage + ew * 32 * kMirrorPitch;
+    uint8_t* stage = mirror_stage + ew * 2 * kPieceBytes;
     uint32_t local = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local) {

@@ -1,0 +1,77 @@
+"""The products' epilogue at the sizes where they can go wrong.
+
+Products are held to the fp64 product of the same 2-byte operands.  One rounding of the result to fp16
+(2^-11 relative) or bf16 (2^-8) and fp32 accumulation of at most 600 terms (below 600 * 2^-24 of the sum
+of magnitudes) bound the difference.
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from dionw_b200 import _native as native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+SENTINEL = 77.0
+
+
+def _padded(n: int) -> int:
+    return (n + 7) // 8 * 8
+
+
+def _operand(gen: torch.Generator, blocks: int, rows: int, cols: int, dtype: torch.dtype) -> torch.Tensor:
+    x = torch.zeros(blocks, rows, _padded(cols), dtype=dtype)
+    x[..., :cols] = (torch.randn(blocks, rows, cols, generator=gen) * 0.1).to(dtype)
+    return x.to(DEV)
+
+
+def _close(got: torch.Tensor, want: torch.Tensor, magnitude: torch.Tensor, dtype: torch.dtype) -> None:
+    rounding = 2.0**-11 if dtype is torch.float16 else 2.0**-8
+    bound = rounding * want.abs() * 1.01 + 600 * 2.0**-24 * magnitude + 1e-7
+    assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m", [1, 8, 31, 33, 64, 127, 130, 256, 257, 517])
+def test_symmetric_products_at_every_edge(m: int, dtype: torch.dtype) -> None:
+    gen = torch.Generator().manual_seed(m)
+    blocks, k = 2, 45 + m
+    a = _operand(gen, blocks, m, k, dtype)
+    a64 = a[..., :k].double()
+    want = a64 @ a64.mT
+    size = a64.abs() @ a64.mT.abs()
+    out = torch.full((blocks, m, _padded(m)), SENTINEL, dtype=dtype, device=DEV)
+    out2 = out.clone()
+    native.symmetric_product(a[..., :k], out[..., :m])
+    _close(out[..., :m], want, size, dtype)
+    assert torch.equal(out[..., :m], out[..., :m].mT) and bool((out[..., m:] == SENTINEL).all())
+    # the polynomial form: Cin, two outputs, the second with a diagonal added to the rounded first
+    g = out.clone()
+    native.symmetric_product(g[..., :m], out[..., :m], cin=g[..., :m], alpha=0.5, beta=-1.25, out2=out2[..., :m], diag=2.5)
+    g64 = g[..., :m].double()
+    _close(out[..., :m], 0.5 * g64 @ g64 - 1.25 * g64, 0.5 * g64.abs() @ g64.abs() + 1.25 * g64.abs(), dtype)
+    eye = torch.eye(m, device=DEV)
+    assert torch.equal(out2[..., :m], (out[..., :m].float() + 2.5 * eye).to(dtype))
+    # B != A, symmetric and commuting (a polynomial of A): exactly symmetric although only one triangle is computed
+    z = out.clone()
+    native.symmetric_product(g[..., :m], out[..., :m], b=z[..., :m], cin=g[..., :m], beta=1.5)
+    z64 = z[..., :m].double()
+    lower = torch.tril(g64 @ z64 + 1.5 * g64)
+    _close(torch.tril(out[..., :m].double()), lower, g64.abs() @ z64.abs() + 1.5 * g64.abs(), dtype)
+    assert torch.equal(out[..., :m], out[..., :m].mT) and bool((out[..., m:] == SENTINEL).all())
+
+
+@pytest.mark.parametrize("m, n, k", [(1, 1, 1), (33, 70, 40), (130, 259, 65), (256, 256, 256), (300, 31, 129)])
+@pytest.mark.parametrize("ld_extra", [0, 8, 3])
+def test_general_products_leave_everything_outside_alone(m: int, n: int, k: int, ld_extra: int) -> None:
+    """Also with an output whose rows are not 16-byte aligned (``ld_extra`` 3)."""
+    gen = torch.Generator().manual_seed(n)
+    a, b = _operand(gen, 2, m, k, torch.float16), _operand(gen, 2, k, n, torch.float16)
+    c = torch.randn(2, m, _padded(n) + ld_extra, generator=gen).half().to(DEV)
+    out = torch.full((2, m, _padded(n) + ld_extra), SENTINEL, dtype=torch.float16, device=DEV)
+    native.batched_gemm(a[..., :k], b[..., :n], out[..., :n], b_is_nk=False, cin=c[..., :n], beta=-0.5)
+    a64, b64, c64 = a[..., :k].double(), b[..., :n].double(), c[..., :n].double()
+    _close(out[..., :n], a64 @ b64 - 0.5 * c64, a64.abs() @ b64.abs() + 0.5 * c64.abs(), torch.float16)
+    assert bool((out[..., n:] == SENTINEL).all())
