@@ -51,6 +51,9 @@ SIGNATURES: dict[str, tuple[object, tuple[object, ...]]] = {
     "dionw_pack_rows": (
         c_int, (c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_float, c_int, c_float, c_float,
                 c_void_p, c_int, c_int64, c_void_p)),
+    "dionw_normalize_pack": (
+        c_int, (c_void_p, c_int, c_int64, c_int64, c_int64, c_float, c_float, c_void_p, c_int, c_int64, c_void_p,
+                c_void_p, c_void_p)),
     "dionw_transpose_2byte": (c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p)),
     "dionw_newton_schulz_workspace_bytes": (c_size_t, (c_int64, c_int64, c_int64, c_int)),
     "dionw_newton_schulz": (
@@ -226,6 +229,16 @@ def pack_rows(src: Tensor, index: Tensor | None, frob: Tensor, k: int, x: Tensor
     _check(library().dionw_pack_rows(src.data_ptr(), _ptr(index), frob.data_ptr(), blocks, rows, k, cols, decay,
                                      int(decay_rows), eps, norm_scale, x.data_ptr(), dtype_code(x.dtype),
                                      x.stride(-2), _stream(src)))
+
+
+def normalize_pack(src: Tensor, x: Tensor, *, eps: float, norm_scale: float = 1.0) -> None:
+    """``x = src / (norm * norm_scale + eps)`` per block, for a contiguous batch of any of the three dtypes."""
+    blocks, rows, cols = src.shape
+    scratch = torch.empty(blocks * rows + blocks, dtype=torch.float32, device=src.device)
+    sums = scratch.data_ptr()
+    _check(library().dionw_normalize_pack(src.data_ptr(), dtype_code(src.dtype), blocks, rows, cols, eps, norm_scale,
+                                          x.data_ptr(), dtype_code(x.dtype), x.stride(-2), sums,
+                                          sums + 4 * blocks * rows, _stream(src)))
 
 
 def transpose_2byte(src: Tensor, dst: Tensor) -> None:

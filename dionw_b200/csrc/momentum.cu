@@ -443,6 +443,167 @@ pack_rows_kernel(float* __restrict__ src, const int32_t* __restrict__ index, con
   for (long long e = cols + lane; e < ldx; e += 32) dst[e] = 0;
 }
 
+// ---------------------------------------------------------------------------
+// normalise + pack a caller's own batch
+// ---------------------------------------------------------------------------
+// 16 bytes of a row as floats: 4 elements of a 4-byte type, 8 of a 2-byte type.
+template <typename S>
+struct Quad;
+template <>
+struct Quad<float> {
+  static constexpr int kCount = 4;
+  static __device__ __forceinline__ void unpack(const uint4& raw, float (&out)[4]) {
+    out[0] = __uint_as_float(raw.x); out[1] = __uint_as_float(raw.y);
+    out[2] = __uint_as_float(raw.z); out[3] = __uint_as_float(raw.w);
+  }
+};
+template <>
+struct Quad<__half> {
+  static constexpr int kCount = 8;
+  static __device__ __forceinline__ void unpack(const uint4& raw, float (&out)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+      out[2 * i] = f.x; out[2 * i + 1] = f.y;
+    }
+  }
+};
+template <>
+struct Quad<__nv_bfloat16> {
+  static constexpr int kCount = 8;
+  static __device__ __forceinline__ void unpack(const uint4& raw, float (&out)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      out[2 * i] = __uint_as_float(w[i] << 16); out[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+  }
+};
+
+// A row in steps of 4 x 16 bytes per lane, all four requested before the first is used; `use` gets the
+// position of the first element and up to kCount elements (`count` of them; 0 past the row end).
+template <typename S, typename Use>
+__device__ __forceinline__ void walk_row(const S* __restrict__ row, long long cols, bool vec, int lane, Use&& use) {
+  constexpr int kUnroll = 4, kCount = Quad<S>::kCount;
+  for (long long e0 = kCount * lane; e0 < cols; e0 += 32 * kCount * kUnroll) {
+    if (vec) {
+      uint4 raw[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const long long e = e0 + 32LL * kCount * u;
+        if (e < cols) raw[u] = *reinterpret_cast<const uint4*>(row + e);
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const long long e = e0 + 32LL * kCount * u;
+        if (e >= cols) break;
+        float v[kCount];
+        Quad<S>::unpack(raw[u], v);
+        use(e, v, kCount);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const long long e = e0 + 32LL * kCount * u;
+        if (e >= cols) break;
+        float v[kCount];
+#pragma unroll
+        for (int i = 0; i < kCount; ++i) v[i] = e + i < cols ? to_float<S>(row[e + i]) : 0.0f;
+        use(e, v, cols - e < kCount ? int(cols - e) : kCount);
+      }
+    }
+  }
+}
+
+// Row sums of squares (of the values rounded to bf16 first for the bf16 iterations) and the normalised
+// 2-byte operand, straight from the caller's dtype.  HBM-bound: two reads of the source and one write
+// of the operand are all the traffic (the norm needs the whole block before the first division).  A
+// conversion to fp32 and a library norm in front of the pack moved 18 bytes per bf16 element instead
+// of 6: 16 blocks of 4096 x 14336 spent 5.4 ms of a 38.7 ms call in those three.
+template <typename S, bool kBf16>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+source_sumsq_kernel(const S* __restrict__ src, long long total_rows, long long cols, float* __restrict__ sumsq,
+                    bool vec) {
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (row >= total_rows) return;
+  float acc[Quad<S>::kCount] = {};
+  walk_row<S>(src + row * cols, cols, vec, lane, [&](long long, const float* v, int) {
+#pragma unroll
+    for (int i = 0; i < Quad<S>::kCount; ++i) {
+      const float x = kBf16 ? bf16_round(v[i]) : v[i];
+      acc[i] = fmaf(x, x, acc[i]);
+    }
+  });
+  float sum = 0.0f;
+#pragma unroll
+  for (int width = Quad<S>::kCount / 2; width >= 1; width >>= 1)
+#pragma unroll
+    for (int i = 0; i < width; ++i) acc[i] += acc[i + width];
+  sum = acc[0];
+#pragma unroll
+  for (int delta = 16; delta >= 1; delta >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, delta);
+  if (lane == 0) sumsq[row] = sum;
+}
+
+template <typename S, bool kBf16>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+source_pack_kernel(const S* __restrict__ src, const float* __restrict__ frob, long long total_rows, long long rows,
+                   long long cols, float eps, float norm_scale, uint16_t* __restrict__ x, long long ldx, bool vec) {
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (row >= total_rows) return;
+  const float norm = frob[row / rows];
+  // The bf16 iterations normalise in bf16: norm, scaled norm and sum are each rounded.
+  const float denom = kBf16 ? bf16_round(bf16_round(bf16_round(norm) * norm_scale) + eps) : __fadd_rn(norm, eps);
+  uint16_t* dst = x + row * ldx;
+  walk_row<S>(src + row * cols, cols, vec, lane, [&](long long e, const float* v, int count) {
+    constexpr int kCount = Quad<S>::kCount;
+    uint32_t w[kCount / 2];
+#pragma unroll
+    for (int i = 0; i < kCount / 2; ++i) {
+      float2 q;
+      q.x = __fdiv_rn(kBf16 ? bf16_round(v[2 * i]) : v[2 * i], denom);
+      q.y = __fdiv_rn(kBf16 ? bf16_round(v[2 * i + 1]) : v[2 * i + 1], denom);
+      if (kBf16) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(q.x, q.y);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+      } else {
+        const __half2 h = __floats2half2_rn(q.x, q.y);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+    }
+    if (vec) {
+      if constexpr (kCount == 8) *reinterpret_cast<uint4*>(dst + e) = make_uint4(w[0], w[1], w[2], w[3]);
+      else *reinterpret_cast<uint2*>(dst + e) = make_uint2(w[0], w[1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kCount; ++i)
+        if (i < count) dst[e + i] = uint16_t(w[i >> 1] >> (16 * (i & 1)));
+    }
+  });
+  for (long long e = cols + lane; e < ldx; e += 32) dst[e] = 0;   // padding adds nothing to any product
+}
+
+template <typename S, bool kBf16>
+int source_pack(const void* src, int64_t blocks, int64_t rows, int64_t cols, float eps, float norm_scale, void* x,
+                int64_t ldx, float* sumsq, float* frob, cudaStream_t stream) {
+  const long long total = blocks * rows;
+  const unsigned grid = unsigned((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  const S* typed = static_cast<const S*>(src);
+  const bool vec = cols % Quad<S>::kCount == 0 && aligned16(src) && aligned16(x);   // ldx is a multiple of 8
+  source_sumsq_kernel<S, kBf16><<<grid, kWarpsPerBlock * 32, 0, stream>>>(typed, total, cols, sumsq, vec);
+  int st = launch_status("source_sumsq_kernel");
+  if (st != DIONW_OK) return st;
+  block_norms_kernel<<<unsigned(blocks), kSelectThreads, 0, stream>>>(sumsq, int(rows), frob);
+  st = launch_status("block_norms_kernel");
+  if (st != DIONW_OK) return st;
+  source_pack_kernel<S, kBf16><<<grid, kWarpsPerBlock * 32, 0, stream>>>(typed, frob, total, rows, cols, eps, norm_scale,
+                                                                         static_cast<uint16_t*>(x), ldx, vec);
+  return launch_status("source_pack_kernel");
+}
+
 __global__ void transpose_2byte_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, long long rows,
                                        long long cols, long long ld_in, long long ld_out) {
   __shared__ uint16_t tile[64][66];
@@ -585,6 +746,25 @@ extern "C" int dionw_pack_rows(float* src, const int32_t* index, const float* fr
                                                                        decay_rows != 0, eps, norm_scale,
                                                                        static_cast<uint16_t*>(x), ldx, vec);
   return launch_status("pack_rows_kernel");
+}
+
+extern "C" int dionw_normalize_pack(const void* src, int src_dtype, int64_t blocks, int64_t rows, int64_t cols,
+                                    float eps, float norm_scale, void* x, int x_dtype, int64_t ldx, float* sumsq,
+                                    float* frob, void* stream_ptr) {
+  DIONW_REQUIRE(blocks > 0 && rows > 0 && cols > 0, "normalize_pack: empty problem");
+  DIONW_REQUIRE(rows < (1LL << 30), "normalize_pack: too many rows");
+  DIONW_REQUIRE(src_dtype >= DIONW_F32 && src_dtype <= DIONW_BF16, "normalize_pack: bad source dtype");
+  DIONW_REQUIRE(x_dtype == DIONW_F16 || x_dtype == DIONW_BF16, "normalize_pack: x must be F16 or BF16");
+  DIONW_REQUIRE(ldx >= cols && ldx % 8 == 0, "normalize_pack: ldx must be >= cols and a multiple of 8");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+#define DIONW_SOURCE(type)                                                                                       \
+  return x_dtype == DIONW_BF16                                                                                   \
+             ? source_pack<type, true>(src, blocks, rows, cols, eps, norm_scale, x, ldx, sumsq, frob, stream)    \
+             : source_pack<type, false>(src, blocks, rows, cols, eps, norm_scale, x, ldx, sumsq, frob, stream)
+  if (src_dtype == DIONW_F32) DIONW_SOURCE(float);
+  if (src_dtype == DIONW_F16) DIONW_SOURCE(__half);
+  DIONW_SOURCE(__nv_bfloat16);
+#undef DIONW_SOURCE
 }
 
 extern "C" int dionw_transpose_2byte(const void* in, void* out, int64_t blocks, int64_t rows, int64_t cols,

@@ -54,14 +54,10 @@ class NativeOrthogonalizer:
         if not matrix.is_cuda:
             raise ValueError("dionw_b200 orthogonalizes on CUDA devices only")
         blocks, rows, cols = matrix.shape
-        src = matrix.float().contiguous()
-        if self.dtype is torch.bfloat16:
-            frob = src.bfloat16().norm(dim=(-2, -1)).float()
-        else:
-            frob = torch.linalg.vector_norm(src, dim=(-2, -1))
+        src = matrix if matrix.dtype in (torch.float32, torch.float16, torch.bfloat16) else matrix.float()
+        src = src.contiguous()
         x = torch.empty(blocks, rows, padded(cols), dtype=self.dtype, device=src.device)
-        _native.pack_rows(src, None, frob, rows, x, decay=1.0, decay_rows=False, eps=epsilon,
-                          norm_scale=self.norm_scale)
+        _native.normalize_pack(src, x, eps=epsilon, norm_scale=self.norm_scale)
         scratch = torch.empty(self.workspace_bytes(blocks, rows, cols), dtype=torch.uint8, device=src.device)
         xt = None
         if rows > cols:

@@ -126,6 +126,15 @@ int dionw_pack_rows(float* src, const int32_t* index, const float* frob,
                     float decay, int decay_rows, float eps, float norm_scale,
                     void* x, int x_dtype, int64_t ldx, void* stream);
 
+/* x = half(src / (||src[b]||_F + eps)) for a caller's own batch src [blocks, rows,
+ * cols] of any of the three dtypes, contiguous; x is [blocks, rows, ldx] in x_dtype
+ * (BF16: the forms described at dionw_pack_rows).  sumsq [blocks * rows] and frob
+ * [blocks] are scratch.  Replaces the cast, norm and division at the head of
+ * src/dionw/_gram.py:85-87 and src/dionw/_polar_express.py:88-92. */
+int dionw_normalize_pack(const void* src, int src_dtype, int64_t blocks, int64_t rows,
+                         int64_t cols, float eps, float norm_scale, void* x, int x_dtype,
+                         int64_t ldx, float* sumsq, float* frob, void* stream);
+
 /* out[b, c, r] = in[b, r, c] for 2-byte elements (tall blocks are iterated in
  * their wide orientation, src/dionw/_gram.py:83-84, :89). */
 int dionw_transpose_2byte(const void* in, void* out, int64_t blocks, int64_t rows,

@@ -1,4 +1,4 @@
-"""The products' epilogue at the sizes where they can go wrong.
+"""The products' epilogue, the tall iteration and the normalising pack at the sizes where they can go wrong.
 
 Products are held to the fp64 product of the same 2-byte operands.  One rounding of the result to fp16
 (2^-11 relative) or bf16 (2^-8) and fp32 accumulation of at most 600 terms (below 600 * 2^-24 of the sum
@@ -75,3 +75,20 @@ def test_general_products_leave_everything_outside_alone(m: int, n: int, k: int,
     a64, b64, c64 = a[..., :k].double(), b[..., :n].double(), c[..., :n].double()
     _close(out[..., :n], a64 @ b64 - 0.5 * c64, a64.abs() @ b64.abs() + 0.5 * c64.abs(), torch.float16)
     assert bool((out[..., n:] == SENTINEL).all())
+
+
+@pytest.mark.parametrize("rows, cols", [(1, 1), (3, 1000), (40, 33), (257, 264), (64, 4100)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_normalize_pack_matches_the_fp32_form(rows: int, cols: int, dtype: torch.dtype) -> None:
+    gen = torch.Generator().manual_seed(cols)
+    src = (torch.randn(2, rows, cols, generator=gen) + 0.1).to(dtype)
+    for out_dtype, scale in ((torch.float16, 1.0), (torch.bfloat16, 1.02)):
+        x = torch.full((2, rows, _padded(cols)), SENTINEL, dtype=out_dtype, device=DEV)
+        native.normalize_pack(src.to(DEV), x, eps=1e-8, norm_scale=scale)
+        value = src.float() if out_dtype is torch.float16 else src.bfloat16().float()
+        norm = value.double().square().sum((1, 2), keepdim=True).sqrt()
+        # the norm's own last bits and, for bf16, three roundings of the divisor and one of the quotient
+        bound = (2.0**-11 if out_dtype is torch.float16 else 4 * 2.0**-8) * 1.02
+        want = value.double() / (norm * scale)
+        assert bool(((x[..., :cols].double().cpu() - want).abs() <= bound * want.abs() + 2.0**-24).all())
+        assert bool((x[..., cols:] == 0).all())
