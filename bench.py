@@ -662,7 +662,7 @@ def run_ns_microbench(args) -> None:
 
         def iteration():
             work.copy_(packed)
-            return run_iteration(fn, work, m, n, scratch, None)
+            return run_iteration(fn, work, m, n, scratch)
 
         def clock(call) -> float:
             for _ in range(args.warmup):

@@ -191,17 +191,14 @@ def open_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any], ar
         "frob": ((count,), torch.float32),
     })
     # Row sums of squares of the orthogonalized rows: the last product's epilogue writes them as
-    # partials per 128 columns when the block is iterated as it lies (wide or square); a tall block
-    # is iterated transposed, and a foreign orthogonalizer knows nothing of this, so those take one
-    # sum per row from a pass of their own.
-    parts = _native.newton_schulz_rowsq_parts(cols) if native and k <= cols else 1
+    # partials per 128 columns; a foreign orthogonalizer knows nothing of this, so its result takes
+    # one sum per row from a pass of its own.
+    parts = _native.newton_schulz_rowsq_parts(cols) if native else 1
     plan["rowsq"] = ((count * k, parts), torch.float32)
     if not selecting:
         plan["u"] = ((count, rows, cols), torch.float32)
     if native:
         plan["ns"] = ((fn.workspace_bytes(count, k, cols),), torch.uint8)
-        if k > cols:
-            plan["xt"] = ((count, cols, padded(k)), dtype)
     momentum = bucket.momentum[blocks]
     return RunContext(
         bucket=bucket, group=group, params=params, grads=grads,
@@ -250,8 +247,7 @@ def run_core(ctx: RunContext) -> RunResult:
     fused = normalize and parts > 1
     if isinstance(fn, NativeOrthogonalizer):
         with _stage("newton_schulz"):
-            orthogonal = run_iteration(fn, buf["x"], k, cols, buf["ns"], buf.get("xt"),
-                                       rowsq=buf["rowsq"] if fused else None)
+            orthogonal = run_iteration(fn, buf["x"], k, cols, buf["ns"], rowsq=buf["rowsq"] if fused else None)
     else:
         orthogonal = _foreign_orthogonalize(fn, ctx.source, ctx.index, float(group[MOMENTUM_KEY]), ctx.selecting,
                                             buf["x"])

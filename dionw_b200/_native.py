@@ -58,6 +58,9 @@ SIGNATURES: dict[str, tuple[object, tuple[object, ...]]] = {
     "dionw_newton_schulz_workspace_bytes": (c_size_t, (c_int64, c_int64, c_int64, c_int)),
     "dionw_newton_schulz": (
         c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_size_t, c_void_p, c_void_p)),
+    "dionw_newton_schulz_tall_workspace_bytes": (c_size_t, (c_int64, c_int64, c_int64, c_int)),
+    "dionw_newton_schulz_tall": (
+        c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_size_t, c_void_p, c_void_p)),
     "dionw_newton_schulz_rowsq_parts": (c_int64, (c_int64,)),
     "dionw_newton_schulz_static": (
         c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p)),
@@ -266,6 +269,18 @@ def newton_schulz(x: Tensor, out: Tensor, m: int, n: int, kind: int, workspace: 
     _check(library().dionw_newton_schulz(x.data_ptr(), out.data_ptr(), x.shape[0], m, n, x.stride(-2), kind,
                                          workspace.data_ptr(), workspace.numel() * workspace.element_size(),
                                          _ptr(rowsq), _stream(x)))
+
+
+def newton_schulz_tall_workspace_bytes(blocks: int, rows: int, cols: int, kind: int) -> int:
+    return int(library().dionw_newton_schulz_tall_workspace_bytes(blocks, rows, cols, kind))
+
+
+def newton_schulz_tall(x: Tensor, out: Tensor, rows: int, cols: int, kind: int, workspace: Tensor,
+                       rowsq: Tensor | None = None) -> None:
+    """``newton_schulz`` on tall ``[blocks, rows, ldx]`` operands (``rows > cols``), as they lie."""
+    _check(library().dionw_newton_schulz_tall(x.data_ptr(), out.data_ptr(), x.shape[0], rows, cols, x.stride(-2), kind,
+                                              workspace.data_ptr(), workspace.numel() * workspace.element_size(),
+                                              _ptr(rowsq), _stream(x)))
 
 
 STATIC_SCRATCH_BYTES = 64 << 20

@@ -223,24 +223,33 @@ int host_sym_tiles(int tiles_m) {
 
 // C = alpha A B^T + beta Cin for a product known to be symmetric (B = A, or A and B symmetric
 // matrices that commute): lower tiles + mirror, optional second output with diag added.
-// b == nullptr means B = A.
-int symmetric_product(const void* a, const void* b, int64_t blocks, int64_t m, int64_t kdim, int64_t lda,
+// b == nullptr means B = A.  `transposed` (with b == nullptr): A is stored [kdim, m] and the product is
+// A^T A.
+int symmetric_product(const void* a, bool transposed, const void* b, int64_t blocks, int64_t m, int64_t kdim, int64_t lda,
                       int64_t a_batch, int64_t ldb, int64_t b_batch, const void* cin, int64_t ldc, int64_t cin_batch, float alpha, float beta, void* out,
                       int64_t ldo, int64_t out_batch, void* out2, float diag, int dtype, cudaStream_t stream) {
   DIONW_REQUIRE(dtype == DIONW_F16 || dtype == DIONW_BF16, "symmetric_product: dtype must be F16 or BF16");
   DIONW_REQUIRE(blocks > 0 && m > 0 && kdim > 0, "symmetric_product: empty problem");
   CUtensorMap map_a, map_b;
-  int st = make_map(&map_a, a, dtype, kdim, m, blocks, lda, a_batch, gemm::kBK, gemm::kBM);
-  if (st != DIONW_OK) return st;
   const bool same = b == nullptr || b == a;
-  if (b == nullptr) {
-    b = a;
-    ldb = lda;
-    b_batch = a_batch;
+  int st;
+  if (transposed) {
+    DIONW_REQUIRE(b == nullptr, "symmetric_product: a transposed operand takes no second one");
+    st = make_map(&map_a, a, dtype, m, kdim, blocks, lda, a_batch, 64, gemm::kBK);
+    if (st != DIONW_OK) return st;
+    map_b = map_a;
+  } else {
+    st = make_map(&map_a, a, dtype, kdim, m, blocks, lda, a_batch, gemm::kBK, gemm::kBM);
+    if (st != DIONW_OK) return st;
+    if (b == nullptr) {
+      b = a;
+      ldb = lda;
+      b_batch = a_batch;
+    }
+    st = make_map(&map_b, b, dtype, kdim, m, blocks, ldb, b_batch, gemm::kBK,
+                  use_cta_pairs() ? gemm2::kHalfN : gemm::kBN);
+    if (st != DIONW_OK) return st;
   }
-  st = make_map(&map_b, b, dtype, kdim, m, blocks, ldb, b_batch, gemm::kBK,
-                use_cta_pairs() ? gemm2::kHalfN : gemm::kBN);
-  if (st != DIONW_OK) return st;
   gemm::Params p{};
   p.cin = cin;
   p.out = out;
@@ -262,6 +271,10 @@ int symmetric_product(const void* a, const void* b, int64_t blocks, int64_t m, i
   p.mirror_diagonal = same ? 0 : 1;
   p.status = device_status_word();
   p.wait_ns = gemm::kWaitLimitNs;
+  if (transposed) {
+    if (dtype == DIONW_F16) return launch_any<__half, __half, true, true>(map_a, map_b, p, stream);
+    return launch_any<__nv_bfloat16, __nv_bfloat16, true, true>(map_a, map_b, p, stream);
+  }
   if (dtype == DIONW_F16) return launch_any<__half, __half, false, true>(map_a, map_b, p, stream);
   return launch_any<__nv_bfloat16, __nv_bfloat16, false, true>(map_a, map_b, p, stream);
 }
@@ -327,7 +340,7 @@ extern "C" int dionw_symmetric_product(const void* a, const void* b, int64_t blo
                                        int64_t lda, int64_t ldb, const void* cin, int64_t ldc, float alpha,
                                        float beta, void* out, int64_t ldo, void* out2, float diag, int dtype,
                                        void* stream) {
-  return dionw::symmetric_product(a, b, blocks, m, kdim, lda, m * lda, ldb, m * ldb, cin, ldc, m * ldc, alpha, beta,
+  return dionw::symmetric_product(a, false, b, blocks, m, kdim, lda, m * lda, ldb, m * ldb, cin, ldc, m * ldc, alpha, beta,
                                   out, ldo, m * ldo, out2, diag, dtype, static_cast<cudaStream_t>(stream));
 }
 

@@ -155,14 +155,15 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
       : "memory");
 }
 
-// Instruction descriptor: fp32 accumulate, A K-major, M = 256 (128 rows in each CTA), N = 256.
-template <typename T, bool kBMajorMN>
+// Instruction descriptor: fp32 accumulate, M = 256 (128 rows in each CTA), N = 256.
+template <typename T, bool kAMajorMN, bool kBMajorMN>
 __device__ __forceinline__ uint32_t make_idesc2() {
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
   uint32_t d = 0;
   d |= 1u << 4;
   d |= fmt << 7;
   d |= fmt << 10;
+  d |= (kAMajorMN ? 1u : 0u) << 15;
   d |= (kBMajorMN ? 1u : 0u) << 16;
   d |= uint32_t(kBN >> 3) << 17;
   d |= uint32_t(kPairM >> 4) << 24;
@@ -229,6 +230,7 @@ template <typename InT, typename OutT, bool kBMajorMN, bool kSym>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
   using namespace gemm;
+  constexpr bool kAMajorMN = kSym && kBMajorMN;   // X^T X, as in the one-CTA kernel
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + size_t(kStages) * kStageBytes);  // leader's: both CTAs' stage landed
@@ -342,7 +344,13 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
           // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
           // because its empty barrier is released by the MMAs that consumed this one.
           if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
-          tma_load_3d_pair(a_dst, &map_a, leader_full, kb * kBK, m0, tile.batch);
+          if constexpr (kAMajorMN) {
+#pragma unroll
+            for (int panel = 0; panel < kBM / 64; ++panel)
+              tma_load_3d_pair(a_dst + panel * kPanelBytes, &map_a, leader_full, m0 + panel * 64, kb * kBK, tile.batch);
+          } else {
+            tma_load_3d_pair(a_dst, &map_a, leader_full, kb * kBK, m0, tile.batch);
+          }
           if constexpr (kBMajorMN) {
 #pragma unroll
             for (int panel = 0; panel < kHalfN / 64; ++panel)
@@ -358,7 +366,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       // the second CTA's MMA warp has nothing to issue
     } else if (lane == 0) {
       // ------------------------------------------------------------ MMA issuer (leader)
-      const uint32_t idesc = make_idesc2<InT, kBMajorMN>();
+      const uint32_t idesc = make_idesc2<InT, kAMajorMN, kBMajorMN>();
       uint32_t it = 0;
       bool ok = true;
       for (uint32_t local = 0; ok; ++local) {
@@ -375,13 +383,15 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + size_t(s) * kStageBytes);
           const uint32_t b_addr = a_addr + kABytes;
-          const uint64_t a_desc = make_smem_desc(a_addr, 16, 1024);
+          const uint64_t a_desc = kAMajorMN ? make_smem_desc(a_addr, kPanelBytes, 1024)
+                                            : make_smem_desc(a_addr, 16, 1024);
           const uint64_t b_desc = kBMajorMN ? make_smem_desc(b_addr, kPanelBytes, 1024)
                                             : make_smem_desc(b_addr, 16, 1024);
 #pragma unroll
           for (int j = 0; j < kBK / kUmmaK; ++j) {
-            const uint64_t a_step = uint64_t((j * kUmmaK * 2) >> 4);
-            const uint64_t b_step = kBMajorMN ? uint64_t((j * kUmmaK * 128) >> 4) : a_step;
+            const uint64_t k_step = uint64_t((j * kUmmaK * 2) >> 4), mn_step = uint64_t((j * kUmmaK * 128) >> 4);
+            const uint64_t a_step = kAMajorMN ? mn_step : k_step;
+            const uint64_t b_step = kBMajorMN ? mn_step : k_step;
             umma2_f16(tmem_d, a_desc + a_step, b_desc + b_step, idesc, (kb > 0 || j > 0) ? 1u : 0u);
           }
           umma2_commit_both(&empty_bar[s]);

@@ -33,7 +33,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;        // 32 KB
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
-constexpr uint32_t kPanelBytes = 64 * kBK * 2;     // one 64-column panel of an MN-major B stage
+constexpr uint32_t kPanelBytes = 64 * kBK * 2;     // one 64-column panel of an MN-major stage
 constexpr uint32_t kPieceBytes = 32 * 32 * 2;      // one 32 x 32 piece of the output, 64 bytes a row
 constexpr uint32_t kMirrorBytes = 8 * 2 * kPieceBytes;  // per epilogue warp: a piece as it lies and its transpose
 constexpr size_t kSmemBytes =
@@ -228,14 +228,15 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr, uint32_t lbo_b
   return d;
 }
 
-// Instruction descriptor for kind::f16: fp32 accumulate, A K-major, M = 128, N = 256.
-template <typename T, bool kBMajorMN>
+// Instruction descriptor for kind::f16: fp32 accumulate, M = 128, N = 256.
+template <typename T, bool kAMajorMN, bool kBMajorMN>
 __device__ __forceinline__ uint32_t make_idesc() {
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
   uint32_t d = 0;
   d |= 1u << 4;                       // D format f32
   d |= fmt << 7;                      // A format
   d |= fmt << 10;                     // B format
+  d |= (kAMajorMN ? 1u : 0u) << 15;   // A major
   d |= (kBMajorMN ? 1u : 0u) << 16;   // B major
   d |= uint32_t(kBN >> 3) << 17;      // N
   d |= uint32_t(kBM >> 4) << 24;      // M
@@ -560,9 +561,11 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
 // ----------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------
+// kSym with kBMajorMN is X^T X: both operands are the row-major [kdim, m] matrix, read MN-major.
 template <typename InT, typename OutT, bool kBMajorMN, bool kSym>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+  constexpr bool kAMajorMN = kSym && kBMajorMN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + size_t(kStages) * kStageBytes);
@@ -618,7 +621,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           uint8_t* a_dst = smem + size_t(s) * kStageBytes;
           uint8_t* b_dst = a_dst + kABytes;
           mbar_expect_tx(&full_bar[s], kStageBytes);
-          tma_load_3d(a_dst, &map_a, &full_bar[s], kb * kBK, m0, tile.batch);
+          if constexpr (kAMajorMN) {
+#pragma unroll
+            for (int panel = 0; panel < kBM / 64; ++panel)
+              tma_load_3d(a_dst + panel * kPanelBytes, &map_a, &full_bar[s], m0 + panel * 64, kb * kBK, tile.batch);
+          } else {
+            tma_load_3d(a_dst, &map_a, &full_bar[s], kb * kBK, m0, tile.batch);
+          }
           if constexpr (kBMajorMN) {
 #pragma unroll
             for (int panel = 0; panel < kBN / 64; ++panel)
@@ -632,7 +641,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      const uint32_t idesc = make_idesc<InT, kBMajorMN>();
+      const uint32_t idesc = make_idesc<InT, kAMajorMN, kBMajorMN>();
       uint32_t it = 0, local = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local) {
@@ -648,15 +657,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + size_t(s) * kStageBytes);
           const uint32_t b_addr = a_addr + kABytes;
-          const uint64_t a_desc = make_smem_desc(a_addr, 16, 1024);
+          const uint64_t a_desc = kAMajorMN ? make_smem_desc(a_addr, kPanelBytes, 1024)
+                                            : make_smem_desc(a_addr, 16, 1024);
           const uint64_t b_desc = kBMajorMN ? make_smem_desc(b_addr, kPanelBytes, 1024)
                                             : make_smem_desc(b_addr, 16, 1024);
 #pragma unroll
           for (int j = 0; j < kBK / kUmmaK; ++j) {
             // K-major: 16 elements = 32 B further along each 128 B row.
             // MN-major: 16 k-rows of 128 B further.
-            const uint64_t a_step = uint64_t((j * kUmmaK * 2) >> 4);
-            const uint64_t b_step = kBMajorMN ? uint64_t((j * kUmmaK * 128) >> 4) : a_step;
+            const uint64_t k_step = uint64_t((j * kUmmaK * 2) >> 4), mn_step = uint64_t((j * kUmmaK * 128) >> 4);
+            const uint64_t a_step = kAMajorMN ? mn_step : k_step;
+            const uint64_t b_step = kBMajorMN ? mn_step : k_step;
             umma_f16(tmem_d, a_desc + a_step, b_desc + b_step, idesc, (kb > 0 || j > 0) ? 1u : 0u);
           }
           umma_commit(&empty_bar[s]);

@@ -59,40 +59,26 @@ class NativeOrthogonalizer:
         x = torch.empty(blocks, rows, padded(cols), dtype=self.dtype, device=src.device)
         _native.normalize_pack(src, x, eps=epsilon, norm_scale=self.norm_scale)
         scratch = torch.empty(self.workspace_bytes(blocks, rows, cols), dtype=torch.uint8, device=src.device)
-        xt = None
-        if rows > cols:
-            xt = torch.empty(blocks, cols, padded(rows), dtype=self.dtype, device=src.device)
-        out = run_iteration(self, x, rows, cols, scratch, xt)
+        out = run_iteration(self, x, rows, cols, scratch)
         return out[..., :cols]
 
     def workspace_bytes(self, blocks: int, rows: int, cols: int) -> int:
-        m, n = min(rows, cols), max(rows, cols)
-        return _native.newton_schulz_workspace_bytes(blocks, m, n, self.code)
+        if rows > cols:
+            return _native.newton_schulz_tall_workspace_bytes(blocks, rows, cols, self.code)
+        return _native.newton_schulz_workspace_bytes(blocks, rows, cols, self.code)
 
 
 def run_iteration(fn: NativeOrthogonalizer, x: Tensor, rows: int, cols: int, scratch: Tensor,
-                  xt: Tensor | None, rowsq: Tensor | None = None) -> Tensor:
-    """Iterate on ``x`` ``[N, rows, ld]`` (normalised, in ``fn.dtype``); returns bf16 ``[N, rows, ld]``.
+                  rowsq: Tensor | None = None) -> Tensor:
+    """Iterate in place on ``x`` ``[N, rows, ld]`` (normalised, in ``fn.dtype``); returns bf16 ``[N, rows, ld]``.
 
-    Wide and square blocks are iterated in place.  Tall ones go through ``xt``, a
-    ``[N, cols, padded(rows)]`` buffer of the same dtype.  ``scratch`` holds
-    ``fn.workspace_bytes(...)`` bytes.  ``rowsq`` (wide and square blocks only):
-    fp32 ``[N * rows, newton_schulz_rowsq_parts(cols)]``, filled with partial row
+    ``scratch`` holds ``fn.workspace_bytes(...)`` bytes.  ``rowsq``: fp32
+    ``[N * rows, newton_schulz_rowsq_parts(cols)]``, filled with partial row
     sums of the squared result by the last product's epilogue.
     """
-    m, n = min(rows, cols), max(rows, cols)
     out = x if x.dtype is torch.bfloat16 else x.view(torch.bfloat16)
-    if rows <= cols:
-        _native.newton_schulz(x, out, m, n, fn.code, scratch, rowsq)
-        return out
-    if rowsq is not None:
-        raise ValueError("row sums come with wide and square blocks only: a tall block is iterated transposed")
-    if xt is None:
-        raise ValueError("tall blocks need the transposed buffer")
-    _native.transpose_2byte(x[..., :cols], xt)
-    xt_out = xt if xt.dtype is torch.bfloat16 else xt.view(torch.bfloat16)
-    _native.newton_schulz(xt, xt_out, m, n, fn.code, scratch)
-    _native.transpose_2byte(xt_out[..., :rows], out)
+    iterate = _native.newton_schulz_tall if rows > cols else _native.newton_schulz
+    iterate(x, out, rows, cols, fn.code, scratch, rowsq)
     return out
 
 

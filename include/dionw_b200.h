@@ -135,8 +135,8 @@ int dionw_normalize_pack(const void* src, int src_dtype, int64_t blocks, int64_t
                          int64_t cols, float eps, float norm_scale, void* x, int x_dtype,
                          int64_t ldx, float* sumsq, float* frob, void* stream);
 
-/* out[b, c, r] = in[b, r, c] for 2-byte elements (tall blocks are iterated in
- * their wide orientation, src/dionw/_gram.py:83-84, :89). */
+/* out[b, c, r] = in[b, r, c] for 2-byte elements (the transposed view of a batch,
+ * src/dionw/_gram.py:83-84, :89, as a copy). */
 int dionw_transpose_2byte(const void* in, void* out, int64_t blocks, int64_t rows,
                           int64_t cols, int64_t ld_in, int64_t ld_out, void* stream);
 
@@ -164,6 +164,16 @@ int dionw_newton_schulz(void* x, void* out, int64_t blocks, int64_t m, int64_t n
                         float* rowsq, void* stream);
 /* Partial sums per output row that dionw_newton_schulz writes into rowsq. */
 int64_t dionw_newton_schulz_rowsq_parts(int64_t n);
+
+/* The same iteration on tall [blocks, rows, ldx] operands (rows > cols) as they lie:
+ * G = X^T X, X <- X Q.  The reference iterates the transposed batch
+ * (src/dionw/_gram.py:83-84, :89); the values are the same.  rowsq (nullable) is
+ * fp32 [blocks * rows, dionw_newton_schulz_rowsq_parts(cols)].  Other arguments as
+ * dionw_newton_schulz; the workspace has its own size. */
+size_t dionw_newton_schulz_tall_workspace_bytes(int64_t blocks, int64_t rows, int64_t cols, int kind);
+int dionw_newton_schulz_tall(void* x, void* out, int64_t blocks, int64_t rows, int64_t cols,
+                             int64_t ldx, int kind, void* workspace, size_t workspace_bytes,
+                             float* rowsq, void* stream);
 
 /* The same iteration for callers that have no scratch to give: a host bound to
  * this ABI without torch's allocator, a serving loop whose memory was budgeted at
@@ -215,8 +225,7 @@ int dionw_batched_gemm(const void* a, int64_t lda, const void* b, int64_t ldb, i
 /* ---- NorMuon and the weight update -------------------------------------- */
 
 /* s[b*k + r] = sum_c o[b, r, c]^2 for a bf16 batch [blocks, k, ldo] (used where
- * dionw_newton_schulz cannot hand the row sums over: tall blocks, which are
- * iterated transposed, and foreign orthogonalizers). */
+ * the iteration does not hand the row sums over: foreign orthogonalizers). */
 int dionw_row_sumsq_bf16(const void* o, int64_t blocks, int64_t k, int64_t cols,
                          int64_t ldo, float* s, void* stream);
 

@@ -77,6 +77,32 @@ def test_general_products_leave_everything_outside_alone(m: int, n: int, k: int,
     assert bool((out[..., n:] == SENTINEL).all())
 
 
+@pytest.mark.parametrize("kind", [native.NS_GRAM, native.NS_GRAM_FULL, native.NS_POLAR_EXPRESS, native.NS_KELLER])
+@pytest.mark.parametrize("rows, cols", [(2, 1), (40, 33), (257, 256), (700, 65), (1531, 517)])
+def test_tall_blocks_equal_the_iteration_of_their_transpose(rows: int, cols: int, kind: int) -> None:
+    """Bit for bit: each element is the same dot product, accumulated in the same order."""
+    gen = torch.Generator().manual_seed(rows)
+    dtype = torch.float16 if kind in (native.NS_GRAM, native.NS_GRAM_FULL) else torch.bfloat16
+    blocks = 3
+    x = torch.randn(blocks, rows, cols, generator=gen)
+    x = (x / x.norm(dim=(1, 2), keepdim=True)).to(dtype).to(DEV)
+    tall = torch.zeros(blocks, rows, _padded(cols), dtype=dtype, device=DEV)
+    tall[..., :cols] = x
+    wide = torch.zeros(blocks, cols, _padded(rows), dtype=dtype, device=DEV)
+    wide[..., :rows] = x.mT
+    parts = native.newton_schulz_rowsq_parts(cols)
+    rowsq = torch.full((blocks * rows, parts), SENTINEL, device=DEV)
+    ws = torch.empty(native.newton_schulz_tall_workspace_bytes(blocks, rows, cols, kind), dtype=torch.uint8, device=DEV)
+    native.newton_schulz_tall(tall, tall.view(torch.bfloat16), rows, cols, kind, ws, rowsq)
+    ws = torch.empty(native.newton_schulz_workspace_bytes(blocks, cols, rows, kind), dtype=torch.uint8, device=DEV)
+    native.newton_schulz(wide, wide.view(torch.bfloat16), cols, rows, kind, ws)
+    got, want = tall.view(torch.bfloat16)[..., :cols], wide.view(torch.bfloat16)[..., :rows].mT
+    assert torch.equal(got, want)
+    # at most 128 fp32 additions per part and two parts: 2^-15 of a sum of squares
+    exact = got.double().square().sum(-1).flatten()
+    assert bool(((rowsq.double().sum(-1) - exact).abs() <= 2.0**-15 * exact + 1e-30).all())
+
+
 @pytest.mark.parametrize("rows, cols", [(1, 1), (3, 1000), (40, 33), (257, 264), (64, 4100)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 def test_normalize_pack_matches_the_fp32_form(rows: int, cols: int, dtype: torch.dtype) -> None:
