@@ -1,0 +1,68 @@
+// Thread-block clusters: rank, barrier, and the other CTAs' shared memory.
+#pragma once
+
+#include <cstdint>
+
+#include <cuda_runtime.h>
+
+namespace dionw {
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  return n;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Address of the same shared-memory object in another CTA of the cluster.
+__device__ __forceinline__ uint32_t peer_address(const void* local, uint32_t rank) {
+  uint32_t out;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(out)
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank));
+  return out;
+}
+
+__device__ __forceinline__ uint32_t peer_load(const void* local, uint32_t rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_address(local, rank)) : "memory");
+  return v;
+}
+
+// CTAs that share one block of `rows` rows: one per `rows_per_cta`, at most the portable cluster size.
+// (The grid stays below 2^31 CTAs.)
+inline unsigned cluster_for(long long blocks, long long rows, long long rows_per_cta) {
+  unsigned n = 1;
+  while (n < 8 && blocks * n * 2 < (1LL << 31) && rows > n * rows_per_cta) n *= 2;
+  return n;
+}
+
+// blocks x cluster CTAs, `cluster` of them to a cluster.
+template <typename... Params, typename... Args>
+cudaError_t launch_clusters(void (*kernel)(Params...), unsigned blocks, unsigned cluster, unsigned threads,
+                            cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(blocks * cluster);
+  config.blockDim = dim3(threads);
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = cluster;
+  attribute.val.clusterDim.y = 1;
+  attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+}  // namespace dionw

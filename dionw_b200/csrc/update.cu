@@ -2,6 +2,7 @@
 // AdamW and the EMA passes.  All HBM-bound streaming kernels.
 #include <type_traits>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "decay_job.cuh"
 
@@ -58,52 +59,82 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
   return total;
 }
 
-// One CTA per block: new row variances, row denominators, block scale.
+// One cluster of up to eight CTAs per block: new row variances, row denominators, block scale.  Eight
+// lanes share a row, so that a warp reads four rows' parts in consecutive words; the parts of a row are
+// added in a fixed order (lane l takes pairs l, l + 8, ..., then the lanes are folded).
+//
+// Bounded by latency: 2 MB at most.  With one CTA per block and a row per thread, one block of 2048 x 28672
+// took 94 us and two of 7168 x 8192 about as long; on eight CTAs they take 14 and 20.
+constexpr int kRowLanes = 8;
+
 __global__ void __launch_bounds__(kReduceThreads)
 normuon_rows_kernel(const float* __restrict__ s, int parts, float* __restrict__ variance,
                     const int32_t* __restrict__ index, int rows, int k, float inv_count_cols, float weight, float eps,
                     float step_host, const float* __restrict__ step_device, bool normalize,
                     float* __restrict__ denom, float* __restrict__ scale) {
   __shared__ float scratch[kReduceThreads];
-  const long long b = blockIdx.x;
+  __shared__ float s_totals[2];
+  const uint32_t rank = cluster_rank(), ctas = cluster_size();
+  const long long b = blockIdx.x / ctas;
   const int tid = threadIdx.x;
   const float step = step_device != nullptr ? *step_device : step_host;
   if (!normalize) {
-    for (int r = tid; r < k; r += kReduceThreads) denom[b * k + r] = 1.0f;
-    if (tid == 0) scale[b] = step;
+    for (int r = int(rank) * kReduceThreads + tid; r < k; r += int(ctas) * kReduceThreads) denom[b * k + r] = 1.0f;
+    if (rank == 0 && tid == 0) scale[b] = step;
     return;
   }
+  const bool pairs = (parts & 1) == 0 && (reinterpret_cast<uintptr_t>(s) & 7u) == 0;
+  const int sub = tid % kRowLanes;
   float n0 = 0.0f, n1 = 0.0f;
-  for (int r = tid; r < k; r += kReduceThreads) {
-    const long long slot = b * rows + (index ? index[b * k + r] : r);
-    // a row's sum of squares arrives whole (parts == 1) or as partials per 128 columns,
-    // added here left to right
-    const float* partial = s + (b * k + r) * parts;
+  constexpr int kRows = kReduceThreads / kRowLanes;   // rows a CTA takes at a time
+  for (int r0 = int(rank) * kRows; r0 < k; r0 += int(ctas) * kRows) {
+    const int r = r0 + tid / kRowLanes;
     float sr = 0.0f;
-    if ((parts & 3) == 0 && (reinterpret_cast<uintptr_t>(s) & 15u) == 0) {
-      for (int j = 0; j < parts; j += 4) {   // same order, four partials per load
-        const float4 q = __ldcs(reinterpret_cast<const float4*>(partial + j));
-        sr = (((sr + q.x) + q.y) + q.z) + q.w;
+    if (r < k) {
+      // a row's sum of squares arrives whole (parts == 1) or as partials per 128 columns
+      const float* partial = s + (b * k + r) * parts;
+      if (pairs) {
+#pragma unroll 4
+        for (int j = 2 * sub; j < parts; j += 2 * kRowLanes) {
+          const float2 q = __ldcs(reinterpret_cast<const float2*>(partial + j));
+          sr += q.x + q.y;
+        }
+      } else {
+        for (int j = sub; j < parts; j += kRowLanes) sr += partial[j];
       }
-    } else {
-      for (int j = 0; j < parts; ++j) sr += partial[j];
     }
-    const float mean = sr * inv_count_cols;
-    const float old = variance[slot];
-    // torch.lerp: start + weight * (end - start) for weight < 0.5, else the mirrored form.
-    const float v = weight < 0.5f ? fmaf(weight, mean - old, old) : mean - (mean - old) * (1.0f - weight);
-    variance[slot] = v;
-    const float d = sqrtf(v) + eps;
-    denom[b * k + r] = d;
-    n0 += sr;
-    n1 += sr / (d * d);
+#pragma unroll
+    for (int delta = kRowLanes / 2; delta >= 1; delta >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, delta);
+    if (r < k && sub == 0) {
+      const long long slot = b * rows + (index ? index[b * k + r] : r);
+      const float mean = sr * inv_count_cols;
+      const float old = variance[slot];
+      // torch.lerp: start + weight * (end - start) for weight < 0.5, else the mirrored form.
+      const float v = weight < 0.5f ? fmaf(weight, mean - old, old) : mean - (mean - old) * (1.0f - weight);
+      variance[slot] = v;
+      const float d = sqrtf(v) + eps;
+      denom[b * k + r] = d;
+      n0 += sr;
+      n1 += sr / (d * d);
+    }
   }
   const float total0 = block_sum(n0, scratch);
   const float total1 = block_sum(n1, scratch);
   if (tid == 0) {
-    const float restore = sqrtf(total0) / fmaxf(sqrtf(total1), eps);
+    s_totals[0] = total0;
+    s_totals[1] = total1;
+  }
+  cluster_sync();
+  if (rank == 0 && tid == 0) {
+    float all0 = 0.0f, all1 = 0.0f;
+    for (uint32_t c = 0; c < ctas; ++c) {
+      all0 += __uint_as_float(peer_load(&s_totals[0], c));
+      all1 += __uint_as_float(peer_load(&s_totals[1], c));
+    }
+    const float restore = sqrtf(all0) / fmaxf(sqrtf(all1), eps);
     scale[b] = restore * step;
   }
+  cluster_sync();   // the other CTAs' shared memory stays until rank 0 has read it
 }
 
 // ---------------------------------------------------------------------------
@@ -435,10 +466,12 @@ extern "C" int dionw_normuon_rows(const float* s, int64_t parts, float* variance
                                   void* stream_ptr) {
   DIONW_REQUIRE(blocks > 0 && rows > 0 && k > 0 && k <= rows && cols > 0 && parts >= 1 && parts <= 4096,
                 "normuon_rows: bad shape");
-  normuon_rows_kernel<<<unsigned(blocks), kReduceThreads, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
-      s, int(parts), variance, index, int(rows), int(k), 1.0f / float(cols), weight, eps, step, step_device,
-      normalize != 0, denom, scale);
-  return launch_status("normuon_rows_kernel");
+  count_launch();
+  return check_cuda(launch_clusters(normuon_rows_kernel, unsigned(blocks), cluster_for(blocks, k, kReduceThreads / kRowLanes),
+                                    kReduceThreads, static_cast<cudaStream_t>(stream_ptr), s, int(parts), variance, index,
+                                    int(rows), int(k), 1.0f / float(cols), weight, eps, step, step_device, normalize != 0,
+                                    denom, scale),
+                    "normuon_rows_kernel");
 }
 
 extern "C" int dionw_apply_round(void* const* weights, const int64_t* rows_per_tensor, const void* const* o,
