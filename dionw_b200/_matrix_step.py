@@ -33,7 +33,7 @@ from dionw_b200.matrix_update import MomentumForm, RowNormalization
 from dionw_b200.newton_schulz import NativeOrthogonalizer, padded, run_iteration
 
 __all__ = ["MAX_RUN_ELEMENTS", "apply_result", "apply_results", "open_run", "prepare_run", "run_core", "run_elements",
-           "run_front", "step_run"]
+           "run_front", "step_run", "step_runs"]
 
 ADAMW_UPDATE_RMS = 0.2        # update RMS of AdamW that matrix steps are matched to
 NEWTON_SCHULZ_EPS = 1e-8      # added to the Frobenius norm; independent of AdamW's eps
@@ -161,6 +161,17 @@ def open_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any], ar
     Raises:
         RuntimeError: If a parameter has no gradient.
     """
+    ctx, plan = _describe_run(bucket, positions, group)
+    fn = bucket.orthogonalize
+    if isinstance(fn, NativeOrthogonalizer):
+        plan["ns"] = ((fn.workspace_bytes(ctx.count, bucket.selected_rows, bucket.cols),), torch.uint8)
+    ctx.buf = _workspace.carve(ctx.momentum.device, plan, arena)
+    return ctx
+
+
+def _describe_run(bucket: Bucket, positions: Sequence[int],
+                  group: dict[str, Any]) -> tuple[RunContext, _workspace.Plan]:
+    """A run's context without its scratch, and the plan of that scratch but for the iteration's own."""
     params = [bucket.params[i] for i in positions]
     grads: list[Tensor] = []
     for param in params:
@@ -197,14 +208,11 @@ def open_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any], ar
     plan["rowsq"] = ((count * k, parts), torch.float32)
     if not selecting:
         plan["u"] = ((count, rows, cols), torch.float32)
-    if native:
-        plan["ns"] = ((fn.workspace_bytes(count, k, cols),), torch.uint8)
     momentum = bucket.momentum[blocks]
     return RunContext(
         bucket=bucket, group=group, params=params, grads=grads,
         rows_per_tensor=[(bucket.slices[i].stop - bucket.slices[i].start) * rows for i in positions],
-        count=count, momentum=momentum, variance=bucket.variance[blocks].view(count, rows), step=step,
-        buf=_workspace.carve(momentum.device, plan, arena))
+        count=count, momentum=momentum, variance=bucket.variance[blocks].view(count, rows), step=step, buf={}), plan
 
 
 def run_front(ctx: RunContext) -> None:
@@ -235,32 +243,95 @@ def run_front(ctx: RunContext) -> None:
                               decay_rows=ctx.selecting, eps=NEWTON_SCHULZ_EPS, norm_scale=fn.norm_scale)
 
 
-def run_core(ctx: RunContext) -> RunResult:
-    """Stages 3-4: the tensor-core part (Newton-Schulz) and the NorMuon scales."""
+def run_core(ctx: RunContext, alone: bool = False) -> RunResult:
+    """Stages 3-4: the tensor-core part (Newton-Schulz) and the NorMuon scales.
+
+    ``alone``: no other stream has work for the GPU meanwhile, so the iteration may be one launch that
+    holds every SM until it is done.  Otherwise it is one launch per product, and what runs beside it
+    (collectives, another run's streaming passes) gets SMs in between."""
     global CURRENT_RUN
-    bucket, group, buf = ctx.bucket, ctx.group, ctx.buf
-    rows, cols, k = bucket.rows, bucket.cols, bucket.selected_rows
-    CURRENT_RUN = (ctx.count, rows, k, cols)
+    bucket, buf = ctx.bucket, ctx.buf
+    CURRENT_RUN = (ctx.count, bucket.rows, bucket.selected_rows, bucket.cols)
     fn = bucket.orthogonalize
-    normalize = RowNormalization(group[ROW_NORMALIZATION_KEY]) is RowNormalization.NORMUON
-    parts = buf["rowsq"].shape[1]
-    fused = normalize and parts > 1
     if isinstance(fn, NativeOrthogonalizer):
         with _stage("newton_schulz"):
-            orthogonal = run_iteration(fn, buf["x"], k, cols, buf["ns"], rowsq=buf["rowsq"] if fused else None)
+            orthogonal = run_iteration(fn, buf["x"], bucket.selected_rows, bucket.cols, buf["ns"],
+                                       rowsq=buf["rowsq"] if _fused_row_sums(ctx) else None, stepwise=not alone)
     else:
-        orthogonal = _foreign_orthogonalize(fn, ctx.source, ctx.index, float(group[MOMENTUM_KEY]), ctx.selecting,
+        orthogonal = _foreign_orthogonalize(fn, ctx.source, ctx.index, float(ctx.group[MOMENTUM_KEY]), ctx.selecting,
                                             buf["x"])
+    return _finish_run(ctx, orthogonal)
+
+
+def _fused_row_sums(ctx: RunContext) -> bool:
+    """Whether the iteration's last product hands NorMuon its row sums."""
+    normalize = RowNormalization(ctx.group[ROW_NORMALIZATION_KEY]) is RowNormalization.NORMUON
+    return normalize and isinstance(ctx.bucket.orthogonalize, NativeOrthogonalizer)
+
+
+def _finish_run(ctx: RunContext, orthogonal: Tensor) -> RunResult:
+    """Stage 4: the orthogonalized rows reduced to one scale per row and one per block."""
+    bucket, group, buf = ctx.bucket, ctx.group, ctx.buf
+    rows, cols, k = bucket.rows, bucket.cols, bucket.selected_rows
+    normalize = RowNormalization(group[ROW_NORMALIZATION_KEY]) is RowNormalization.NORMUON
+    fused = _fused_row_sums(ctx)
     with _stage("finish"):
         if normalize and not fused:
             _native.row_sumsq_bf16(orthogonal, cols, buf["rowsq"])
         _native.normuon_rows(buf["rowsq"], ctx.variance, ctx.index, blocks=ctx.count, rows=rows, k=k, cols=cols,
                              weight=1.0 - float(group[MUON_BETA2_KEY]), eps=NORMALIZATION_EPS, step=ctx.step,
                              normalize=normalize, denom=buf["denom"], scale=buf["scale"],
-                             parts=parts if fused else 1, step_device=bucket.step_device)
+                             parts=buf["rowsq"].shape[1] if fused else 1, step_device=bucket.step_device)
     return RunResult(params=ctx.params, rows_per_tensor=ctx.rows_per_tensor, count=ctx.count, rows=rows, k=k,
                      cols=cols, orthogonal=orthogonal, rowmap=ctx.rowmap, denom=buf["denom"], scale=buf["scale"],
                      decay_device=bucket.decay_device)
+
+
+def groups_of_runs(runs: Sequence[tuple[Bucket, Sequence[int]]],
+                   limit: int = MAX_RUN_ELEMENTS) -> list[list[tuple[Bucket, Sequence[int]]]]:
+    """``runs`` in order, split into groups that ``step_runs`` takes together: built-in iterations of
+    one dtype on one device, at most ``NS_GROUP_MAX`` of them and, so that the transient memory of a
+    step stays bounded as it is for one run, at most ``limit`` update elements together."""
+    groups: list[list[tuple[Bucket, Sequence[int]]]] = []
+    key: Any = None
+    elements = 0
+    for bucket, positions in runs:
+        fn = bucket.orthogonalize
+        this = (fn.dtype, bucket.momentum.device) if isinstance(fn, NativeOrthogonalizer) else None
+        size = sum(run_elements(bucket, position) for position in positions)
+        if (groups and this is not None and this == key and len(groups[-1]) < _native.NS_GROUP_MAX
+                and elements + size <= limit):
+            groups[-1].append((bucket, positions))
+            elements += size
+        else:
+            groups.append([(bucket, positions)])
+            key, elements = this, size
+    return groups
+
+
+def step_runs(runs: Sequence[tuple[Bucket, Sequence[int]]], param_groups: Sequence[dict[str, Any]]) -> None:
+    """One Dion step for several runs of one group (``groups_of_runs``), stage by stage.
+
+    Their Newton-Schulz iterations run as one launch.  An iteration is a chain of 15 to 18 products;
+    on small blocks each is one part-filled wave and most of its time is the way from one product to
+    the next, which the products of the other runs fill.  Same kernels on the same values: the
+    results are those of ``step_run`` on each."""
+    described = [_describe_run(bucket, positions, param_groups[bucket.group_index]) for bucket, positions in runs]
+    contexts = [ctx for ctx, _ in described]
+    shapes = [(ctx.count, ctx.bucket.selected_rows, ctx.bucket.cols) for ctx in contexts]
+    kinds = [ctx.bucket.orthogonalize.code for ctx in contexts]
+    plan: _workspace.Plan = {f"{i}.{name}": entry for i, (_, own) in enumerate(described) for name, entry in own.items()}
+    plan["ns"] = ((_native.newton_schulz_group_workspace_bytes(shapes, kinds),), torch.uint8)
+    buf = _workspace.carve(contexts[0].momentum.device, plan)
+    for i, (ctx, own) in enumerate(described):
+        ctx.buf = {name: buf[f"{i}.{name}"] for name in own}
+        run_front(ctx)
+    outs = [ctx.buf["x"].view(torch.bfloat16) for ctx in contexts]
+    with _stage("newton_schulz"):
+        _native.newton_schulz_group([ctx.buf["x"] for ctx in contexts], outs, shapes, kinds, buf["ns"],
+                                    [ctx.buf["rowsq"] if _fused_row_sums(ctx) else None for ctx in contexts])
+    for ctx, out in zip(contexts, outs):
+        apply_result(_finish_run(ctx, out), ctx.group)
 
 
 def prepare_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any],
@@ -268,7 +339,7 @@ def prepare_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any],
     """Stages 1-4 of a run, one after the other on the current stream."""
     ctx = open_run(bucket, positions, group, arena)
     run_front(ctx)
-    return run_core(ctx)
+    return run_core(ctx, alone=True)
 
 
 def apply_result(result: RunResult, group: dict[str, Any]) -> None:

@@ -20,6 +20,7 @@ LIBRARY_PATH = Path(__file__).resolve().parent / "lib" / "libdionw_b200.so"
 
 F32, F16, BF16 = 0, 1, 2
 NS_GRAM, NS_POLAR_EXPRESS, NS_KELLER, NS_GRAM_FULL = 0, 1, 2, 3
+NS_STEPWISE = 256   # added to a kind: one launch per product
 _DTYPE_CODE = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
 
 _ERRORS = {
@@ -61,6 +62,9 @@ SIGNATURES: dict[str, tuple[object, tuple[object, ...]]] = {
     "dionw_newton_schulz_tall_workspace_bytes": (c_size_t, (c_int64, c_int64, c_int64, c_int)),
     "dionw_newton_schulz_tall": (
         c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_size_t, c_void_p, c_void_p)),
+    "dionw_newton_schulz_group_workspace_bytes": (c_size_t, (c_int, _I64P, _I64P, _I64P, POINTER(c_int))),
+    "dionw_newton_schulz_group": (
+        c_int, (c_int, _PP, _PP, _I64P, _I64P, _I64P, POINTER(c_int), c_void_p, c_size_t, _PP, c_void_p)),
     "dionw_newton_schulz_rowsq_parts": (c_int64, (c_int64,)),
     "dionw_newton_schulz_static": (
         c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p)),
@@ -281,6 +285,26 @@ def newton_schulz_tall(x: Tensor, out: Tensor, rows: int, cols: int, kind: int, 
     _check(library().dionw_newton_schulz_tall(x.data_ptr(), out.data_ptr(), x.shape[0], rows, cols, x.stride(-2), kind,
                                               workspace.data_ptr(), workspace.numel() * workspace.element_size(),
                                               _ptr(rowsq), _stream(x)))
+
+
+NS_GROUP_MAX = 6   # DIONW_NS_GROUP_MAX
+
+
+def newton_schulz_group_workspace_bytes(shapes: Sequence[tuple[int, int, int]], kinds: Sequence[int]) -> int:
+    """Scratch for one launch over batches of ``(blocks, rows, cols)``."""
+    n = len(shapes)
+    return int(library().dionw_newton_schulz_group_workspace_bytes(
+        n, *(_i64_array([shape[i] for shape in shapes]) for i in range(3)), (c_int * n)(*kinds)))
+
+
+def newton_schulz_group(xs: Sequence[Tensor], outs: Sequence[Tensor], shapes: Sequence[tuple[int, int, int]],
+                        kinds: Sequence[int], workspace: Tensor, rowsqs: Sequence[Tensor | None]) -> None:
+    """The iterations of up to ``NS_GROUP_MAX`` batches as one launch (``x`` ``[blocks, rows, padded cols]``)."""
+    n = len(shapes)
+    _check(library().dionw_newton_schulz_group(
+        n, _ptr_array(xs), _ptr_array(outs), *(_i64_array([shape[i] for shape in shapes]) for i in range(3)),
+        (c_int * n)(*kinds), workspace.data_ptr(), workspace.numel() * workspace.element_size(),
+        (c_void_p * n)(*[_ptr(r) for r in rowsqs]), _stream(xs[0])))
 
 
 STATIC_SCRATCH_BYTES = 64 << 20

@@ -1,5 +1,6 @@
 // Host side of the tcgen05 GEMMs: tensor maps, launches, and the Newton-Schulz
 // product schedules built from them.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <map>
@@ -7,6 +8,7 @@
 #include <utility>
 
 #include "gemm2_sm100.cuh"
+#include "products.cuh"
 
 namespace dionw {
 namespace {
@@ -166,28 +168,19 @@ bool use_cta_pairs() {
   return on;
 }
 
-template <typename InT, typename OutT, bool kBMajorMN, bool kSym>
-int launch2(const CUtensorMap& map_a, const CUtensorMap& map_b, gemm::Params p, cudaStream_t stream) {
-  auto kernel = gemm2::gemm2_kernel<InT, OutT, kBMajorMN, kSym>;
+// Runs a filled plan as clusters of two CTAs.
+template <typename InT, int kMaps, int kSteps>
+int launch_plan(const gemm2::Plan<kMaps, kSteps>& plan, cudaStream_t stream) {
+  static_assert(sizeof(plan) <= 32764, "kernel parameters are limited to 32764 bytes");
+  auto kernel = gemm2::gemm2_kernel<InT, kMaps, kSteps>;
   static std::atomic<bool> configured[kMaxDevices];   // the attribute is per device
   const int device = current_device();
   if (!configured[device].load(std::memory_order_acquire)) {
     DIONW_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm2::kSmemBytes)));
     configured[device].store(true, std::memory_order_release);
   }
-  // Pair tiles are 256 x 256.
-  p.tiles_m = (p.m + gemm2::kPairM - 1) / gemm2::kPairM;
-  p.tiles_n = (p.n + gemm2::kBN - 1) / gemm2::kBN;
-  p.tiles_per_batch = kSym ? p.tiles_m * (p.tiles_m + 1) / 2 : p.tiles_m * p.tiles_n;
-  const int total = p.tiles_per_batch * p.batches;
-  if (total == 0) return DIONW_OK;
   const int pairs_max = sm_count() / 2;
-  const int pairs = total < pairs_max ? total : pairs_max;
-  // Tiles from a counter only where a pair takes more than one: a one-wave product gains nothing
-  // from it and would pay the hand-out's latency on its critical path.
-  p.tile_counter = (use_dynamic_tiles() && total > pairs) ? tile_counters(stream) : nullptr;
-  // The streaming job rides on products whose main loop is long enough to hide a row behind it.
-  p.job = (p.kdim >= 24 * gemm2::kBK) ? t_side_job : nullptr;
+  const int pairs = plan.total_tiles < pairs_max ? plan.total_tiles : pairs_max;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(unsigned(2 * pairs));
   config.blockDim = dim3(gemm2::kThreads);
@@ -201,137 +194,216 @@ int launch2(const CUtensorMap& map_a, const CUtensorMap& map_b, gemm::Params p, 
   attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
-  config.numAttrs = use_dependent_launch() ? 2 : 1;
+  // A plan of several products follows the clearing of its counters, which is no kernel.
+  config.numAttrs = kSteps == 1 && use_dependent_launch() ? 2 : 1;
   count_launch();
-  return check_cuda(cudaLaunchKernelEx(&config, kernel, map_a, map_b, p), "gemm2_kernel launch");
+  return check_cuda(cudaLaunchKernelEx(&config, kernel, plan), "gemm2_kernel launch");
 }
 
-// The one-CTA kernel, or the two-CTA kernel when it is switched on.  The tensor map of B is
-// built by the caller for the variant in use (their B boxes differ).
-template <typename InT, typename OutT, bool kBMajorMN, bool kSym>
-int launch_any(const CUtensorMap& map_a, const CUtensorMap& map_b, const gemm::Params& p, cudaStream_t stream) {
-  if (use_cta_pairs()) return launch2<InT, OutT, kBMajorMN, kSym>(map_a, map_b, p, stream);
-  return launch<InT, OutT, kBMajorMN, kSym>(map_a, map_b, p, stream);
+// The epilogue's side of a product; the tile counts are the caller's.
+gemm::Params params_of(const Product& product) {
+  gemm::Params p{};
+  p.cin = product.cin.base;
+  p.out = const_cast<void*>(product.out.base);
+  p.out2 = product.out2;
+  p.ldc = product.cin.ld;
+  p.ldo = product.out.ld;
+  p.cin_batch = product.cin.batch;
+  p.out_batch = product.out.batch;
+  p.alpha = product.alpha;
+  p.beta = product.beta;
+  p.diag = product.diag;
+  p.m = int(product.m);
+  p.n = int(product.n);
+  p.kdim = int(product.k);
+  p.batches = int(product.blocks);
+  p.mirror_diagonal = product.same_operands ? 0 : 1;
+  p.rowsq = product.rowsq;
+  p.rowsq_parts = int(2 * ((product.n + gemm::kBN - 1) / gemm::kBN));
+  p.status = device_status_word();
+  p.wait_ns = gemm::kWaitLimitNs;
+  return p;
 }
 
-int host_sym_tiles(int tiles_m) {
-  const int q = tiles_m / 2;
-  return q * (q + 1) + ((tiles_m & 1) ? q + 1 : 0);
+// Operand A is stored [m, k] (or [k, m]: a_mn), B is stored [n, k] (or [k, n]: b_mn).
+int operand_map(CUtensorMap* map, const Operand& x, int dtype, bool mn, int64_t outer, int64_t k, int64_t blocks,
+                uint32_t box_outer) {
+  if (mn) return make_map(map, x.base, dtype, outer, k, blocks, x.ld, x.batch, 64, gemm::kBK);
+  return make_map(map, x.base, dtype, k, outer, blocks, x.ld, x.batch, gemm::kBK, box_outer);
+}
+
+int run_one_cta(const Product& product, int dtype, cudaStream_t stream) {
+  const int64_t blocks = product.blocks;
+  CUtensorMap map_a, map_b;
+  int st = operand_map(&map_a, product.a, dtype, product.a_mn, product.m, product.k, blocks, gemm::kBM);
+  if (st != DIONW_OK) return st;
+  st = operand_map(&map_b, product.b, dtype, product.b_mn, product.n, product.k, blocks, gemm::kBN);
+  if (st != DIONW_OK) return st;
+  gemm::Params p = params_of(product);
+  p.tiles_m = (p.m + gemm::kBM - 1) / gemm::kBM;
+  p.tiles_n = (p.n + gemm::kBN - 1) / gemm::kBN;
+  const int q = p.tiles_m / 2;
+  p.tiles_per_batch = product.symmetric ? q * (q + 1) + ((p.tiles_m & 1) ? q + 1 : 0) : p.tiles_m * p.tiles_n;
+  const bool f16 = dtype == DIONW_F16, same = product.out_dtype == dtype;
+  if (product.symmetric) {
+    if (product.b_mn)
+      return f16 ? launch<__half, __half, true, true>(map_a, map_b, p, stream)
+                 : launch<__nv_bfloat16, __nv_bfloat16, true, true>(map_a, map_b, p, stream);
+    return f16 ? launch<__half, __half, false, true>(map_a, map_b, p, stream)
+               : launch<__nv_bfloat16, __nv_bfloat16, false, true>(map_a, map_b, p, stream);
+  }
+  if (product.b_mn) {
+    if (f16 && same) return launch<__half, __half, true, false>(map_a, map_b, p, stream);
+    if (f16) return launch<__half, __nv_bfloat16, true, false>(map_a, map_b, p, stream);
+    return launch<__nv_bfloat16, __nv_bfloat16, true, false>(map_a, map_b, p, stream);
+  }
+  if (f16 && same) return launch<__half, __half, false, false>(map_a, map_b, p, stream);
+  if (f16) return launch<__half, __nv_bfloat16, false, false>(map_a, map_b, p, stream);
+  return launch<__nv_bfloat16, __nv_bfloat16, false, false>(map_a, map_b, p, stream);
+}
+
+// Tiles of 256 x 256.
+int64_t wide_tiles(const Product& product) {
+  const int64_t tm = (product.m + gemm2::kPairM - 1) / gemm2::kPairM, tn = (product.n + gemm2::kBN - 1) / gemm2::kBN;
+  return product.blocks * (product.symmetric ? tm * (tm + 1) / 2 : tm * tn);
+}
+
+// Width of the tiles of a product that runs beside products of `tiles` 256-wide tiles in all (its own
+// among them).  256 columns are the better use of the memory system (a k-block of a 256 x 256 tile brings
+// 32 KB into each SM, one of two 256 x 128 tiles 24 KB each), so they are taken wherever they fill the GPU.
+// Where they would leave half of the SM pairs without a tile, twice as many pairs with half the columns each
+// finish sooner: main loop and epilogue are then half as long.  Row sums come in parts of 128 columns per
+// warp: 256-wide tiles.  In a chain, 128 against 256 columns: 1 block of 256^3 with Cin 7.1 against 8.0 us,
+// with two outputs 8.1 against 10.7; 1 block of 2048^3 18.0 against 26.5 us.
+int tile_width(const Product& product, int64_t tiles) {
+  if (product.rowsq != nullptr) return gemm2::kBN;
+  if (product.n <= gemm2::kBN / 2) return gemm2::kBN / 2;
+  return 2 * tiles <= sm_count() / 2 ? gemm2::kBN / 2 : gemm2::kBN;
+}
+
+// Fills a plan with `count` products.  `counters` (device memory, see plan_counter_bytes) is needed for more
+// than one; a single product draws its tiles from the stream's own counters when that is switched on.
+template <typename InT, int kMaps, int kSteps>
+int run_plan(const Product* const* products, int count, int dtype, unsigned* counters, cudaStream_t stream) {
+  gemm2::Plan<kMaps, kSteps> plan;
+  struct Mapped {
+    Operand x;
+    int64_t inner, rows;
+    uint32_t box;
+  } mapped[kMaps];
+  int maps = 0;
+  int64_t tiles = 0;
+  int64_t matrices = 0;
+  uint64_t done[kMaxChains] = {}, need[kMaxChains] = {};   // reports of a matrix: by the products so far; before this one
+  for (int i = 0; i < count; ++i) {
+    const Product& product = *products[i];
+    const int64_t blocks = product.blocks;
+    // the products that run at the same time: the neighbours at the same position of other chains
+    int64_t together = 0;
+    for (int j = i; j >= 0 && (j == i || products[j]->chain < products[j + 1]->chain); --j) together += wide_tiles(*products[j]);
+    for (int j = i + 1; j < count && products[j]->chain > products[j - 1]->chain; ++j) together += wide_tiles(*products[j]);
+    gemm2::Step& step = plan.steps[i];
+    // One map serves an operand in several products: the dimensions are those of memory, and boxes of 64
+    // rows suit both an MN-major operand and the half of B that a CTA loads of a 128-wide tile.
+    auto map_of = [&](const Operand& x, bool mn, int64_t outer, uint32_t box, int* index) {
+      const int64_t inner = mn ? outer : product.k, rows = mn ? product.k : outer;
+      for (int j = 0; j < maps; ++j)
+        if (mapped[j].x.base == x.base && mapped[j].x.ld == x.ld && mapped[j].x.batch == x.batch &&
+            mapped[j].inner == inner && mapped[j].rows == rows && mapped[j].box == box) {
+          *index = j;
+          return int(DIONW_OK);
+        }
+      if (maps == kMaps) {
+        set_error("a plan of %d products needs more than %d tensor maps", count, kMaps);
+        return int(DIONW_ERR_UNSUPPORTED);
+      }
+      const int st = operand_map(&plan.maps[maps], x, dtype, mn, outer, product.k, blocks, box);
+      if (st != DIONW_OK) return st;
+      mapped[maps] = {x, inner, rows, box};
+      *index = maps++;
+      return int(DIONW_OK);
+    };
+    step.tile_n = short(tile_width(product, together));
+    int st = map_of(product.a, product.a_mn, product.m, product.a_mn ? 64 : gemm2::kBM, &step.map_a);
+    if (st != DIONW_OK) return st;
+    st = map_of(product.b, product.b_mn, product.n, product.b_mn ? 64 : step.tile_n / 2, &step.map_b);
+    if (st != DIONW_OK) return st;
+    step.p = params_of(product);
+    step.p.tiles_m = (step.p.m + gemm2::kPairM - 1) / gemm2::kPairM;
+    step.p.tiles_n = (step.p.n + step.tile_n - 1) / step.tile_n;
+    step.p.tiles_per_batch = product.symmetric ? (gemm2::kBN / step.tile_n) * (step.p.tiles_m * (step.p.tiles_m + 1) / 2)
+                                               : step.p.tiles_m * step.p.tiles_n;
+    step.symmetric = product.symmetric;
+    step.a_major_mn = product.a_mn;
+    step.b_major_mn = product.b_mn;
+    step.out_bf16 = product.out_dtype == DIONW_BF16;
+    if (!product.beside_previous) need[product.chain] = done[product.chain];
+    done[product.chain] += uint64_t(step.p.tiles_per_batch) * gemm2::kReportsPerTile;
+    step.need = unsigned(need[product.chain]);
+    step.progress = counters != nullptr ? counters + 2 + product.first_block : nullptr;
+    if (product.first_block + blocks > matrices) matrices = product.first_block + blocks;
+    step.first_tile = int(tiles);
+    tiles += int64_t(step.p.tiles_per_batch) * blocks;
+    DIONW_REQUIRE(tiles < (1LL << 31) && done[product.chain] < (1ULL << 32), "the products of one launch have too many tiles");
+  }
+  for (int i = maps; i < kMaps; ++i) plan.maps[i] = plan.maps[0];   // every map is prefetched
+  if (tiles == 0) return DIONW_OK;
+  plan.count = count;
+  plan.total_tiles = int(tiles);
+  plan.job = t_side_job;
+  plan.status = device_status_word();
+  plan.wait_ns = gemm::kWaitLimitNs;
+  if (count > 1) {
+    plan.tile_counter = reinterpret_cast<int*>(counters);
+    DIONW_CUDA(cudaMemsetAsync(counters, 0, plan_counter_bytes(matrices), stream));
+  } else {
+    // Tiles from a counter only where a pair takes more than one: a one-wave product gains nothing
+    // from it and would pay the hand-out's latency on its critical path.
+    plan.tile_counter = (use_dynamic_tiles() && tiles > sm_count() / 2) ? tile_counters(stream) : nullptr;
+  }
+  return launch_plan<InT>(plan, stream);
 }
 
 }  // namespace
 
-// C = alpha A B^T + beta Cin for a product known to be symmetric (B = A, or A and B symmetric
-// matrices that commute): lower tiles + mirror, optional second output with diag added.
-// b == nullptr means B = A.  `transposed` (with b == nullptr): A is stored [kdim, m] and the product is
-// A^T A.
-int symmetric_product(const void* a, bool transposed, const void* b, int64_t blocks, int64_t m, int64_t kdim, int64_t lda,
-                      int64_t a_batch, int64_t ldb, int64_t b_batch, const void* cin, int64_t ldc, int64_t cin_batch, float alpha, float beta, void* out,
-                      int64_t ldo, int64_t out_batch, void* out2, float diag, int dtype, cudaStream_t stream) {
-  DIONW_REQUIRE(dtype == DIONW_F16 || dtype == DIONW_BF16, "symmetric_product: dtype must be F16 or BF16");
-  DIONW_REQUIRE(blocks > 0 && m > 0 && kdim > 0, "symmetric_product: empty problem");
-  CUtensorMap map_a, map_b;
-  const bool same = b == nullptr || b == a;
-  int st;
-  if (transposed) {
-    DIONW_REQUIRE(b == nullptr, "symmetric_product: a transposed operand takes no second one");
-    st = make_map(&map_a, a, dtype, m, kdim, blocks, lda, a_batch, 64, gemm::kBK);
-    if (st != DIONW_OK) return st;
-    map_b = map_a;
-  } else {
-    st = make_map(&map_a, a, dtype, kdim, m, blocks, lda, a_batch, gemm::kBK, gemm::kBM);
-    if (st != DIONW_OK) return st;
-    if (b == nullptr) {
-      b = a;
-      ldb = lda;
-      b_batch = a_batch;
-    }
-    st = make_map(&map_b, b, dtype, kdim, m, blocks, ldb, b_batch, gemm::kBK,
-                  use_cta_pairs() ? gemm2::kHalfN : gemm::kBN);
-    if (st != DIONW_OK) return st;
-  }
-  gemm::Params p{};
-  p.cin = cin;
-  p.out = out;
-  p.out2 = out2;
-  p.ldc = ldc;
-  p.ldo = ldo;
-  p.cin_batch = cin_batch;
-  p.out_batch = out_batch;
-  p.alpha = alpha;
-  p.beta = beta;
-  p.diag = diag;
-  p.m = int(m);
-  p.n = int(m);
-  p.kdim = int(kdim);
-  p.batches = int(blocks);
-  p.tiles_m = int((m + gemm::kBM - 1) / gemm::kBM);
-  p.tiles_n = int((m + gemm::kBN - 1) / gemm::kBN);
-  p.tiles_per_batch = host_sym_tiles(p.tiles_m);
-  p.mirror_diagonal = same ? 0 : 1;
-  p.status = device_status_word();
-  p.wait_ns = gemm::kWaitLimitNs;
-  if (transposed) {
-    if (dtype == DIONW_F16) return launch_any<__half, __half, true, true>(map_a, map_b, p, stream);
-    return launch_any<__nv_bfloat16, __nv_bfloat16, true, true>(map_a, map_b, p, stream);
-  }
-  if (dtype == DIONW_F16) return launch_any<__half, __half, false, true>(map_a, map_b, p, stream);
-  return launch_any<__nv_bfloat16, __nv_bfloat16, false, true>(map_a, map_b, p, stream);
-}
+size_t plan_counter_bytes(int64_t blocks) { return blocks <= kMaxPlanBlocks ? size_t(blocks + 2) * sizeof(unsigned) : 0; }
 
-// C = A B + beta Cin.
-int batched_gemm(const void* a, int64_t lda, int64_t a_batch, const void* b, int64_t ldb, int64_t b_batch,
-                 bool b_is_nk, const void* cin, int64_t ldc, int64_t cin_batch, float beta, void* out, int64_t ldo,
-                 int64_t out_batch, int64_t blocks, int64_t m, int64_t n, int64_t kdim, int in_dtype, int out_dtype,
-                 float* rowsq, cudaStream_t stream) {
-  DIONW_REQUIRE(in_dtype == DIONW_F16 || in_dtype == DIONW_BF16, "batched_gemm: input dtype must be F16 or BF16");
-  DIONW_REQUIRE(out_dtype == DIONW_F16 || out_dtype == DIONW_BF16, "batched_gemm: output dtype must be F16 or BF16");
-  DIONW_REQUIRE(blocks > 0 && m > 0 && n > 0 && kdim > 0, "batched_gemm: empty problem");
-  CUtensorMap map_a, map_b;
-  int st = make_map(&map_a, a, in_dtype, kdim, m, blocks, lda, a_batch, gemm::kBK, gemm::kBM);
-  if (st != DIONW_OK) return st;
-  if (b_is_nk) {
-    st = make_map(&map_b, b, in_dtype, kdim, n, blocks, ldb, b_batch, gemm::kBK,
-                  use_cta_pairs() ? gemm2::kHalfN : gemm::kBN);
-  } else {
-    st = make_map(&map_b, b, in_dtype, n, kdim, blocks, ldb, b_batch, 64, gemm::kBK);
+int run_products(const Product* products, int count, int dtype, void* counters, cudaStream_t stream) {
+  const bool f16 = dtype == DIONW_F16;
+  // position in the chain first, then the chain
+  const Product* ordered[kMaxChains * kMaxChainProducts];
+  int position[kMaxChains * kMaxChainProducts], seen[kMaxChains] = {};
+  int64_t matrices = 0;
+  int chains = 0;
+  DIONW_REQUIRE(count <= kMaxChains * kMaxChainProducts, "products: too many in one call");
+  for (int i = 0; i < count; ++i) {
+    DIONW_REQUIRE(products[i].blocks > 0, "products: empty batch");
+    position[i] = seen[products[i].chain]++;
+    matrices = std::max(matrices, products[i].first_block + products[i].blocks);
+    chains = std::max(chains, products[i].chain + 1);
   }
-  if (st != DIONW_OK) return st;
-  gemm::Params p{};
-  p.cin = cin;
-  p.out = out;
-  p.out2 = nullptr;
-  p.ldc = ldc;
-  p.ldo = ldo;
-  p.cin_batch = cin_batch;
-  p.out_batch = out_batch;
-  p.alpha = 1.0f;
-  p.beta = beta;
-  p.diag = 0.0f;
-  p.m = int(m);
-  p.n = int(n);
-  p.kdim = int(kdim);
-  p.batches = int(blocks);
-  p.tiles_m = int((m + gemm::kBM - 1) / gemm::kBM);
-  p.tiles_n = int((n + gemm::kBN - 1) / gemm::kBN);
-  p.tiles_per_batch = p.tiles_m * p.tiles_n;
-  p.rowsq = rowsq;
-  p.rowsq_parts = 2 * p.tiles_n;   // both kernels' tiles are 256 columns wide
-  p.status = device_status_word();
-  p.wait_ns = gemm::kWaitLimitNs;
-  const bool f16 = in_dtype == DIONW_F16;
-  const bool out_same = out_dtype == in_dtype;
-  if (b_is_nk) {
-    if (f16 && out_same) return launch_any<__half, __half, false, false>(map_a, map_b, p, stream);
-    if (f16) return launch_any<__half, __nv_bfloat16, false, false>(map_a, map_b, p, stream);
-    if (out_same) return launch_any<__nv_bfloat16, __nv_bfloat16, false, false>(map_a, map_b, p, stream);
-  } else {
-    if (f16 && out_same) return launch_any<__half, __half, true, false>(map_a, map_b, p, stream);
-    if (f16) return launch_any<__half, __nv_bfloat16, true, false>(map_a, map_b, p, stream);
-    if (out_same) return launch_any<__nv_bfloat16, __nv_bfloat16, true, false>(map_a, map_b, p, stream);
+  int n = 0;
+  for (int level = 0; level < kMaxChainProducts; ++level)
+    for (int i = 0; i < count; ++i)
+      if (position[i] == level) ordered[n++] = products + i;
+  DIONW_REQUIRE(n == count, "products: a chain is too long");
+  if (use_cta_pairs() && count > 1 && matrices <= kMaxPlanBlocks && counters != nullptr) {
+    unsigned* c = static_cast<unsigned*>(counters);
+    constexpr int kMaps = kMaxChainMaps, kSteps = kMaxChainProducts;
+    if (chains == 1)
+      return f16 ? run_plan<__half, kMaps, kSteps>(ordered, count, dtype, c, stream)
+                 : run_plan<__nv_bfloat16, kMaps, kSteps>(ordered, count, dtype, c, stream);
+    return f16 ? run_plan<__half, kMaxChains * kMaps, kMaxChains * kSteps>(ordered, count, dtype, c, stream)
+               : run_plan<__nv_bfloat16, kMaxChains * kMaps, kMaxChains * kSteps>(ordered, count, dtype, c, stream);
   }
-  set_error("batched_gemm: bf16 inputs with an fp16 output are not supported");
-  return DIONW_ERR_UNSUPPORTED;
+  for (int i = 0; i < count; ++i) {
+    int st;
+    if (!use_cta_pairs()) st = run_one_cta(products[i], dtype, stream);
+    else if (f16) st = run_plan<__half, 2, 1>(ordered + i, 1, dtype, nullptr, stream);
+    else st = run_plan<__nv_bfloat16, 2, 1>(ordered + i, 1, dtype, nullptr, stream);
+    if (st != DIONW_OK) return st;
+  }
+  return DIONW_OK;
 }
 
 }  // namespace dionw
@@ -340,17 +412,51 @@ extern "C" int dionw_symmetric_product(const void* a, const void* b, int64_t blo
                                        int64_t lda, int64_t ldb, const void* cin, int64_t ldc, float alpha,
                                        float beta, void* out, int64_t ldo, void* out2, float diag, int dtype,
                                        void* stream) {
-  return dionw::symmetric_product(a, false, b, blocks, m, kdim, lda, m * lda, ldb, m * ldb, cin, ldc, m * ldc, alpha, beta,
-                                  out, ldo, m * ldo, out2, diag, dtype, static_cast<cudaStream_t>(stream));
+  using namespace dionw;
+  DIONW_REQUIRE(dtype == DIONW_F16 || dtype == DIONW_BF16, "symmetric_product: dtype must be F16 or BF16");
+  DIONW_REQUIRE(blocks > 0 && m > 0 && kdim > 0, "symmetric_product: empty problem");
+  Product product;
+  product.a = {a, lda, m * lda};
+  product.same_operands = b == nullptr || b == a;
+  product.b = b == nullptr ? product.a : Operand{b, ldb, m * ldb};
+  product.symmetric = true;
+  product.cin = {cin, ldc, m * ldc};
+  product.alpha = alpha;
+  product.beta = beta;
+  product.out = {out, ldo, m * ldo};
+  product.out2 = out2;
+  product.diag = diag;
+  product.m = product.n = m;
+  product.k = kdim;
+  product.out_dtype = dtype;
+  product.blocks = blocks;
+  return run_products(&product, 1, dtype, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int dionw_batched_gemm(const void* a, int64_t lda, const void* b, int64_t ldb, int b_is_nk,
                                   const void* cin, int64_t ldc, float beta, void* out, int64_t ldo, int64_t blocks,
                                   int64_t m, int64_t n, int64_t kdim, int in_dtype, int out_dtype, void* stream) {
-  const int64_t b_rows = b_is_nk ? n : kdim;
-  return dionw::batched_gemm(a, lda, m * lda, b, ldb, b_rows * ldb, b_is_nk != 0, cin, ldc, m * ldc, beta, out, ldo,
-                             m * ldo, blocks, m, n, kdim, in_dtype, out_dtype, nullptr,
-                             static_cast<cudaStream_t>(stream));
+  using namespace dionw;
+  DIONW_REQUIRE(in_dtype == DIONW_F16 || in_dtype == DIONW_BF16, "batched_gemm: input dtype must be F16 or BF16");
+  DIONW_REQUIRE(out_dtype == DIONW_F16 || out_dtype == DIONW_BF16, "batched_gemm: output dtype must be F16 or BF16");
+  DIONW_REQUIRE(blocks > 0 && m > 0 && n > 0 && kdim > 0, "batched_gemm: empty problem");
+  if (in_dtype == DIONW_BF16 && out_dtype != DIONW_BF16) {
+    set_error("batched_gemm: bf16 inputs with an fp16 output are not supported");
+    return DIONW_ERR_UNSUPPORTED;
+  }
+  Product product;
+  product.a = {a, lda, m * lda};
+  product.b = {b, ldb, (b_is_nk ? n : kdim) * ldb};
+  product.b_mn = b_is_nk == 0;
+  product.cin = {cin, ldc, m * ldc};
+  product.beta = beta;
+  product.out = {out, ldo, m * ldo};
+  product.m = m;
+  product.n = n;
+  product.k = kdim;
+  product.out_dtype = out_dtype;
+  product.blocks = blocks;
+  return run_products(&product, 1, in_dtype, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 namespace dionw {

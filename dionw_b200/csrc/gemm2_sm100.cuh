@@ -6,7 +6,8 @@
 //
 // Roles per CTA: warp 0 = TMA producer for this CTA's operands; warp 1 = in the leader
 // CTA (cluster rank 0) the MMA issuer (idle in the other CTA); warps 2-9 = epilogue of this
-// CTA's 128 accumulator rows (the epilogue code is shared with the one-CTA kernel).  Every
+// CTA's 128 accumulator rows (the epilogue code is shared with the one-CTA kernel); warp 10 = in a plan
+// of several products the reporter of stored tiles.  Every
 // TMA load is a per-CTA load into the CTA's own shared memory (no multicast); both CTAs' loads
 // of a stage complete on ONE barrier, in the leader, which the .cta_group::2 form of the copy
 // permits; only the leader's producer announces the pair's byte count on it.  The other
@@ -21,9 +22,32 @@
 // optimizer step 97.5-100.5 ms instead of 100.0-103.1.  It is the default; DIONW_GEMM_CTA_PAIRS=0
 // selects the one-CTA kernel.
 //
+// A launch runs a PLAN: one product, or the whole Newton-Schulz iterations of up to six batches (chains of
+// up to 18 products that depend on one another, matrix by matrix).  In a plan of several products the tiles
+// of all of them form one sequence, ordered by position in the chain and then by chain, which the pairs draw
+// from a counter; `progress[b]` counts what has been stored for matrix b, and a tile's loads start once
+// everything its product reads from matrix b is there.  What that buys, against one launch per product: pairs
+// that run out of tiles of one product go on with the next one's, so only the last product of a plan ends in a
+// part-filled wave; the start of a product (launch, descriptor fetch, first loads) and the end of the one
+// before (last epilogue, teardown) overlap across matrices; and the host makes one launch where it made 15 to 18.
+// Measured, an iteration as one launch per product against one plan: 16 blocks of 1024^2 453 -> 380 us,
+// 16 of 1024 x 4096 805 -> 720 us, 1 of 256 x 1024 146 -> 143 us; the four batches of a 12-layer 768-wide
+// language model 1259 -> 900 us, the six of a 1100-wide image encoder 3.3 -> 1.9 ms, a 4-layer 4096-wide
+// one's four 8.9 -> 8.0 ms.  A plan's matrices need not lie in L2 for that: running them in cohorts of two
+// waves of tiles, each through all its products, changed nothing.
+//
+// What bounds a plan of small matrices now is the epilogue's chain of latencies: with clocks read inside the
+// kernel, an epilogue warp spent 4000 of 15000 cycles per 768-deep tile waiting for its accumulator.  Sixteen
+// epilogue warps, each with half the columns, were 10 to 25 % slower (96 registers a thread: spills).
+//
+// Why a plan cannot deadlock, whatever else runs on the GPU: tiles are drawn in order by pairs that are
+// already running, and a tile depends only on tiles before it.  The earliest unfinished tile is therefore
+// held by a running pair whose wait is over.
+//
 // Every spin-wait is bounded, as in the one-CTA kernel.
 #pragma once
 
+#include "cluster.cuh"
 #include "gemm_sm100.cuh"
 
 namespace dionw {
@@ -36,33 +60,17 @@ constexpr int kPairM = 256;                        // rows of a pair's tile
 constexpr int kBM = 128;                           // rows per CTA
 constexpr int kBN = 256;
 constexpr int kBK = 64;
-constexpr int kHalfN = 128;                        // columns of B each CTA loads
 constexpr int kStages = 6;
-constexpr int kThreads = 320;
-constexpr int kEpilogueThreads = 256;
+constexpr int kEpilogueWarps = 8;
+constexpr int kReporterWarp = 2 + kEpilogueWarps;
+constexpr int kThreads = 32 * (kReporterWarp + 1);
+constexpr uint32_t kBarrierBytes = 512;
 constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
-constexpr uint32_t kBBytes = kHalfN * kBK * 2;     // 16 KB
+constexpr uint32_t kBBytes = (kBN / 2) * kBK * 2;  // 16 KB: the half of B's columns that each CTA loads
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
-constexpr uint32_t kPanelBytes = 64 * kBK * 2;
-constexpr size_t kSmemBytes = size_t(kStages) * kStageBytes + 1024 + 256 + gemm::kMirrorBytes;
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Address of the same shared-memory object in another CTA of the cluster.
-__device__ __forceinline__ uint32_t peer_address(const void* local, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(gemm::smem_u32(local)), "r"(rank));
-  return out;
-}
+constexpr uint32_t kPanelBytes = 64 * kBK * 2;     // one 64-column panel of an MN-major operand
+constexpr size_t kSmemBytes = size_t(kStages) * kStageBytes + 1024 + kBarrierBytes +
+                              kEpilogueWarps * 2 * gemm::kPieceBytes;
 
 __device__ __forceinline__ void remote_arrive(uint32_t cluster_address) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
@@ -73,6 +81,12 @@ __device__ __forceinline__ void remote_arrive(uint32_t cluster_address) {
 // acquire at cluster scope.  Used once per tile (the tile hand-out), never per stage.
 __device__ __forceinline__ void remote_arrive_release(uint32_t cluster_address) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
+}
+
+// Relaxed arrive that is issued once `loaded`, the result of a load, is there.
+__device__ __forceinline__ void remote_arrive_after(uint32_t cluster_address, int loaded) {
+  asm volatile("{\n.reg .b32 t;\nmov.b32 t, %1;\nmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}\n"
+               ::"r"(cluster_address), "r"(loaded) : "memory");
 }
 
 __device__ __forceinline__ void remote_store_s32(uint32_t cluster_address, int value) {
@@ -155,22 +169,50 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
       : "memory");
 }
 
-// Instruction descriptor: fp32 accumulate, M = 256 (128 rows in each CTA), N = 256.
-template <typename T, bool kAMajorMN, bool kBMajorMN>
-__device__ __forceinline__ uint32_t make_idesc2() {
+// Instruction descriptor: fp32 accumulate, M = 256 (128 rows in each CTA), N = 256 or 128.
+template <typename T>
+__device__ __forceinline__ uint32_t make_idesc2(bool a_major_mn, bool b_major_mn, int tile_n) {
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
   uint32_t d = 0;
   d |= 1u << 4;
   d |= fmt << 7;
   d |= fmt << 10;
-  d |= (kAMajorMN ? 1u : 0u) << 15;
-  d |= (kBMajorMN ? 1u : 0u) << 16;
-  d |= uint32_t(kBN >> 3) << 17;
+  d |= (a_major_mn ? 1u : 0u) << 15;
+  d |= (b_major_mn ? 1u : 0u) << 16;
+  d |= uint32_t(tile_n >> 3) << 17;
   d |= uint32_t(kPairM >> 4) << 24;
   return d;
 }
 
-// Pair tiles are 256 x 256.  General: groups of 4 tile rows sweep the columns.
+// ----------------------------------------------------------------------------
+// plans
+// ----------------------------------------------------------------------------
+struct Step {
+  Params p;               // tiles_m, tiles_n, tiles_per_batch count tiles of 256 x tile_n
+  int map_a, map_b;       // indices into the plan's maps
+  int first_tile;         // tiles of the plan before this product
+  unsigned need;          // progress of a matrix from which on this product may read it
+  unsigned* progress;     // of the chain's matrices: zero at the start of the launch (null: one product only)
+  short tile_n;           // 256 or 128
+  bool symmetric;         // only tiles on and below the diagonal
+  bool a_major_mn, b_major_mn;
+  bool out_bf16;          // the result is bf16 although the operands are fp16
+};
+
+template <int kMaps, int kSteps>
+struct Plan {
+  CUtensorMap maps[kMaps];
+  Step steps[kSteps];
+  int count;
+  int total_tiles;
+  int* tile_counter;      // {next tile, pairs done} in global memory, or null for a fixed stride (one product only)
+  DecayJob* job;          // streaming job the epilogue warps work on while they wait, or null
+  int* status;
+  uint64_t wait_ns;
+};
+constexpr unsigned kReportsPerTile = 2;   // each CTA reports its half
+
+// General: groups of 4 tile rows sweep the columns.
 __device__ __forceinline__ Tile general_tile(int t, const Params& p) {
   Tile tile;
   tile.batch = t / p.tiles_per_batch;
@@ -186,20 +228,58 @@ __device__ __forceinline__ Tile general_tile(int t, const Params& p) {
   return tile;
 }
 
-// Symmetric: tile row i needs tile columns 0..i; i(i+1)/2 tiles precede row i.  (Walking the
-// triangle in groups of four tile rows swept by columns, as the general schedule does, was measured
-// and dropped: 18 blocks of 3584^2, K = 3584, 664 / 707 / 801 / 804 us against 646 / 733 / 776 / 740 us
-// for A A^T plain / with Cin / with two outputs / with B != A -- no better on balance.)
-__device__ __forceinline__ Tile sym_tile(int t, const Params& p) {
+// Symmetric: tile row i needs the columns up to its own end, (i + 1) * per_row tiles (per_row = 256 / tile_n);
+// per_row * i(i+1)/2 tiles precede row i.  (Walking the triangle in groups of four tile rows swept by
+// columns, as the general schedule does, was measured and dropped: 18 blocks of 3584^2, K = 3584,
+// 664 / 707 / 801 / 804 us against 646 / 733 / 776 / 740 us for A A^T plain / with Cin / with two
+// outputs / with B != A -- no better on balance.)
+__device__ __forceinline__ Tile sym_tile(int t, const Params& p, int per_row) {
   Tile tile;
   tile.batch = t / p.tiles_per_batch;
   const int r = t - tile.batch * p.tiles_per_batch;
-  int i = int((sqrtf(8.0f * float(r) + 1.0f) - 1.0f) * 0.5f);
-  while (i * (i + 1) / 2 > r) --i;
-  while ((i + 1) * (i + 2) / 2 <= r) ++i;
+  const int u = r / per_row;
+  int i = int((sqrtf(8.0f * float(u) + 1.0f) - 1.0f) * 0.5f);
+  while (i * (i + 1) / 2 > u) --i;
+  while ((i + 1) * (i + 2) / 2 <= u) ++i;
   tile.tm = i;
-  tile.tn = r - i * (i + 1) / 2;
+  tile.tn = r - per_row * (i * (i + 1) / 2);
   return tile;
+}
+
+__device__ __forceinline__ Tile tile_of(int t, const Step& step) {
+  return step.symmetric ? gemm2::sym_tile(t, step.p, kBN / step.tile_n) : gemm2::general_tile(t, step.p);
+}
+
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void add_release(unsigned* p, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// Orders this thread's accesses through the generic proxy (ordinary loads and stores) with those of the
+// async proxy (TMA) on both sides.
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// Bounded wait until the progress of a matrix has reached `need`.
+__device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned need, volatile int* abort_flag,
+                                              int* status, uint64_t limit_ns) {
+  uint32_t spins = 0;
+  uint64_t start = 0;
+  while (load_acquire(progress) < need) {
+    if ((++spins & 255u) == 0) {
+      if (*abort_flag != 0) return false;
+      const uint64_t now = gemm::global_ns();
+      if (start == 0) start = now;
+      else if (now - start > limit_ns) {
+        *abort_flag = 1;
+        if (status != nullptr) atomicExch(status, gemm::kWaitCode);
+        return false;
+      }
+    }
+  }
+  return true;
 }
 
 // ----------------------------------------------------------------------------
@@ -215,22 +295,32 @@ __device__ __forceinline__ Tile sym_tile(int t, const Params& p) {
 // through a ring of kTileSlots entries kept in BOTH CTAs' shared memory: it writes the entry (its own
 // copy and, through the cluster's shared-memory window, the peer's), then arrives with release at
 // cluster scope on the slot's `tile_full` barrier of each CTA.  Consumers -- the leader's MMA thread,
-// the peer's producer thread and the eight epilogue warps of each CTA, 18 in all -- wait on their own
+// the peer's producer thread and the epilogue warps of each CTA -- wait on their own
 // CTA's `tile_full` (acquire at cluster scope), read the entry and arrive on the LEADER's `tile_empty`
-// barrier of the slot; the producer reuses a slot after all 18 have done so.  -1 ends the pair's work.
+// barrier of the slot; the producer reuses a slot after all of them have done so.  -1 ends the pair's work.
 // When a pair has drawn its -1 it adds one to a second counter; the pair that brings that to the number
 // of pairs knows that nobody will draw again and clears both counters for the next launch on the stream.
-constexpr int kTileSlots = 4;
-constexpr uint32_t kTileConsumers = 2 * (1 + kEpilogueThreads / 32);
+// In a plan of several products each CTA's producer then waits for what the tile depends on, and tells its
+// own CTA's epilogue warps, which read Cin, through the slot's `ready` barrier.  (Waiting before the tile is
+// published, so that the ring itself carries the news, put the ring's two cluster-scope hops on the path
+// from one product to the next.)  An epilogue warp reports the slot as read after it has seen `ready`, so
+// that the barrier is never more than one phase ahead of it.
+//
+// A CTA's half of a tile is reported by a warp of its own, once the eight epilogue warps have arrived on the
+// slot's `stored` barrier: the release at GPU scope waits until the stores have reached L2, and took an
+// epilogue warp 2700 cycles of every tile.  The reporter, too, reports the slot as read only then.
+// For the same reason the arrivals on `tile_empty` are relaxed: they follow a load whose value is in use, not
+// the stores of the tile before (as a release at cluster scope each cost the warp 2000 cycles per tile).
+constexpr int kTileSlots = 8;
+constexpr uint32_t kTileConsumers = 2 * (1 + kEpilogueWarps);   // and the reporters, in a plan of several products
 
 // ----------------------------------------------------------------------------
 // the kernel (launched as clusters of two CTAs)
 // ----------------------------------------------------------------------------
-template <typename InT, typename OutT, bool kBMajorMN, bool kSym>
+template <typename InT, int kMaps, int kSteps>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   using namespace gemm;
-  constexpr bool kAMajorMN = kSym && kBMajorMN;   // X^T X, as in the one-CTA kernel
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + size_t(kStages) * kStageBytes);  // leader's: both CTAs' stage landed
@@ -239,19 +329,20 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   uint64_t* acc_empty = acc_full + 2;         // [2] leader only: both CTAs' epilogues drained it
   uint64_t* tile_full = acc_empty + 2;        // [kTileSlots] both: the slot's tile index is written
   uint64_t* tile_empty = tile_full + kTileSlots;  // [kTileSlots] leader only: every consumer has read the slot
-  int* tile_ring = reinterpret_cast<int*>(tile_empty + kTileSlots);  // [kTileSlots]
+  uint64_t* ready = tile_empty + kTileSlots;      // [kTileSlots] both: what the slot's tile reads is there
+  uint64_t* stored = ready + kTileSlots;          // [kTileSlots] both: this CTA's half of the slot's tile is stored
+  int* tile_ring = reinterpret_cast<int*>(stored + kTileSlots);  // [kTileSlots]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tile_ring + kTileSlots);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint8_t* mirror_stage = smem + size_t(kStages) * kStageBytes + 256;
+  uint8_t* mirror_stage = smem + size_t(kStages) * kStageBytes + kBarrierBytes;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();       // 0 = leader
   const int pair = blockIdx.x >> 1;
   const int pairs = gridDim.x >> 1;
-  const int total_tiles = p.tiles_per_batch * p.batches;
-  const int k_blocks = (p.kdim + kBK - 1) / kBK;
-  const bool dynamic = p.tile_counter != nullptr;
+  const int total_tiles = plan.total_tiles;
+  const bool dynamic = plan.tile_counter != nullptr;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -260,20 +351,19 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 2 * kEpilogueThreads);
+      mbar_init(&acc_empty[a], 2 * kEpilogueWarps);
     }
     for (int s = 0; s < kTileSlots; ++s) {
       mbar_init(&tile_full[s], 1);
-      mbar_init(&tile_empty[s], kTileConsumers);
+      mbar_init(&tile_empty[s], kTileConsumers + (kSteps > 1 ? 2 : 0));
+      mbar_init(&ready[s], 1);
+      mbar_init(&stored[s], kEpilogueWarps);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (threadIdx.x == 0) {
-    prefetch_map(&map_a);
-    prefetch_map(&map_b);
-  }
+  if (warp == 2 && lane < (kMaps < 32 ? kMaps : 32)) prefetch_map(&plan.maps[lane]);
   if (warp == 1) tmem_alloc2(tmem_slot, kTmemCols);
   tc_fence_before();
   __syncthreads();
@@ -283,19 +373,30 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
   gemm::griddep_wait();     // set-up above overlaps the tail of the previous product; global memory from here on
   gemm::griddep_launch();
 
+  // The product that tile t belongs to; each role keeps its own position, and its tiles only ever grow.
+  auto step_at = [&](int t, int& at) -> const Step& {
+    if constexpr (kSteps > 1) {
+      while (at + 1 < plan.count && t >= plan.steps[at + 1].first_tile) ++at;
+    }
+    return plan.steps[at];
+  };
+
   // The n-th tile of this pair for a consumer: its index, -1 when the pair is done, -2 when the wait
   // gave up.  Called by ONE thread per consumer (the single-thread roles themselves, lane 0 of an
   // epilogue warp), which also reports the slot as read.
   const uint32_t leader_tile_empty = peer_address(&tile_empty[0], 0);
-  auto take_tile = [&](uint32_t n) -> int {
+  auto take_tile = [&](uint32_t n, bool when_ready) -> int {
     if (!dynamic) {
       const long long t = (long long)pair + (long long)n * pairs;
       return t < total_tiles ? int(t) : -1;
     }
     const uint32_t slot = n % kTileSlots;
-    if (!mbar_wait_cluster(&tile_full[slot], (n / kTileSlots) & 1u, abort_flag, p.status, p.wait_ns)) return -2;
+    if (!mbar_wait_cluster(&tile_full[slot], (n / kTileSlots) & 1u, abort_flag, plan.status, plan.wait_ns)) return -2;
     const int t = tile_ring[slot];
-    remote_arrive_release(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)));
+    if (kSteps > 1 && when_ready && t >= 0 &&
+        !mbar_wait(&ready[slot], (n / kTileSlots) & 1u, abort_flag, plan.status, plan.wait_ns))
+      return -2;
+    remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), t);
     return t;
   };
 
@@ -303,62 +404,96 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
     // ------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
       uint32_t it = 0;
+      int at = 0;
       bool ok = true;
-      // The draw for tile n + 1 is issued before the loads of tile n: its latency hides behind them.
-      int drawn = (dynamic && rank == 0) ? atomicAdd(p.tile_counter, 1) : 0;
-      for (uint32_t n = 0; ok; ++n) {
-        int t;
-        if (dynamic && rank == 0) {
-          // publish the tile drawn last to the pair
-          const uint32_t slot = n % kTileSlots;
-          if (!mbar_wait_cluster(&tile_empty[slot], ((n / kTileSlots) & 1u) ^ 1u, abort_flag, p.status, p.wait_ns)) break;
-          t = drawn < total_tiles ? drawn : -1;
-          if (t >= 0) drawn = atomicAdd(p.tile_counter, 1);
-          tile_ring[slot] = t;
-          remote_store_s32(peer_address(&tile_ring[slot], 1), t);
-          remote_arrive_release(peer_address(&tile_full[slot], 0));
-          remote_arrive_release(peer_address(&tile_full[slot], 1));
-          if (t < 0) {
-            // nobody of this pair draws again; the last pair to get here clears the counters
-            if (atomicAdd(p.tile_counter + 1, 1) == pairs - 1) {
-              p.tile_counter[0] = 0;
-              p.tile_counter[1] = 0;
-              __threadfence();
-            }
+      // The leader publishes tile n + 1 before it loads tile n, and draws tile n + 2 then: neither the
+      // draw nor the way through the ring lies between two tiles.
+      auto publish = [&](uint32_t n, int t) -> bool {
+        const uint32_t slot = n % kTileSlots;
+        if (!mbar_wait_cluster(&tile_empty[slot], ((n / kTileSlots) & 1u) ^ 1u, abort_flag, plan.status, plan.wait_ns))
+          return false;
+        tile_ring[slot] = t;
+        remote_store_s32(peer_address(&tile_ring[slot], 1), t);
+        remote_arrive_release(peer_address(&tile_full[slot], 0));
+        remote_arrive_release(peer_address(&tile_full[slot], 1));
+        if (t < 0) {
+          // nobody of this pair draws again; the last pair to get here clears the counters
+          if (atomicAdd(plan.tile_counter + 1, 1) == pairs - 1) {
+            plan.tile_counter[0] = 0;
+            plan.tile_counter[1] = 0;
+            __threadfence();
           }
+        }
+        return true;
+      };
+      const bool leads = dynamic && rank == 0;
+      auto draw = [&] { return atomicAdd(plan.tile_counter, 1); };
+      auto valid = [&](int t) { return t < total_tiles ? t : -1; };
+      int current = -1, next = -1;
+      if (leads) {
+        current = valid(draw());
+        if (current >= 0) next = draw();
+        ok = publish(0, current);
+      }
+      for (uint32_t n = 0; ok; ++n) {
+        int t = current;
+        if (leads) {
+          if (t < 0) break;
+          current = valid(next);
+          if (!publish(n + 1, current)) break;
+          if (current >= 0) next = draw();
         } else {
-          t = take_tile(n);
+          t = take_tile(n, false);
         }
         if (t < 0) break;
-        const Tile tile = kSym ? gemm2::sym_tile(t, p) : gemm2::general_tile(t, p);
-        const int m0 = tile.tm * kPairM + int(rank) * kBM;
-        const int n0 = tile.tn * kBN + int(rank) * kHalfN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t phase = (it / kStages) & 1u;
-          if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, p.status, p.wait_ns)) { ok = false; break; }
-          uint8_t* a_dst = smem + size_t(s) * kStageBytes;
-          uint8_t* b_dst = a_dst + kABytes;
-          const uint32_t leader_full = peer_address(&full_bar[s], 0);
-          // The peer's bytes may land before the leader has announced them: the phase still
-          // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
-          // because its empty barrier is released by the MMAs that consumed this one.
-          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
-          if constexpr (kAMajorMN) {
-#pragma unroll
-            for (int panel = 0; panel < kBM / 64; ++panel)
-              tma_load_3d_pair(a_dst + panel * kPanelBytes, &map_a, leader_full, m0 + panel * 64, kb * kBK, tile.batch);
-          } else {
-            tma_load_3d_pair(a_dst, &map_a, leader_full, kb * kBK, m0, tile.batch);
+        const Step& step = step_at(t, at);
+        const Tile tile = tile_of(t - step.first_tile, step);
+        if constexpr (kSteps > 1) {
+          if (step.need != 0) {
+            if (!progress_wait(&step.progress[tile.batch], step.need, abort_flag, plan.status, plan.wait_ns)) break;
+            proxy_fence();   // what the tile reads was stored through the generic proxy, by other SMs
           }
-          if constexpr (kBMajorMN) {
-#pragma unroll
-            for (int panel = 0; panel < kHalfN / 64; ++panel)
-              tma_load_3d_pair(b_dst + panel * kPanelBytes, &map_b, leader_full, n0 + panel * 64, kb * kBK, tile.batch);
-          } else {
-            tma_load_3d_pair(b_dst, &map_b, leader_full, kb * kBK, n0, tile.batch);
-          }
+          mbar_arrive(&ready[n % kTileSlots]);
         }
+        const CUtensorMap* map_a = &plan.maps[step.map_a];
+        const CUtensorMap* map_b = &plan.maps[step.map_b];
+        const int half_n = step.tile_n / 2;
+        const int m0 = tile.tm * kPairM + int(rank) * kBM;
+        const int n0 = tile.tn * step.tile_n + int(rank) * half_n;
+        const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
+        const uint32_t pair_bytes = 2 * (kABytes + uint32_t(half_n) * kBK * 2);
+        // The layout of the operands is a constant inside the loop.
+        auto load_loop = [&](auto a_major_mn, auto b_major_mn) {
+          for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+            const int s = it % kStages;
+            const uint32_t phase = (it / kStages) & 1u;
+            if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
+            uint8_t* a_dst = smem + size_t(s) * kStageBytes;
+            uint8_t* b_dst = a_dst + kABytes;
+            const uint32_t leader_full = peer_address(&full_bar[s], 0);
+            // The peer's bytes may land before the leader has announced them: the phase still
+            // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
+            // because its empty barrier is released by the MMAs that consumed this one.
+            if (rank == 0) mbar_expect_tx(&full_bar[s], pair_bytes);
+            const int k0 = kb * kBK;
+            if constexpr (decltype(a_major_mn)::value) {
+#pragma unroll
+              for (int panel = 0; panel < kBM / 64; ++panel)
+                tma_load_3d_pair(a_dst + panel * kPanelBytes, map_a, leader_full, m0 + panel * 64, k0, tile.batch);
+            } else {
+              tma_load_3d_pair(a_dst, map_a, leader_full, k0, m0, tile.batch);
+            }
+            if constexpr (decltype(b_major_mn)::value) {
+              tma_load_3d_pair(b_dst, map_b, leader_full, n0, k0, tile.batch);
+              if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, leader_full, n0 + 64, k0, tile.batch);
+            } else {
+              tma_load_3d_pair(b_dst, map_b, leader_full, k0, n0, tile.batch);
+            }
+          }
+        };
+        if (step.a_major_mn) load_loop(std::true_type(), std::true_type());
+        else if (step.b_major_mn) load_loop(std::false_type(), std::true_type());
+        else load_loop(std::false_type(), std::false_type());
       }
     }
   } else if (warp == 1) {
@@ -366,75 +501,116 @@ gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ 
       // the second CTA's MMA warp has nothing to issue
     } else if (lane == 0) {
       // ------------------------------------------------------------ MMA issuer (leader)
-      const uint32_t idesc = make_idesc2<InT, kAMajorMN, kBMajorMN>();
       uint32_t it = 0;
+      int at = 0;
       bool ok = true;
       for (uint32_t local = 0; ok; ++local) {
-        if (take_tile(local) < 0) break;
+        const int t = take_tile(local, false);
+        if (t < 0) break;
+        const Step& step = step_at(t, at);
+        const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
+        const int tile_n = step.tile_n;
         const uint32_t acc = local & 1u;
         const uint32_t acc_phase = (local >> 1) & 1u;
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, p.wait_ns)) { ok = false; break; }
+        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * uint32_t(kBN);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t phase = (it / kStages) & 1u;
-          if (!mbar_wait(&full_bar[s], phase, abort_flag, p.status, p.wait_ns)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + size_t(s) * kStageBytes);
-          const uint32_t b_addr = a_addr + kABytes;
-          const uint64_t a_desc = kAMajorMN ? make_smem_desc(a_addr, kPanelBytes, 1024)
-                                            : make_smem_desc(a_addr, 16, 1024);
-          const uint64_t b_desc = kBMajorMN ? make_smem_desc(b_addr, kPanelBytes, 1024)
-                                            : make_smem_desc(b_addr, 16, 1024);
+        // The layout of the operands is a constant inside the loop.
+        auto main_loop = [&](auto a_major_mn, auto b_major_mn) {
+          constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
+          const uint32_t idesc = make_idesc2<InT>(kAMN, kBMN, tile_n);
+          for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+            const int s = it % kStages;
+            const uint32_t phase = (it / kStages) & 1u;
+            if (!mbar_wait(&full_bar[s], phase, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + size_t(s) * kStageBytes);
+            const uint32_t b_addr = a_addr + kABytes;
+            const uint64_t a_desc = make_smem_desc(a_addr, kAMN ? kPanelBytes : 16, 1024);
+            const uint64_t b_desc = make_smem_desc(b_addr, kBMN ? kPanelBytes : 16, 1024);
 #pragma unroll
-          for (int j = 0; j < kBK / kUmmaK; ++j) {
-            const uint64_t k_step = uint64_t((j * kUmmaK * 2) >> 4), mn_step = uint64_t((j * kUmmaK * 128) >> 4);
-            const uint64_t a_step = kAMajorMN ? mn_step : k_step;
-            const uint64_t b_step = kBMajorMN ? mn_step : k_step;
-            umma2_f16(tmem_d, a_desc + a_step, b_desc + b_step, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+            for (int j = 0; j < kBK / kUmmaK; ++j) {
+              const uint64_t k_step = uint64_t((j * kUmmaK * 2) >> 4), mn_step = uint64_t((j * kUmmaK * 128) >> 4);
+              umma2_f16(tmem_d, a_desc + (kAMN ? mn_step : k_step), b_desc + (kBMN ? mn_step : k_step), idesc,
+                        (kb > 0 || j > 0) ? 1u : 0u);
+            }
+            umma2_commit_both(&empty_bar[s]);
           }
-          umma2_commit_both(&empty_bar[s]);
-        }
+        };
+        if (step.a_major_mn) main_loop(std::true_type(), std::true_type());
+        else if (step.b_major_mn) main_loop(std::false_type(), std::true_type());
+        else main_loop(std::false_type(), std::false_type());
         if (ok) umma2_commit_both(&acc_full[acc]);
+      }
+    }
+  } else if (warp == kReporterWarp) {
+    // ------------------------------------------------------------ reporter (both CTAs)
+    if (kSteps > 1 && lane == 0) {
+      int at = 0;
+      for (uint32_t n = 0;; ++n) {
+        const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
+        if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
+        const int t = tile_ring[slot];
+        if (t < 0) break;
+        const Step& step = step_at(t, at);
+        unsigned* progress = &step.progress[(t - step.first_tile) / step.p.tiles_per_batch];
+        if (!mbar_wait(&stored[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
+        // The tile's stores are there for later tiles once it is counted (their producers order the
+        // proxies: the stores went through the generic one, TMA reads through the async one).
+        add_release(progress, 1u);
+        remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), t);
       }
     }
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int ew = warp - 2;
     const int sub = warp & 3;
-    const int first_chunk = (ew >> 2) * (kBN / 64);
     uint8_t* stage = mirror_stage + ew * 2 * kPieceBytes;
     const uint32_t leader_empty[2] = {peer_address(&acc_empty[0], 0), peer_address(&acc_empty[1], 0)};
-    bool ok = true;
-    for (uint32_t local = 0; ok; ++local) {
+    int at = 0;
+    for (uint32_t local = 0;; ++local) {
       int t = 0;
-      if (lane == 0) t = take_tile(local);   // one lane waits, reads and reports; the warp follows it
+      if (lane == 0) t = take_tile(local, true);   // one lane waits, reads and reports; the warp follows it
       t = __shfl_sync(0xffffffffu, t, 0);
       if (t < 0) break;
-      const Tile tile = kSym ? gemm2::sym_tile(t, p) : gemm2::general_tile(t, p);
+      const Step& step = step_at(t, at);
+      const Params& p = step.p;
+      const Tile tile = tile_of(t - step.first_tile, step);
+      const int chunks = step.tile_n / (32 * kEpilogueWarps / 4);
+      const int first_chunk = (ew >> 2) * chunks;
       const uint32_t acc = local & 1u;
       const uint32_t acc_phase = (local >> 1) & 1u;
-      if (p.job != nullptr) {
+      // The streaming job rides on products whose main loop is long enough to hide a row behind it.
+      if (plan.job != nullptr && p.kdim >= 24 * kBK) {
         // The accumulator of this tile is still being summed: take rows of the streaming job
         // meanwhile, at most `per_wait` of them, one at a time, looking at the barrier in between.
-        const int limit = p.job->per_wait;
+        const int limit = plan.job->per_wait;
         for (int taken = 0; taken < limit; ++taken) {
           long long row = -1;
-          if (lane == 0 && !mbar_try(&acc_full[acc], acc_phase)) row = atomicAdd(&p.job->cursor, 1);
+          if (lane == 0 && !mbar_try(&acc_full[acc], acc_phase)) row = atomicAdd(&plan.job->cursor, 1);
           row = __shfl_sync(0xffffffffu, row, 0);
-          if (row < 0 || row >= p.job->total_rows) break;
-          decay_job_row(p.job, row, lane);
+          if (row < 0 || row >= plan.job->total_rows) break;
+          decay_job_row(plan.job, row, lane);
         }
       }
-      if (!epilogue_tile<InT, OutT, kSym>(p, tile.batch, tile.tm * kPairM + int(rank) * kBM, tile.tn * kBN,
-                                          tmem_base + acc * uint32_t(kBN), &acc_full[acc], acc_phase, abort_flag,
-                                          stage, sub, lane, first_chunk)) {
-        ok = false;
-        break;
+      const int m_base = tile.tm * kPairM + int(rank) * kBM, n_base = tile.tn * step.tile_n;
+      const uint32_t tmem_acc = tmem_base + acc * uint32_t(kBN);
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) remote_arrive(leader_empty[acc]);
+      };
+      auto epilogue = [&](auto symmetric) {
+        return epilogue_tile<InT, decltype(symmetric)::value, kEpilogueWarps / 8>(
+            p, tile.batch, m_base, n_base, tmem_acc, &acc_full[acc], acc_phase, abort_flag, stage, sub, lane, first_chunk,
+            chunks, step.out_bf16, release);
+      };
+      const bool done = step.symmetric ? epilogue(std::true_type()) : epilogue(std::false_type());
+      if (!done) break;
+      if constexpr (kSteps > 1) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&stored[local % kTileSlots]);
       }
-      tc_fence_before();
-      remote_arrive(leader_empty[acc]);
     }
   }
 

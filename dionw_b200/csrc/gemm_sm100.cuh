@@ -57,8 +57,6 @@ struct Params {
   int mirror_diagonal;   // symmetric schedule with B != A: also mirror inside the diagonal sub-blocks
   float* rowsq;          // nullable, general products only: [batches, m, rowsq_parts] partial row sums of out^2
   int rowsq_parts;       // = 2 * tiles_n: one partial per 128 columns, written once each, summed by the reader
-  int* tile_counter;     // two-CTA kernel: {next tile, pairs done} in global memory, or null for a fixed stride
-  DecayJob* job;         // two-CTA kernel: streaming job the epilogue warps work on while they wait, or null
   int* status;           // device status word (may be null: the code is then not recorded)
   uint64_t wait_ns;      // limit of every bounded wait, in nanoseconds of %globaltimer
 };
@@ -317,10 +315,11 @@ __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
 }
 
 // ----------------------------------------------------------------------------
-// epilogue of one accumulator: 128 rows (m_base ..) x 256 columns (n_base ..) of batch
+// epilogue of one accumulator: 128 rows (m_base ..) x tile_n columns (n_base ..) of batch
 // ``batch``, read from TMEM at ``tmem_acc`` by the warp that owns sub-partition ``sub``;
-// this warp handles chunks first_chunk .. first_chunk+3 of the eight 32-column chunks.
-// Returns false when the bounded wait for the accumulator ran out.
+// this warp handles `chunks` of the tile's 32-column chunks from first_chunk on.  `release` is called once,
+// when the warp has read all it needs of the accumulator.  kPartWarps warps in a row of the tile share the
+// 128 columns of one part of the row sums.  Returns false when the bounded wait for the accumulator ran out.
 //
 // A warp works on 32 x 32 pieces.  The accumulator is read in the mma result layout, because
 // stmatrix turns that into rows of the piece and, with .trans, into rows of its mirror image at four
@@ -336,13 +335,28 @@ __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
 // through per-element loops: a 256^3 mirrored product with Cin took 15.7 us in a chain of products,
 // this takes 8.1; 6 blocks of 517^3 17.8 us against 12.6.
 // ----------------------------------------------------------------------------
-template <typename InT, typename OutT, bool kSym>
+template <typename InT, bool kSym, int kPartWarps, typename Release>
 __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_base, int n_base, uint32_t tmem_acc,
                                               uint64_t* acc_full_bar, uint32_t acc_phase, volatile int* abort_flag,
-                                              uint8_t* stage, int sub, int lane, int first_chunk) {
+                                              uint8_t* stage, int sub, int lane, int first_chunk, int chunks,
+                                              bool to_bf16, Release&& release) {
+  // A general product of fp16 operands has a bf16 result where `to_bf16` says so.  (As a template argument the
+  // second general form cost the kernel that holds all of them its registers.)
+  auto pack_out = [&](float a, float b) -> uint32_t {
+    if constexpr (kSym || std::is_same<InT, __nv_bfloat16>::value) return pack2<InT>(a, b);
+    return to_bf16 ? pack2<__nv_bfloat16>(a, b) : pack2<InT>(a, b);
+  };
+  auto unpack_out = [&](uint32_t w) -> float2 {
+    if constexpr (kSym || std::is_same<InT, __nv_bfloat16>::value) return unpack2<InT>(w);
+    return to_bf16 ? unpack2<__nv_bfloat16>(w) : unpack2<InT>(w);
+  };
   const uint16_t* cin = p.cin ? reinterpret_cast<const uint16_t*>(p.cin) + size_t(batch) * p.cin_batch : nullptr;
   uint16_t* out = reinterpret_cast<uint16_t*>(p.out) + size_t(batch) * p.out_batch;
   uint16_t* out2 = kSym && p.out2 ? reinterpret_cast<uint16_t*>(p.out2) + size_t(batch) * p.out_batch : nullptr;
+  // What every piece needs, held in registers: the parameters themselves lie where a load takes a while.
+  const int m = p.m, n = p.n;
+  const int64_t ldo = p.ldo, ldc = p.ldc;
+  const float alpha = p.alpha, beta = p.beta, diag = p.diag;
   const int row0 = m_base + sub * 32;
   // Class of the 32 x 32 piece at (row0, col0) under the symmetric schedule:
   // 0 stored as it is; 1 strictly below the diagonal: stored and stored transposed;
@@ -355,64 +369,74 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
     if (col0 >= row0 + 32) return 2;
     return p.mirror_diagonal != 0 ? 3 : 0;
   };
-  const bool out_aligned = (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 &&
+  // Chunks past the matrix, and under the symmetric schedule those above the diagonal, come last.
+  int end_chunk = first_chunk;
+  while (end_chunk < first_chunk + chunks && n_base + end_chunk * 32 < n && row0 < m &&
+         class_of(n_base + end_chunk * 32) != 2)
+    ++end_chunk;
+  const bool out_aligned = (ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 &&
                            (reinterpret_cast<uintptr_t>(out2) & 15u) == 0;
-  const bool cin_aligned = (p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(cin) & 15u) == 0;
+  const bool cin_aligned = (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(cin) & 15u) == 0;
   const int piece_row = lane >> 2, piece_unit = lane & 3, piece_col = piece_unit * 8;
-  // 16 bytes of Cin at (r, c): elements outside the matrix read as zero.
+  // 16 bytes of Cin at (r, c): elements outside the matrix read as zero.  Read from L2: in a plan of
+  // several products the bytes were written by another SM during this launch.
   auto get = [&](int r, int c) -> uint4 {
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (r >= p.m || c >= p.n) return v;
-    const uint16_t* at = cin + size_t(r) * p.ldc + c;
-    if (cin_aligned && c + 8 <= p.n) return *reinterpret_cast<const uint4*>(at);
+    if (r >= m || c >= n) return v;
+    const uint16_t* at = cin + size_t(r) * ldc + c;
+    if (cin_aligned && c + 8 <= n) return __ldcg(reinterpret_cast<const uint4*>(at));
     uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (c + j < p.n) w[j >> 1] |= uint32_t(at[j]) << (16 * (j & 1));
+      if (c + j < n) w[j >> 1] |= uint32_t(__ldcg(at + j)) << (16 * (j & 1));
     return make_uint4(w[0], w[1], w[2], w[3]);
   };
   auto put = [&](uint16_t* base, int r, int c, const uint4& v) {
-    if (r >= p.m || c >= p.n) return;
-    uint16_t* at = base + size_t(r) * p.ldo + c;
-    if (out_aligned && c + 8 <= p.n) {
+    if (r >= m || c >= n) return;
+    uint16_t* at = base + size_t(r) * ldo + c;
+    if (out_aligned && c + 8 <= n) {
       *reinterpret_cast<uint4*>(at) = v;
       return;
     }
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (c + j < p.n) at[j] = uint16_t(w[j >> 1] >> (16 * (j & 1)));
+      if (c + j < n) at[j] = uint16_t(w[j >> 1] >> (16 * (j & 1)));
   };
   auto unit_at = [](int row, int unit) -> uint32_t { return uint32_t(row * 64 + ((unit ^ ((row >> 1) & 3)) << 4)); };
-  uint8_t* mirror = stage + kPieceBytes;
-  const uint32_t stage_u32 = smem_u32(stage), mirror_u32 = smem_u32(mirror);
+  // Places in the staging tiles, from one base each: 16 rows on are 1024 bytes, which leaves the swizzle
+  // alone, and two units on are the same place with bit 5 flipped.
+  uint8_t* const my_piece = stage + unit_at(piece_row, piece_unit);   // + 512 * it
+  uint8_t* const my_mirror = my_piece + kPieceBytes;
   // This lane's row addresses for the four matrices of one ldmatrix / stmatrix: rows 16h + 8 * (i % 2),
-  // columns 16 * pair + 8 * (i / 2) of the piece, i = lane / 8.
-  auto matrix_at = [&](int h, int pair) { return unit_at(16 * h + ((lane >> 3) & 1) * 8 + (lane & 7), 2 * pair + (lane >> 4)); };
-  auto mirror_at = [&](int h, int pair) { return unit_at(16 * pair + (lane >> 4) * 8 + (lane & 7), 2 * h + ((lane >> 3) & 1)); };
+  // columns 16 * pair + 8 * (i / 2) of the piece, i = lane / 8; and their places in the mirror image.
+  const uint32_t matrix_base = smem_u32(stage) + unit_at(((lane >> 3) & 1) * 8 + (lane & 7), lane >> 4);
+  const uint32_t mirror_base = smem_u32(stage) + kPieceBytes + unit_at((lane >> 4) * 8 + (lane & 7), (lane >> 3) & 1);
+  auto matrix_at = [&](int h, int pair) { return (matrix_base ^ uint32_t(pair << 5)) + uint32_t(h << 10); };
+  auto mirror_at = [&](int h, int pair) { return (mirror_base ^ uint32_t(h << 5)) + uint32_t(pair << 10); };
 
   // The Cin piece of the next chunk is requested before the current chunk is worked on.
   uint4 ahead[4];
   auto prefetch = [&](int chunk) {
     const int col0 = n_base + chunk * 32;
-    if (cin == nullptr || class_of(col0) == 2) return;
+    if (cin == nullptr || chunk >= end_chunk) return;
 #pragma unroll
     for (int it = 0; it < 4; ++it) ahead[it] = get(row0 + 8 * it + piece_row, col0 + piece_col);
   };
   prefetch(first_chunk);   // does not depend on the accumulator: overlaps the wait below
   if (!mbar_wait(acc_full_bar, acc_phase, abort_flag, p.status, p.wait_ns)) return false;
   tc_fence_after();
-  // Sums of the squares of the rounded results over the warp's 128 columns, for NorMuon: the values are
+  if (end_chunk == first_chunk) release();
+  // Sums of the squares of the rounded results over the warp's columns, for NorMuon: the values are
   // in registers here, so the row statistics need no second pass over the output.  Lane l sums its
   // columns of rows l/4 + 8i; the four lanes of a row are added at the end: the order is fixed.
-  const bool want_sq = !kSym && p.rowsq != nullptr;
+  const bool want_sq = !kSym && p.rowsq != nullptr;   // 256-column tiles only
   float sq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
-  for (int chunk = first_chunk; chunk < first_chunk + kBN / 64; ++chunk) {
+  for (int chunk = first_chunk; chunk < end_chunk; ++chunk) {
     const int col0 = n_base + chunk * 32;
-    if (col0 >= p.n || row0 >= p.m) break;   // uniform over the warp
-    const int cls = class_of(col0);
-    if (cls == 2) break;          // uniform over the warp; the chunks after it lie above the diagonal too
+    const int cls = class_of(col0);   // uniform over the warp
+    // (Requesting the next chunk's accumulator before this one is stored was measured: 1-2 % slower.)
     uint32_t v[32];
     const uint32_t taddr = tmem_acc + (uint32_t(sub * 32) << 16) + uint32_t(chunk * 32);
     tmem_load_16x32(taddr, v);
@@ -421,39 +445,38 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
     if (cin != nullptr) {
 #pragma unroll
       for (int it = 0; it < 4; ++it)
-        *reinterpret_cast<uint4*>(stage + unit_at(8 * it + piece_row, piece_unit)) = ahead[it];
-      if (chunk + 1 < first_chunk + kBN / 64) prefetch(chunk + 1);
+        *reinterpret_cast<uint4*>(my_piece + 512 * it) = ahead[it];
+      prefetch(chunk + 1);
       __syncwarp();
-      uint32_t c[16];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int pair = 0; pair < 2; ++pair) {
-          uint32_t* f = c + 8 * h + 4 * pair;
-          ldmatrix4(stage_u32 + matrix_at(h, pair), f[0], f[1], f[2], f[3]);
-        }
       tmem_wait(v);
+      if (chunk + 1 == end_chunk) release();
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float2 cf = unpack2<InT>(c[j]);
-        r[j] = pack2<OutT>(fmaf(p.beta, cf.x, p.alpha * __uint_as_float(v[2 * j])),
-                           fmaf(p.beta, cf.y, p.alpha * __uint_as_float(v[2 * j + 1])));
+      for (int f = 0; f < 16; f += 4) {   // (h, pair) = (f / 8, f / 4 % 2)
+        uint32_t c[4];
+        ldmatrix4(matrix_at(f >> 3, (f >> 2) & 1), c[0], c[1], c[2], c[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 cf = unpack2<InT>(c[j]);
+          r[f + j] = pack_out(fmaf(beta, cf.x, alpha * __uint_as_float(v[2 * (f + j)])),
+                                 fmaf(beta, cf.y, alpha * __uint_as_float(v[2 * (f + j) + 1])));
+        }
       }
       __syncwarp();               // every lane has its part of Cin: the staging tile is free
     } else {
       tmem_wait(v);
+      if (chunk + 1 == end_chunk) release();
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        r[j] = pack2<OutT>(p.alpha * __uint_as_float(v[2 * j]), p.alpha * __uint_as_float(v[2 * j + 1]));
+        r[j] = pack_out(alpha * __uint_as_float(v[2 * j]), alpha * __uint_as_float(v[2 * j + 1]));
     }
     if (want_sq) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int column = col0 + (j >> 1 & 3) * 8 + (lane & 3) * 2;
-        const float2 f = unpack2<OutT>(r[j]);
+        const float2 f = unpack_out(r[j]);
         float& sum = sq[2 * (j >> 3) + (j & 1)];
-        if (column < p.n) sum = fmaf(f.x, f.x, sum);
-        if (column + 1 < p.n) sum = fmaf(f.y, f.y, sum);
+        if (column < n) sum = fmaf(f.x, f.x, sum);
+        if (column + 1 < n) sum = fmaf(f.y, f.y, sum);
       }
     }
 #pragma unroll
@@ -461,30 +484,30 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
 #pragma unroll
       for (int pair = 0; pair < 2; ++pair) {
         const uint32_t* f = r + 8 * h + 4 * pair;
-        stmatrix4(stage_u32 + matrix_at(h, pair), f[0], f[1], f[2], f[3]);
-        if (kSym && cls != 0) stmatrix4_trans(mirror_u32 + mirror_at(h, pair), f[0], f[1], f[2], f[3]);
+        stmatrix4(matrix_at(h, pair), f[0], f[1], f[2], f[3]);
+        if (kSym && cls != 0) stmatrix4_trans(mirror_at(h, pair), f[0], f[1], f[2], f[3]);
       }
     __syncwarp();
     // Whole pieces, which are nearly all, go out with plain 16-byte stores, the four loads first.
-    const bool whole = out_aligned && row0 + 32 <= p.m && col0 + 32 <= p.n;   // uniform over the warp
+    const bool whole = out_aligned && row0 + 32 <= m && col0 + 32 <= n;   // uniform over the warp
     uint4 piece[4];
 #pragma unroll
     for (int it = 0; it < 4; ++it)
-      piece[it] = *reinterpret_cast<const uint4*>(stage + unit_at(8 * it + piece_row, piece_unit));
+      piece[it] = *reinterpret_cast<const uint4*>(my_piece + 512 * it);
     if constexpr (kSym) {
       if (cls != 0) {
         uint4 other[4];
 #pragma unroll
         for (int it = 0; it < 4; ++it)
-          other[it] = *reinterpret_cast<const uint4*>(mirror + unit_at(8 * it + piece_row, piece_unit));
+          other[it] = *reinterpret_cast<const uint4*>(my_mirror + 512 * it);
         if (cls == 1) {
           if (whole) {
-            const size_t at = size_t(col0 + piece_row) * p.ldo + row0 + piece_col;
+            const size_t at = size_t(col0 + piece_row) * ldo + row0 + piece_col;
 #pragma unroll
-            for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out + at + size_t(8 * it) * p.ldo) = other[it];
+            for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out + at + size_t(8 * it) * ldo) = other[it];
             if (out2 != nullptr) {
 #pragma unroll
-              for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out2 + at + size_t(8 * it) * p.ldo) = other[it];
+              for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out2 + at + size_t(8 * it) * ldo) = other[it];
             }
           } else {
 #pragma unroll
@@ -510,10 +533,10 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
         }
       }
     }
-    const size_t at = size_t(row0 + piece_row) * p.ldo + col0 + piece_col;
+    const size_t at = size_t(row0 + piece_row) * ldo + col0 + piece_col;
     if (whole) {
 #pragma unroll
-      for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out + at + size_t(8 * it) * p.ldo) = piece[it];
+      for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out + at + size_t(8 * it) * ldo) = piece[it];
     } else {
 #pragma unroll
       for (int it = 0; it < 4; ++it) put(out, row0 + 8 * it + piece_row, col0 + piece_col, piece[it]);
@@ -527,15 +550,15 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
             const int d = 8 * it + piece_row - piece_col;   // its position inside the 8 elements
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const float2 f = unpack2<OutT>(w[j]);
-              if (d == 2 * j) w[j] = pack2<OutT>(f.x + p.diag, f.y);
-              if (d == 2 * j + 1) w[j] = pack2<OutT>(f.x, f.y + p.diag);
+              const float2 f = unpack_out(w[j]);
+              if (d == 2 * j) w[j] = pack_out(f.x + diag, f.y);
+              if (d == 2 * j + 1) w[j] = pack_out(f.x, f.y + diag);
             }
           }
         }
         if (whole) {
 #pragma unroll
-          for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out2 + at + size_t(8 * it) * p.ldo) = piece[it];
+          for (int it = 0; it < 4; ++it) *reinterpret_cast<uint4*>(out2 + at + size_t(8 * it) * ldo) = piece[it];
         } else {
 #pragma unroll
           for (int it = 0; it < 4; ++it) put(out2, row0 + 8 * it + piece_row, col0 + piece_col, piece[it]);
@@ -548,11 +571,32 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
     const int part = 2 * (n_base / kBN) + first_chunk / (kBN / 64);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      float sum = sq[i];
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 1);
+      sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 2);
+    }
+    bool writer = piece_unit == 0;
+    if constexpr (kPartWarps == 2) {
+      // The second warp of a part hands its sums to the first through its staging tile (the warps of one
+      // sub-partition are four apart, and so are their tiles).
+      const bool second = (first_chunk / chunks) % 2 != 0;
+      const int barrier = 1 + 4 * (first_chunk / (2 * chunks)) + sub;
+      float* theirs = reinterpret_cast<float*>(second ? stage : stage + 4 * 2 * kPieceBytes);
+      if (second && writer) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) theirs[8 * i + piece_row] = sq[i];
+      }
+      asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+      if (!second && writer) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sq[i] += theirs[8 * i + piece_row];
+      }
+      asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
+      writer = writer && !second;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
       const int row = row0 + 8 * i + piece_row;
-      if (piece_unit == 0 && row < p.m) p.rowsq[(size_t(batch) * p.m + row) * p.rowsq_parts + part] = sum;
+      if (writer && row < m) p.rowsq[(size_t(batch) * m + row) * p.rowsq_parts + part] = sq[i];
     }
   }
   return true;
@@ -689,13 +733,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       const Tile tile = kSym ? sym_tile(t, p) : general_tile(t, p);
       const uint32_t acc = local & 1u;
       const uint32_t acc_phase = (local >> 1) & 1u;
-      if (!epilogue_tile<InT, OutT, kSym>(p, tile.batch, tile.tm * kBM, tile.tn * kBN, tmem_base + acc * uint32_t(kBN),
-                                          &acc_full[acc], acc_phase, abort_flag, stage, sub, lane, first_chunk)) {
+      auto release = [&] {
+        tc_fence_before();
+        mbar_arrive(&acc_empty[acc]);
+      };
+      if (!epilogue_tile<InT, kSym, 1>(p, tile.batch, tile.tm * kBM, tile.tn * kBN, tmem_base + acc * uint32_t(kBN),
+                                             &acc_full[acc], acc_phase, abort_flag, stage, sub, lane, first_chunk,
+                                             kBN / 64, std::is_same<OutT, __nv_bfloat16>::value, release)) {
         ok = false;
         break;
       }
-      tc_fence_before();
-      mbar_arrive(&acc_empty[acc]);
     }
   }
 

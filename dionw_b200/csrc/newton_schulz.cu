@@ -1,17 +1,8 @@
-// The Newton-Schulz product schedules, launched product by product on the
-// tcgen05 GEMMs of gemm.cu.
-#include "common.cuh"
+// The Newton-Schulz product schedules: which products, in which order.  gemm.cu runs them, all of one
+// iteration as one launch.
+#include "products.cuh"
 
 namespace dionw {
-
-int symmetric_product(const void* a, bool transposed, const void* b, int64_t blocks, int64_t m, int64_t kdim, int64_t lda,
-                      int64_t a_batch, int64_t ldb, int64_t b_batch, const void* cin, int64_t ldc, int64_t cin_batch, float alpha, float beta, void* out,
-                      int64_t ldo, int64_t out_batch, void* out2, float diag, int dtype, cudaStream_t stream);
-int batched_gemm(const void* a, int64_t lda, int64_t a_batch, const void* b, int64_t ldb, int64_t b_batch,
-                 bool b_is_nk, const void* cin, int64_t ldc, int64_t cin_batch, float beta, void* out, int64_t ldo,
-                 int64_t out_batch, int64_t blocks, int64_t m, int64_t n, int64_t kdim, int in_dtype, int out_dtype,
-                 float* rowsq, cudaStream_t stream);
-
 namespace {
 
 struct Coeff {
@@ -69,22 +60,28 @@ size_t bytes_of(const Layout& l) {
   return l.gram ? l.x_bytes + 5 * l.g_bytes : 2 * l.x_bytes + 2 * l.g_bytes;
 }
 
-// The schedule on a batch of rows x cols blocks of either orientation, as they lie.  A wide block is
+// A batch of rows x cols blocks and where its result goes.
+struct Problem {
+  void* x;
+  void* out;
+  int64_t blocks, rows, cols, ldx;
+  int kind;
+  float* rowsq;
+};
+
+// The schedule on a batch of either orientation, as it lies: appends its products to `list`.  A wide block is
 // multiplied from the left (G = X X^T, X <- Q X), a tall one from the right (G = X^T X, X <- X Q): every
 // matrix among G, Q and the polynomials is stored exactly symmetric, so Q serves as the K-major second
 // operand of X Q as it is, and the only product that needs transposed reads is X^T X, which takes both
 // operands MN-major.  Value for value the same as iterating the transposed copy of a tall block, without
 // the two transposing passes, which took 102 us each on 12 blocks of 3072 x 768.
-int iterate(void* x, void* out, int64_t blocks, int64_t rows, int64_t cols, int64_t ldx, int kind, void* workspace,
-            size_t workspace_bytes, float* rowsq, cudaStream_t stream) {
-  const Layout l = layout_of(blocks, rows, cols, ldx, kind);
-  uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  const size_t lost = size_t(ws - reinterpret_cast<uint8_t*>(workspace));
-  if (workspace == nullptr || workspace_bytes < bytes_of(l) + lost) {
-    set_error("newton_schulz: workspace of %zu bytes is smaller than the %zu needed", workspace_bytes,
-              bytes_of(l) + lost);
-    return DIONW_ERR_WORKSPACE;
-  }
+void append_products(const Problem& problem, int chain, int64_t first_block, const Layout& l, uint8_t* ws, Product* list,
+                     int& count) {
+  void* const x = problem.x;
+  void* const out = problem.out;
+  const int64_t blocks = problem.blocks, rows = problem.rows, cols = problem.cols, ldx = problem.ldx;
+  const int kind = problem.kind;
+  float* const rowsq = problem.rowsq;
   const bool gram = kind == DIONW_NS_GRAM || kind == DIONW_NS_GRAM_FULL;
   const int dt = gram ? DIONW_F16 : DIONW_BF16;
   // Every m x m matrix of the Gram schedule is a polynomial in one symmetric G, so the
@@ -96,112 +93,171 @@ int iterate(void* x, void* out, int64_t blocks, int64_t rows, int64_t cols, int6
   const int64_t xb = rows * ldx;    // batch strides in elements
   const int64_t gb = m * l.ldg;
   const int64_t ldg = l.ldg;
-  int st = DIONW_OK;
-#define DIONW_STEP(call)            \
-  do {                              \
-    st = (call);                    \
-    if (st != DIONW_OK) return st;  \
-  } while (0)
-  // G = X X^T (wide), X^T X (tall)
+  auto next_product = [&]() -> Product& {
+    Product& p = list[count++];
+    p.blocks = blocks;
+    p.chain = chain;
+    p.first_block = first_block;
+    return p;
+  };
+  auto small = [&](const void* base) { return Operand{base, ldg, gb}; };   // an m x m matrix
+  auto block = [&](const void* base) { return Operand{base, ldx, xb}; };   // a rows x cols matrix
+  // to = X X^T (wide), X^T X (tall)
   auto gram_of = [&](const void* from, void* to) {
-    return symmetric_product(from, tall, nullptr, blocks, m, n, ldx, xb, 0, 0, nullptr, 0, 0, 1.0f, 0.0f, to, ldg, gb,
-                             nullptr, 0.0f, dt, stream);
+    Product& p = next_product();
+    p.a = p.b = block(from);
+    p.a_mn = p.b_mn = tall;
+    p.symmetric = p.same_operands = true;
+    p.out = small(to);
+    p.m = p.n = m;
+    p.k = n;
+    p.out_dtype = dt;
+  };
+  // to = alpha A B + beta A-or-B's polynomial `cin`, all m x m and symmetric; a == b: the square of a matrix
+  auto combine = [&](const void* a, const void* b, double alpha, const void* cin, double beta, void* to) -> Product& {
+    Product& p = next_product();
+    p.a = small(a);
+    p.b = small(b);
+    p.symmetric = a == b || mirror;
+    p.same_operands = a == b;
+    p.alpha = float(alpha);
+    p.cin = small(cin);
+    p.beta = float(beta);
+    p.out = small(to);
+    p.m = p.n = p.k = m;
+    p.out_dtype = dt;
+    return p;
   };
   // to = S from + beta from (wide), from S + beta from (tall) with a symmetric S; beta = 0: no second term
-  auto multiply = [&](const void* s, const void* from, float beta, void* to, int out_dtype, float* sums) {
-    const void* cin = beta != 0.0f ? from : nullptr;
-    if (tall)
-      return batched_gemm(from, ldx, xb, s, ldg, gb, true, cin, ldx, xb, beta, to, ldx, xb, blocks, n, m, m, dt,
-                          out_dtype, sums, stream);
-    return batched_gemm(s, ldg, gb, from, ldx, xb, false, cin, ldx, xb, beta, to, ldx, xb, blocks, m, n, m, dt,
-                        out_dtype, sums, stream);
+  auto multiply = [&](const void* s, const void* from, double beta, void* to, int out_dtype, float* sums) {
+    Product& p = next_product();
+    p.a = tall ? block(from) : small(s);
+    p.b = tall ? small(s) : block(from);
+    p.b_mn = !tall;
+    if (beta != 0.0) p.cin = block(from);
+    p.beta = float(beta);
+    p.out = block(to);
+    p.m = rows;
+    p.n = cols;
+    p.k = m;
+    p.out_dtype = out_dtype;
+    p.rowsq = sums;
   };
 
   if (l.gram) {
-    void* x0 = x;
     void* x1 = ws;
     void* g = ws + l.x_bytes;
     void* z = ws + l.x_bytes + l.g_bytes;
-    void* q0 = ws + l.x_bytes + 2 * l.g_bytes;
-    void* q1 = ws + l.x_bytes + 3 * l.g_bytes;
+    void* q = ws + l.x_bytes + 2 * l.g_bytes;
+    void* qnext = ws + l.x_bytes + 3 * l.g_bytes;
     void* rz = ws + l.x_bytes + 4 * l.g_bytes;
-    void* xcur = x0;
-    void* q = q0;
-    void* qnext = q1;
-    DIONW_STEP(gram_of(xcur, g));
+    const void* xcur = x;
+    gram_of(xcur, g);
     for (int i = 0; i < 5; ++i) {
       const Coeff k = kGram[i];
-      if (i == kRestart) {
-        // restart: X <- Q X and its Gram matrix
-        DIONW_STEP(multiply(q, xcur, 0.0f, x1, dt, nullptr));
+      if (i == kRestart) {   // X <- Q X and its Gram matrix
+        multiply(q, xcur, 0.0, x1, dt, nullptr);
         xcur = x1;
-        DIONW_STEP(gram_of(xcur, g));
+        gram_of(xcur, g);
       }
-      const bool fresh_q = (i == 0 || i == kRestart);
       // Z = c G G^T + b G; on a fresh start also Q = Z + a I.  The diagonal is round(fp32(Z) + fp32(a)),
       // as the reference's compiled GPU step forms `z + a * eye` (its eager CPU run rounds `a` to
       // fp16 first, which costs 4e-3 of accuracy on 256 x 4096 operands).
-      DIONW_STEP(symmetric_product(g, false, nullptr, blocks, m, m, ldg, gb, 0, 0, g, ldg, gb, float(k.c), float(k.b), z, ldg, gb,
-                                   fresh_q ? q : nullptr, float(k.a), dt, stream));
+      const bool fresh_q = i == 0 || i == kRestart;
+      Product& zp = combine(g, g, k.c, g, k.b, z);
+      if (fresh_q) {
+        zp.out2 = q;
+        zp.diag = float(k.a);
+      }
       if (!fresh_q) {
-        // Q <- a Q + Q Z   (Z is stored symmetric, so Z^T == Z bit for bit)
-        if (mirror)
-          DIONW_STEP(symmetric_product(q, false, z, blocks, m, m, ldg, gb, ldg, gb, q, ldg, gb, 1.0f, float(k.a), qnext, ldg,
-                                       gb, nullptr, 0.0f, dt, stream));
-        else
-          DIONW_STEP(batched_gemm(q, ldg, gb, z, ldg, gb, true, q, ldg, gb, float(k.a), qnext, ldg, gb, blocks, m,
-                                  m, m, dt, dt, nullptr, stream));
+        // Q <- a Q + Q Z
+        combine(q, z, 1.0, q, k.a, qnext);
         void* t = q;
         q = qnext;
         qnext = t;
       }
       if (i < 4 && i + 1 != kRestart) {
-        // RZ = a G + G Z ; G <- a RZ + Z RZ
-        if (mirror) {
-          DIONW_STEP(symmetric_product(g, false, z, blocks, m, m, ldg, gb, ldg, gb, g, ldg, gb, 1.0f, float(k.a), rz, ldg,
-                                       gb, nullptr, 0.0f, dt, stream));
-          DIONW_STEP(symmetric_product(z, false, rz, blocks, m, m, ldg, gb, ldg, gb, rz, ldg, gb, 1.0f, float(k.a), g, ldg,
-                                       gb, nullptr, 0.0f, dt, stream));
-        } else {
-          DIONW_STEP(batched_gemm(g, ldg, gb, z, ldg, gb, true, g, ldg, gb, float(k.a), rz, ldg, gb, blocks, m, m,
-                                  m, dt, dt, nullptr, stream));
-          DIONW_STEP(batched_gemm(z, ldg, gb, rz, ldg, gb, false, rz, ldg, gb, float(k.a), g, ldg, gb, blocks, m,
-                                  m, m, dt, dt, nullptr, stream));
-        }
+        // RZ = a G + G Z, which does not touch Q; G <- a RZ + Z RZ.  (RZ is stored exactly symmetric by the
+        // mirrored products only, so the full ones read it as the [k, n] operand that it is.)
+        combine(g, z, 1.0, g, k.a, rz).beside_previous = !fresh_q;
+        combine(z, rz, 1.0, rz, k.a, g).b_mn = !mirror;
       }
     }
-    // out = Q X in bf16
-    DIONW_STEP(multiply(q, xcur, 0.0f, out, DIONW_BF16, rowsq));
-    return DIONW_OK;
+    multiply(q, xcur, 0.0, out, DIONW_BF16, rowsq);   // out = Q X
+  } else {
+    // Standard iteration: X <- a X + (b G + c G^2) X with G = X X^T.
+    const Coeff* table = gram ? kGram : (kind == DIONW_NS_POLAR_EXPRESS ? kPolarExpress : kKeller);
+    void* x1 = ws;
+    void* x2 = ws + l.x_bytes;
+    void* g = ws + 2 * l.x_bytes;
+    void* poly = ws + 2 * l.x_bytes + l.g_bytes;
+    const void* cur = x;
+    for (int i = 0; i < 5; ++i) {
+      const Coeff k = table[i];
+      void* next = i == 4 ? out : (cur == x1 ? x2 : x1);
+      gram_of(cur, g);
+      combine(g, g, k.c, g, k.b, poly);
+      multiply(poly, cur, k.a, next, i == 4 ? DIONW_BF16 : dt, i == 4 ? rowsq : nullptr);
+      cur = next;
+    }
   }
+}
 
-  // Standard iteration: X <- a X + (b G + c G^2) X with G = X X^T.
-  const Coeff* table = gram ? kGram : (kind == DIONW_NS_POLAR_EXPRESS ? kPolarExpress : kKeller);
-  void* x1 = ws;
-  void* x2 = ws + l.x_bytes;
-  void* g = ws + 2 * l.x_bytes;
-  void* poly = ws + 2 * l.x_bytes + l.g_bytes;
-  void* cur = x;
-  for (int i = 0; i < 5; ++i) {
-    const Coeff k = table[i];
-    void* next = (i == 4) ? out : ((cur == x1) ? x2 : x1);
-    DIONW_STEP(gram_of(cur, g));
-    DIONW_STEP(symmetric_product(g, false, nullptr, blocks, m, m, ldg, gb, 0, 0, g, ldg, gb, float(k.c), float(k.b), poly, ldg, gb,
-                                 nullptr, 0.0f, dt, stream));
-    DIONW_STEP(multiply(poly, cur, float(k.a), next, i == 4 ? DIONW_BF16 : dt, i == 4 ? rowsq : nullptr));
-    cur = next;
+size_t group_bytes(const Problem* problems, int n) {
+  int64_t matrices = 0;
+  size_t bytes = 0;
+  for (int i = 0; i < n; ++i) {
+    matrices += problems[i].blocks;
+    bytes += bytes_of(layout_of(problems[i].blocks, problems[i].rows, problems[i].cols, problems[i].ldx, problems[i].kind));
   }
-#undef DIONW_STEP
-  return DIONW_OK;
+  return bytes + align256(plan_counter_bytes(matrices));
+}
+
+// Up to kMaxChains batches that are iterated in the same dtype, as one launch, or product by product.
+int iterate(const Problem* problems, int n, bool stepwise, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
+  const size_t lost = size_t(ws - reinterpret_cast<uint8_t*>(workspace));
+  const size_t need = group_bytes(problems, n);
+  if (workspace == nullptr || workspace_bytes < need + lost) {
+    set_error("newton_schulz: workspace of %zu bytes is smaller than the %zu needed", workspace_bytes, need + lost);
+    return DIONW_ERR_WORKSPACE;
+  }
+  int64_t matrices = 0;
+  for (int i = 0; i < n; ++i) matrices += problems[i].blocks;
+  const size_t counter_bytes = align256(plan_counter_bytes(matrices));
+  void* counters = counter_bytes != 0 && !stepwise ? ws : nullptr;
+  ws += counter_bytes;
+  Product list[kMaxChains * kMaxChainProducts];
+  int count = 0;
+  int64_t first_block = 0;
+  for (int i = 0; i < n; ++i) {
+    const Layout l = layout_of(problems[i].blocks, problems[i].rows, problems[i].cols, problems[i].ldx, problems[i].kind);
+    append_products(problems[i], i, first_block, l, ws, list, count);
+    ws += bytes_of(l);
+    first_block += problems[i].blocks;
+  }
+  const bool gram = problems[0].kind == DIONW_NS_GRAM || problems[0].kind == DIONW_NS_GRAM_FULL;
+  return run_products(list, count, gram ? DIONW_F16 : DIONW_BF16, counters, stream);
+}
+
+bool known_kind(int kind) {
+  kind &= ~DIONW_NS_STEPWISE;
+  return kind == DIONW_NS_GRAM || kind == DIONW_NS_POLAR_EXPRESS || kind == DIONW_NS_KELLER || kind == DIONW_NS_GRAM_FULL;
 }
 
 }  // namespace
 }  // namespace dionw
 
+namespace dionw {
+// Part of dionw_newton_schulz_workspace_bytes that is not operands (newton_schulz_static.cu keeps it apart).
+size_t newton_schulz_counter_bytes(int64_t blocks) { return align256(plan_counter_bytes(blocks)); }
+}  // namespace dionw
+
 extern "C" size_t dionw_newton_schulz_workspace_bytes(int64_t blocks, int64_t m, int64_t n, int kind) {
   using namespace dionw;
   if (blocks <= 0 || m <= 0 || n <= 0) return 0;
-  return bytes_of(layout_of(blocks, m, n, round_up(n, 8), kind)) + 256;
+  const Problem problem{nullptr, nullptr, blocks, m, n, round_up(n, 8), kind & ~DIONW_NS_STEPWISE, nullptr};
+  return group_bytes(&problem, 1) + 256;
 }
 
 extern "C" int64_t dionw_newton_schulz_rowsq_parts(int64_t n) { return n <= 0 ? 0 : 2 * ((n + 255) / 256); }
@@ -209,36 +265,74 @@ extern "C" int64_t dionw_newton_schulz_rowsq_parts(int64_t n) { return n <= 0 ? 
 extern "C" int dionw_newton_schulz(void* x, void* out, int64_t blocks, int64_t m, int64_t n, int64_t ldx, int kind,
                                    void* workspace, size_t workspace_bytes, float* rowsq, void* stream_ptr) {
   using namespace dionw;
-  DIONW_REQUIRE(kind == DIONW_NS_GRAM || kind == DIONW_NS_POLAR_EXPRESS || kind == DIONW_NS_KELLER ||
-                    kind == DIONW_NS_GRAM_FULL,
-                "newton_schulz: unknown kind %d", kind);
+  DIONW_REQUIRE(known_kind(kind), "newton_schulz: unknown kind %d", kind);
   DIONW_REQUIRE(blocks > 0 && m > 0 && n >= m, "newton_schulz: needs blocks > 0 and 0 < m <= n (got %lld, %lld, %lld)",
                 (long long)blocks, (long long)m, (long long)n);
   DIONW_REQUIRE(ldx >= n && ldx % 8 == 0, "newton_schulz: ldx must be >= n and a multiple of 8");
   DIONW_REQUIRE(aligned16(x) && aligned16(out), "newton_schulz: x and out must be 16-byte aligned");
-  return iterate(x, out, blocks, m, n, ldx, kind, workspace, workspace_bytes, rowsq,
-                 static_cast<cudaStream_t>(stream_ptr));
+  const Problem problem{x, out, blocks, m, n, ldx, kind & ~DIONW_NS_STEPWISE, rowsq};
+  return iterate(&problem, 1, (kind & DIONW_NS_STEPWISE) != 0, workspace, workspace_bytes, static_cast<cudaStream_t>(stream_ptr));
 }
 
 extern "C" size_t dionw_newton_schulz_tall_workspace_bytes(int64_t blocks, int64_t rows, int64_t cols, int kind) {
   using namespace dionw;
   if (blocks <= 0 || rows <= 0 || cols <= 0) return 0;
-  return bytes_of(layout_of(blocks, rows, cols, round_up(cols, 8), kind)) + 256;
+  const Problem problem{nullptr, nullptr, blocks, rows, cols, round_up(cols, 8), kind & ~DIONW_NS_STEPWISE, nullptr};
+  return group_bytes(&problem, 1) + 256;
 }
 
 extern "C" int dionw_newton_schulz_tall(void* x, void* out, int64_t blocks, int64_t rows, int64_t cols, int64_t ldx,
                                         int kind, void* workspace, size_t workspace_bytes, float* rowsq,
                                         void* stream) {
   using namespace dionw;
-  DIONW_REQUIRE(kind == DIONW_NS_GRAM || kind == DIONW_NS_POLAR_EXPRESS || kind == DIONW_NS_KELLER ||
-                    kind == DIONW_NS_GRAM_FULL,
-                "newton_schulz_tall: unknown kind %d", kind);
+  DIONW_REQUIRE(known_kind(kind), "newton_schulz_tall: unknown kind %d", kind);
   DIONW_REQUIRE(blocks > 0 && cols > 0 && rows > cols,
                 "newton_schulz_tall: needs blocks > 0 and 0 < cols < rows (got %lld, %lld, %lld)", (long long)blocks,
                 (long long)rows, (long long)cols);
   DIONW_REQUIRE(blocks <= 65535, "newton_schulz_tall: more than 65535 blocks in one call");
   DIONW_REQUIRE(ldx >= cols && ldx % 8 == 0, "newton_schulz_tall: ldx must be >= cols and a multiple of 8");
   DIONW_REQUIRE(aligned16(x) && aligned16(out), "newton_schulz_tall: x and out must be 16-byte aligned");
-  return iterate(x, out, blocks, rows, cols, ldx, kind, workspace, workspace_bytes, rowsq,
-                 static_cast<cudaStream_t>(stream));
+  const Problem problem{x, out, blocks, rows, cols, ldx, kind & ~DIONW_NS_STEPWISE, rowsq};
+  return iterate(&problem, 1, (kind & DIONW_NS_STEPWISE) != 0, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+namespace dionw {
+namespace {
+// Fills `problems`; the message says what is wrong with a bad group.
+int read_group(int n, const int64_t* blocks, const int64_t* rows, const int64_t* cols, const int* kinds, Problem* problems) {
+  DIONW_REQUIRE(n >= 1 && n <= kMaxChains, "newton_schulz_group: takes 1 to %d batches (got %d)", kMaxChains, n);
+  auto is_gram = [](int kind) { return kind == DIONW_NS_GRAM || kind == DIONW_NS_GRAM_FULL; };
+  for (int i = 0; i < n; ++i) {
+    DIONW_REQUIRE(known_kind(kinds[i]) && (kinds[i] & DIONW_NS_STEPWISE) == 0, "newton_schulz_group: unknown kind %d", kinds[i]);
+    DIONW_REQUIRE(is_gram(kinds[i]) == is_gram(kinds[0]), "newton_schulz_group: fp16 and bf16 iterations in one group");
+    DIONW_REQUIRE(blocks[i] > 0 && rows[i] > 0 && cols[i] > 0, "newton_schulz_group: empty batch");
+    problems[i] = Problem{nullptr, nullptr, blocks[i], rows[i], cols[i], round_up(cols[i], 8), kinds[i], nullptr};
+  }
+  return DIONW_OK;
+}
+}  // namespace
+}  // namespace dionw
+
+extern "C" size_t dionw_newton_schulz_group_workspace_bytes(int n, const int64_t* blocks, const int64_t* rows,
+                                                            const int64_t* cols, const int* kinds) {
+  using namespace dionw;
+  Problem problems[kMaxChains];
+  if (read_group(n, blocks, rows, cols, kinds, problems) != DIONW_OK) return 0;
+  return group_bytes(problems, n) + 256;
+}
+
+extern "C" int dionw_newton_schulz_group(int n, void* const* x, void* const* out, const int64_t* blocks,
+                                         const int64_t* rows, const int64_t* cols, const int* kinds, void* workspace,
+                                         size_t workspace_bytes, float* const* rowsq, void* stream) {
+  using namespace dionw;
+  Problem problems[kMaxChains];
+  const int st = read_group(n, blocks, rows, cols, kinds, problems);
+  if (st != DIONW_OK) return st;
+  for (int i = 0; i < n; ++i) {
+    DIONW_REQUIRE(aligned16(x[i]) && aligned16(out[i]), "newton_schulz_group: x and out must be 16-byte aligned");
+    problems[i].x = x[i];
+    problems[i].out = out[i];
+    problems[i].rowsq = rowsq != nullptr ? rowsq[i] : nullptr;
+  }
+  return iterate(problems, n, false, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }

@@ -24,13 +24,19 @@
 #include "common.cuh"
 
 namespace dionw {
+
+size_t newton_schulz_counter_bytes(int64_t blocks);   // newton_schulz.cu
+
 namespace {
 
 // 64 MiB: enough for, e.g., 2 blocks of 1024 x 4096, 8 blocks of 512 x 2048 or
 // 1 block of 1536 x 4096 (dionw_newton_schulz_workspace_bytes gives the need).
 constexpr size_t kStaticScratchBytes = DIONW_STATIC_SCRATCH_BYTES;
 
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// The tile counters of a launch lie beside it: the ceiling is on the operands' scratch alone.
+constexpr size_t kStaticCounterBytes = 128 << 10;
+
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes + kStaticCounterBytes];
 
 // Device address of g_static_scratch per device ordinal.  The symbol's name is
 // only a host-side handle: the address a kernel can use has to be asked for,
@@ -56,7 +62,8 @@ int scratch_for_current_device(void** out) {
 extern "C" int dionw_newton_schulz_static(void* x, void* out, int64_t blocks, int64_t m, int64_t n, int64_t ldx,
                                           int kind, void* stream) {
   using namespace dionw;
-  const size_t need = dionw_newton_schulz_workspace_bytes(blocks, m, n, kind);
+  size_t need = dionw_newton_schulz_workspace_bytes(blocks, m, n, kind);
+  if (need != 0) need -= newton_schulz_counter_bytes(blocks);   // at most 65 KiB
   if (need == 0) {
     set_error("newton_schulz_static: needs blocks > 0, m > 0, n > 0");
     return DIONW_ERR_ARGUMENT;
@@ -84,5 +91,6 @@ extern "C" int dionw_newton_schulz_static(void* x, void* out, int64_t blocks, in
   // Nothing in the scratch has to start at zero: every product of the schedule
   // writes the whole of its output before a later product reads it, so what the
   // previous call left behind is never looked at.
-  return dionw_newton_schulz(x, out, blocks, m, n, ldx, kind, scratch, kStaticScratchBytes, nullptr, stream);
+  return dionw_newton_schulz(x, out, blocks, m, n, ldx, kind, scratch, kStaticScratchBytes + kStaticCounterBytes, nullptr,
+                             stream);
 }

@@ -69,16 +69,17 @@ class NativeOrthogonalizer:
 
 
 def run_iteration(fn: NativeOrthogonalizer, x: Tensor, rows: int, cols: int, scratch: Tensor,
-                  rowsq: Tensor | None = None) -> Tensor:
+                  rowsq: Tensor | None = None, stepwise: bool = False) -> Tensor:
     """Iterate in place on ``x`` ``[N, rows, ld]`` (normalised, in ``fn.dtype``); returns bf16 ``[N, rows, ld]``.
 
     ``scratch`` holds ``fn.workspace_bytes(...)`` bytes.  ``rowsq``: fp32
     ``[N * rows, newton_schulz_rowsq_parts(cols)]``, filled with partial row
-    sums of the squared result by the last product's epilogue.
+    sums of the squared result by the last product's epilogue.  ``stepwise``: one
+    launch per product, for a call that runs beside other streams' kernels.
     """
     out = x if x.dtype is torch.bfloat16 else x.view(torch.bfloat16)
     iterate = _native.newton_schulz_tall if rows > cols else _native.newton_schulz
-    iterate(x, out, rows, cols, fn.code, scratch, rowsq)
+    iterate(x, out, rows, cols, fn.code + (_native.NS_STEPWISE if stepwise else 0), scratch, rowsq)
     return out
 
 

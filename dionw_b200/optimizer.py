@@ -31,7 +31,8 @@ from dionw_b200._keys import (
     NUM_HEADS_KEY, ROUTE_KEY, ROW_NORMALIZATION_KEY, STRUCTURAL_KEYS,
 )
 from dionw_b200._matrix_step import (
-    MAX_RUN_ELEMENTS, apply_result, open_run, run_core, run_elements, run_front, step_run, step_size,
+    MAX_RUN_ELEMENTS, apply_result, groups_of_runs, open_run, run_core, run_elements, run_front, step_run, step_runs,
+    step_size,
 )
 from dionw_b200.ema import EMAConfig, IntegratedEMAOptimizer, ProfileRegion, no_profile
 from dionw_b200.matrix_update import DION3_UPDATE, MatrixUpdate, MomentumForm, RowNormalization
@@ -256,9 +257,15 @@ class _DionCore(Optimizer):
         return loss
 
     def _step_in_sequence(self, runs: list[tuple[Bucket, list[int]]]) -> None:
-        for bucket, run in runs:
+        # An observer of stages wants its figures per run, and a replaced ``step_run`` gets every run.
+        together = step_run is _sequential_step_run and _matrix_step.STAGE_HOOK is None
+        for members in groups_of_runs(runs, MAX_RUN_ELEMENTS) if together else [[run] for run in runs]:
             # the library looks up per-device facts (SM count, status word) for the current device
-            with torch.cuda.device(bucket.momentum.device):
+            with torch.cuda.device(members[0][0].momentum.device):
+                if len(members) > 1:
+                    step_runs(members, self.param_groups)
+                    continue
+                bucket, run = members[0]
                 step_run(bucket, run, self.param_groups[bucket.group_index], self.state)
         self._step_adamw_groups()
 

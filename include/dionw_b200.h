@@ -47,6 +47,11 @@ extern "C" {
 /* GRAM with the products among symmetric matrices computed in full, as the
  * reference's cuBLAS calls do, instead of on one triangle of tiles. */
 #define DIONW_NS_GRAM_FULL 3
+/* Added to the kind of dionw_newton_schulz or dionw_newton_schulz_tall: one launch per
+ * product instead of one for the iteration, for a call that other streams' kernels
+ * run beside -- they get SMs between two products, where one launch holds them all
+ * until the iteration is done.  Same results. */
+#define DIONW_NS_STEPWISE 256
 
 /* Text of the last error on the calling thread (copied, NUL-terminated). */
 void dionw_last_error(char* buffer, size_t size);
@@ -174,6 +179,18 @@ size_t dionw_newton_schulz_tall_workspace_bytes(int64_t blocks, int64_t rows, in
 int dionw_newton_schulz_tall(void* x, void* out, int64_t blocks, int64_t rows, int64_t cols,
                              int64_t ldx, int kind, void* workspace, size_t workspace_bytes,
                              float* rowsq, void* stream);
+
+/* The iterations of up to DIONW_NS_GROUP_MAX batches of different shapes (wide, square or tall, ldx =
+ * cols rounded up to 8) as one launch: the products of one batch fill the GPU while those of another
+ * wait for one another.  All kinds of a group iterate in the same dtype.  rowsq (nullable) holds one
+ * nullable pointer per batch.  Arrays are host arrays of n entries; results are those of n single calls. */
+#define DIONW_NS_GROUP_MAX 6
+size_t dionw_newton_schulz_group_workspace_bytes(int n, const int64_t* blocks, const int64_t* rows,
+                                                 const int64_t* cols, const int* kinds);
+int dionw_newton_schulz_group(int n, void* const* x, void* const* out, const int64_t* blocks,
+                              const int64_t* rows, const int64_t* cols, const int* kinds,
+                              void* workspace, size_t workspace_bytes, float* const* rowsq,
+                              void* stream);
 
 /* The same iteration for callers that have no scratch to give: a host bound to
  * this ABI without torch's allocator, a serving loop whose memory was budgeted at

@@ -118,3 +118,68 @@ def test_normalize_pack_matches_the_fp32_form(rows: int, cols: int, dtype: torch
         want = value.double() / (norm * scale)
         assert bool(((x[..., :cols].double().cpu() - want).abs() <= bound * want.abs() + 2.0**-24).all())
         assert bool((x[..., cols:] == 0).all())
+
+
+@pytest.mark.parametrize("kinds", [(native.NS_GRAM,), (native.NS_POLAR_EXPRESS, native.NS_KELLER)])
+def test_a_group_of_batches_equals_its_members_alone(kinds: tuple[int, ...]) -> None:
+    """One launch over wide, square and tall batches, of one tile and of many, against one launch each,
+    bit for bit; repeated, because what could differ is the order in which tiles run."""
+    shapes = [(3, 130, 300), (1, 1, 1), (2, 256, 256), (5, 700, 65), (1, 1030, 2100), (40, 64, 192)]
+    assert len(shapes) == native.NS_GROUP_MAX
+    gen = torch.Generator().manual_seed(5)
+    dtype = torch.float16 if native.NS_GRAM in kinds else torch.bfloat16
+    codes = [kinds[i % len(kinds)] for i in range(len(shapes))]
+    sources, want, sums = [], [], []
+    for (blocks, rows, cols), kind in zip(shapes, codes):
+        x = torch.zeros(blocks, rows, _padded(cols), dtype=dtype)
+        values = torch.randn(blocks, rows, cols, generator=gen)
+        x[..., :cols] = (values / values.norm(dim=(1, 2), keepdim=True)).to(dtype)
+        x = x.to(DEV)
+        sources.append(x)
+        alone = x.clone()
+        rowsq = torch.empty(blocks * rows, native.newton_schulz_rowsq_parts(cols), device=DEV)
+        tall = rows > cols
+        need = (native.newton_schulz_tall_workspace_bytes if tall else native.newton_schulz_workspace_bytes)
+        ws = torch.empty(need(blocks, rows, cols, kind), dtype=torch.uint8, device=DEV)
+        run = native.newton_schulz_tall if tall else native.newton_schulz
+        run(alone, alone.view(torch.bfloat16), rows, cols, kind, ws, rowsq)
+        want.append(alone.view(torch.bfloat16)[..., :cols])
+        sums.append(rowsq)
+        stepwise, out = x.clone(), torch.empty_like(x).view(torch.bfloat16)
+        run(stepwise, out, rows, cols, kind + native.NS_STEPWISE, ws)
+        assert torch.equal(out[..., :cols], want[-1])
+    ws = torch.empty(native.newton_schulz_group_workspace_bytes(shapes, codes), dtype=torch.uint8, device=DEV)
+    for _ in range(5):
+        ws.fill_(255)   # neither the counters nor the matrices may have to start at anything
+        xs = [x.clone() for x in sources]
+        rowsqs = [None if i == 2 else torch.full_like(s, SENTINEL) for i, s in enumerate(sums)]
+        native.newton_schulz_group(xs, [x.view(torch.bfloat16) for x in xs], shapes, codes, ws, rowsqs)
+        for i, (x, (_, _, cols)) in enumerate(zip(xs, shapes)):
+            assert torch.equal(x.view(torch.bfloat16)[..., :cols], want[i])
+            assert rowsqs[i] is None or torch.equal(rowsqs[i], sums[i])
+    assert native.device_status() == 0
+    with pytest.raises(ValueError, match="fp16 and bf16"):
+        native.newton_schulz_group(xs[:2], xs[:2], shapes[:2], [native.NS_GRAM, native.NS_KELLER], ws, [None, None])
+
+
+@pytest.mark.parametrize("update", ["DION3_UPDATE", "MUON_UPDATE"])
+def test_a_step_in_groups_equals_a_step_run_by_run(update: str, monkeypatch: pytest.MonkeyPatch) -> None:
+    import dionw_b200 as dionw
+
+    shapes = [(1024, 1100), (1024, 1100), (96, 40), (40, 96), (64, 64), (1200, 1030), (8, 300), (33, 17), (20, 20)]
+    results = []
+    for group_max in (native.NS_GROUP_MAX, 1):
+        monkeypatch.setattr(native, "NS_GROUP_MAX", group_max)
+        gen = torch.Generator().manual_seed(11)
+        model = torch.nn.ParameterList([torch.nn.Parameter((torch.randn(s, generator=gen) * 0.02).to(DEV)) for s in shapes])
+        extra = {"fraction": 1.0} if update == "MUON_UPDATE" else {}
+        optimizer = dionw.Dion(dionw.param_groups(model, **extra)[0], lr=1e-2, weight_decay=0.1,
+                               matrix_update=getattr(dionw, update))
+        for _ in range(3):
+            for p in model:
+                p.grad = (torch.randn(p.shape, generator=gen) * 1e-3).to(DEV)
+            optimizer.step()
+        results.append([t.clone() for p in model for t in (p.detach(), optimizer.state[p]["momentum"],
+                                                           optimizer.state[p]["variance"])])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
