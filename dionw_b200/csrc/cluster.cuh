@@ -1,4 +1,4 @@
-// Thread-block clusters: rank, barrier, and the other CTAs' shared memory.
+// Kernel launches: clusters (rank, barrier, the other CTAs' shared memory) and programmatic dependence.
 #pragma once
 
 #include <cstdint>
@@ -47,6 +47,30 @@ inline unsigned cluster_for(long long blocks, long long rows, long long rows_per
   return n;
 }
 
+// Programmatic dependent launch: a kernel launched by launch_dependent or launch_clusters may have CTAs
+// resident while the kernel before it in the stream still runs, and waits here before it touches global
+// memory; the wait returns once that kernel has completed and its writes are visible.  A step of small
+// matrices is a chain of 5 to 20 us kernels with 2 to 3 us between them: @PDLFIGURES@
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, cudaStream_t stream,
+                             Args... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(threads);
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // blocks x cluster CTAs, `cluster` of them to a cluster.
 template <typename... Params, typename... Args>
 cudaError_t launch_clusters(void (*kernel)(Params...), unsigned blocks, unsigned cluster, unsigned threads,
@@ -55,13 +79,15 @@ cudaError_t launch_clusters(void (*kernel)(Params...), unsigned blocks, unsigned
   config.gridDim = dim3(blocks * cluster);
   config.blockDim = dim3(threads);
   config.stream = stream;
-  cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = cluster;
-  attribute.val.clusterDim.y = 1;
-  attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = cluster;
+  attributes[0].val.clusterDim.y = 1;
+  attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = 2;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 

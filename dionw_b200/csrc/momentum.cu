@@ -125,6 +125,7 @@ template <typename G>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 accumulate_row_l1_kernel(const RowTable tab, float* __restrict__ momentum, float* __restrict__ scores,
                          float* __restrict__ sumsq, long long cols, long long total_rows, bool vec) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= total_rows) return;
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 accumulate_copy_decay_kernel(const RowTable tab, float* __restrict__ momentum, float* __restrict__ u,
                              float* __restrict__ sumsq, long long cols, long long total_rows, float decay,
                              bool nesterov, bool vec) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= total_rows) return;
@@ -246,6 +248,7 @@ constexpr int kKeep = 4;
 __global__ void __launch_bounds__(kSelectThreads)
 select_rows_kernel(const float* __restrict__ scores, const float* __restrict__ sumsq, int rows, int k,
                    int32_t* __restrict__ index, int32_t* __restrict__ rowmap, float* __restrict__ frob) {
+  after_previous();
   __shared__ uint32_t hist[4][256];
   __shared__ uint32_t s_prefix, s_remaining;
   __shared__ uint32_t warp_totals[32];
@@ -404,6 +407,7 @@ select_rows_kernel(const float* __restrict__ scores, const float* __restrict__ s
 
 __global__ void __launch_bounds__(kSelectThreads)
 block_norms_kernel(const float* __restrict__ sumsq, int rows, float* __restrict__ frob) {
+  after_previous();
   __shared__ float partial[kSelectThreads];
   const int tid = threadIdx.x;
   const float* ss = sumsq + (long long)blockIdx.x * rows;
@@ -428,6 +432,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 pack_rows_kernel(float* __restrict__ src, const int32_t* __restrict__ index, const float* __restrict__ frob,
                  long long rows, long long k, long long cols, long long total, float decay, bool decay_rows,
                  float eps, float norm_scale, uint16_t* __restrict__ x, long long ldx, bool vec) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (item >= total) return;
@@ -570,6 +575,7 @@ template <typename S, bool kBf16>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 source_sumsq_kernel(const S* __restrict__ src, long long total_rows, long long cols, float* __restrict__ sumsq,
                     bool vec) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= total_rows) return;
@@ -596,6 +602,7 @@ template <typename S, bool kBf16>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 source_pack_kernel(const S* __restrict__ src, const float* __restrict__ frob, long long total_rows, long long rows,
                    long long cols, float eps, float norm_scale, uint16_t* __restrict__ x, long long ldx, bool vec) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= total_rows) return;
@@ -638,13 +645,13 @@ int source_pack(const void* src, int64_t blocks, int64_t rows, int64_t cols, flo
   const unsigned grid = unsigned((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
   const S* typed = static_cast<const S*>(src);
   const bool vec = cols % Quad<S>::kCount == 0 && aligned16(src) && aligned16(x);   // ldx is a multiple of 8
-  source_sumsq_kernel<S, kBf16><<<grid, kWarpsPerBlock * 32, 0, stream>>>(typed, total, cols, sumsq, vec);
+  launch_dependent(source_sumsq_kernel<S, kBf16>, grid, kWarpsPerBlock * 32, stream, typed, total, cols, sumsq, vec);
   int st = launch_status("source_sumsq_kernel");
   if (st != DIONW_OK) return st;
-  block_norms_kernel<<<unsigned(blocks), kSelectThreads, 0, stream>>>(sumsq, int(rows), frob);
+  launch_dependent(block_norms_kernel, unsigned(blocks), kSelectThreads, stream, sumsq, int(rows), frob);
   st = launch_status("block_norms_kernel");
   if (st != DIONW_OK) return st;
-  source_pack_kernel<S, kBf16><<<grid, kWarpsPerBlock * 32, 0, stream>>>(typed, frob, total, rows, cols, eps, norm_scale,
+  launch_dependent(source_pack_kernel<S, kBf16>, grid, kWarpsPerBlock * 32, stream, typed, frob, total, rows, cols, eps, norm_scale,
                                                                          static_cast<uint16_t*>(x), ldx, vec);
   return launch_status("source_pack_kernel");
 }
@@ -724,11 +731,11 @@ extern "C" int dionw_accumulate_row_l1_run(const void* const* grads, int grad_dt
     const unsigned grid = unsigned((nrows + kWarpsPerBlock - 1) / kWarpsPerBlock);
     float* m = momentum + row0 * cols;
     if (grad_dtype == DIONW_F32)
-      accumulate_row_l1_kernel<float><<<grid, kWarpsPerBlock * 32, 0, stream>>>(tab, m, scores + row0, sumsq + row0, cols, nrows, vec);
+      launch_dependent(accumulate_row_l1_kernel<float>, grid, kWarpsPerBlock * 32, stream, tab, m, scores + row0, sumsq + row0, cols, nrows, vec);
     else if (grad_dtype == DIONW_F16)
-      accumulate_row_l1_kernel<__half><<<grid, kWarpsPerBlock * 32, 0, stream>>>(tab, m, scores + row0, sumsq + row0, cols, nrows, vec);
+      launch_dependent(accumulate_row_l1_kernel<__half>, grid, kWarpsPerBlock * 32, stream, tab, m, scores + row0, sumsq + row0, cols, nrows, vec);
     else
-      accumulate_row_l1_kernel<__nv_bfloat16><<<grid, kWarpsPerBlock * 32, 0, stream>>>(tab, m, scores + row0, sumsq + row0, cols, nrows, vec);
+      launch_dependent(accumulate_row_l1_kernel<__nv_bfloat16>, grid, kWarpsPerBlock * 32, stream, tab, m, scores + row0, sumsq + row0, cols, nrows, vec);
     return launch_status("accumulate_row_l1_kernel");
   });
 }
@@ -748,11 +755,11 @@ extern "C" int dionw_accumulate_copy_decay_run(const void* const* grads, int gra
     float* out = u + row0 * cols;
     const bool nest = nesterov != 0;
     if (grad_dtype == DIONW_F32)
-      accumulate_copy_decay_kernel<float><<<grid, kWarpsPerBlock * 32, 0, stream>>>(tab, m, out, sumsq + row0, cols, nrows, decay, nest, vec);
+      launch_dependent(accumulate_copy_decay_kernel<float>, grid, kWarpsPerBlock * 32, stream, tab, m, out, sumsq + row0, cols, nrows, decay, nest, vec);
     else if (grad_dtype == DIONW_F16)
-      accumulate_copy_decay_kernel<__half><<<grid, kWarpsPerBlock * 32, 0, stream>>>(tab, m, out, sumsq + row0, cols, nrows, decay, nest, vec);
+      launch_dependent(accumulate_copy_decay_kernel<__half>, grid, kWarpsPerBlock * 32, stream, tab, m, out, sumsq + row0, cols, nrows, decay, nest, vec);
     else
-      accumulate_copy_decay_kernel<__nv_bfloat16><<<grid, kWarpsPerBlock * 32, 0, stream>>>(tab, m, out, sumsq + row0, cols, nrows, decay, nest, vec);
+      launch_dependent(accumulate_copy_decay_kernel<__nv_bfloat16>, grid, kWarpsPerBlock * 32, stream, tab, m, out, sumsq + row0, cols, nrows, decay, nest, vec);
     return launch_status("accumulate_copy_decay_kernel");
   });
 }
@@ -770,7 +777,7 @@ extern "C" int dionw_select_rows(const float* scores, const float* sumsq, int64_
 
 extern "C" int dionw_block_norms(const float* sumsq, int64_t blocks, int64_t rows, float* frob, void* stream_ptr) {
   DIONW_REQUIRE(blocks > 0 && rows > 0, "block_norms: empty problem");
-  block_norms_kernel<<<unsigned(blocks), kSelectThreads, 0, static_cast<cudaStream_t>(stream_ptr)>>>(sumsq, int(rows), frob);
+  launch_dependent(block_norms_kernel, unsigned(blocks), kSelectThreads, static_cast<cudaStream_t>(stream_ptr), sumsq, int(rows), frob);
   return launch_status("block_norms_kernel");
 }
 
@@ -785,11 +792,11 @@ extern "C" int dionw_pack_rows(float* src, const int32_t* index, const float* fr
   const unsigned grid = unsigned((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   if (x_dtype == DIONW_BF16)
-    pack_rows_kernel<true><<<grid, kWarpsPerBlock * 32, 0, stream>>>(src, index, frob, rows, k, cols, total, decay,
+    launch_dependent(pack_rows_kernel<true>, grid, kWarpsPerBlock * 32, stream, src, index, frob, rows, k, cols, total, decay,
                                                                       decay_rows != 0, eps, norm_scale,
                                                                       static_cast<uint16_t*>(x), ldx, vec);
   else
-    pack_rows_kernel<false><<<grid, kWarpsPerBlock * 32, 0, stream>>>(src, index, frob, rows, k, cols, total, decay,
+    launch_dependent(pack_rows_kernel<false>, grid, kWarpsPerBlock * 32, stream, src, index, frob, rows, k, cols, total, decay,
                                                                        decay_rows != 0, eps, norm_scale,
                                                                        static_cast<uint16_t*>(x), ldx, vec);
   return launch_status("pack_rows_kernel");

@@ -72,6 +72,7 @@ normuon_rows_kernel(const float* __restrict__ s, int parts, float* __restrict__ 
                     const int32_t* __restrict__ index, int rows, int k, float inv_count_cols, float weight, float eps,
                     float step_host, const float* __restrict__ step_device, bool normalize,
                     float* __restrict__ denom, float* __restrict__ scale) {
+  after_previous();
   __shared__ float scratch[kReduceThreads];
   __shared__ float s_totals[2];
   const uint32_t rank = cluster_rank(), ctas = cluster_size();
@@ -163,6 +164,7 @@ struct ApplyTable {
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
 apply_run_kernel(const ApplyTable tab, long long total_rows, int ldo, int rows, int k, int cols, float decay_host,
                  const float* __restrict__ decay_device, bool has_decay, bool vec, const DecayJob* __restrict__ job) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;   // one row per warp; the launch chooses the CTA size
   const long long stride = (long long)gridDim.x * warps;
@@ -254,6 +256,7 @@ struct AdamTable {
 };
 
 __global__ void adamw_bump_steps_kernel(const AdamTable tab) {
+  after_previous();
   const int i = threadIdx.x;
   if (i < tab.n) *tab.step[i] += 1.0f;
 }
@@ -271,6 +274,7 @@ __device__ __forceinline__ void adamw_math(float& p, float g, float& m, float& v
 __global__ void __launch_bounds__(kAdamThreads)
 adamw_multi_kernel(const AdamTable tab, float lr_host, float beta1, float beta2, float weight_decay_host, float eps,
                    const float* __restrict__ hyper_device) {
+  after_previous();
   // learning rate and weight decay come from device memory when the caller keeps them there
   const float lr = hyper_device != nullptr ? hyper_device[0] : lr_host;
   const float weight_decay = hyper_device != nullptr ? hyper_device[1] : weight_decay_host;
@@ -506,7 +510,7 @@ extern "C" int dionw_apply_round(void* const* weights, const int64_t* rows_per_t
     if (acc > 0) {
       long long grid = (acc + warps - 1) / warps;
       if (grid > 0x7FFFFFFFll) grid = 0x7FFFFFFFll;   // the kernel walks the rows with a stride
-      apply_run_kernel<<<unsigned(grid), warps * 32, 0, stream>>>(tab, acc, int(ldo), int(rows), int(k), int(cols),
+      launch_dependent(apply_run_kernel, unsigned(grid), warps * 32, stream, tab, acc, int(ldo), int(rows), int(k), int(cols),
                                                                   decay_factor, decay_device, has_decay != 0, vec,
                                                                   static_cast<const DecayJob*>(decay_job));
       const int st = launch_status("apply_run_kernel");
@@ -622,10 +626,10 @@ extern "C" int dionw_adamw_multi(void* const* params, const void* const* grads, 
         tab.step[slot] = static_cast<float*>(steps[i]);
       },
       [&](const AdamTable& tab, unsigned blocks) {
-        adamw_bump_steps_kernel<<<1, kAdamTable, 0, stream>>>(tab);
+        launch_dependent(adamw_bump_steps_kernel, 1, kAdamTable, stream, tab);
         int st = launch_status("adamw_bump_steps_kernel");
         if (st != DIONW_OK) return st;
-        adamw_multi_kernel<<<blocks, kAdamThreads, 0, stream>>>(tab, lr, beta1, beta2, weight_decay, eps,
+        launch_dependent(adamw_multi_kernel, blocks, kAdamThreads, stream, tab, lr, beta1, beta2, weight_decay, eps,
                                                                 hyper_device);
         return launch_status("adamw_multi_kernel");
       });
