@@ -239,13 +239,21 @@ def pack_rows(src: Tensor, index: Tensor | None, frob: Tensor, k: int, x: Tensor
 
 
 def normalize_pack(src: Tensor, x: Tensor, *, eps: float, norm_scale: float = 1.0) -> None:
-    """``x = src / (norm * norm_scale + eps)`` per block, for a contiguous batch of any of the three dtypes."""
+    """``x = src / (norm * norm_scale + eps)`` per block, for a contiguous batch of any of the three dtypes.
+
+    The norm is torch's, as in src/dionw/_gram.py:85-87 and src/dionw/_polar_express.py:88-92: a norm
+    summed in another order differs in its last bit, which moves single roundings of ``x`` and with them
+    1e-3 of the polar factor.  Torch sums the 2-byte batches in fp32 without a copy, in the order of
+    the fp32 copy.
+    """
     blocks, rows, cols = src.shape
-    scratch = torch.empty(blocks * rows + blocks, dtype=torch.float32, device=src.device)
-    sums = scratch.data_ptr()
+    if x.dtype is torch.bfloat16:
+        frob = src.bfloat16().norm(dim=(-2, -1)).float()
+    else:
+        frob = torch.linalg.vector_norm(src, dim=(-2, -1), dtype=torch.float32)
     _check(library().dionw_normalize_pack(src.data_ptr(), dtype_code(src.dtype), blocks, rows, cols, eps, norm_scale,
-                                          x.data_ptr(), dtype_code(x.dtype), x.stride(-2), sums,
-                                          sums + 4 * blocks * rows, _stream(src)))
+                                          x.data_ptr(), dtype_code(x.dtype), x.stride(-2), None, frob.data_ptr(),
+                                          _stream(src)))
 
 
 def transpose_2byte(src: Tensor, dst: Tensor) -> None:

@@ -566,11 +566,11 @@ __device__ __forceinline__ void walk_row(const S* __restrict__ row, long long co
   }
 }
 
-// Row sums of squares (of the values rounded to bf16 first for the bf16 iterations) and the normalised
-// 2-byte operand, straight from the caller's dtype.  HBM-bound: two reads of the source and one write
-// of the operand are all the traffic (the norm needs the whole block before the first division).  A
-// conversion to fp32 and a library norm in front of the pack moved 18 bytes per bf16 element instead
-// of 6: 16 blocks of 4096 x 14336 spent 5.4 ms of a 38.7 ms call in those three.
+// Row sums of squares (of the values rounded to bf16 first for the bf16 iterations), for a caller that has no
+// norms, and the normalised 2-byte operand, straight from the caller's dtype.  HBM-bound: two reads of the
+// source (the norm needs the whole block before the first division) and one write of the operand are all the
+// traffic.  A conversion to fp32 in front of norm and pack moved 18 bytes per bf16 element instead of 6: 16
+// blocks of 4096 x 14336 spent 5.4 ms of a 38.7 ms call in conversion, norm and pack.
 template <typename S, bool kBf16>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 source_sumsq_kernel(const S* __restrict__ src, long long total_rows, long long cols, float* __restrict__ sumsq,
@@ -645,12 +645,14 @@ int source_pack(const void* src, int64_t blocks, int64_t rows, int64_t cols, flo
   const unsigned grid = unsigned((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
   const S* typed = static_cast<const S*>(src);
   const bool vec = cols % Quad<S>::kCount == 0 && aligned16(src) && aligned16(x);   // ldx is a multiple of 8
-  launch_dependent(source_sumsq_kernel<S, kBf16>, grid, kWarpsPerBlock * 32, stream, typed, total, cols, sumsq, vec);
-  int st = launch_status("source_sumsq_kernel");
-  if (st != DIONW_OK) return st;
-  launch_dependent(block_norms_kernel, unsigned(blocks), kSelectThreads, stream, sumsq, int(rows), frob);
-  st = launch_status("block_norms_kernel");
-  if (st != DIONW_OK) return st;
+  if (sumsq != nullptr) {
+    launch_dependent(source_sumsq_kernel<S, kBf16>, grid, kWarpsPerBlock * 32, stream, typed, total, cols, sumsq, vec);
+    int st = launch_status("source_sumsq_kernel");
+    if (st != DIONW_OK) return st;
+    launch_dependent(block_norms_kernel, unsigned(blocks), kSelectThreads, stream, sumsq, int(rows), frob);
+    st = launch_status("block_norms_kernel");
+    if (st != DIONW_OK) return st;
+  }
   launch_dependent(source_pack_kernel<S, kBf16>, grid, kWarpsPerBlock * 32, stream, typed, frob, total, rows, cols, eps, norm_scale,
                                                                          static_cast<uint16_t*>(x), ldx, vec);
   return launch_status("source_pack_kernel");

@@ -133,8 +133,10 @@ int dionw_pack_rows(float* src, const int32_t* index, const float* frob,
 
 /* x = half(src / (||src[b]||_F + eps)) for a caller's own batch src [blocks, rows,
  * cols] of any of the three dtypes, contiguous; x is [blocks, rows, ldx] in x_dtype
- * (BF16: the forms described at dionw_pack_rows).  sumsq [blocks * rows] and frob
- * [blocks] are scratch.  Replaces the cast, norm and division at the head of
+ * (BF16: the forms described at dionw_pack_rows).  frob [blocks] holds the Frobenius
+ * norms if sumsq is null; otherwise sumsq [blocks * rows] and frob are scratch and the
+ * norms are taken here.  (They differ from another summation's in the last bit, which
+ * moves single roundings of x.)  Replaces the cast, norm and division at the head of
  * src/dionw/_gram.py:85-87 and src/dionw/_polar_express.py:88-92. */
 int dionw_normalize_pack(const void* src, int src_dtype, int64_t blocks, int64_t rows,
                          int64_t cols, float eps, float norm_scale, void* x, int x_dtype,

@@ -120,6 +120,44 @@ def test_normalize_pack_matches_the_fp32_form(rows: int, cols: int, dtype: torch
         assert bool((x[..., cols:] == 0).all())
 
 
+@pytest.mark.parametrize("blocks, rows, cols", [(1, 256, 1024), (6, 1531, 517), (16, 1024, 1024), (40, 65, 4000), (3, 1, 9)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_normalize_pack_has_the_bits_of_the_fp32_form(blocks: int, rows: int, cols: int, dtype: torch.dtype) -> None:
+    """Bit for bit what the batch's fp32 copy gives, divided by torch's norm of that copy."""
+    for seed in range(3):
+        gen = torch.Generator(device=DEV).manual_seed(seed)
+        src = torch.randn(blocks, rows, cols, device=DEV, generator=gen)
+        if seed > 0:
+            src /= torch.linalg.vector_norm(src, dim=(1, 2), keepdim=True)
+        src = src.to(dtype)
+        copy = src.float()
+        for out_dtype, scale in ((torch.float16, 1.0), (torch.bfloat16, 1.02)):
+            half = out_dtype is torch.float16
+            norm = torch.linalg.vector_norm(copy, dim=(1, 2)) if half else copy.bfloat16().norm(dim=(1, 2)).float()
+            x, want = (torch.empty(blocks, rows, _padded(cols), dtype=out_dtype, device=DEV) for _ in range(2))
+            native.normalize_pack(src, x, eps=1e-8, norm_scale=scale)
+            native.pack_rows(copy, None, norm, rows, want, decay=1.0, decay_rows=False, eps=1e-8, norm_scale=scale)
+            assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_the_library_takes_the_norms_of_a_caller_without_them(dtype: torch.dtype) -> None:
+    """With a buffer for row sums the norms come from fp32 sums of 40 x 333 squares: 2^-12 at the most."""
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    src = torch.randn(3, 40, 333, device=DEV, generator=gen).to(dtype)
+    x = torch.empty(3, 40, 336, dtype=torch.float16, device=DEV)
+    sums, frob = torch.empty(120, device=DEV), torch.empty(3, device=DEV)
+    status = native.library().dionw_normalize_pack(
+        src.data_ptr(), native.dtype_code(dtype), 3, 40, 333, 1e-8, 1.0, x.data_ptr(), native.F16, 336, sums.data_ptr(),
+        frob.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert status == 0
+    norm = src.double().square().sum((1, 2)).sqrt()
+    assert bool(((frob.double() - norm).abs() <= 2.0**-12 * norm).all())
+    want = torch.empty_like(x)
+    native.pack_rows(src.float(), None, frob, 40, want, decay=1.0, decay_rows=False, eps=1e-8)
+    assert torch.equal(x, want)
+
+
 @pytest.mark.parametrize("kinds", [(native.NS_GRAM,), (native.NS_POLAR_EXPRESS, native.NS_KELLER)])
 def test_a_group_of_batches_equals_its_members_alone(kinds: tuple[int, ...]) -> None:
     """One launch over wide, square and tall batches, of one tile and of many, against one launch each,
