@@ -83,10 +83,15 @@ __device__ __forceinline__ void remote_arrive_release(uint32_t cluster_address) 
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 
-// Relaxed arrive that is issued once `loaded`, the result of a load, is there.
+// Relaxed arrive that is issued once `loaded`, the result of a load, is there: the arrive is predicated on the
+// value, which is never kNoTile.  (Relaxed, so the memory model does not order the load before it; the
+// dependency does, since an instruction is not issued before its predicate is known.  The comparison is with
+// the largest integer because no branch on the sign of a tile's index decides it.)
+constexpr int kNoTile = 0x7FFFFFFF;   // a plan has fewer than 2^31 tiles
 __device__ __forceinline__ void remote_arrive_after(uint32_t cluster_address, int loaded) {
-  asm volatile("{\n.reg .b32 t;\nmov.b32 t, %1;\nmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}\n"
-               ::"r"(cluster_address), "r"(loaded) : "memory");
+  asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %1, %2;\n"
+               "@p mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}\n"
+               ::"r"(cluster_address), "r"(loaded), "n"(kNoTile) : "memory");
 }
 
 __device__ __forceinline__ void remote_store_s32(uint32_t cluster_address, int value) {
@@ -309,8 +314,9 @@ __device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned
 // A CTA's half of a tile is reported by a warp of its own, once the eight epilogue warps have arrived on the
 // slot's `stored` barrier: the release at GPU scope waits until the stores have reached L2, and took an
 // epilogue warp 2700 cycles of every tile.  The reporter, too, reports the slot as read only then.
-// For the same reason the arrivals on `tile_empty` are relaxed: they follow a load whose value is in use, not
-// the stores of the tile before (as a release at cluster scope each cost the warp 2000 cycles per tile).
+// For the same reason the arrivals on `tile_empty` are relaxed: they have to follow the read of the slot, which
+// their predicate depends on, and not the stores of the tile before (as a release at cluster scope each cost
+// the warp 2000 cycles per tile).
 constexpr int kTileSlots = 8;
 constexpr uint32_t kTileConsumers = 2 * (1 + kEpilogueWarps);   // and the reporters, in a plan of several products
 

@@ -200,6 +200,25 @@ def test_a_group_of_batches_equals_its_members_alone(kinds: tuple[int, ...]) -> 
         native.newton_schulz_group(xs[:2], xs[:2], shapes[:2], [native.NS_GRAM, native.NS_KELLER], ws, [None, None])
 
 
+@pytest.mark.parametrize("blocks, rows, cols", [(4000, 40, 64), (1500, 64, 40), (700, 130, 257)])
+def test_a_plan_of_many_tiles_equals_its_products_alone(blocks: int, rows: int, cols: int) -> None:
+    """Hundreds of tiles per SM pair, each shorter than the way of its index to the pair's consumers: an
+    entry of the tile ring that is written before it has been read everywhere shows as a wrong tile."""
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    x = torch.zeros(blocks, rows, _padded(cols), dtype=torch.float16, device=DEV)
+    values = torch.randn(blocks, rows, cols, device=DEV, generator=gen)
+    x[..., :cols] = values / values.norm(dim=(1, 2), keepdim=True)
+    run = native.newton_schulz_tall if rows > cols else native.newton_schulz
+    need = native.newton_schulz_tall_workspace_bytes if rows > cols else native.newton_schulz_workspace_bytes
+    ws = torch.empty(need(blocks, rows, cols, native.NS_GRAM), dtype=torch.uint8, device=DEV)
+    want, got = (torch.empty_like(x).view(torch.bfloat16) for _ in range(2))
+    run(x.clone(), want, rows, cols, native.NS_GRAM + native.NS_STEPWISE, ws)
+    for _ in range(3):
+        run(x.clone(), got, rows, cols, native.NS_GRAM, ws)
+        assert torch.equal(got[..., :cols], want[..., :cols])
+    assert native.device_status() == 0
+
+
 @pytest.mark.parametrize("update", ["DION3_UPDATE", "MUON_UPDATE"])
 def test_a_step_in_groups_equals_a_step_run_by_run(update: str, monkeypatch: pytest.MonkeyPatch) -> None:
     import dionw_b200 as dionw
