@@ -578,6 +578,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
       int t = 0;
       if (lane == 0) t = take_tile(local, true);   // one lane waits, reads and reports; the warp follows it
       t = __shfl_sync(0xffffffffu, t, 0);
+      __syncwarp();   // the other lanes read Cin too, which lane 0's wait alone has acquired: a shuffle orders no memory
       if (t < 0) break;
       const Step& step = step_at(t, at);
       const Params& p = step.p;

@@ -219,6 +219,29 @@ def test_a_plan_of_many_tiles_equals_its_products_alone(blocks: int, rows: int, 
     assert native.device_status() == 0
 
 
+@pytest.mark.parametrize("blocks, rows, cols", [(1, 256, 520), (1, 500, 300), (2, 1000, 1100)])
+def test_a_chain_of_one_matrix_reads_what_was_just_stored(blocks: int, rows: int, cols: int) -> None:
+    """One or two matrices, so that every product starts the moment the one before it is stored: each lane of
+    an epilogue warp must see the second term that other SMs wrote, iteration after iteration."""
+    gen = torch.Generator(device=DEV).manual_seed(cols)
+    x = torch.zeros(blocks, rows, _padded(cols), dtype=torch.float16, device=DEV)
+    values = torch.randn(blocks, rows, cols, device=DEV, generator=gen)
+    x[..., :cols] = values / values.norm(dim=(1, 2), keepdim=True)
+    run = native.newton_schulz_tall if rows > cols else native.newton_schulz
+    need = native.newton_schulz_tall_workspace_bytes if rows > cols else native.newton_schulz_workspace_bytes
+    ws = torch.empty(need(blocks, rows, cols, native.NS_GRAM), dtype=torch.uint8, device=DEV)
+    want = torch.empty_like(x).view(torch.bfloat16)
+    run(x.clone(), want, rows, cols, native.NS_GRAM + native.NS_STEPWISE, ws)
+    outs = []
+    for i in range(64):
+        ws.fill_(i)   # what the last iteration left in the scratch must not pass for this one's
+        out = torch.empty_like(want)
+        run(x.clone(), out, rows, cols, native.NS_GRAM, ws)
+        outs.append(out)
+    assert all(torch.equal(out[..., :cols], want[..., :cols]) for out in outs)
+    assert native.device_status() == 0
+
+
 @pytest.mark.parametrize("update", ["DION3_UPDATE", "MUON_UPDATE"])
 def test_a_step_in_groups_equals_a_step_run_by_run(update: str, monkeypatch: pytest.MonkeyPatch) -> None:
     import dionw_b200 as dionw
