@@ -164,9 +164,22 @@ def open_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any], ar
     ctx, plan = _describe_run(bucket, positions, group)
     fn = bucket.orthogonalize
     if isinstance(fn, NativeOrthogonalizer):
-        plan["ns"] = ((fn.workspace_bytes(ctx.count, bucket.selected_rows, bucket.cols),), torch.uint8)
+        plan = _with_iteration(plan, fn.workspace_bytes(ctx.count, bucket.selected_rows, bucket.cols), ["u"])
     ctx.buf = _workspace.carve(ctx.momentum.device, plan, arena)
     return ctx
+
+
+def _with_iteration(plan: _workspace.Plan, ns_bytes: int, sources: Sequence[str]) -> _workspace.Plan:
+    """``plan`` with the iteration's scratch, and the fp32 copies of whole blocks named in ``sources`` over it.
+
+    A copy is written by the accumulating pass and last read by the pack, run after run, and the iteration
+    begins after the last pack: the copies can share its scratch, and one another's."""
+    copies = {name: plan[name] for name in sources if name in plan}
+    longest = max((math.prod(shape) * dtype.itemsize for shape, dtype in copies.values()), default=0)
+    out = {name: entry for name, entry in plan.items() if name not in copies}
+    out["ns"] = ((max(ns_bytes, longest),), torch.uint8)
+    out.update({name: (*entry, "ns") for name, entry in copies.items()})
+    return out
 
 
 def _describe_run(bucket: Bucket, positions: Sequence[int],
@@ -290,8 +303,12 @@ def _finish_run(ctx: RunContext, orthogonal: Tensor) -> RunResult:
 def groups_of_runs(runs: Sequence[tuple[Bucket, Sequence[int]]],
                    limit: int = MAX_RUN_ELEMENTS) -> list[list[tuple[Bucket, Sequence[int]]]]:
     """``runs`` in order, split into groups that ``step_runs`` takes together: built-in iterations of
-    one dtype on one device, at most ``NS_GROUP_MAX`` of them and, so that the transient memory of a
-    step stays bounded as it is for one run, at most ``limit`` update elements together."""
+    one dtype on one device, at most ``NS_GROUP_MAX`` of them and at most ``limit`` update elements together.
+
+    The members hold their operands and the iteration's scratch at the same time, so the transient memory
+    of a step of many small runs is that of their sum and not of the largest: 0.60 GB instead of 0.19 for a
+    12-layer 768-wide language model, 2.0 instead of 1.5 for four layers of 4096.  ``limit`` bounds it as it
+    bounds one run (``optimizer.MAX_RUN_ELEMENTS``)."""
     groups: list[list[tuple[Bucket, Sequence[int]]]] = []
     key: Any = None
     elements = 0
@@ -309,8 +326,17 @@ def groups_of_runs(runs: Sequence[tuple[Bucket, Sequence[int]]],
     return groups
 
 
+def _group_plan(plans: Sequence[_workspace.Plan], shapes: Sequence[tuple[int, int, int]],
+                kinds: Sequence[int]) -> _workspace.Plan:
+    """The scratch of several runs together: entry ``name`` of run ``i`` is ``i.name``."""
+    plan = {f"{i}.{name}": entry for i, own in enumerate(plans) for name, entry in own.items()}
+    return _with_iteration(plan, _native.newton_schulz_group_workspace_bytes(shapes, kinds),
+                           [f"{i}.u" for i in range(len(plans))])
+
+
 def step_runs(runs: Sequence[tuple[Bucket, Sequence[int]]], param_groups: Sequence[dict[str, Any]]) -> None:
-    """One Dion step for several runs of one group (``groups_of_runs``), stage by stage.
+    """One Dion step for several runs (one entry of ``groups_of_runs``; their parameter groups may differ),
+    stage by stage.
 
     Their Newton-Schulz iterations run as one launch.  An iteration is a chain of 15 to 18 products;
     on small blocks each is one part-filled wave and most of its time is the way from one product to
@@ -320,9 +346,7 @@ def step_runs(runs: Sequence[tuple[Bucket, Sequence[int]]], param_groups: Sequen
     contexts = [ctx for ctx, _ in described]
     shapes = [(ctx.count, ctx.bucket.selected_rows, ctx.bucket.cols) for ctx in contexts]
     kinds = [ctx.bucket.orthogonalize.code for ctx in contexts]
-    plan: _workspace.Plan = {f"{i}.{name}": entry for i, (_, own) in enumerate(described) for name, entry in own.items()}
-    plan["ns"] = ((_native.newton_schulz_group_workspace_bytes(shapes, kinds),), torch.uint8)
-    buf = _workspace.carve(contexts[0].momentum.device, plan)
+    buf = _workspace.carve(contexts[0].momentum.device, _group_plan([own for _, own in described], shapes, kinds))
     for i, (ctx, own) in enumerate(described):
         ctx.buf = {name: buf[f"{i}.{name}"] for name in own}
         run_front(ctx)

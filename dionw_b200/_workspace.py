@@ -5,7 +5,9 @@ reused by every later run and step: runs execute one after another on one
 stream, so they can share it, and the caching allocator is not asked for
 gigabytes every step.  A plan is an ordered ``name -> (shape, dtype)`` mapping;
 its entries are laid out in order, each starting on a 256-byte boundary, so two
-processes that build the same plan agree on every offset.
+processes that build the same plan agree on every offset.  An entry ``(shape,
+dtype, other)`` lies over the start of the earlier entry ``other``, which is at
+least as long: the two are not in use at the same time.
 """
 
 from __future__ import annotations
@@ -25,7 +27,7 @@ _CARVED_MAX = 64
 # addresses and is only valid while this number stands.
 generation = 0
 
-Plan = dict[str, tuple[tuple[int, ...], torch.dtype]]
+Plan = dict[str, tuple[tuple[int, ...], torch.dtype] | tuple[tuple[int, ...], torch.dtype, str]]
 
 
 def _round(n: int) -> int:
@@ -36,8 +38,14 @@ def layout(plan: Plan) -> tuple[dict[str, tuple[int, int]], int]:
     """``name -> (byte offset, byte size)`` of every entry, and the total bytes."""
     offsets: dict[str, tuple[int, int]] = {}
     cursor = 0
-    for name, (shape, dtype) in plan.items():
+    for name, (shape, dtype, *over) in plan.items():
         nbytes = math.prod(shape) * dtype.itemsize
+        if over:
+            start, room = offsets[over[0]]
+            if nbytes > room:
+                raise ValueError(f"{name} needs {nbytes} bytes, {over[0]} under it has {room}")
+            offsets[name] = (start, nbytes)
+            continue
         offsets[name] = (cursor, nbytes)
         cursor += _round(nbytes)
     return offsets, cursor
@@ -47,7 +55,7 @@ def views(buffer: Tensor, plan: Plan, base: int = 0) -> dict[str, Tensor]:
     """Typed views of ``buffer`` (a byte tensor) for every entry of ``plan``, laid out from ``base``."""
     offsets, _ = layout(plan)
     out: dict[str, Tensor] = {}
-    for name, (shape, dtype) in plan.items():
+    for name, (shape, dtype, *_) in plan.items():
         start, nbytes = offsets[name]
         out[name] = buffer[base + start : base + start + nbytes].view(dtype).view(shape)
     return out
