@@ -41,14 +41,19 @@ def padded(n: int) -> int:
 @dataclass(frozen=True)
 class NativeOrthogonalizer:
     """A built-in iteration.  ``Dion`` recognises it and feeds it from its fused
-    pack kernel; called directly it orthogonalizes any ``[N, rows, cols]`` batch."""
+    pack kernel; called directly it orthogonalizes any ``[N, rows, cols]`` batch.
+
+    A direct call is one launch that holds every SM until the iteration is done.  With
+    ``stepwise=True`` it is one launch per product, between which kernels of other streams
+    (collectives, a data loader's copies) get SMs; the result is the same bit for bit.
+    """
 
     kind: NewtonSchulz
     code: int             # DIONW_NS_* of the C ABI
     dtype: torch.dtype    # element type of the iteration
     norm_scale: float     # factor on the Frobenius norm before normalising
 
-    def __call__(self, matrix: Tensor, epsilon: float) -> Tensor:
+    def __call__(self, matrix: Tensor, epsilon: float, *, stepwise: bool = False) -> Tensor:
         if matrix.ndim != 3:
             raise ValueError(f"expected a [N, rows, cols] batch, got shape {tuple(matrix.shape)}")
         if not matrix.is_cuda:
@@ -59,7 +64,7 @@ class NativeOrthogonalizer:
         x = torch.empty(blocks, rows, padded(cols), dtype=self.dtype, device=src.device)
         _native.normalize_pack(src, x, eps=epsilon, norm_scale=self.norm_scale)
         scratch = torch.empty(self.workspace_bytes(blocks, rows, cols), dtype=torch.uint8, device=src.device)
-        out = run_iteration(self, x, rows, cols, scratch)
+        out = run_iteration(self, x, rows, cols, scratch, stepwise=stepwise)
         return out[..., :cols]
 
     def workspace_bytes(self, blocks: int, rows: int, cols: int) -> int:

@@ -242,6 +242,25 @@ def test_a_chain_of_one_matrix_reads_what_was_just_stored(blocks: int, rows: int
     assert native.device_status() == 0
 
 
+@pytest.mark.parametrize("rows, cols", [(130, 257), (257, 130), (96, 96)])
+def test_a_direct_call_can_leave_room_for_other_streams(rows: int, cols: int) -> None:
+    """``stepwise``: one launch per product, the same result."""
+    from dionw_b200.newton_schulz import NewtonSchulz, newton_schulz_fn
+
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    x = torch.randn(3, rows, cols, device=DEV, generator=gen)
+    for kind in (NewtonSchulz.GRAM, NewtonSchulz.KELLER):
+        call = newton_schulz_fn(kind)
+        counts, outs = [], []
+        for extra in ({}, {"stepwise": True}):
+            before = native.launch_count()
+            outs.append(call(x, 1e-8, **extra))
+            counts.append(native.launch_count() - before)
+        products = 18 if kind is NewtonSchulz.GRAM and rows != cols else 15
+        assert counts[1] - counts[0] == products - 1
+        assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("update", ["DION3_UPDATE", "MUON_UPDATE"])
 def test_a_step_in_groups_equals_a_step_run_by_run(update: str, monkeypatch: pytest.MonkeyPatch) -> None:
     import dionw_b200 as dionw
