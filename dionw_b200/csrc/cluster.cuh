@@ -47,6 +47,9 @@ inline unsigned cluster_for(long long blocks, long long rows, long long rows_per
   return n;
 }
 
+// Whether kernels are launched with programmatic dependence: yes, unless DIONW_GEMM_PDL=0 (gemm.cu).
+bool use_dependent_launch();
+
 // Programmatic dependent launch: a kernel launched by launch_dependent or launch_clusters may have CTAs
 // resident while the kernel before it in the stream still runs, and waits here before it touches global
 // memory; the wait returns once that kernel has completed and its writes are visible.  A step of small
@@ -69,7 +72,7 @@ cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned 
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
-  config.numAttrs = 1;
+  config.numAttrs = use_dependent_launch() ? 1 : 0;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
@@ -89,7 +92,7 @@ cudaError_t launch_clusters(void (*kernel)(Params...), unsigned blocks, unsigned
   attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
-  config.numAttrs = 2;
+  config.numAttrs = use_dependent_launch() ? 2 : 1;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 

@@ -11,6 +11,19 @@
 #include "products.cuh"
 
 namespace dionw {
+
+// Products, and the other kernels of a step (cluster.cuh), are launched with programmatic stream serialization:
+// they wait with griddepcontrol.wait before they touch global memory.  DIONW_GEMM_PDL=0 turns that off.
+// Measured on the Llama-3-8B-shaped step, for the products when each was a launch of its own (about 290 per
+// step): 95.1-96.2 ms with it, 98.3-99.0 ms without.
+bool use_dependent_launch() {
+  static const bool on = [] {
+    const char* v = std::getenv("DIONW_GEMM_PDL");
+    return v == nullptr || v[0] != '0';
+  }();
+  return on;
+}
+
 namespace {
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -70,17 +83,6 @@ int current_device() {
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) device = 0;
   return device;
-}
-
-// Products are launched with programmatic stream serialization (the kernels wait with
-// griddepcontrol.wait before they touch global memory), unless DIONW_GEMM_PDL=0.  Measured on the
-// Llama-3-8B-shaped step: 95.1-96.2 ms with it, 98.3-99.0 ms without (about 290 product launches per step).
-bool use_dependent_launch() {
-  static const bool on = [] {
-    const char* v = std::getenv("DIONW_GEMM_PDL");
-    return v == nullptr || v[0] != '0';
-  }();
-  return on;
 }
 
 template <typename InT, typename OutT, bool kBMajorMN, bool kSym>
