@@ -289,7 +289,6 @@ extern "C" int dionw_newton_schulz_tall(void* x, void* out, int64_t blocks, int6
   DIONW_REQUIRE(blocks > 0 && cols > 0 && rows > cols,
                 "newton_schulz_tall: needs blocks > 0 and 0 < cols < rows (got %lld, %lld, %lld)", (long long)blocks,
                 (long long)rows, (long long)cols);
-  DIONW_REQUIRE(blocks <= 65535, "newton_schulz_tall: more than 65535 blocks in one call");
   DIONW_REQUIRE(ldx >= cols && ldx % 8 == 0, "newton_schulz_tall: ldx must be >= cols and a multiple of 8");
   DIONW_REQUIRE(aligned16(x) && aligned16(out), "newton_schulz_tall: x and out must be 16-byte aligned");
   const Problem problem{x, out, blocks, rows, cols, ldx, kind & ~DIONW_NS_STEPWISE, rowsq};

@@ -261,6 +261,26 @@ def test_a_direct_call_can_leave_room_for_other_streams(rows: int, cols: int) ->
         assert torch.equal(*outs)
 
 
+@pytest.mark.parametrize("rows, cols", [(9, 8), (8, 9)])
+def test_more_blocks_than_a_grid_dimension_holds(rows: int, cols: int) -> None:
+    """Either orientation takes any number of blocks; each comes out as it does in a small batch."""
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    blocks = 65536 + 9
+    x = torch.zeros(blocks, rows, _padded(cols), dtype=torch.float16, device=DEV)
+    x[..., :cols] = torch.randn(blocks, rows, cols, device=DEV, generator=gen) / 9.0
+    run = native.newton_schulz_tall if rows > cols else native.newton_schulz
+    need = native.newton_schulz_tall_workspace_bytes if rows > cols else native.newton_schulz_workspace_bytes
+    ws = torch.empty(need(blocks, rows, cols, native.NS_GRAM), dtype=torch.uint8, device=DEV)
+    out = torch.empty_like(x).view(torch.bfloat16)
+    few = [x[:50].clone(), x[-50:].clone()]
+    run(x, out, rows, cols, native.NS_GRAM, ws)
+    for part, got in zip(few, (out[:50], out[-50:])):
+        want = torch.empty_like(part).view(torch.bfloat16)
+        run(part, want, rows, cols, native.NS_GRAM, ws)
+        assert torch.equal(got[..., :cols], want[..., :cols])
+    assert native.device_status() == 0
+
+
 @pytest.mark.parametrize("update", ["DION3_UPDATE", "MUON_UPDATE"])
 def test_a_step_in_groups_equals_a_step_run_by_run(update: str, monkeypatch: pytest.MonkeyPatch) -> None:
     import dionw_b200 as dionw
