@@ -291,7 +291,7 @@ __device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned
 // tile hand-out
 // ----------------------------------------------------------------------------
 // A pair takes its tiles either in a fixed stride (tile = pair, pair + pairs, ...: no shared state)
-// or from a counter in global memory, one atomicAdd per tile (Params::tile_counter non-null).  The
+// or from a counter in global memory, one atomicAdd per tile (Plan::tile_counter non-null).  The
 // second form is for products that run beside other kernels (NCCL's, another stream's): a pair whose
 // CTAs become resident late, or not before the others are done, simply takes fewer tiles, where the
 // fixed stride makes the whole product wait for it.
@@ -608,7 +608,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
         if (lane == 0) remote_arrive(leader_empty[acc]);
       };
       auto epilogue = [&](auto symmetric) {
-        return epilogue_tile<InT, decltype(symmetric)::value, kEpilogueWarps / 8>(
+        return epilogue_tile<InT, decltype(symmetric)::value>(
             p, tile.batch, m_base, n_base, tmem_acc, &acc_full[acc], acc_phase, abort_flag, stage, sub, lane, first_chunk,
             chunks, step.out_bf16, release);
       };

@@ -267,11 +267,6 @@ __device__ __forceinline__ Tile general_tile(int t, const Params& p) {
 
 // Symmetric product: tile row i (128 rows) needs tile columns 0..i/2 (256
 // columns each).  Rows 2q and 2q+1 hold q+1 tiles each, q(q+1) tiles precede them.
-__device__ __forceinline__ int sym_tiles(int tiles_m) {
-  const int q = tiles_m / 2;
-  return q * (q + 1) + ((tiles_m & 1) ? q + 1 : 0);
-}
-
 __device__ __forceinline__ Tile sym_tile(int t, const Params& p) {
   Tile tile;
   tile.batch = t / p.tiles_per_batch;
@@ -318,8 +313,8 @@ __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
 // epilogue of one accumulator: 128 rows (m_base ..) x tile_n columns (n_base ..) of batch
 // ``batch``, read from TMEM at ``tmem_acc`` by the warp that owns sub-partition ``sub``;
 // this warp handles `chunks` of the tile's 32-column chunks from first_chunk on.  `release` is called once,
-// when the warp has read all it needs of the accumulator.  kPartWarps warps in a row of the tile share the
-// 128 columns of one part of the row sums.  Returns false when the bounded wait for the accumulator ran out.
+// when the warp has read all it needs of the accumulator.  Returns false when the bounded wait for the
+// accumulator ran out.
 //
 // A warp works on 32 x 32 pieces.  The accumulator is read in the mma result layout, because
 // stmatrix turns that into rows of the piece and, with .trans, into rows of its mirror image at four
@@ -335,7 +330,7 @@ __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
 // through per-element loops: a 256^3 mirrored product with Cin took 15.7 us in a chain of products,
 // this takes 8.1; 6 blocks of 517^3 17.8 us against 12.6.
 // ----------------------------------------------------------------------------
-template <typename InT, bool kSym, int kPartWarps, typename Release>
+template <typename InT, bool kSym, typename Release>
 __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_base, int n_base, uint32_t tmem_acc,
                                               uint64_t* acc_full_bar, uint32_t acc_phase, volatile int* abort_flag,
                                               uint8_t* stage, int sub, int lane, int first_chunk, int chunks,
@@ -574,29 +569,10 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
       sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 1);
       sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 2);
     }
-    bool writer = piece_unit == 0;
-    if constexpr (kPartWarps == 2) {
-      // The second warp of a part hands its sums to the first through its staging tile (the warps of one
-      // sub-partition are four apart, and so are their tiles).
-      const bool second = (first_chunk / chunks) % 2 != 0;
-      const int barrier = 1 + 4 * (first_chunk / (2 * chunks)) + sub;
-      float* theirs = reinterpret_cast<float*>(second ? stage : stage + 4 * 2 * kPieceBytes);
-      if (second && writer) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) theirs[8 * i + piece_row] = sq[i];
-      }
-      asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
-      if (!second && writer) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sq[i] += theirs[8 * i + piece_row];
-      }
-      asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory");
-      writer = writer && !second;
-    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = row0 + 8 * i + piece_row;
-      if (writer && row < m) p.rowsq[(size_t(batch) * m + row) * p.rowsq_parts + part] = sq[i];
+      if (piece_unit == 0 && row < m) p.rowsq[(size_t(batch) * m + row) * p.rowsq_parts + part] = sq[i];
     }
   }
   return true;
@@ -737,9 +713,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         tc_fence_before();
         mbar_arrive(&acc_empty[acc]);
       };
-      if (!epilogue_tile<InT, kSym, 1>(p, tile.batch, tile.tm * kBM, tile.tn * kBN, tmem_base + acc * uint32_t(kBN),
-                                             &acc_full[acc], acc_phase, abort_flag, stage, sub, lane, first_chunk,
-                                             kBN / 64, std::is_same<OutT, __nv_bfloat16>::value, release)) {
+      if (!epilogue_tile<InT, kSym>(p, tile.batch, tile.tm * kBM, tile.tn * kBN, tmem_base + acc * uint32_t(kBN),
+                                    &acc_full[acc], acc_phase, abort_flag, stage, sub, lane, first_chunk, kBN / 64,
+                                    std::is_same<OutT, __nv_bfloat16>::value, release)) {
         ok = false;
         break;
       }

@@ -143,7 +143,8 @@ int dionw_normalize_pack(const void* src, int src_dtype, int64_t blocks, int64_t
                          int64_t ldx, float* sumsq, float* frob, void* stream);
 
 /* out[b, c, r] = in[b, r, c] for 2-byte elements (the transposed view of a batch,
- * src/dionw/_gram.py:83-84, :89, as a copy). */
+ * src/dionw/_gram.py:83-84, :89, as a copy).  For callers of this ABI: the package
+ * iterates tall blocks as they lie and does not call it. */
 int dionw_transpose_2byte(const void* in, void* out, int64_t blocks, int64_t rows,
                           int64_t cols, int64_t ld_in, int64_t ld_out, void* stream);
 
