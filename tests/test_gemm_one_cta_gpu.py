@@ -87,3 +87,46 @@ def test_one_cta_gemm_in_child_process(tmp_path):
     err = float((o.float() - theirs.float()).norm() / o.float().norm())
     # same arithmetic per product; only the order of fp32 accumulation inside a tile may differ
     assert err < 2e-3, err
+
+
+CHILD_TALL = r"""
+import sys, torch
+from dionw_b200 import _native as nat
+dev = "cuda"
+got = {}
+for kind, dtype in ((nat.NS_GRAM, torch.float16), (nat.NS_KELLER, torch.bfloat16)):
+    for rows, cols in ((700, 65), (1531, 517), (300, 256)):
+        gen = torch.Generator(dev).manual_seed(rows)
+        ld = (cols + 7) // 8 * 8
+        x = torch.zeros(3, rows, ld, dtype=dtype, device=dev)
+        values = torch.randn(3, rows, cols, device=dev, generator=gen)
+        x[..., :cols] = values / values.norm(dim=(1, 2), keepdim=True)
+        out = torch.empty(3, rows, ld, dtype=torch.bfloat16, device=dev)
+        rowsq = torch.empty(3 * rows, nat.newton_schulz_rowsq_parts(cols), device=dev)
+        ws = torch.empty(nat.newton_schulz_tall_workspace_bytes(3, rows, cols, kind), dtype=torch.uint8, device=dev)
+        nat.newton_schulz_tall(x, out, rows, cols, kind, ws, rowsq)
+        got[kind, rows, cols] = out[..., :cols].cpu(), rowsq.cpu()
+torch.cuda.synchronize()
+assert nat.device_status() == 0
+torch.save(got, sys.argv[1])
+"""
+
+
+def test_one_cta_gemm_iterates_tall_blocks(tmp_path):
+    """X^T X with both operands MN-major, X Q with Q K-major, and the row sums, against the default kernel."""
+    results = []
+    for pairs in ("0", "1"):
+        out_file = tmp_path / f"tall_{pairs}.pt"
+        env = dict(os.environ, DIONW_GEMM_CTA_PAIRS=pairs, PYTHONPATH=ROOT)
+        done = subprocess.run([sys.executable, "-c", CHILD_TALL, str(out_file)], env=env, capture_output=True,
+                              text=True, timeout=600, cwd=ROOT)
+        assert done.returncode == 0, done.stdout + done.stderr
+        results.append(torch.load(out_file))
+    for (kind, rows, cols), (out, rowsq) in results[0].items():
+        theirs, _ = results[1][kind, rows, cols]
+        err = float((out.float() - theirs.float()).norm() / theirs.float().norm())
+        # as above; the iterations in bf16 round 2^3 times as coarsely
+        assert err < (2e-3 if kind == 0 else 1.6e-2), (kind, rows, cols, err)
+        exact = out.double().square().sum(-1).flatten()
+        # at most 128 fp32 additions per part of 128 columns, the parts added in fp64 here: 2^-15 of a sum of squares
+        assert bool(((rowsq.double().sum(-1) - exact).abs() <= 2.0**-15 * exact + 1e-30).all())

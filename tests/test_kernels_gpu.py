@@ -113,6 +113,40 @@ def test_select_rows_breaks_ties_toward_lower_rows(native) -> None:
     assert expect[0].tolist() == [0, 1, 2, 3, 4, 5, 6, 7, 8, 17]
 
 
+@pytest.mark.parametrize("rows, k, above", [(9000, 4000, 700), (9000, 701, 700), (40001, 20000, 3), (40001, 40001, 9), (1025, 600, 0)])
+def test_select_rows_breaks_ties_across_the_ctas_of_a_block(native, rows, k, above) -> None:
+    """Two values, the lower one at the threshold and in the rows of every CTA of the cluster; 40001 rows are
+    more than the CTAs keep in registers."""
+    g = _gen(rows + k)
+    scores = torch.full((2, rows), 0.5)
+    scores.scatter_(1, torch.rand(2, rows, generator=g).topk(above).indices, 2.0)
+    sumsq = torch.rand(2, rows, generator=g)
+    expect = oracle.select_rows(scores, k)
+    index = torch.empty(2, k, dtype=torch.int32, device=DEV)
+    rowmap = torch.empty(2, rows, dtype=torch.int32, device=DEV)
+    frob = torch.empty(2, device=DEV)
+    native.select_rows(scores.to(DEV), sumsq.to(DEV), k, index, rowmap, frob)
+    assert torch.equal(index.cpu().long(), expect)
+    expect_map = torch.full((2, rows), -1, dtype=torch.int32)
+    expect_map.scatter_(1, expect, torch.arange(k, dtype=torch.int32).expand(2, k))
+    assert torch.equal(rowmap.cpu(), expect_map)
+    # at most 40 additions per thread, 10 in the block, 8 over the cluster: 58 * 2^-24 of the sum, half of that of
+    # its root, and the root's own rounding
+    torch.testing.assert_close(frob.double().cpu(), torch.gather(sumsq, 1, expect).double().sum(-1).sqrt(),
+                               rtol=60 * 2.0**-25, atol=0)
+
+
+def test_select_rows_of_more_rows_than_stay_in_registers(native) -> None:
+    g = _gen(12)
+    scores, sumsq = torch.rand(1, 50003, generator=g) + 0.5, torch.rand(1, 50003, generator=g)
+    expect = oracle.select_rows(scores, 12501)
+    index = torch.empty(1, 12501, dtype=torch.int32, device=DEV)
+    rowmap = torch.empty(1, 50003, dtype=torch.int32, device=DEV)
+    frob = torch.empty(1, device=DEV)
+    native.select_rows(scores.to(DEV), sumsq.to(DEV), 12501, index, rowmap, frob)
+    assert torch.equal(index.cpu().long(), expect)
+
+
 def test_pack_rows_decays_and_normalises(native) -> None:
     g = _gen(4)
     blocks, rows, k, cols = 2, 64, 16, 520

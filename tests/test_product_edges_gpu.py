@@ -98,7 +98,7 @@ def test_tall_blocks_equal_the_iteration_of_their_transpose(rows: int, cols: int
     native.newton_schulz(wide, wide.view(torch.bfloat16), cols, rows, kind, ws)
     got, want = tall.view(torch.bfloat16)[..., :cols], wide.view(torch.bfloat16)[..., :rows].mT
     assert torch.equal(got, want)
-    # at most 128 fp32 additions per part and two parts: 2^-15 of a sum of squares
+    # at most 128 fp32 additions per part of 128 columns (the parts are added in fp64 here): 2^-15 of a sum of squares
     exact = got.double().square().sum(-1).flatten()
     assert bool(((rowsq.double().sum(-1) - exact).abs() <= 2.0**-15 * exact + 1e-30).all())
 
