@@ -302,3 +302,17 @@ def test_a_step_in_groups_equals_a_step_run_by_run(update: str, monkeypatch: pyt
                                                            optimizer.state[p]["variance"])])
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m", [100, 128, 129, 384, 385, 640, 641])
+def test_symmetric_products_whose_last_narrow_tile_is_left_out(m: int) -> None:
+    """Up to 128 columns into its last tile row a product of 128-wide tiles has no tile for the rest of it;
+    one matrix and 300 of them, which take 128- and 256-wide tiles."""
+    gen = torch.Generator().manual_seed(m)
+    for blocks in (1, 300 if m <= 129 else 40):
+        a = _operand(gen, blocks, m, 72, torch.float16)
+        out = torch.full((blocks, m, _padded(m)), SENTINEL, dtype=torch.float16, device=DEV)
+        native.symmetric_product(a[..., :72], out[..., :m])
+        a64 = a[..., :72].double()
+        _close(out[..., :m], a64 @ a64.mT, a64.abs() @ a64.mT.abs(), torch.float16)
+        assert torch.equal(out[..., :m], out[..., :m].mT) and bool((out[..., m:] == SENTINEL).all())
