@@ -1,5 +1,7 @@
 // The Newton-Schulz product schedules: which products, in which order.  gemm.cu runs them, all of one
 // iteration as one launch.
+#include <algorithm>
+
 #include "products.cuh"
 
 namespace dionw {
@@ -203,6 +205,14 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
   }
 }
 
+// A batch of blocks up to this wide on their shorter side goes product by product.  A plan pays about 10 us at its
+// start (its counters are cleared, and it is launched without programmatic dependence) and a hop through ring and
+// progress per tile; it gets that back where other tiles fill the wait, and a product on one 64 x 64 tile per
+// matrix is over in 4 us.  Plan against one launch per product: 1 block of 64^2 92 against 74 us, 16 of
+// 64 x 1024 123 against 117, 1000 of 64^2 691 against 588; on wider blocks 1 of 192 x 768 126 against 123, 16 of
+// 192 x 768 132 against 134, 300 of 256^2 363 against 432.  (The batches of a group fill one another's waits.)
+constexpr int64_t kStepwiseSide = 64;
+
 size_t group_bytes(const Problem* problems, int n) {
   int64_t matrices = 0;
   size_t bytes = 0;
@@ -225,7 +235,8 @@ int iterate(const Problem* problems, int n, bool stepwise, void* workspace, size
   int64_t matrices = 0;
   for (int i = 0; i < n; ++i) matrices += problems[i].blocks;
   const size_t counter_bytes = align256(plan_counter_bytes(matrices));
-  void* counters = counter_bytes != 0 && !stepwise ? ws : nullptr;
+  const bool small = n == 1 && std::min(problems[0].rows, problems[0].cols) <= kStepwiseSide;
+  void* counters = counter_bytes != 0 && !stepwise && !small ? ws : nullptr;
   ws += counter_bytes;
   Product list[kMaxChains * kMaxChainProducts];
   int count = 0;

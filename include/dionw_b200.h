@@ -50,7 +50,8 @@ extern "C" {
 /* Added to the kind of dionw_newton_schulz or dionw_newton_schulz_tall: one launch per
  * product instead of one for the iteration, for a call that other streams' kernels
  * run beside -- they get SMs between two products, where one launch holds them all
- * until the iteration is done.  Same results. */
+ * until the iteration is done.  Same results.  (Blocks of up to 64 on their shorter
+ * side always take one launch per product: on those it is the faster.) */
 #define DIONW_NS_STEPWISE 256
 
 /* Text of the last error on the calling thread (copied, NUL-terminated). */

@@ -200,7 +200,7 @@ def test_a_group_of_batches_equals_its_members_alone(kinds: tuple[int, ...]) -> 
         native.newton_schulz_group(xs[:2], xs[:2], shapes[:2], [native.NS_GRAM, native.NS_KELLER], ws, [None, None])
 
 
-@pytest.mark.parametrize("blocks, rows, cols", [(4000, 40, 64), (1500, 64, 40), (700, 130, 257)])
+@pytest.mark.parametrize("blocks, rows, cols", [(4000, 66, 72), (1500, 72, 66), (700, 130, 257)])
 def test_a_plan_of_many_tiles_equals_its_products_alone(blocks: int, rows: int, cols: int) -> None:
     """Hundreds of tiles per SM pair, each shorter than the way of its index to the pair's consumers: an
     entry of the tile ring that is written before it has been read everywhere shows as a wrong tile."""
@@ -316,3 +316,24 @@ def test_symmetric_products_whose_last_narrow_tile_is_left_out(m: int) -> None:
         a64 = a[..., :72].double()
         _close(out[..., :m], a64 @ a64.mT, a64.abs() @ a64.mT.abs(), torch.float16)
         assert torch.equal(out[..., :m], out[..., :m].mT) and bool((out[..., m:] == SENTINEL).all())
+
+
+@pytest.mark.parametrize("rows, cols, launches", [(64, 256, 18), (300, 64, 18), (64, 64, 15), (65, 256, 1), (65, 65, 1)])
+def test_small_blocks_go_product_by_product(rows: int, cols: int, launches: int) -> None:
+    """A plan's start costs more than it saves on them; in a group they are part of the plan all the same."""
+    x = torch.zeros(2, rows, _padded(cols), dtype=torch.float16, device=DEV)
+    x[..., :cols] = torch.randn(2, rows, cols, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)) / 64
+    run = native.newton_schulz_tall if rows > cols else native.newton_schulz
+    need = native.newton_schulz_tall_workspace_bytes if rows > cols else native.newton_schulz_workspace_bytes
+    ws = torch.empty(need(2, rows, cols, native.NS_GRAM), dtype=torch.uint8, device=DEV)
+    out = torch.empty_like(x).view(torch.bfloat16)
+    before = native.launch_count()
+    run(x.clone(), out, rows, cols, native.NS_GRAM, ws)
+    assert native.launch_count() - before == launches
+    shapes, kinds = [(2, rows, cols)] * 2, [native.NS_GRAM] * 2
+    ws = torch.empty(native.newton_schulz_group_workspace_bytes(shapes, kinds), dtype=torch.uint8, device=DEV)
+    xs = [x.clone(), x.clone()]
+    before = native.launch_count()
+    native.newton_schulz_group(xs, [v.view(torch.bfloat16) for v in xs], shapes, kinds, ws, [None, None])
+    assert native.launch_count() - before == 1
+    assert all(torch.equal(v.view(torch.bfloat16)[..., :cols], out[..., :cols]) for v in xs)
