@@ -412,8 +412,14 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
       uint32_t it = 0;
       int at = 0;
       bool ok = true;
-      // The leader publishes tile n + 1 before it loads tile n, and draws tile n + 2 then: neither the
-      // draw nor the way through the ring lies between two tiles.
+      // The leader draws its next tile once what the current one reads is there, and publishes it after the
+      // current one's loads.  Not earlier: a pair that waits for a product's inputs would take two of its
+      // tiles while other pairs get none, and a product of 66 tiles on 74 pairs take two tiles' time (1 block
+      // of 2816 x 2927: 788 us so, 514 now, 512 to 570 as one launch per product; 2496^2, 15 products: 585,
+      // 437, 417).  On long main loops it draws after the loads, when six stages are still to be multiplied,
+      // and so it does for its first tile, which waits for nothing while other pairs may not have started.
+      // (On the products of small matrices neither the draw nor the ring shows: 12-layer 768-wide steps
+      // 1804 us with two tiles drawn ahead, 1809 with this.)
       auto publish = [&](uint32_t n, int t) -> bool {
         const uint32_t slot = n % kTileSlots;
         if (!mbar_wait_cluster(&tile_empty[slot], ((n / kTileSlots) & 1u) ^ 1u, abort_flag, plan.status, plan.wait_ns))
@@ -435,22 +441,13 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
       const bool leads = dynamic && rank == 0;
       auto draw = [&] { return atomicAdd(plan.tile_counter, 1); };
       auto valid = [&](int t) { return t < total_tiles ? t : -1; };
-      int current = -1, next = -1;
+      int current = -1;
       if (leads) {
         current = valid(draw());
-        if (current >= 0) next = draw();
         ok = publish(0, current);
       }
       for (uint32_t n = 0; ok; ++n) {
-        int t = current;
-        if (leads) {
-          if (t < 0) break;
-          current = valid(next);
-          if (!publish(n + 1, current)) break;
-          if (current >= 0) next = draw();
-        } else {
-          t = take_tile(n, false);
-        }
+        const int t = leads ? current : take_tile(n, false);
         if (t < 0) break;
         const Step& step = step_at(t, at);
         const Tile tile = tile_of(t - step.first_tile, step);
@@ -467,6 +464,9 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
         const int m0 = tile.tm * kPairM + int(rank) * kBM;
         const int n0 = tile.tn * step.tile_n + int(rank) * half_n;
         const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
+        const bool late = n == 0 || k_blocks >= 2 * kStages;
+        int next = -1;
+        if (leads && !late) next = draw();
         const uint32_t pair_bytes = 2 * (kABytes + uint32_t(half_n) * kBK * 2);
         // The layout of the operands is a constant inside the loop.
         auto load_loop = [&](auto a_major_mn, auto b_major_mn) {
@@ -500,6 +500,11 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
         if (step.a_major_mn) load_loop(std::true_type(), std::true_type());
         else if (step.b_major_mn) load_loop(std::false_type(), std::true_type());
         else load_loop(std::false_type(), std::false_type());
+        if (leads && ok) {
+          if (late) next = draw();
+          current = valid(next);
+          ok = publish(n + 1, current);
+        }
       }
     }
   } else if (warp == 1) {
