@@ -63,8 +63,9 @@ constexpr int kBK = 64;
 constexpr int kStages = 6;
 constexpr int kEpilogueWarps = 8;
 constexpr int kReporterWarp = 2 + kEpilogueWarps;
-constexpr int kThreads = 32 * (kReporterWarp + 1);
-constexpr uint32_t kBarrierBytes = 512;
+constexpr int kSchedulerWarp = kReporterWarp + 1;
+constexpr int kThreads = 32 * (kSchedulerWarp + 1);
+constexpr uint32_t kBarrierBytes = 640;
 constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
 constexpr uint32_t kBBytes = (kBN / 2) * kBK * 2;  // 16 KB: the half of B's columns that each CTA loads
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
@@ -76,26 +77,35 @@ __device__ __forceinline__ void remote_arrive(uint32_t cluster_address) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 
-// Arrive with release semantics at cluster scope: what this thread wrote before (its own or the
-// peer's shared memory) is visible to a thread of either CTA that then observes the phase with an
-// acquire at cluster scope.  Used once per tile (the tile hand-out), never per stage.
-__device__ __forceinline__ void remote_arrive_release(uint32_t cluster_address) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
-}
-
 // Relaxed arrive that is issued once `loaded`, the result of a load, is there: the arrive is predicated on the
 // value, which is never kNoTile.  (Relaxed, so the memory model does not order the load before it; the
 // dependency does, since an instruction is not issued before its predicate is known.  The comparison is with
-// the largest integer because no branch on the sign of a tile's index decides it.)
-constexpr int kNoTile = 0x7FFFFFFF;   // a plan has fewer than 2^31 tiles
+// the largest integer because no branch on the sign of an entry's step decides it.)
+constexpr int kNoTile = 0x7FFFFFFF;   // no step has this number
 __device__ __forceinline__ void remote_arrive_after(uint32_t cluster_address, int loaded) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %1, %2;\n"
                "@p mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}\n"
                ::"r"(cluster_address), "r"(loaded), "n"(kNoTile) : "memory");
 }
 
-__device__ __forceinline__ void remote_store_s32(uint32_t cluster_address, int value) {
-  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cluster_address), "r"(value) : "memory");
+// An entry of the tile ring: the product of the plan (negative: no more tiles) and the tile of it.
+struct alignas(16) Entry {
+  int step, batch, tm, tn;
+};
+
+// Stores an entry in the peer's shared memory and counts its bytes on a barrier there, which releases it: the
+// sender waits for nothing.  (A store and an arrive with release at cluster scope took the sender 1700 cycles.)
+__device__ __forceinline__ void send_entry(uint32_t cluster_address, uint32_t cluster_bar, const Entry& e) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(cluster_address), "r"(e.step), "r"(e.batch), "r"(e.tm), "r"(e.tn), "r"(cluster_bar) : "memory");
+}
+
+// One instruction: what depends on one field of the entry depends on all of them.
+__device__ __forceinline__ Entry load_entry(const Entry* from) {
+  Entry e;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(e.step), "=r"(e.batch), "=r"(e.tm), "=r"(e.tn) : "r"(gemm::smem_u32(from)) : "memory");
+  return e;
 }
 
 __device__ __forceinline__ bool mbar_try_cluster(uint64_t* bar, uint32_t parity) {
@@ -296,20 +306,29 @@ __device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned
 // CTAs become resident late, or not before the others are done, simply takes fewer tiles, where the
 // fixed stride makes the whole product wait for it.
 //
-// The leader CTA's producer thread draws the index and publishes it to every consumer of the pair
-// through a ring of kTileSlots entries kept in BOTH CTAs' shared memory: it writes the entry (its own
-// copy and, through the cluster's shared-memory window, the peer's), then arrives with release at
-// cluster scope on the slot's `tile_full` barrier of each CTA.  Consumers -- the leader's MMA thread,
-// the peer's producer thread and the epilogue warps of each CTA -- wait on their own
+// A warp of its own in each CTA, the scheduler, does the hand-out, ahead of the loads.  The leader's draws the
+// index, finds the product and the tile that it stands for, and publishes them to every consumer of the pair
+// through a ring of kTileSlots entries kept in BOTH CTAs' shared memory: it writes its own copy and arrives on
+// the slot's `tile_full` barrier, and sends the peer's, where the bytes themselves complete the phase that the
+// peer's scheduler has armed.  Consumers -- the leader's MMA thread, the producer thread and the epilogue warps
+// of each CTA, the peer's scheduler -- wait on their own
 // CTA's `tile_full` (acquire at cluster scope), read the entry and arrive on the LEADER's `tile_empty`
-// barrier of the slot; the producer reuses a slot after all of them have done so.  -1 ends the pair's work.
-// When a pair has drawn its -1 it adds one to a second counter; the pair that brings that to the number
+// barrier of the slot; the scheduler reuses a slot after all of them have done so.  A negative step ends the pair's work.
+// When a pair has drawn its end it adds one to a second counter; the pair that brings that to the number
 // of pairs knows that nobody will draw again and clears both counters for the next launch on the stream.
-// In a plan of several products each CTA's producer then waits for what the tile depends on, and tells its
-// own CTA's epilogue warps, which read Cin, through the slot's `ready` barrier.  (Waiting before the tile is
+// In a plan of several products each CTA's scheduler then waits for what the tile depends on, and tells its
+// own CTA's producer and its epilogue warps, which read Cin, through the slot's `ready` barrier.  (Waiting before the tile is
 // published, so that the ring itself carries the news, put the ring's two cluster-scope hops on the path
-// from one product to the next.)  An epilogue warp reports the slot as read after it has seen `ready`, so
+// from one product to the next.)  Who waits for `ready` reports the slot as read only then, so
 // that the barrier is never more than one phase ahead of it.
+//
+// When the leader draws its next tile: once what the current one reads is there, and not before the current
+// one's loads are within kDrawAhead k-blocks of their end (its first tile, which waits for nothing while other
+// pairs may not have started: at their end).  Earlier, a pair that waits for a product's inputs would take two of
+// its tiles while other pairs get none, and a product of 66 tiles on 74 pairs take two tiles' time (1 block of
+// 2816 x 2927: 788 us so, 514 without).  Later, the way from the draw to the first load is not hidden behind the
+// current tile: when the producer itself drew, decoded, published, waited and loaded in turn, the tensor pipe had
+// nothing to do for 4500 of the 15000 cycles of a 1024-deep tile.
 //
 // A CTA's half of a tile is reported by a warp of its own, once the eight epilogue warps have arrived on the
 // slot's `stored` barrier: the release at GPU scope waits until the stores have reached L2, and took an
@@ -318,7 +337,8 @@ __device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned
 // their predicate depends on, and not the stores of the tile before (as a release at cluster scope each cost
 // the warp 2000 cycles per tile).
 constexpr int kTileSlots = 8;
-constexpr uint32_t kTileConsumers = 2 * (1 + kEpilogueWarps);   // and the reporters, in a plan of several products
+constexpr uint32_t kTileConsumers = 2 + 2 * (1 + kEpilogueWarps);   // and the reporters, in a plan of several products
+constexpr int kDrawAhead = 24;
 
 // ----------------------------------------------------------------------------
 // the kernel (launched as clusters of two CTAs)
@@ -337,8 +357,9 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   uint64_t* tile_empty = tile_full + kTileSlots;  // [kTileSlots] leader only: every consumer has read the slot
   uint64_t* ready = tile_empty + kTileSlots;      // [kTileSlots] both: what the slot's tile reads is there
   uint64_t* stored = ready + kTileSlots;          // [kTileSlots] both: this CTA's half of the slot's tile is stored
-  int* tile_ring = reinterpret_cast<int*>(stored + kTileSlots);  // [kTileSlots]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tile_ring + kTileSlots);
+  Entry* tile_ring = reinterpret_cast<Entry*>(stored + kTileSlots);  // [kTileSlots] both
+  uint64_t* may_draw = reinterpret_cast<uint64_t*>(tile_ring + kTileSlots);   // leader's: its scheduler may draw again
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(may_draw + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* mirror_stage = smem + size_t(kStages) * kStageBytes + kBarrierBytes;
 
@@ -348,7 +369,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   const int pair = blockIdx.x >> 1;
   const int pairs = gridDim.x >> 1;
   const int total_tiles = plan.total_tiles;
-  const bool dynamic = plan.tile_counter != nullptr;
+  const bool dynamic = kSteps > 1 || plan.tile_counter != nullptr;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -365,6 +386,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
       mbar_init(&ready[s], 1);
       mbar_init(&stored[s], kEpilogueWarps);
     }
+    mbar_init(may_draw, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -379,94 +401,43 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   gemm::griddep_wait();     // set-up above overlaps the tail of the previous product; global memory from here on
   gemm::griddep_launch();
 
-  // The product that tile t belongs to; each role keeps its own position, and its tiles only ever grow.
-  auto step_at = [&](int t, int& at) -> const Step& {
-    if constexpr (kSteps > 1) {
-      while (at + 1 < plan.count && t >= plan.steps[at + 1].first_tile) ++at;
-    }
-    return plan.steps[at];
-  };
-
-  // The n-th tile of this pair for a consumer: its index, -1 when the pair is done, -2 when the wait
+  // The n-th tile of this pair for a consumer; its step is -1 when the pair is done and -2 when the wait
   // gave up.  Called by ONE thread per consumer (the single-thread roles themselves, lane 0 of an
   // epilogue warp), which also reports the slot as read.
   const uint32_t leader_tile_empty = peer_address(&tile_empty[0], 0);
-  auto take_tile = [&](uint32_t n, bool when_ready) -> int {
+  auto take_tile = [&](uint32_t n, bool when_ready) -> Entry {
     if (!dynamic) {
       const long long t = (long long)pair + (long long)n * pairs;
-      return t < total_tiles ? int(t) : -1;
+      if (t >= total_tiles) return Entry{-1, 0, 0, 0};
+      const Tile tile = tile_of(int(t), plan.steps[0]);
+      return Entry{0, tile.batch, tile.tm, tile.tn};
     }
-    const uint32_t slot = n % kTileSlots;
-    if (!mbar_wait_cluster(&tile_full[slot], (n / kTileSlots) & 1u, abort_flag, plan.status, plan.wait_ns)) return -2;
-    const int t = tile_ring[slot];
-    if (kSteps > 1 && when_ready && t >= 0 &&
-        !mbar_wait(&ready[slot], (n / kTileSlots) & 1u, abort_flag, plan.status, plan.wait_ns))
-      return -2;
-    remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), t);
-    return t;
+    const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
+    if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) return Entry{-2, 0, 0, 0};
+    const Entry e = load_entry(&tile_ring[slot]);
+    if (kSteps > 1 && when_ready && e.step >= 0 && !mbar_wait(&ready[slot], phase, abort_flag, plan.status, plan.wait_ns))
+      return Entry{-2, 0, 0, 0};
+    remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), e.step);
+    return e;
   };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
       uint32_t it = 0;
-      int at = 0;
       bool ok = true;
-      // The leader draws its next tile once what the current one reads is there, and publishes it after the
-      // current one's loads.  Not earlier: a pair that waits for a product's inputs would take two of its
-      // tiles while other pairs get none, and a product of 66 tiles on 74 pairs take two tiles' time (1 block
-      // of 2816 x 2927: 788 us so, 514 now, 512 to 570 as one launch per product; 2496^2, 15 products: 585,
-      // 437, 417).  On long main loops it draws after the loads, when six stages are still to be multiplied,
-      // and so it does for its first tile, which waits for nothing while other pairs may not have started.
-      // (On the products of small matrices neither the draw nor the ring shows: 12-layer 768-wide steps
-      // 1804 us with two tiles drawn ahead, 1809 with this.)
-      auto publish = [&](uint32_t n, int t) -> bool {
-        const uint32_t slot = n % kTileSlots;
-        if (!mbar_wait_cluster(&tile_empty[slot], ((n / kTileSlots) & 1u) ^ 1u, abort_flag, plan.status, plan.wait_ns))
-          return false;
-        tile_ring[slot] = t;
-        remote_store_s32(peer_address(&tile_ring[slot], 1), t);
-        remote_arrive_release(peer_address(&tile_full[slot], 0));
-        remote_arrive_release(peer_address(&tile_full[slot], 1));
-        if (t < 0) {
-          // nobody of this pair draws again; the last pair to get here clears the counters
-          if (atomicAdd(plan.tile_counter + 1, 1) == pairs - 1) {
-            plan.tile_counter[0] = 0;
-            plan.tile_counter[1] = 0;
-            __threadfence();
-          }
-        }
-        return true;
-      };
-      const bool leads = dynamic && rank == 0;
-      auto draw = [&] { return atomicAdd(plan.tile_counter, 1); };
-      auto valid = [&](int t) { return t < total_tiles ? t : -1; };
-      int current = -1;
-      if (leads) {
-        current = valid(draw());
-        ok = publish(0, current);
-      }
       for (uint32_t n = 0; ok; ++n) {
-        const int t = leads ? current : take_tile(n, false);
-        if (t < 0) break;
-        const Step& step = step_at(t, at);
-        const Tile tile = tile_of(t - step.first_tile, step);
-        if constexpr (kSteps > 1) {
-          if (step.need != 0) {
-            if (!progress_wait(&step.progress[tile.batch], step.need, abort_flag, plan.status, plan.wait_ns)) break;
-            proxy_fence();   // what the tile reads was stored through the generic proxy, by other SMs
-          }
-          mbar_arrive(&ready[n % kTileSlots]);
-        }
+        const Entry tile = take_tile(n, true);
+        if (tile.step < 0) break;
+        const Step& step = plan.steps[tile.step];
         const CUtensorMap* map_a = &plan.maps[step.map_a];
         const CUtensorMap* map_b = &plan.maps[step.map_b];
         const int half_n = step.tile_n / 2;
         const int m0 = tile.tm * kPairM + int(rank) * kBM;
         const int n0 = tile.tn * step.tile_n + int(rank) * half_n;
         const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
-        const bool late = n == 0 || k_blocks >= 2 * kStages;
-        int next = -1;
-        if (leads && !late) next = draw();
+        // the k-block after whose loads this pair's next tile may be drawn
+        const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? k_blocks - 1 : max(0, k_blocks - kDrawAhead);
         const uint32_t pair_bytes = 2 * (kABytes + uint32_t(half_n) * kBK * 2);
         // The layout of the operands is a constant inside the loop.
         auto load_loop = [&](auto a_major_mn, auto b_major_mn) {
@@ -495,16 +466,12 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
             } else {
               tma_load_3d_pair(b_dst, map_b, leader_full, k0, n0, tile.batch);
             }
+            if (kb == draw_at) mbar_arrive(may_draw);
           }
         };
         if (step.a_major_mn) load_loop(std::true_type(), std::true_type());
         else if (step.b_major_mn) load_loop(std::false_type(), std::true_type());
         else load_loop(std::false_type(), std::false_type());
-        if (leads && ok) {
-          if (late) next = draw();
-          current = valid(next);
-          ok = publish(n + 1, current);
-        }
       }
     }
   } else if (warp == 1) {
@@ -513,12 +480,11 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
     } else if (lane == 0) {
       // ------------------------------------------------------------ MMA issuer (leader)
       uint32_t it = 0;
-      int at = 0;
       bool ok = true;
       for (uint32_t local = 0; ok; ++local) {
-        const int t = take_tile(local, false);
-        if (t < 0) break;
-        const Step& step = step_at(t, at);
+        const Entry tile = take_tile(local, false);
+        if (tile.step < 0) break;
+        const Step& step = plan.steps[tile.step];
         const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
         const int tile_n = step.tile_n;
         const uint32_t acc = local & 1u;
@@ -557,19 +523,67 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   } else if (warp == kReporterWarp) {
     // ------------------------------------------------------------ reporter (both CTAs)
     if (kSteps > 1 && lane == 0) {
-      int at = 0;
       for (uint32_t n = 0;; ++n) {
         const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
         if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
-        const int t = tile_ring[slot];
-        if (t < 0) break;
-        const Step& step = step_at(t, at);
-        unsigned* progress = &step.progress[(t - step.first_tile) / step.p.tiles_per_batch];
+        const Entry tile = load_entry(&tile_ring[slot]);
+        if (tile.step < 0) break;
+        unsigned* progress = &plan.steps[tile.step].progress[tile.batch];
         if (!mbar_wait(&stored[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
         // The tile's stores are there for later tiles once it is counted (their producers order the
         // proxies: the stores went through the generic one, TMA reads through the async one).
         add_release(progress, 1u);
-        remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), t);
+        remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), tile.step);
+      }
+    }
+  } else if (warp == kSchedulerWarp) {
+    // ------------------------------------------------------------ scheduler (both CTAs)
+    if (dynamic && lane == 0) {
+      if (rank != 0) mbar_expect_tx(&tile_full[0], sizeof(Entry));
+      int at = 0;   // the product of the last tile drawn: tiles only ever grow
+      for (uint32_t n = 0;; ++n) {
+        const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
+        Entry e;
+        if (rank == 0) {
+          if (n != 0 && !mbar_wait(may_draw, (n - 1) & 1u, abort_flag, plan.status, plan.wait_ns)) break;
+          const int t = atomicAdd(plan.tile_counter, 1);
+          if (t < total_tiles) {
+            if constexpr (kSteps > 1) {
+              while (at + 1 < plan.count && t >= plan.steps[at + 1].first_tile) ++at;
+            }
+            const Tile tile = tile_of(t - plan.steps[at].first_tile, plan.steps[at]);
+            e = Entry{at, tile.batch, tile.tm, tile.tn};
+          } else {
+            e = Entry{-1, 0, 0, 0};
+          }
+          if (!mbar_wait_cluster(&tile_empty[slot], phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) break;
+          send_entry(peer_address(&tile_ring[slot], 1), peer_address(&tile_full[slot], 1), e);
+          tile_ring[slot] = e;
+          mbar_arrive(&tile_full[slot]);
+          if (e.step < 0) {
+            // nobody of this pair draws again; the last pair to get here clears the counters
+            if (atomicAdd(plan.tile_counter + 1, 1) == pairs - 1) {
+              plan.tile_counter[0] = 0;
+              plan.tile_counter[1] = 0;
+              __threadfence();
+            }
+            break;
+          }
+        } else {
+          if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
+          e = load_entry(&tile_ring[slot]);
+          remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), e.step);
+          if (e.step < 0) break;
+          mbar_expect_tx(&tile_full[(n + 1) % kTileSlots], sizeof(Entry));   // its last phase is over: this thread has seen it
+        }
+        if constexpr (kSteps > 1) {
+          const Step& step = plan.steps[e.step];
+          if (step.need != 0) {
+            if (!progress_wait(&step.progress[e.batch], step.need, abort_flag, plan.status, plan.wait_ns)) break;
+            proxy_fence();   // what the tile reads was stored through the generic proxy, by other SMs
+          }
+          mbar_arrive(&ready[slot]);
+        }
       }
     }
   } else {
@@ -578,16 +592,17 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
     const int sub = warp & 3;
     uint8_t* stage = mirror_stage + ew * 2 * kPieceBytes;
     const uint32_t leader_empty[2] = {peer_address(&acc_empty[0], 0), peer_address(&acc_empty[1], 0)};
-    int at = 0;
     for (uint32_t local = 0;; ++local) {
-      int t = 0;
-      if (lane == 0) t = take_tile(local, true);   // one lane waits, reads and reports; the warp follows it
-      t = __shfl_sync(0xffffffffu, t, 0);
+      Entry tile{};
+      if (lane == 0) tile = take_tile(local, true);   // one lane waits, reads and reports; the warp follows it
+      tile.step = __shfl_sync(0xffffffffu, tile.step, 0);
+      tile.batch = __shfl_sync(0xffffffffu, tile.batch, 0);
+      tile.tm = __shfl_sync(0xffffffffu, tile.tm, 0);
+      tile.tn = __shfl_sync(0xffffffffu, tile.tn, 0);
       __syncwarp();   // the other lanes read Cin too, which lane 0's wait alone has acquired: a shuffle orders no memory
-      if (t < 0) break;
-      const Step& step = step_at(t, at);
+      if (tile.step < 0) break;
+      const Step& step = plan.steps[tile.step];
       const Params& p = step.p;
-      const Tile tile = tile_of(t - step.first_tile, step);
       const int chunks = step.tile_n / (32 * kEpilogueWarps / 4);
       const int first_chunk = (ew >> 2) * chunks;
       const uint32_t acc = local & 1u;
