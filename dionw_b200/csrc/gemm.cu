@@ -220,6 +220,7 @@ gemm::Params params_of(const Product& product) {
   p.kdim = int(product.k);
   p.batches = int(product.blocks);
   p.mirror_diagonal = product.same_operands ? 0 : 1;
+  p.lower_only = 0;
   p.rowsq = product.rowsq;
   p.rowsq_parts = int(2 * ((product.n + gemm::kBN - 1) / gemm::kBN));
   p.status = device_status_word();
@@ -316,12 +317,12 @@ int run_plan(const Product* const* products, int count, int dtype, unsigned* cou
     gemm2::Step& step = plan.steps[i];
     // One map serves an operand in several products: the dimensions are those of memory, and boxes of 64
     // rows suit both an MN-major operand and the half of B that a CTA loads of a 128-wide tile.
-    auto map_of = [&](const Operand& x, bool mn, int64_t outer, uint32_t box, int* index) {
+    auto map_of = [&](const Operand& x, bool mn, int64_t outer, uint32_t box, short* index) {
       const int64_t inner = mn ? outer : product.k, rows = mn ? product.k : outer;
       for (int j = 0; j < maps; ++j)
         if (mapped[j].x.base == x.base && mapped[j].x.ld == x.ld && mapped[j].x.batch == x.batch &&
             mapped[j].inner == inner && mapped[j].rows == rows && mapped[j].box == box) {
-          *index = j;
+          *index = short(j);
           return int(DIONW_OK);
         }
       if (maps == kMaps) {
@@ -331,7 +332,7 @@ int run_plan(const Product* const* products, int count, int dtype, unsigned* cou
       const int st = operand_map(&plan.maps[maps], x, dtype, mn, outer, product.k, blocks, box);
       if (st != DIONW_OK) return st;
       mapped[maps] = {x, inner, rows, box};
-      *index = maps++;
+      *index = short(maps++);
       return int(DIONW_OK);
     };
     step.tile_n = short(tile_width(product, together));
@@ -339,13 +340,24 @@ int run_plan(const Product* const* products, int count, int dtype, unsigned* cou
     if (st != DIONW_OK) return st;
     st = map_of(product.b, product.b_mn, product.n, product.b_mn ? 64 : step.tile_n / 2, &step.map_b);
     if (st != DIONW_OK) return st;
+    if (product.a_lower) st = map_of(product.a, true, product.m, 64, &step.map_a_t);
+    if (st != DIONW_OK) return st;
+    if (product.b_lower) st = map_of(product.b, true, product.n, 64, &step.map_b_t);
+    if (st != DIONW_OK) return st;
+    DIONW_REQUIRE((!product.a_lower || (!product.a_mn && product.m == product.k)) &&
+                      (!product.b_lower || (!product.b_mn && product.n == product.k)),
+                  "a lower operand is square and read in rows");
     step.p = params_of(product);
+    step.p.lower_only = product.out_lower ? 1 : 0;
     step.p.tiles_m = (step.p.m + gemm2::kPairM - 1) / gemm2::kPairM;
     step.p.tiles_n = (step.p.n + step.tile_n - 1) / step.tile_n;
     step.p.tiles_per_batch = product.symmetric ? symmetric_tiles(product.n, step.tile_n) : step.p.tiles_m * step.p.tiles_n;
     step.symmetric = product.symmetric;
     step.a_major_mn = product.a_mn;
     step.b_major_mn = product.b_mn;
+    step.a_lower = product.a_lower;
+    step.b_lower = product.b_lower;
+    step.same_operands = product.symmetric && product.same_operands;
     step.out_bf16 = product.out_dtype == DIONW_BF16;
     if (!product.beside_previous) need[product.chain] = done[product.chain];
     done[product.chain] += uint64_t(step.p.tiles_per_batch) * gemm2::kReportsPerTile;
@@ -409,8 +421,8 @@ int run_products(const Product* products, int count, int dtype, void* counters, 
   for (int i = 0; i < count; ++i) {
     int st;
     if (!use_cta_pairs()) st = run_one_cta(products[i], dtype, stream);
-    else if (f16) st = run_plan<__half, 2, 1>(ordered + i, 1, dtype, nullptr, stream);
-    else st = run_plan<__nv_bfloat16, 2, 1>(ordered + i, 1, dtype, nullptr, stream);
+    else if (f16) st = run_plan<__half, 4, 1>(ordered + i, 1, dtype, nullptr, stream);
+    else st = run_plan<__nv_bfloat16, 4, 1>(ordered + i, 1, dtype, nullptr, stream);
     if (st != DIONW_OK) return st;
   }
   return DIONW_OK;

@@ -204,13 +204,16 @@ __device__ __forceinline__ uint32_t make_idesc2(bool a_major_mn, bool b_major_mn
 // ----------------------------------------------------------------------------
 struct Step {
   Params p;               // tiles_m, tiles_n, tiles_per_batch count tiles of 256 x tile_n
-  int map_a, map_b;       // indices into the plan's maps
+  short map_a, map_b;     // indices into the plan's maps
+  short map_a_t, map_b_t; // of a lower operand: the map for the blocks that are read transposed
   int first_tile;         // tiles of the plan before this product
   unsigned need;          // progress of a matrix from which on this product may read it
   unsigned* progress;     // of the chain's matrices: zero at the start of the launch (null: one product only)
   short tile_n;           // 256 or 128
   bool symmetric;         // only tiles on and below the diagonal
   bool a_major_mn, b_major_mn;
+  bool a_lower, b_lower;  // the operand is a symmetric matrix of which only the 256 x 256 blocks up to the diagonal are stored
+  bool same_operands;     // a tile on the diagonal has the same rows of A and of B
   bool out_bf16;          // the result is bf16 although the operands are fp16
 };
 
@@ -263,6 +266,27 @@ __device__ __forceinline__ Tile sym_tile(int t, const Params& p, int per_row) {
 
 __device__ __forceinline__ Tile tile_of(int t, const Step& step) {
   return step.symmetric ? gemm2::sym_tile(t, step.p, kBN / step.tile_n) : gemm2::general_tile(t, step.p);
+}
+
+// How a tile's k-blocks are read: A in rows (K-major) up to a_end and B up to b_end, and in columns (MN-major)
+// from there on.  Of a symmetric matrix that a product of the plan left, only the 256 x 256 blocks up to the
+// diagonal exist: what lies right of the diagonal in a row is read from the column it is equal to.  The tensor
+// cores take either order, so nothing is stored twice: a mirrored copy was half of all bytes the products wrote,
+// and the write path, at 20 to 25 bytes per cycle and SM, what their epilogues waited for (1300 to 2900 of 2500 to
+// 4600 cycles per 32-column chunk).
+struct Ranges {
+  int k_blocks, a_end, b_end;   // b_end <= a_end in every product there is
+  bool shared;                  // A's rows serve as B's
+};
+__device__ __forceinline__ Ranges ranges_of(const Step& step, int tm, int tn) {
+  constexpr int kPerBlock = kPairM / kBK;
+  Ranges r;
+  r.k_blocks = (step.p.kdim + kBK - 1) / kBK;
+  const int column_block = step.tile_n == kBN ? tn : tn >> 1;
+  r.a_end = step.a_major_mn ? 0 : step.a_lower ? min(r.k_blocks, (tm + 1) * kPerBlock) : r.k_blocks;
+  r.b_end = step.b_major_mn ? 0 : step.b_lower ? min(r.k_blocks, (column_block + 1) * kPerBlock) : r.k_blocks;
+  r.shared = step.same_operands && step.tile_n == kBN && tm == tn;
+  return r;
 }
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
@@ -430,18 +454,20 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
         const Entry tile = take_tile(n, true);
         if (tile.step < 0) break;
         const Step& step = plan.steps[tile.step];
-        const CUtensorMap* map_a = &plan.maps[step.map_a];
-        const CUtensorMap* map_b = &plan.maps[step.map_b];
+        const Ranges range = ranges_of(step, tile.tm, tile.tn);
         const int half_n = step.tile_n / 2;
         const int m0 = tile.tm * kPairM + int(rank) * kBM;
         const int n0 = tile.tn * step.tile_n + int(rank) * half_n;
-        const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
         // the k-block after whose loads this pair's next tile may be drawn
-        const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? k_blocks - 1 : max(0, k_blocks - kDrawAhead);
-        const uint32_t pair_bytes = 2 * (kABytes + uint32_t(half_n) * kBK * 2);
+        const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? range.k_blocks - 1 : max(0, range.k_blocks - kDrawAhead);
+        const uint32_t pair_bytes = 2 * (kABytes + (range.shared ? 0u : uint32_t(half_n) * kBK * 2));
         // The layout of the operands is a constant inside the loop.
-        auto load_loop = [&](auto a_major_mn, auto b_major_mn) {
-          for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        auto load_loop = [&](int begin, int end, auto a_major_mn, auto b_major_mn) {
+          constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
+          if (!ok || begin >= end) return;
+          const CUtensorMap* map_a = &plan.maps[kAMN && step.a_lower ? step.map_a_t : step.map_a];
+          const CUtensorMap* map_b = &plan.maps[kBMN && step.b_lower ? step.map_b_t : step.map_b];
+          for (int kb = begin; kb < end; ++kb, ++it) {
             const int s = it % kStages;
             const uint32_t phase = (it / kStages) & 1u;
             if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
@@ -453,25 +479,27 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
             // because its empty barrier is released by the MMAs that consumed this one.
             if (rank == 0) mbar_expect_tx(&full_bar[s], pair_bytes);
             const int k0 = kb * kBK;
-            if constexpr (decltype(a_major_mn)::value) {
+            if constexpr (kAMN) {
 #pragma unroll
               for (int panel = 0; panel < kBM / 64; ++panel)
                 tma_load_3d_pair(a_dst + panel * kPanelBytes, map_a, leader_full, m0 + panel * 64, k0, tile.batch);
             } else {
               tma_load_3d_pair(a_dst, map_a, leader_full, k0, m0, tile.batch);
             }
-            if constexpr (decltype(b_major_mn)::value) {
-              tma_load_3d_pair(b_dst, map_b, leader_full, n0, k0, tile.batch);
-              if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, leader_full, n0 + 64, k0, tile.batch);
-            } else {
-              tma_load_3d_pair(b_dst, map_b, leader_full, k0, n0, tile.batch);
+            if (!range.shared) {
+              if constexpr (kBMN) {
+                tma_load_3d_pair(b_dst, map_b, leader_full, n0, k0, tile.batch);
+                if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, leader_full, n0 + 64, k0, tile.batch);
+              } else {
+                tma_load_3d_pair(b_dst, map_b, leader_full, k0, n0, tile.batch);
+              }
             }
             if (kb == draw_at) mbar_arrive(may_draw);
           }
         };
-        if (step.a_major_mn) load_loop(std::true_type(), std::true_type());
-        else if (step.b_major_mn) load_loop(std::false_type(), std::true_type());
-        else load_loop(std::false_type(), std::false_type());
+        load_loop(0, range.b_end, std::false_type(), std::false_type());
+        load_loop(range.b_end, range.a_end, std::false_type(), std::true_type());
+        load_loop(range.a_end, range.k_blocks, std::true_type(), std::true_type());
       }
     }
   } else if (warp == 1) {
@@ -485,24 +513,25 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
         const Entry tile = take_tile(local, false);
         if (tile.step < 0) break;
         const Step& step = plan.steps[tile.step];
-        const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
-        const int tile_n = step.tile_n;
+        const Ranges range = ranges_of(step, tile.tm, tile.tn);
         const uint32_t acc = local & 1u;
         const uint32_t acc_phase = (local >> 1) & 1u;
         if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * uint32_t(kBN);
+        const uint32_t b_offset = range.shared ? 0u : kABytes;
         // The layout of the operands is a constant inside the loop.
-        auto main_loop = [&](auto a_major_mn, auto b_major_mn) {
+        auto main_loop = [&](int begin, int end, auto a_major_mn, auto b_major_mn) {
           constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
-          const uint32_t idesc = make_idesc2<InT>(kAMN, kBMN, tile_n);
-          for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          if (!ok) return;
+          const uint32_t idesc = make_idesc2<InT>(kAMN, kBMN, step.tile_n);
+          for (int kb = begin; kb < end; ++kb, ++it) {
             const int s = it % kStages;
             const uint32_t phase = (it / kStages) & 1u;
             if (!mbar_wait(&full_bar[s], phase, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
             tc_fence_after();
             const uint32_t a_addr = smem_u32(smem + size_t(s) * kStageBytes);
-            const uint32_t b_addr = a_addr + kABytes;
+            const uint32_t b_addr = a_addr + b_offset;
             const uint64_t a_desc = make_smem_desc(a_addr, kAMN ? kPanelBytes : 16, 1024);
             const uint64_t b_desc = make_smem_desc(b_addr, kBMN ? kPanelBytes : 16, 1024);
 #pragma unroll
@@ -514,9 +543,9 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
             umma2_commit_both(&empty_bar[s]);
           }
         };
-        if (step.a_major_mn) main_loop(std::true_type(), std::true_type());
-        else if (step.b_major_mn) main_loop(std::false_type(), std::true_type());
-        else main_loop(std::false_type(), std::false_type());
+        main_loop(0, range.b_end, std::false_type(), std::false_type());
+        main_loop(range.b_end, range.a_end, std::false_type(), std::true_type());
+        main_loop(range.a_end, range.k_blocks, std::true_type(), std::true_type());
         if (ok) umma2_commit_both(&acc_full[acc]);
       }
     }

@@ -55,6 +55,7 @@ struct Params {
   int batches;
   int tiles_m, tiles_n, tiles_per_batch;
   int mirror_diagonal;   // symmetric schedule with B != A: also mirror inside the diagonal sub-blocks
+  int lower_only;        // symmetric schedule: no mirror image outside the 256 x 256 blocks on the diagonal
   float* rowsq;          // nullable, general products only: [batches, m, rowsq_parts] partial row sums of out^2
   int rowsq_parts;       // = 2 * tiles_n: one partial per 128 columns, written once each, summed by the reader
   int* status;           // device status word (may be null: the code is then not recorded)
@@ -354,13 +355,14 @@ __device__ __forceinline__ bool epilogue_tile(const Params& p, int batch, int m_
   const float alpha = p.alpha, beta = p.beta, diag = p.diag;
   const int row0 = m_base + sub * 32;
   // Class of the 32 x 32 piece at (row0, col0) under the symmetric schedule:
-  // 0 stored as it is; 1 strictly below the diagonal: stored and stored transposed;
+  // 0 stored as it is (also below the diagonal, outside of its 256 x 256 blocks, where readers want no mirror
+  // image); 1 strictly below the diagonal: stored and stored transposed;
   // 2 strictly above: skipped (its mirror image writes it); 3 on the diagonal of a product with
   // B != A, which is symmetric only up to rounding: the lower triangle is stored and mirrored, so
   // that the stored matrix is exactly symmetric.
   auto class_of = [&](int col0) -> int {
     if constexpr (!kSym) return 0;
-    if (col0 + 32 <= row0) return 1;
+    if (col0 + 32 <= row0) return p.lower_only != 0 && (col0 ^ row0) >= 256 ? 0 : 1;
     if (col0 >= row0 + 32) return 2;
     return p.mirror_diagonal != 0 ? 3 : 0;
   };

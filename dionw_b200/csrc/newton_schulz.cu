@@ -90,6 +90,8 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
   // products among them are symmetric too: GRAM computes their lower tiles and mirrors,
   // GRAM_FULL computes them as general products, as the reference's cuBLAS calls do.
   const bool mirror = kind == DIONW_NS_GRAM;
+  // Where every m x m product is on the triangle, nothing reads past the diagonal.
+  const bool lower = kind != DIONW_NS_GRAM_FULL || !l.gram;
   const bool tall = rows > cols;
   const int64_t m = l.m, n = l.n;
   const int64_t xb = rows * ldx;    // batch strides in elements
@@ -110,6 +112,7 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
     p.a = p.b = block(from);
     p.a_mn = p.b_mn = tall;
     p.symmetric = p.same_operands = true;
+    p.out_lower = lower;
     p.out = small(to);
     p.m = p.n = m;
     p.k = n;
@@ -122,6 +125,7 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
     p.b = small(b);
     p.symmetric = a == b || mirror;
     p.same_operands = a == b;
+    p.a_lower = p.b_lower = p.out_lower = lower;
     p.alpha = float(alpha);
     p.cin = small(cin);
     p.beta = float(beta);
@@ -136,6 +140,8 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
     p.a = tall ? block(from) : small(s);
     p.b = tall ? small(s) : block(from);
     p.b_mn = !tall;
+    p.a_lower = lower && !tall;
+    p.b_lower = lower && tall;
     if (beta != 0.0) p.cin = block(from);
     p.beta = float(beta);
     p.out = block(to);

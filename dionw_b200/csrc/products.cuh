@@ -18,6 +18,9 @@ struct Product {
   bool a_mn = false;             // A stored [k, m] (symmetric products of one operand only: A^T A)
   bool b_mn = false;             // B stored [k, n]
   bool symmetric = false;        // known to be symmetric: lower tiles + mirror
+  // An operand or the result is symmetric and only its 256 x 256 blocks up to the diagonal are stored.  (The
+  // one-CTA kernel stores mirror images everywhere and reads whole matrices.)
+  bool a_lower = false, b_lower = false, out_lower = false;
   bool same_operands = false;    // symmetric: A and B are the same matrix, so diagonal tiles come out symmetric
   Operand cin;                   // base null: no second term
   float alpha = 1.0f, beta = 0.0f;
