@@ -65,7 +65,7 @@ constexpr int kEpilogueWarps = 8;
 constexpr int kReporterWarp = 2 + kEpilogueWarps;
 constexpr int kSchedulerWarp = kReporterWarp + 1;
 constexpr int kThreads = 32 * (kSchedulerWarp + 1);
-constexpr uint32_t kBarrierBytes = 640;
+constexpr uint32_t kBarrierBytes = 832;
 constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
 constexpr uint32_t kBBytes = (kBN / 2) * kBK * 2;  // 16 KB: the half of B's columns that each CTA loads
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
@@ -88,23 +88,40 @@ __device__ __forceinline__ void remote_arrive_after(uint32_t cluster_address, in
                ::"r"(cluster_address), "r"(loaded), "n"(kNoTile) : "memory");
 }
 
-// An entry of the tile ring: the product of the plan (negative: no more tiles) and the tile of it.
+// An entry of the tile ring: the product of the plan (negative: no more tiles), the tile of it, and what the
+// loads and the main loop need to know about the two (see Ranges), so that neither waits for the parameters of a
+// product it has not met yet: read from the kernel's arguments they took 700 cycles between tile and first load.
 struct alignas(16) Entry {
   int step, batch, tm, tn;
+  int k_blocks, a_end, b_end, flags;
+  int map_a, map_b, map_a_mn, map_b_mn;
 };
+constexpr int kSharedFlag = 1, kWideFlag = 2;
+constexpr int kEntryWords = sizeof(Entry) / sizeof(int4);
 
 // Stores an entry in the peer's shared memory and counts its bytes on a barrier there, which releases it: the
 // sender waits for nothing.  (A store and an arrive with release at cluster scope took the sender 1700 cycles.)
 __device__ __forceinline__ void send_entry(uint32_t cluster_address, uint32_t cluster_bar, const Entry& e) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-               ::"r"(cluster_address), "r"(e.step), "r"(e.batch), "r"(e.tm), "r"(e.tn), "r"(cluster_bar) : "memory");
+  const int4* words = reinterpret_cast<const int4*>(&e);
+#pragma unroll
+  for (int i = 0; i < kEntryWords; ++i)
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(cluster_address + 16 * i), "r"(words[i].x), "r"(words[i].y), "r"(words[i].z), "r"(words[i].w),
+                 "r"(cluster_bar) : "memory");
 }
 
-// One instruction: what depends on one field of the entry depends on all of them.
-__device__ __forceinline__ Entry load_entry(const Entry* from) {
-  Entry e;
+// Word i of an entry; one instruction, so what depends on one of its fields depends on all of them.
+__device__ __forceinline__ void load_entry_word(const Entry* from, int i, Entry& e) {
+  int4& w = reinterpret_cast<int4*>(&e)[i];
   asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(e.step), "=r"(e.batch), "=r"(e.tm), "=r"(e.tn) : "r"(gemm::smem_u32(from)) : "memory");
+               : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(gemm::smem_u32(from) + 16 * i) : "memory");
+}
+// The entry, but for its last word(s) where they are not needed; the word that readers report on is read last.
+template <int kWords>
+__device__ __forceinline__ Entry load_entry(const Entry* from) {
+  Entry e{};
+#pragma unroll
+  for (int i = kWords - 1; i >= 0; --i) load_entry_word(from, i, e);
   return e;
 }
 
@@ -144,11 +161,11 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 
 // TMA load into this CTA's shared memory whose completion is signalled on a barrier of the
 // pair's leader CTA (the .cta_group::2 form allows the barrier to be the peer's).
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t leader_bar, int c0,
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t smem_dst, const CUtensorMap* map, uint32_t leader_bar, int c0,
                                                  int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(gemm::smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(c0), "r"(c1), "r"(c2)
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 
@@ -268,25 +285,31 @@ __device__ __forceinline__ Tile tile_of(int t, const Step& step) {
   return step.symmetric ? gemm2::sym_tile(t, step.p, kBN / step.tile_n) : gemm2::general_tile(t, step.p);
 }
 
-// How a tile's k-blocks are read: A in rows (K-major) up to a_end and B up to b_end, and in columns (MN-major)
-// from there on.  Of a symmetric matrix that a product of the plan left, only the 256 x 256 blocks up to the
+// How a tile's k-blocks are read: A in rows (K-major) up to a_end and B up to b_end <= a_end, and in columns
+// (MN-major) from there on; with kSharedFlag A's rows serve as B's.  Of a symmetric matrix that a product of the plan left, only the 256 x 256 blocks up to the
 // diagonal exist: what lies right of the diagonal in a row is read from the column it is equal to.  The tensor
 // cores take either order, so nothing is stored twice: a mirrored copy was half of all bytes the products wrote,
 // and the write path, at 20 to 25 bytes per cycle and SM, what their epilogues waited for (1300 to 2900 of 2500 to
 // 4600 cycles per 32-column chunk).
-struct Ranges {
-  int k_blocks, a_end, b_end;   // b_end <= a_end in every product there is
-  bool shared;                  // A's rows serve as B's
-};
-__device__ __forceinline__ Ranges ranges_of(const Step& step, int tm, int tn) {
+__device__ __forceinline__ Entry entry_of(const Step& step, int at, const Tile& tile) {
   constexpr int kPerBlock = kPairM / kBK;
-  Ranges r;
-  r.k_blocks = (step.p.kdim + kBK - 1) / kBK;
-  const int column_block = step.tile_n == kBN ? tn : tn >> 1;
-  r.a_end = step.a_major_mn ? 0 : step.a_lower ? min(r.k_blocks, (tm + 1) * kPerBlock) : r.k_blocks;
-  r.b_end = step.b_major_mn ? 0 : step.b_lower ? min(r.k_blocks, (column_block + 1) * kPerBlock) : r.k_blocks;
-  r.shared = step.same_operands && step.tile_n == kBN && tm == tn;
-  return r;
+  const int k_blocks = (step.p.kdim + kBK - 1) / kBK;
+  const int column_block = step.tile_n == kBN ? tile.tn : tile.tn >> 1;
+  const bool shared = step.same_operands && step.tile_n == kBN && tile.tm == tile.tn;
+  Entry e;
+  e.step = at;
+  e.batch = tile.batch;
+  e.tm = tile.tm;
+  e.tn = tile.tn;
+  e.k_blocks = k_blocks;
+  e.a_end = step.a_major_mn ? 0 : step.a_lower ? min(k_blocks, (tile.tm + 1) * kPerBlock) : k_blocks;
+  e.b_end = step.b_major_mn ? 0 : step.b_lower ? min(k_blocks, (column_block + 1) * kPerBlock) : k_blocks;
+  e.flags = (shared ? kSharedFlag : 0) | (step.tile_n == kBN ? kWideFlag : 0);
+  e.map_a = step.map_a;
+  e.map_b = step.map_b;
+  e.map_a_mn = step.a_lower ? step.map_a_t : step.map_a;
+  e.map_b_mn = step.b_lower ? step.map_b_t : step.map_b;
+  return e;
 }
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
@@ -297,9 +320,16 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
 __device__ __forceinline__ void add_release(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// One lane of a converged warp, as the compiler understands it.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+
 // Orders this thread's accesses through the generic proxy (ordinary loads and stores) with those of the
 // async proxy (TMA) on both sides.
-__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 // Bounded wait until the progress of a matrix has reached `need`.
 __device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned need, volatile int* abort_flag,
@@ -429,124 +459,150 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   // gave up.  Called by ONE thread per consumer (the single-thread roles themselves, lane 0 of an
   // epilogue warp), which also reports the slot as read.
   const uint32_t leader_tile_empty = peer_address(&tile_empty[0], 0);
-  auto take_tile = [&](uint32_t n, bool when_ready) -> Entry {
+  auto take_tile = [&](uint32_t n, bool when_ready, auto words) -> Entry {
+    Entry none{};
+    none.step = -1;
     if (!dynamic) {
       const long long t = (long long)pair + (long long)n * pairs;
-      if (t >= total_tiles) return Entry{-1, 0, 0, 0};
-      const Tile tile = tile_of(int(t), plan.steps[0]);
-      return Entry{0, tile.batch, tile.tm, tile.tn};
+      if (t >= total_tiles) return none;
+      return entry_of(plan.steps[0], 0, tile_of(int(t), plan.steps[0]));
     }
+    none.step = -2;
     const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
-    if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) return Entry{-2, 0, 0, 0};
-    const Entry e = load_entry(&tile_ring[slot]);
+    if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) return none;
+    const Entry e = load_entry<decltype(words)::value>(&tile_ring[slot]);
     if (kSteps > 1 && when_ready && e.step >= 0 && !mbar_wait(&ready[slot], phase, abort_flag, plan.status, plan.wait_ns))
-      return Entry{-2, 0, 0, 0};
+      return none;
     remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), e.step);
     return e;
+  };
+
+  // The same for a warp: one lane waits, reads and reports, the others follow it.
+  auto take_tile_warp = [&](uint32_t n, bool when_ready, auto words) -> Entry {
+    Entry e{};
+    if (lane == 0) e = take_tile(n, when_ready, words);
+    int* fields = reinterpret_cast<int*>(&e);
+#pragma unroll
+    for (int i = 0; i < 4 * decltype(words)::value; ++i) fields[i] = __shfl_sync(0xffffffffu, fields[i], 0);
+    __syncwarp();   // what lane 0's wait has acquired is the other lanes' too: a shuffle orders no memory
+    return e;
+  };
+  const std::integral_constant<int, 1> kTileOnly{};
+  const std::integral_constant<int, 2> kTileAndRanges{};
+  const std::integral_constant<int, 3> kWholeEntry{};
+  // All lanes wait; false for all of them when one gave up.
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, plan.status, plan.wait_ns)) != 0;
   };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
-      uint32_t it = 0;
+      int s = 0;                 // stage of the ring, and the parity that its slot's next release has
+      uint32_t released = 1;
       bool ok = true;
+      const uint32_t ring = smem_u32(smem), leader_full = peer_address(full_bar, 0);
       for (uint32_t n = 0; ok; ++n) {
-        const Entry tile = take_tile(n, true);
+        const Entry tile = take_tile(n, true, kWholeEntry);
         if (tile.step < 0) break;
-        const Step& step = plan.steps[tile.step];
-        const Ranges range = ranges_of(step, tile.tm, tile.tn);
-        const int half_n = step.tile_n / 2;
+        const bool shared = (tile.flags & kSharedFlag) != 0;
+        const int tile_n = (tile.flags & kWideFlag) != 0 ? kBN : kBN / 2, half_n = tile_n / 2;
         const int m0 = tile.tm * kPairM + int(rank) * kBM;
-        const int n0 = tile.tn * step.tile_n + int(rank) * half_n;
+        const int n0 = tile.tn * tile_n + int(rank) * half_n;
         // the k-block after whose loads this pair's next tile may be drawn
-        const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? range.k_blocks - 1 : max(0, range.k_blocks - kDrawAhead);
-        const uint32_t pair_bytes = 2 * (kABytes + (range.shared ? 0u : uint32_t(half_n) * kBK * 2));
+        const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? tile.k_blocks - 1 : max(0, tile.k_blocks - kDrawAhead);
+        const uint32_t pair_bytes = 2 * (kABytes + (shared ? 0u : uint32_t(half_n) * kBK * 2));
         // The layout of the operands is a constant inside the loop.
         auto load_loop = [&](int begin, int end, auto a_major_mn, auto b_major_mn) {
           constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
           if (!ok || begin >= end) return;
-          const CUtensorMap* map_a = &plan.maps[kAMN && step.a_lower ? step.map_a_t : step.map_a];
-          const CUtensorMap* map_b = &plan.maps[kBMN && step.b_lower ? step.map_b_t : step.map_b];
-          for (int kb = begin; kb < end; ++kb, ++it) {
-            const int s = it % kStages;
-            const uint32_t phase = (it / kStages) & 1u;
-            if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
-            uint8_t* a_dst = smem + size_t(s) * kStageBytes;
-            uint8_t* b_dst = a_dst + kABytes;
-            const uint32_t leader_full = peer_address(&full_bar[s], 0);
-            // The peer's bytes may land before the leader has announced them: the phase still
-            // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
-            // because its empty barrier is released by the MMAs that consumed this one.
-            if (rank == 0) mbar_expect_tx(&full_bar[s], pair_bytes);
+          const CUtensorMap* map_a = &plan.maps[kAMN ? tile.map_a_mn : tile.map_a];
+          const CUtensorMap* map_b = &plan.maps[kBMN ? tile.map_b_mn : tile.map_b];
+          for (int kb = begin; kb < end; ++kb) {
+            if (!mbar_wait(&empty_bar[s], released, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
+            const uint32_t a_dst = ring + uint32_t(s) * kStageBytes, b_dst = a_dst + kABytes;
+            const uint32_t landed = leader_full + uint32_t(s) * uint32_t(sizeof(uint64_t));
             const int k0 = kb * kBK;
-            if constexpr (kAMN) {
+            {
+              // The peer's bytes may land before the leader has announced them: the phase still
+              // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
+              // because its empty barrier is released by the MMAs that consumed this one.
+              if (rank == 0) mbar_expect_tx(&full_bar[s], pair_bytes);
+              if constexpr (kAMN) {
 #pragma unroll
-              for (int panel = 0; panel < kBM / 64; ++panel)
-                tma_load_3d_pair(a_dst + panel * kPanelBytes, map_a, leader_full, m0 + panel * 64, k0, tile.batch);
-            } else {
-              tma_load_3d_pair(a_dst, map_a, leader_full, k0, m0, tile.batch);
-            }
-            if (!range.shared) {
-              if constexpr (kBMN) {
-                tma_load_3d_pair(b_dst, map_b, leader_full, n0, k0, tile.batch);
-                if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, leader_full, n0 + 64, k0, tile.batch);
+                for (int panel = 0; panel < kBM / 64; ++panel)
+                  tma_load_3d_pair(a_dst + panel * kPanelBytes, map_a, landed, m0 + panel * 64, k0, tile.batch);
               } else {
-                tma_load_3d_pair(b_dst, map_b, leader_full, k0, n0, tile.batch);
+                tma_load_3d_pair(a_dst, map_a, landed, k0, m0, tile.batch);
               }
+              if (!shared) {
+                if constexpr (kBMN) {
+                  tma_load_3d_pair(b_dst, map_b, landed, n0, k0, tile.batch);
+                  if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, landed, n0 + 64, k0, tile.batch);
+                } else {
+                  tma_load_3d_pair(b_dst, map_b, landed, k0, n0, tile.batch);
+                }
+              }
+              if (kb == draw_at) mbar_arrive(may_draw);
             }
-            if (kb == draw_at) mbar_arrive(may_draw);
+            if (++s == kStages) s = 0, released ^= 1u;
           }
         };
-        load_loop(0, range.b_end, std::false_type(), std::false_type());
-        load_loop(range.b_end, range.a_end, std::false_type(), std::true_type());
-        load_loop(range.a_end, range.k_blocks, std::true_type(), std::true_type());
+        load_loop(0, tile.b_end, std::false_type(), std::false_type());
+        load_loop(tile.b_end, tile.a_end, std::false_type(), std::true_type());
+        load_loop(tile.a_end, tile.k_blocks, std::true_type(), std::true_type());
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank != 0) {
-      // the second CTA's MMA warp has nothing to issue
-    } else if (lane == 0) {
+    if (rank == 0) {   // the second CTA's MMA warp has nothing to issue
       // ------------------------------------------------------------ MMA issuer (leader)
-      uint32_t it = 0;
+      // The whole warp goes through the loop and one elected lane issues: the descriptors of an MMA are uniform
+      // registers, which the compiler can only keep there where the warp is converged.  Issued by a thread of its own,
+      // an MMA took 140 to 190 cycles to issue and 128 to run (64 on a tile of 128 columns).
+      int s = 0;                 // stage of the ring, and the parity that its next load completes
+      uint32_t loaded = 0;
       bool ok = true;
+      const uint32_t ring = smem_u32(smem);
       for (uint32_t local = 0; ok; ++local) {
-        const Entry tile = take_tile(local, false);
+        const Entry tile = take_tile_warp(local, false, kTileAndRanges);
         if (tile.step < 0) break;
-        const Step& step = plan.steps[tile.step];
-        const Ranges range = ranges_of(step, tile.tm, tile.tn);
         const uint32_t acc = local & 1u;
         const uint32_t acc_phase = (local >> 1) & 1u;
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
+        if (!warp_wait(&acc_empty[acc], acc_phase ^ 1u)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * uint32_t(kBN);
-        const uint32_t b_offset = range.shared ? 0u : kABytes;
+        const uint32_t b_offset = (tile.flags & kSharedFlag) != 0 ? 0u : kABytes;
+        const int tile_n = (tile.flags & kWideFlag) != 0 ? kBN : kBN / 2;
         // The layout of the operands is a constant inside the loop.
         auto main_loop = [&](int begin, int end, auto a_major_mn, auto b_major_mn) {
           constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
           if (!ok) return;
-          const uint32_t idesc = make_idesc2<InT>(kAMN, kBMN, step.tile_n);
-          for (int kb = begin; kb < end; ++kb, ++it) {
-            const int s = it % kStages;
-            const uint32_t phase = (it / kStages) & 1u;
-            if (!mbar_wait(&full_bar[s], phase, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
+          const uint32_t idesc = make_idesc2<InT>(kAMN, kBMN, tile_n);
+          for (int kb = begin; kb < end; ++kb) {
+            if (!warp_wait(&full_bar[s], loaded)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(smem + size_t(s) * kStageBytes);
+            const uint32_t a_addr = ring + uint32_t(s) * kStageBytes;
             const uint32_t b_addr = a_addr + b_offset;
             const uint64_t a_desc = make_smem_desc(a_addr, kAMN ? kPanelBytes : 16, 1024);
             const uint64_t b_desc = make_smem_desc(b_addr, kBMN ? kPanelBytes : 16, 1024);
+            if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < kBK / kUmmaK; ++j) {
-              const uint64_t k_step = uint64_t((j * kUmmaK * 2) >> 4), mn_step = uint64_t((j * kUmmaK * 128) >> 4);
-              umma2_f16(tmem_d, a_desc + (kAMN ? mn_step : k_step), b_desc + (kBMN ? mn_step : k_step), idesc,
-                        (kb > 0 || j > 0) ? 1u : 0u);
+              for (int j = 0; j < kBK / kUmmaK; ++j) {
+                const uint64_t k_step = uint64_t((j * kUmmaK * 2) >> 4), mn_step = uint64_t((j * kUmmaK * 128) >> 4);
+                umma2_f16(tmem_d, a_desc + (kAMN ? mn_step : k_step), b_desc + (kBMN ? mn_step : k_step), idesc,
+                          (kb > 0 || j > 0) ? 1u : 0u);
+              }
+              umma2_commit_both(&empty_bar[s]);
             }
-            umma2_commit_both(&empty_bar[s]);
+            __syncwarp();
+            if (++s == kStages) s = 0, loaded ^= 1u;
           }
         };
-        main_loop(0, range.b_end, std::false_type(), std::false_type());
-        main_loop(range.b_end, range.a_end, std::false_type(), std::true_type());
-        main_loop(range.a_end, range.k_blocks, std::true_type(), std::true_type());
-        if (ok) umma2_commit_both(&acc_full[acc]);
+        main_loop(0, tile.b_end, std::false_type(), std::false_type());
+        main_loop(tile.b_end, tile.a_end, std::false_type(), std::true_type());
+        main_loop(tile.a_end, tile.k_blocks, std::true_type(), std::true_type());
+        if (ok && elect_one()) umma2_commit_both(&acc_full[acc]);
+        __syncwarp();
       }
     }
   } else if (warp == kReporterWarp) {
@@ -555,7 +611,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
       for (uint32_t n = 0;; ++n) {
         const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
         if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
-        const Entry tile = load_entry(&tile_ring[slot]);
+        const Entry tile = load_entry<1>(&tile_ring[slot]);
         if (tile.step < 0) break;
         unsigned* progress = &plan.steps[tile.step].progress[tile.batch];
         if (!mbar_wait(&stored[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
@@ -580,10 +636,10 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
             if constexpr (kSteps > 1) {
               while (at + 1 < plan.count && t >= plan.steps[at + 1].first_tile) ++at;
             }
-            const Tile tile = tile_of(t - plan.steps[at].first_tile, plan.steps[at]);
-            e = Entry{at, tile.batch, tile.tm, tile.tn};
+            e = entry_of(plan.steps[at], at, tile_of(t - plan.steps[at].first_tile, plan.steps[at]));
           } else {
-            e = Entry{-1, 0, 0, 0};
+            e = Entry{};
+            e.step = -1;
           }
           if (!mbar_wait_cluster(&tile_empty[slot], phase ^ 1u, abort_flag, plan.status, plan.wait_ns)) break;
           send_entry(peer_address(&tile_ring[slot], 1), peer_address(&tile_full[slot], 1), e);
@@ -600,7 +656,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
           }
         } else {
           if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) break;
-          e = load_entry(&tile_ring[slot]);
+          e = load_entry<1>(&tile_ring[slot]);
           remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), e.step);
           if (e.step < 0) break;
           mbar_expect_tx(&tile_full[(n + 1) % kTileSlots], sizeof(Entry));   // its last phase is over: this thread has seen it
@@ -622,13 +678,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
     uint8_t* stage = mirror_stage + ew * 2 * kPieceBytes;
     const uint32_t leader_empty[2] = {peer_address(&acc_empty[0], 0), peer_address(&acc_empty[1], 0)};
     for (uint32_t local = 0;; ++local) {
-      Entry tile{};
-      if (lane == 0) tile = take_tile(local, true);   // one lane waits, reads and reports; the warp follows it
-      tile.step = __shfl_sync(0xffffffffu, tile.step, 0);
-      tile.batch = __shfl_sync(0xffffffffu, tile.batch, 0);
-      tile.tm = __shfl_sync(0xffffffffu, tile.tm, 0);
-      tile.tn = __shfl_sync(0xffffffffu, tile.tn, 0);
-      __syncwarp();   // the other lanes read Cin too, which lane 0's wait alone has acquired: a shuffle orders no memory
+      const Entry tile = take_tile_warp(local, true, kTileOnly);
       if (tile.step < 0) break;
       const Step& step = plan.steps[tile.step];
       const Params& p = step.p;
