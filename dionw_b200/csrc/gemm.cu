@@ -8,6 +8,7 @@
 #include <utility>
 
 #include "gemm2_sm100.cuh"
+#include "onchip_sm100.cuh"
 #include "products.cuh"
 
 namespace dionw {
@@ -426,6 +427,121 @@ int run_products(const Product* products, int count, int dtype, void* counters, 
     if (st != DIONW_OK) return st;
   }
   return DIONW_OK;
+}
+
+namespace {
+
+// Clusters of `pairs` SM pairs that the current device runs at a time, 0 where it cannot be told.
+int onchip_clusters(int pairs) {
+  static std::atomic<int> known[kMaxDevices][onchip::kMaxPairs + 1];   // + 1; zero: not asked yet
+  std::atomic<int>& slot = known[current_device()][pairs];
+  int value = slot.load(std::memory_order_acquire);
+  if (value != 0) return value - 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(onchip::kSmemBytes)) == cudaSuccess) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(unsigned(2 * pairs));
+    config.blockDim = dim3(onchip::kThreads);
+    config.dynamicSmemBytes = onchip::kSmemBytes;
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = unsigned(2 * pairs);
+    attribute.val.clusterDim.y = 1;
+    attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&clusters, onchip::iteration_kernel, &config) != cudaSuccess) clusters = 0;
+  }
+  cudaGetLastError();   // what went wrong here shows at the launch
+  slot.store(clusters + 1, std::memory_order_release);
+  return clusters;
+}
+
+// As many pairs to a matrix as it has column blocks, while all clusters run at the same time.
+int pairs_per_matrix(int64_t blocks, int64_t tiles) {
+  for (int pairs = int(std::min<int64_t>(tiles, onchip::kMaxPairs)); pairs > 1; --pairs)
+    if (blocks <= onchip_clusters(pairs)) return pairs;
+  return 1;
+}
+
+}  // namespace
+
+// On chip a chain of products takes 14 x 2.4 us whatever the rest of the GPU does, but every pair sums the whole Gram
+// matrix (0.26 us per 64 columns of n) and a batch takes whole waves of clusters.  Iteration as a plan against on
+// chip, us, m = 256: 1 block of n = 1024 107 and 69, 4096 129 and 109, 8192 157 and 162; 37 blocks 130 and 84, 192 and
+// 162, 285 and 296; 74 blocks (one wave) 182 and 89, 318 and 220, 463 and 388; 160 (two and a bit) of 1024 282 and 261,
+// of 2048 379 and 412.  m = 96: 1 block of 1024 89 and 43, of 8192 138 and 126; 160 of 1024 196 and 152.
+constexpr int64_t kOnChipColumns = 6144, kOnChipColumnsInWaves = 1024;
+
+bool runs_on_chip(int64_t blocks, int64_t m, int64_t n) {
+  if (!use_cta_pairs() || m > onchip::kSide) return false;
+  const int wave = onchip_clusters(1);
+  return wave > 0 && n <= (blocks <= wave ? kOnChipColumns : kOnChipColumnsInWaves);
+}
+
+int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* slots, int n_slots, bool tall, cudaStream_t stream) {
+  auto slot_of = [&](const void* base) -> int {
+    for (int i = 0; i < n_slots; ++i)
+      if (slots[i].base == base) return slots[i].slot;
+    return -1;
+  };
+  onchip::Iteration it{};
+  const int64_t blocks = list[0].blocks, m = list[0].m, n = list[0].k;
+  it.tall = tall;
+  it.m = int(m);
+  it.n = int(n);
+  it.status = device_status_word();
+  it.wait_ns = gemm::kWaitLimitNs;
+  for (int part = 0; part < 2; ++part) {
+    const Product& gram = *list++;
+    const int64_t cols = tall ? m : n, rows = tall ? n : m;
+    const uint32_t boxes[2] = {uint32_t(onchip::kRows), 64};
+    for (int box = 0; box < 2; ++box) {
+      const int st = make_map(&it.x[part][box], gram.a.base, DIONW_F16, cols, rows, blocks, gram.a.ld, gram.a.batch, 64, boxes[box]);
+      if (st != DIONW_OK) return st;
+    }
+    it.count[part] = 1 + chain_length[part];
+    DIONW_REQUIRE(it.count[part] <= onchip::kMaxOps, "a chain has at most %d products", onchip::kMaxOps - 1);
+    it.ops[part][0] = {-1, -1, -1, 0, -1, gram.alpha, 0.0f, 0.0f};
+    DIONW_REQUIRE(slot_of(gram.out.base) == 0, "the Gram matrix is the first slot's");
+    for (int i = 1; i < it.count[part]; ++i) {
+      const Product& p = *list++;
+      onchip::Op& op = it.ops[part][i];
+      op.a = int8_t(slot_of(p.a.base));
+      op.b = int8_t(slot_of(p.b.base));
+      op.cin = int8_t(slot_of(p.cin.base));
+      op.out = int8_t(slot_of(p.out.base));
+      op.out2 = int8_t(p.out2 != nullptr ? slot_of(p.out2) : -1);
+      op.alpha = p.alpha;
+      op.beta = p.beta;
+      op.diag = p.diag;
+      DIONW_REQUIRE(p.symmetric && p.m == m && p.n == m && p.k == m && op.a >= 0 && op.b >= 0 && op.cin >= 0 && op.out >= 0 &&
+                        (p.out2 == nullptr || op.out2 >= 0),
+                    "a chain is of symmetric products of one size on known matrices");
+    }
+    const Product& result = *list++;
+    DIONW_REQUIRE(slot_of(tall ? result.b.base : result.a.base) == 2, "Q is the third slot's");
+    it.result[part] = params_of(result);
+    it.result_bf16[part] = result.out_dtype == DIONW_BF16;
+  }
+  const int64_t tiles = (n + onchip::kSide - 1) / onchip::kSide;
+  it.pairs = pairs_per_matrix(blocks, tiles);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(unsigned(2 * it.pairs * blocks));
+  config.blockDim = dim3(onchip::kThreads);
+  config.dynamicSmemBytes = onchip::kSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = unsigned(2 * it.pairs);
+  attributes[0].val.clusterDim.y = 1;
+  attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = use_dependent_launch() ? 2 : 1;
+  count_launch();
+  return check_cuda(cudaLaunchKernelEx(&config, onchip::iteration_kernel, it), "iteration_kernel launch");
 }
 
 }  // namespace dionw

@@ -229,6 +229,15 @@ size_t group_bytes(const Problem* problems, int n) {
   return bytes + align256(plan_counter_bytes(matrices));
 }
 
+// The list that append_products makes of a Gram iteration, on chip: products 1 to 5 and 8 to 16 are on m x m matrices.
+int iterate_on_chip(const Product* list, int count, bool tall, cudaStream_t stream) {
+  const int lengths[2] = {5, 9};
+  DIONW_REQUIRE(count == 4 + lengths[0] + lengths[1], "newton_schulz: the Gram schedule has 18 products");
+  // G and RZ, Z, both Qs: RZ is written from G and G from RZ, each for the last time
+  const ChainSlot slots[] = {{list[0].out.base, 0}, {list[2].out.base, 0}, {list[1].out.base, 1}, {list[1].out2, 2}, {list[5].out.base, 2}};
+  return run_on_chip(list, lengths, slots, 5, tall, stream);
+}
+
 // Up to kMaxChains batches that are iterated in the same dtype, as one launch, or product by product.
 int iterate(const Problem* problems, int n, bool stepwise, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
@@ -254,6 +263,11 @@ int iterate(const Problem* problems, int n, bool stepwise, void* workspace, size
     first_block += problems[i].blocks;
   }
   const bool gram = problems[0].kind == DIONW_NS_GRAM || problems[0].kind == DIONW_NS_GRAM_FULL;
+  if (n == 1 && counters != nullptr && problems[0].kind == DIONW_NS_GRAM) {
+    const Layout l = layout_of(problems[0].blocks, problems[0].rows, problems[0].cols, problems[0].ldx, problems[0].kind);
+    if (l.gram && runs_on_chip(problems[0].blocks, l.m, l.n))
+      return iterate_on_chip(list, count, problems[0].rows > problems[0].cols, stream);
+  }
   return run_products(list, count, gram ? DIONW_F16 : DIONW_BF16, counters, stream);
 }
 

@@ -51,4 +51,14 @@ size_t plan_counter_bytes(int64_t blocks);
 // `counters` (plan_counter_bytes of all chains' matrices, 4-byte aligned) is given and the limits hold.
 int run_products(const Product* products, int count, int dtype, void* counters, cudaStream_t stream);
 
+// The Gram schedule of a batch on chip (onchip_sm100.cuh): X X^T, a chain of fp16 symmetric products, Q X, twice.
+// Each m x m matrix is in one of three places; several may share a place where the one is no longer read when the
+// other is written.
+struct ChainSlot {
+  const void* base;
+  int slot;
+};
+bool runs_on_chip(int64_t blocks, int64_t m, int64_t n);   // whether that is the faster way
+int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* slots, int n_slots, bool tall, cudaStream_t stream);
+
 }  // namespace dionw
