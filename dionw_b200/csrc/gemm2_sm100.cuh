@@ -455,9 +455,16 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   gemm::griddep_wait();     // set-up above overlaps the tail of the previous product; global memory from here on
   gemm::griddep_launch();
 
-  // The n-th tile of this pair for a consumer; its step is -1 when the pair is done and -2 when the wait
-  // gave up.  Called by ONE thread per consumer (the single-thread roles themselves, lane 0 of an
-  // epilogue warp), which also reports the slot as read.
+  // All lanes of a warp wait; false for all of them when one gave up.
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, plan.status, plan.wait_ns)) != 0;
+  };
+  auto warp_wait_cluster = [&](uint64_t* bar, uint32_t parity) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, plan.status, plan.wait_ns)) != 0;
+  };
+  // The n-th tile of this pair for a consumer; its step is -1 when the pair is done and -2 when the wait gave up.
+  // Called by whole warps: every lane waits and reads, and one reports the slot as read once all of them have.
+  // (Where one lane handed the entry to the others by shuffles the first load of a tile came 650 cycles later.)
   const uint32_t leader_tile_empty = peer_address(&tile_empty[0], 0);
   auto take_tile = [&](uint32_t n, bool when_ready, auto words) -> Entry {
     Entry none{};
@@ -469,35 +476,21 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
     }
     none.step = -2;
     const uint32_t slot = n % kTileSlots, phase = (n / kTileSlots) & 1u;
-    if (!mbar_wait_cluster(&tile_full[slot], phase, abort_flag, plan.status, plan.wait_ns)) return none;
+    if (!warp_wait_cluster(&tile_full[slot], phase)) return none;
     const Entry e = load_entry<decltype(words)::value>(&tile_ring[slot]);
-    if (kSteps > 1 && when_ready && e.step >= 0 && !mbar_wait(&ready[slot], phase, abort_flag, plan.status, plan.wait_ns))
-      return none;
-    remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), e.step);
-    return e;
-  };
-
-  // The same for a warp: one lane waits, reads and reports, the others follow it.
-  auto take_tile_warp = [&](uint32_t n, bool when_ready, auto words) -> Entry {
-    Entry e{};
-    if (lane == 0) e = take_tile(n, when_ready, words);
-    int* fields = reinterpret_cast<int*>(&e);
-#pragma unroll
-    for (int i = 0; i < 4 * decltype(words)::value; ++i) fields[i] = __shfl_sync(0xffffffffu, fields[i], 0);
-    __syncwarp();   // what lane 0's wait has acquired is the other lanes' too: a shuffle orders no memory
+    if (kSteps > 1 && when_ready && e.step >= 0 && !warp_wait(&ready[slot], phase)) return none;
+    const int seen = __any_sync(0xffffffffu, e.step == kNoTile) ? kNoTile : 0;   // a value of every lane's load
+    if (lane == 0) remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), seen);
     return e;
   };
   const std::integral_constant<int, 1> kTileOnly{};
   const std::integral_constant<int, 2> kTileAndRanges{};
   const std::integral_constant<int, 3> kWholeEntry{};
-  // All lanes wait; false for all of them when one gave up.
-  auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, plan.status, plan.wait_ns)) != 0;
-  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    // A whole warp of which one elected lane issues, as in the MMA issuer.
+    {
       int s = 0;                 // stage of the ring, and the parity that its slot's next release has
       uint32_t released = 1;
       bool ok = true;
@@ -519,11 +512,11 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
           const CUtensorMap* map_a = &plan.maps[kAMN ? tile.map_a_mn : tile.map_a];
           const CUtensorMap* map_b = &plan.maps[kBMN ? tile.map_b_mn : tile.map_b];
           for (int kb = begin; kb < end; ++kb) {
-            if (!mbar_wait(&empty_bar[s], released, abort_flag, plan.status, plan.wait_ns)) { ok = false; break; }
+            if (!warp_wait(&empty_bar[s], released)) { ok = false; break; }
             const uint32_t a_dst = ring + uint32_t(s) * kStageBytes, b_dst = a_dst + kABytes;
             const uint32_t landed = leader_full + uint32_t(s) * uint32_t(sizeof(uint64_t));
             const int k0 = kb * kBK;
-            {
+            if (elect_one()) {
               // The peer's bytes may land before the leader has announced them: the phase still
               // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
               // because its empty barrier is released by the MMAs that consumed this one.
@@ -545,6 +538,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
               }
               if (kb == draw_at) mbar_arrive(may_draw);
             }
+            __syncwarp();
             if (++s == kStages) s = 0, released ^= 1u;
           }
         };
@@ -564,7 +558,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
       bool ok = true;
       const uint32_t ring = smem_u32(smem);
       for (uint32_t local = 0; ok; ++local) {
-        const Entry tile = take_tile_warp(local, false, kTileAndRanges);
+        const Entry tile = take_tile(local, false, kTileAndRanges);
         if (tile.step < 0) break;
         const uint32_t acc = local & 1u;
         const uint32_t acc_phase = (local >> 1) & 1u;
@@ -678,7 +672,7 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
     uint8_t* stage = mirror_stage + ew * 2 * kPieceBytes;
     const uint32_t leader_empty[2] = {peer_address(&acc_empty[0], 0), peer_address(&acc_empty[1], 0)};
     for (uint32_t local = 0;; ++local) {
-      const Entry tile = take_tile_warp(local, true, kTileOnly);
+      const Entry tile = take_tile(local, true, kTileOnly);
       if (tile.step < 0) break;
       const Step& step = plan.steps[tile.step];
       const Params& p = step.p;
