@@ -60,6 +60,55 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// kCount floats, and kCount 2-byte words, as one access each: streamed past the caches.
+template <int kCount>
+struct Span;
+template <>
+struct Span<4> {
+  static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
+    const float4 q = __ldcs(reinterpret_cast<const float4*>(p));
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  }
+  static __device__ __forceinline__ void store(float* p, const float (&v)[4]) {
+    __stcs(reinterpret_cast<float4*>(p), make_float4(v[0], v[1], v[2], v[3]));
+  }
+  static __device__ __forceinline__ void load(const uint16_t* p, uint32_t (&h)[4]) {
+    const uint2 q = __ldcs(reinterpret_cast<const uint2*>(p));
+    h[0] = q.x & 0xFFFFu; h[1] = q.x >> 16; h[2] = q.y & 0xFFFFu; h[3] = q.y >> 16;
+  }
+  static __device__ __forceinline__ void store(uint16_t* p, const uint32_t (&h)[4]) {
+    __stcs(reinterpret_cast<uint2*>(p), make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16)));
+  }
+};
+template <>
+struct Span<2> {
+  static __device__ __forceinline__ void load(const float* p, float (&v)[2]) {
+    const float2 q = __ldcs(reinterpret_cast<const float2*>(p));
+    v[0] = q.x; v[1] = q.y;
+  }
+  static __device__ __forceinline__ void store(float* p, const float (&v)[2]) {
+    __stcs(reinterpret_cast<float2*>(p), make_float2(v[0], v[1]));
+  }
+  static __device__ __forceinline__ void load(const uint16_t* p, uint32_t (&h)[2]) {
+    const uint32_t q = __ldcs(reinterpret_cast<const unsigned int*>(p));
+    h[0] = q & 0xFFFFu; h[1] = q >> 16;
+  }
+  static __device__ __forceinline__ void store(uint16_t* p, const uint32_t (&h)[2]) {
+    __stcs(reinterpret_cast<unsigned int*>(p), h[0] | (h[1] << 16));
+  }
+};
+template <>
+struct Span<1> {
+  static __device__ __forceinline__ void load(const float* p, float (&v)[1]) { v[0] = __ldcs(p); }
+  static __device__ __forceinline__ void store(float* p, const float (&v)[1]) { __stcs(p, v[0]); }
+  static __device__ __forceinline__ void load(const uint16_t* p, uint32_t (&h)[1]) { h[0] = __ldcs(p); }
+  static __device__ __forceinline__ void store(uint16_t* p, const uint32_t (&h)[1]) { __stcs(p, uint16_t(h[0])); }
+};
+
+// Elements of one access to rows of `cols` floats and rows of 2-byte words `ld` apart, both from 16-byte (words:
+// 8-byte) boundaries on: what divides every row's start.
+inline int span_of(long long cols, long long ld) { return cols % 4 == 0 && ld % 4 == 0 ? 4 : cols % 2 == 0 && ld % 2 == 0 ? 2 : 1; }
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 template <typename T>

@@ -1,0 +1,104 @@
+"""The streaming passes with a CTA to a row, at the lengths where their accesses, chunks and row groups end.
+
+Held to torch with the same single operations in fp32, bit for bit; the fp32 row sums, whose order torch does not
+have, to the oracle's order (scores) and to fp64 within n * 2^-24 of a sum of n non-negative terms (squares).
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from dionw_b200 import _native as native
+from oracle import dion_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+# cols on both sides of every line at which the launch changes, of chunks of 1024, and of 16-, 8- and 4-byte accesses
+COLS = [299, 300, 302, 767, 768, 1022, 1024, 1025, 1028, 2047, 2048, 2052, 2558, 2560, 4095, 4096, 4097, 4100, 5002]
+
+
+def _gen(cols: int) -> torch.Generator:
+    return torch.Generator(device=DEV).manual_seed(cols)
+
+
+@pytest.mark.parametrize("cols", COLS)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_accumulate(cols: int, dtype: torch.dtype) -> None:
+    gen = _gen(cols)
+    rows = [3, 1, 6]   # groups of two and four rows end in the middle of the second and third tensor
+    grads = [torch.randn(r, cols, device=DEV, generator=gen).to(dtype) for r in rows]
+    start = torch.randn(1, sum(rows), cols, device=DEV, generator=gen)
+    total = start[0] + torch.cat(grads).float()
+
+    def squares_close(sums: torch.Tensor, of: torch.Tensor) -> bool:
+        exact = of.double().square().sum(-1)
+        return bool(((sums.flatten().double() - exact).abs() <= 2 * cols * 2.0**-24 * exact).all())
+
+    momentum = start.clone()
+    scores, sumsq = (torch.full((1, sum(rows)), 7.0, device=DEV) for _ in range(2))
+    native.accumulate_row_l1_run(grads, rows, momentum, scores, sumsq, cols)
+    assert torch.equal(momentum[0], total)
+    assert torch.equal(scores.cpu(), oracle.row_scores(total.cpu()).view(1, -1))
+    assert squares_close(sumsq, total)
+    for nesterov in (False, True):
+        momentum, u = start.clone(), torch.empty_like(start)
+        native.accumulate_copy_decay_run(grads, rows, momentum, u, sumsq, cols, 0.95, nesterov)
+        assert torch.equal(momentum[0], total * 0.95)
+        assert torch.equal(u[0], torch.cat(grads).float() + total * 0.95 if nesterov else total)
+        assert squares_close(sumsq, u[0])
+
+
+@pytest.mark.parametrize("cols", COLS)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("selecting", [False, True])
+def test_pack(cols: int, dtype: torch.dtype, selecting: bool) -> None:
+    gen = _gen(cols)
+    blocks, rows, k, ld = 2, 9, 5 if selecting else 9, (cols + 7) // 8 * 8
+    source = torch.randn(blocks, rows, cols, device=DEV, generator=gen)
+    index = torch.stack([torch.randperm(rows, device=DEV, generator=gen)[:k].sort().values for _ in range(blocks)]).int()
+    frob = torch.tensor([3.7, 11.0], device=DEV)
+    x = torch.full((blocks, k, ld), 77.0, dtype=dtype, device=DEV)
+    after = source.clone()
+    native.pack_rows(after, index if selecting else None, frob, k, x, decay=0.95, decay_rows=selecting, eps=1e-3, norm_scale=1.02)
+    chosen = torch.stack([s[i.long()] for s, i in zip(source, index)]) if selecting else source
+    if dtype is torch.bfloat16:
+        denom = (frob.bfloat16() * 1.02 + 1e-3)[:, None, None]   # rounded after each step, as torch rounds
+        want = chosen.bfloat16() / denom
+    else:
+        want = (chosen / (frob + 1e-3)[:, None, None]).half()
+    assert torch.equal(x[..., :cols], want) and bool((x[..., cols:] == 0).all())
+    if selecting:
+        for s, i in zip(source, index):
+            s[i.long()] *= 0.95
+    assert torch.equal(after, source)
+
+
+@pytest.mark.parametrize("cols", COLS)
+@pytest.mark.parametrize("selecting", [False, True])
+@pytest.mark.parametrize("decay", [None, 0.9])
+def test_apply(cols: int, selecting: bool, decay: float | None) -> None:
+    gen = _gen(cols)
+    rows, counts, ld = 7, [1, 2], (cols + 7) // 8 * 8
+    blocks, k = sum(counts), 3 if selecting else 7
+    weights = [torch.randn(n * rows, cols, device=DEV, generator=gen) for n in counts]
+    update = torch.randn(blocks, k, ld, device=DEV, generator=gen).bfloat16()
+    denom, scale = torch.rand(blocks * k, device=DEV, generator=gen) + 0.5, torch.rand(blocks, device=DEV, generator=gen)
+    rowmap = torch.full((blocks, rows), -1, dtype=torch.int32, device=DEV)
+    chosen = [torch.randperm(rows, device=DEV, generator=gen)[:k].sort().values for _ in range(blocks)]
+    if selecting:
+        for m, c in zip(rowmap, chosen):
+            m[c] = torch.arange(k, dtype=torch.int32, device=DEV)
+    else:
+        chosen = [torch.arange(rows, device=DEV)] * blocks
+    want = torch.cat(weights).view(blocks, rows, cols).clone()
+    if decay is not None:
+        want *= decay
+    for b in range(blocks):
+        want[b, chosen[b]] += update[b, :, :cols].float() / denom[b * k:(b + 1) * k, None] * scale[b]
+    first = [0, counts[0]]
+    native.apply_round(weights, [n * rows for n in counts], [update[b].data_ptr() for b in first],
+                       [rowmap[b].data_ptr() for b in first] if selecting else None,
+                       [denom[b * k:].data_ptr() for b in first], [scale[b:].data_ptr() for b in first], ldo=ld, rows=rows, k=k,
+                       cols=cols, decay_factor=decay or 1.0, has_decay=decay is not None, decay_device=None, cta_warps=0, decay_job=None)
+    assert torch.equal(torch.cat(weights).view(blocks, rows, cols), want)
