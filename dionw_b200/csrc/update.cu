@@ -313,7 +313,11 @@ team_apply_run_kernel(const ApplyTable tab, int ldo, int rows, int k, int cols, 
 // ---------------------------------------------------------------------------
 constexpr int kAdamTable = 48;
 constexpr int kAdamThreads = 256;
-constexpr int kAdamChunk = kAdamThreads * 16;  // elements per CTA
+// 16-byte accesses of a thread to each array.  HBM-bound where enough CTAs are resident that some load while others go
+// through two divisions and a square root per element: with four accesses and two CTAs of 87 registers an SM 131 M elements
+// took 582 us, 590 to 630 at the clock that products leave behind; with two and four of 64 it is 567 (6.8 TB/s), 568 to 587.
+constexpr int kAdamUnroll = 2;
+constexpr int kAdamChunk = kAdamThreads * 4 * kAdamUnroll;  // elements per CTA
 
 struct AdamTable {
   float* p[kAdamTable];
@@ -342,7 +346,7 @@ __device__ __forceinline__ void adamw_math(float& p, float g, float& m, float& v
   p -= step_size * m / denom;
 }
 
-__global__ void __launch_bounds__(kAdamThreads)
+__global__ void __launch_bounds__(kAdamThreads, 4)
 adamw_multi_kernel(const AdamTable tab, float lr_host, float beta1, float beta2, float weight_decay_host, float eps,
                    const float* __restrict__ hyper_device) {
   after_previous();
@@ -368,9 +372,9 @@ adamw_multi_kernel(const AdamTable tab, float lr_host, float beta1, float beta2,
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
                      reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
   if (vec && base + kAdamChunk <= n) {
-    float4 pv[4], gv[4], mv[4], vv[4];
+    float4 pv[kAdamUnroll], gv[kAdamUnroll], mv[kAdamUnroll], vv[kAdamUnroll];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < kAdamUnroll; ++j) {
       const long long e = base + 4LL * (threadIdx.x + j * kAdamThreads);
       pv[j] = __ldcs(reinterpret_cast<const float4*>(p + e));
       gv[j] = __ldcs(reinterpret_cast<const float4*>(g + e));
@@ -378,7 +382,7 @@ adamw_multi_kernel(const AdamTable tab, float lr_host, float beta1, float beta2,
       vv[j] = __ldcs(reinterpret_cast<const float4*>(v + e));
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < kAdamUnroll; ++j) {
       const long long e = base + 4LL * (threadIdx.x + j * kAdamThreads);
       adamw_math(pv[j].x, gv[j].x, mv[j].x, vv[j].x, lr, beta1, beta2, weight_decay, eps, step_size, bc2_sqrt);
       adamw_math(pv[j].y, gv[j].y, mv[j].y, vv[j].y, lr, beta1, beta2, weight_decay, eps, step_size, bc2_sqrt);
