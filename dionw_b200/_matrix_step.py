@@ -230,30 +230,41 @@ def _describe_run(bucket: Bucket, positions: Sequence[int],
 
 def run_front(ctx: RunContext) -> None:
     """Stages 1-2 and the pack: the HBM-bound front of a run (reads G, updates M, writes the operand)."""
+    _accumulate(ctx)
+    buf = ctx.buf
+    if ctx.selecting:
+        with _stage("select"):
+            _native.select_rows(buf["scores"], buf["sumsq"], ctx.bucket.selected_rows, buf["index"], buf["rowmap"], buf["frob"])
+    else:
+        with _stage("accumulate"):
+            _native.block_norms(buf["sumsq"], buf["frob"])
+    _pack(ctx)
+
+
+def _accumulate(ctx: RunContext) -> None:
+    """Stage 1."""
     global CURRENT_RUN
     bucket, group, buf = ctx.bucket, ctx.group, ctx.buf
-    cols, k = bucket.cols, bucket.selected_rows
-    CURRENT_RUN = (ctx.count, bucket.rows, k, cols)
-    decay = float(group[MOMENTUM_KEY])
-    if ctx.selecting:
-        with _stage("accumulate"):
-            _native.accumulate_row_l1_run(ctx.grads, ctx.rows_per_tensor, ctx.momentum, buf["scores"],
-                                          buf["sumsq"], cols)
-        with _stage("select"):
-            _native.select_rows(buf["scores"], buf["sumsq"], k, buf["index"], buf["rowmap"], buf["frob"])
-        ctx.index, ctx.rowmap, ctx.source = buf["index"], buf["rowmap"], ctx.momentum
-    else:
-        nesterov = MomentumForm(group[MOMENTUM_FORM_KEY]) is MomentumForm.NESTEROV
-        with _stage("accumulate"):
-            _native.accumulate_copy_decay_run(ctx.grads, ctx.rows_per_tensor, ctx.momentum, buf["u"],
-                                              buf["sumsq"], cols, decay, nesterov)
-            _native.block_norms(buf["sumsq"], buf["frob"])
-        ctx.index, ctx.rowmap, ctx.source = None, None, buf["u"]
-    fn = bucket.orthogonalize
+    CURRENT_RUN = (ctx.count, bucket.rows, bucket.selected_rows, bucket.cols)
+    with _stage("accumulate"):
+        if ctx.selecting:
+            _native.accumulate_row_l1_run(ctx.grads, ctx.rows_per_tensor, ctx.momentum, buf["scores"], buf["sumsq"], bucket.cols)
+            ctx.index, ctx.rowmap, ctx.source = buf["index"], buf["rowmap"], ctx.momentum
+        else:
+            nesterov = MomentumForm(group[MOMENTUM_FORM_KEY]) is MomentumForm.NESTEROV
+            _native.accumulate_copy_decay_run(ctx.grads, ctx.rows_per_tensor, ctx.momentum, buf["u"], buf["sumsq"], bucket.cols,
+                                              float(group[MOMENTUM_KEY]), nesterov)
+            ctx.index, ctx.rowmap, ctx.source = None, None, buf["u"]
+
+
+def _pack(ctx: RunContext) -> None:
+    """The operand of a built-in iteration, from the selected rows and their norms."""
+    fn = ctx.bucket.orthogonalize
     if isinstance(fn, NativeOrthogonalizer):
         with _stage("pack"):
-            _native.pack_rows(ctx.source, ctx.index, buf["frob"], k, buf["x"], decay=decay,
-                              decay_rows=ctx.selecting, eps=NEWTON_SCHULZ_EPS, norm_scale=fn.norm_scale)
+            _native.pack_rows(ctx.source, ctx.index, ctx.buf["frob"], ctx.bucket.selected_rows, ctx.buf["x"],
+                              decay=float(ctx.group[MOMENTUM_KEY]), decay_rows=ctx.selecting, eps=NEWTON_SCHULZ_EPS,
+                              norm_scale=fn.norm_scale)
 
 
 def run_core(ctx: RunContext, alone: bool = False) -> RunResult:
@@ -284,20 +295,32 @@ def _fused_row_sums(ctx: RunContext) -> bool:
 
 def _finish_run(ctx: RunContext, orthogonal: Tensor) -> RunResult:
     """Stage 4: the orthogonalized rows reduced to one scale per row and one per block."""
-    bucket, group, buf = ctx.bucket, ctx.group, ctx.buf
-    rows, cols, k = bucket.rows, bucket.cols, bucket.selected_rows
-    normalize = RowNormalization(group[ROW_NORMALIZATION_KEY]) is RowNormalization.NORMUON
-    fused = _fused_row_sums(ctx)
+    bucket, buf = ctx.bucket, ctx.buf
+    scales = _scale_arguments(ctx)
     with _stage("finish"):
-        if normalize and not fused:
-            _native.row_sumsq_bf16(orthogonal, cols, buf["rowsq"])
-        _native.normuon_rows(buf["rowsq"], ctx.variance, ctx.index, blocks=ctx.count, rows=rows, k=k, cols=cols,
-                             weight=1.0 - float(group[MUON_BETA2_KEY]), eps=NORMALIZATION_EPS, step=ctx.step,
-                             normalize=normalize, denom=buf["denom"], scale=buf["scale"],
-                             parts=buf["rowsq"].shape[1] if fused else 1, step_device=bucket.step_device)
-    return RunResult(params=ctx.params, rows_per_tensor=ctx.rows_per_tensor, count=ctx.count, rows=rows, k=k,
-                     cols=cols, orthogonal=orthogonal, rowmap=ctx.rowmap, denom=buf["denom"], scale=buf["scale"],
-                     decay_device=bucket.decay_device)
+        if scales["normalize"] and not _fused_row_sums(ctx):
+            _native.row_sumsq_bf16(orthogonal, bucket.cols, buf["rowsq"])
+        _native.normuon_rows(**scales, eps=NORMALIZATION_EPS)
+    return _result(ctx, orthogonal)
+
+
+def _scale_arguments(ctx: RunContext) -> dict[str, Any]:
+    """The arguments of ``_native.normuon_rows`` for a run whose row sums are there."""
+    bucket, buf = ctx.bucket, ctx.buf
+    return {
+        "s": buf["rowsq"], "variance": ctx.variance, "index": ctx.index, "blocks": ctx.count, "rows": bucket.rows,
+        "k": bucket.selected_rows, "cols": bucket.cols, "weight": 1.0 - float(ctx.group[MUON_BETA2_KEY]), "step": ctx.step,
+        "normalize": RowNormalization(ctx.group[ROW_NORMALIZATION_KEY]) is RowNormalization.NORMUON, "denom": buf["denom"],
+        "scale": buf["scale"], "parts": buf["rowsq"].shape[1] if _fused_row_sums(ctx) else 1,
+        "step_device": bucket.step_device,
+    }
+
+
+def _result(ctx: RunContext, orthogonal: Tensor) -> RunResult:
+    bucket, buf = ctx.bucket, ctx.buf
+    return RunResult(params=ctx.params, rows_per_tensor=ctx.rows_per_tensor, count=ctx.count, rows=bucket.rows,
+                     k=bucket.selected_rows, cols=bucket.cols, orthogonal=orthogonal, rowmap=ctx.rowmap, denom=buf["denom"],
+                     scale=buf["scale"], decay_device=bucket.decay_device)
 
 
 def groups_of_runs(runs: Sequence[tuple[Bucket, Sequence[int]]],
@@ -338,7 +361,8 @@ def step_runs(runs: Sequence[tuple[Bucket, Sequence[int]]], param_groups: Sequen
     """One Dion step for several runs (one entry of ``groups_of_runs``; their parameter groups may differ),
     stage by stage.
 
-    Their Newton-Schulz iterations run as one launch.  An iteration is a chain of 15 to 18 products;
+    Their row selections, their Newton-Schulz iterations and their NorMuon scales run as one launch each: the
+    first and the last are a few blocks that wait for memory, 5 to 15 us each on their own.  An iteration is a chain of 15 to 18 products;
     on small blocks each is one part-filled wave and most of its time is the way from one product to
     the next, which the products of the other runs fill.  Same kernels on the same values: the
     results are those of ``step_run`` on each."""
@@ -349,13 +373,25 @@ def step_runs(runs: Sequence[tuple[Bucket, Sequence[int]]], param_groups: Sequen
     buf = _workspace.carve(contexts[0].momentum.device, _group_plan([own for _, own in described], shapes, kinds))
     for i, (ctx, own) in enumerate(described):
         ctx.buf = {name: buf[f"{i}.{name}"] for name in own}
-        run_front(ctx)
+        if not ctx.selecting:
+            run_front(ctx)   # to its end: the copies of whole blocks share their scratch
+    selecting = [ctx for ctx in contexts if ctx.selecting]
+    if selecting:
+        for ctx in selecting:
+            _accumulate(ctx)
+        with _stage("select"):
+            _native.select_rows_group([(ctx.buf["scores"], ctx.buf["sumsq"], ctx.bucket.selected_rows, ctx.buf["index"],
+                                        ctx.buf["rowmap"], ctx.buf["frob"]) for ctx in selecting])
+        for ctx in selecting:
+            _pack(ctx)
     outs = [ctx.buf["x"].view(torch.bfloat16) for ctx in contexts]
     with _stage("newton_schulz"):
         _native.newton_schulz_group([ctx.buf["x"] for ctx in contexts], outs, shapes, kinds, buf["ns"],
                                     [ctx.buf["rowsq"] if _fused_row_sums(ctx) else None for ctx in contexts])
+    with _stage("finish"):
+        _native.normuon_rows_group([_scale_arguments(ctx) for ctx in contexts], NORMALIZATION_EPS)
     for ctx, out in zip(contexts, outs):
-        apply_result(_finish_run(ctx, out), ctx.group)
+        apply_result(_result(ctx, out), ctx.group)
 
 
 def prepare_run(bucket: Bucket, positions: Sequence[int], group: dict[str, Any],

@@ -11,7 +11,7 @@ from __future__ import annotations
 import ctypes
 from ctypes import POINTER, c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_uint8, c_void_p
 from pathlib import Path
-from typing import Sequence
+from typing import Any, Sequence
 
 import torch
 from torch import Tensor
@@ -48,6 +48,7 @@ SIGNATURES: dict[str, tuple[object, tuple[object, ...]]] = {
     "dionw_accumulate_copy_decay_run": (
         c_int, (_PP, c_int, _I64P, c_int, c_void_p, c_void_p, c_void_p, c_int64, c_float, c_int, c_void_p)),
     "dionw_select_rows": (c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p)),
+    "dionw_select_rows_group": (c_int, (c_int, _PP, _PP, _I64P, _I64P, _I64P, _PP, _PP, _PP, c_void_p)),
     "dionw_block_norms": (c_int, (c_void_p, c_int64, c_int64, c_void_p, c_void_p)),
     "dionw_pack_rows": (
         c_int, (c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_float, c_int, c_float, c_float,
@@ -78,6 +79,9 @@ SIGNATURES: dict[str, tuple[object, tuple[object, ...]]] = {
     "dionw_normuon_rows": (
         c_int, (c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_float, c_float, c_float,
                 c_void_p, c_int, c_void_p, c_void_p, c_void_p)),
+    "dionw_normuon_rows_group": (
+        c_int, (c_int, _PP, _I64P, _PP, _PP, _I64P, _I64P, _I64P, _I64P, POINTER(c_float), c_float, POINTER(c_float), _PP,
+                POINTER(c_int), _PP, _PP, c_void_p)),
     "dionw_apply_round": (
         c_int, (_PP, _I64P, _PP, _PP, _PP, _PP, c_int, c_int64, c_int64, c_int64, c_int64, c_float, c_void_p, c_int,
                 c_int, c_void_p, c_void_p)),
@@ -147,6 +151,10 @@ def _ptr(t: Tensor | None) -> int | None:
 
 def _ptr_array(tensors: Sequence[Tensor]):
     return (c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+
+def _optional_ptr_array(tensors: Sequence[Tensor | None]):
+    return (c_void_p * len(tensors))(*map(_ptr, tensors))
 
 
 def _i64_array(values: Sequence[int]):
@@ -223,6 +231,15 @@ def select_rows(scores: Tensor, sumsq: Tensor, k: int, index: Tensor, rowmap: Te
     blocks, rows = scores.shape
     _check(library().dionw_select_rows(scores.data_ptr(), sumsq.data_ptr(), blocks, rows, k, index.data_ptr(),
                                        rowmap.data_ptr(), frob.data_ptr(), _stream(scores)))
+
+
+def select_rows_group(runs: Sequence[tuple[Tensor, Tensor, int, Tensor, Tensor, Tensor]]) -> None:
+    """``select_rows`` of up to ``NS_GROUP_MAX`` runs in one launch; a run is the arguments of that."""
+    scores, sumsq, ks, index, rowmap, frob = zip(*runs)
+    _check(library().dionw_select_rows_group(
+        len(runs), _ptr_array(scores), _ptr_array(sumsq), _i64_array([t.shape[0] for t in sumsq]),
+        _i64_array([t.shape[1] for t in sumsq]), _i64_array(ks), _ptr_array(index), _ptr_array(rowmap),
+        _ptr_array(frob), _stream(frob[0])))
 
 
 def block_norms(sumsq: Tensor, frob: Tensor) -> None:
@@ -359,6 +376,21 @@ def normuon_rows(s: Tensor, variance: Tensor, index: Tensor | None, *, blocks: i
     _check(library().dionw_normuon_rows(s.data_ptr(), parts, variance.data_ptr(), _ptr(index), blocks, rows, k, cols,
                                         weight, eps, step, _ptr(step_device), int(normalize), denom.data_ptr(),
                                         scale.data_ptr(), _stream(s)))
+
+
+def normuon_rows_group(runs: Sequence[dict[str, Any]], eps: float) -> None:
+    """``normuon_rows`` of up to ``NS_GROUP_MAX`` runs in one launch; a run is its arguments by name."""
+    def values(key: str) -> list[Any]:
+        return [run[key] for run in runs]
+
+    n = len(runs)
+    floats = (c_float * n)
+    _check(library().dionw_normuon_rows_group(
+        n, _ptr_array(values("s")), _i64_array(values("parts")), _ptr_array(values("variance")),
+        _optional_ptr_array(values("index")), _i64_array(values("blocks")), _i64_array(values("rows")), _i64_array(values("k")),
+        _i64_array(values("cols")), floats(*values("weight")), eps, floats(*values("step")),
+        _optional_ptr_array(values("step_device")), (c_int * n)(*map(int, values("normalize"))), _ptr_array(values("denom")),
+        _ptr_array(values("scale")), _stream(runs[0]["s"])))
 
 
 def apply_run(weights: Sequence[Tensor], rows_per_tensor: Sequence[int], o: Tensor, rowmap: Tensor | None,

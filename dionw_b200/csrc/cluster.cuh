@@ -39,6 +39,9 @@ __device__ __forceinline__ uint32_t peer_load(const void* local, uint32_t rank) 
   return v;
 }
 
+// Runs whose per-block kernels (row selection, NorMuon scales) share a launch: as many as a plan takes batches.
+constexpr int kGroupRuns = 6;
+
 // CTAs that share one block of `rows` rows: one per `rows_per_cta`, at most the portable cluster size.
 // (The grid stays below 2^31 CTAs.)
 inline unsigned cluster_for(long long blocks, long long rows, long long rows_per_cta) {

@@ -409,11 +409,29 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 // rows in 28 dependent steps per pass: the four selections of a one-layer 8192-wide model took 254 us, on
 // clusters they take 141.  A CTA per 1024 rows, because below that a pass is one step and a larger cluster
 // only adds barriers.
+//
+// A launch takes the blocks of up to six runs: the selections of a step are some 10 us of latency each on a few SMs,
+// and side by side they take the time of one.  Every run keeps the cluster that its own rows ask for (the first CTAs of
+// the launch's), so that its sums have one order.
 constexpr int kKeep = 4;
 
+struct SelectRun {
+  const float* scores;
+  const float* sumsq;
+  int32_t* index;
+  int32_t* rowmap;
+  float* frob;
+  int rows, k;
+  unsigned ctas;         // of a cluster that work on a block
+  unsigned first_block;  // blocks of the runs before
+};
+struct SelectTable {
+  SelectRun run[kGroupRuns];
+  int n;
+};
+
 __global__ void __launch_bounds__(kSelectThreads)
-select_rows_kernel(const float* __restrict__ scores, const float* __restrict__ sumsq, int rows, int k,
-                   int32_t* __restrict__ index, int32_t* __restrict__ rowmap, float* __restrict__ frob) {
+select_rows_kernel(const __grid_constant__ SelectTable tab) {
   after_previous();
   __shared__ uint32_t hist[4][256];
   __shared__ uint32_t s_prefix, s_remaining;
@@ -421,10 +439,18 @@ select_rows_kernel(const float* __restrict__ scores, const float* __restrict__ s
   __shared__ uint32_t s_gt, s_eq;          // this CTA's rows above and at the threshold
   __shared__ float partial[kSelectThreads];
   const int tid = threadIdx.x;
-  const uint32_t rank = cluster_rank(), ctas = cluster_size();
-  const long long b = blockIdx.x / ctas;
-  const float* sc = scores + b * rows;
-  const float* ss = sumsq + b * rows;
+  const uint32_t rank = cluster_rank();
+  const unsigned block = blockIdx.x / cluster_size();
+  int at = 0;
+  while (at + 1 < tab.n && block >= tab.run[at + 1].first_block) ++at;
+  const SelectRun& run = tab.run[at];
+  const int rows = run.rows, k = run.k;
+  const uint32_t ctas = run.ctas;
+  int32_t* __restrict__ const index = run.index;
+  int32_t* __restrict__ const rowmap = run.rowmap;
+  const long long b = block - run.first_block;
+  const float* ss = run.sumsq + b * rows;
+  const float* sc = run.scores + b * rows;
   const int per = (rows + int(ctas) - 1) / int(ctas);
   const int first = min(rows, int(rank) * per), last = min(rows, first + per);
 
@@ -566,7 +592,7 @@ select_rows_kernel(const float* __restrict__ scores, const float* __restrict__ s
   if (rank == 0 && tid == 0) {
     float total = 0.0f;
     for (uint32_t c = 0; c < ctas; ++c) total = __fadd_rn(total, __uint_as_float(peer_load(&partial[0], c)));
-    frob[b] = sqrtf(total);
+    run.frob[b] = sqrtf(total);
   }
   cluster_sync();   // the other CTAs' shared memory stays until rank 0 has read it
 }
@@ -1002,15 +1028,31 @@ extern "C" int dionw_accumulate_copy_decay_run(const void* const* grads, int gra
   });
 }
 
+extern "C" int dionw_select_rows_group(int n, const float* const* scores, const float* const* sumsq, const int64_t* blocks,
+                                       const int64_t* rows, const int64_t* k, int32_t* const* index, int32_t* const* rowmap,
+                                       float* const* frob, void* stream_ptr) {
+  DIONW_REQUIRE(n >= 1 && n <= kGroupRuns, "select_rows_group: takes 1 to %d runs (got %d)", kGroupRuns, n);
+  SelectTable tab;
+  tab.n = n;
+  long long total = 0;
+  unsigned widest = 1;
+  for (int i = 0; i < n; ++i) {
+    DIONW_REQUIRE(blocks[i] > 0 && rows[i] > 0 && k[i] > 0 && k[i] <= rows[i], "select_rows: need 0 < k <= rows and blocks > 0");
+    DIONW_REQUIRE(rows[i] < (1LL << 30), "select_rows: too many rows");
+    const unsigned ctas = cluster_for(blocks[i], rows[i], kSelectThreads);
+    tab.run[i] = SelectRun{scores[i], sumsq[i], index[i], rowmap[i], frob[i], int(rows[i]), int(k[i]), ctas, unsigned(total)};
+    total += blocks[i];
+    widest = ctas > widest ? ctas : widest;
+  }
+  DIONW_REQUIRE(total * widest < (1LL << 31), "select_rows: too many blocks");
+  count_launch();
+  return check_cuda(launch_clusters(select_rows_kernel, unsigned(total), widest, kSelectThreads, static_cast<cudaStream_t>(stream_ptr), tab),
+                    "select_rows_kernel");
+}
+
 extern "C" int dionw_select_rows(const float* scores, const float* sumsq, int64_t blocks, int64_t rows, int64_t k,
                                  int32_t* index, int32_t* rowmap, float* frob, void* stream_ptr) {
-  DIONW_REQUIRE(blocks > 0 && rows > 0 && k > 0 && k <= rows, "select_rows: need 0 < k <= rows and blocks > 0");
-  DIONW_REQUIRE(rows < (1LL << 30), "select_rows: too many rows");
-  count_launch();
-  return check_cuda(launch_clusters(select_rows_kernel, unsigned(blocks), cluster_for(blocks, rows, kSelectThreads),
-                                    kSelectThreads, static_cast<cudaStream_t>(stream_ptr), scores, sumsq, int(rows), int(k), index, rowmap,
-                                    frob),
-                    "select_rows_kernel");
+  return dionw_select_rows_group(1, &scores, &sumsq, &blocks, &rows, &k, &index, &rowmap, &frob, stream_ptr);
 }
 
 extern "C" int dionw_block_norms(const float* sumsq, int64_t blocks, int64_t rows, float* frob, void* stream_ptr) {

@@ -65,21 +65,58 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 //
 // Bounded by latency: 2 MB at most.  With one CTA per block and a row per thread, one block of 2048 x 28672
 // took 94 us and two of 7168 x 8192 about as long; on eight CTAs they take 14 and 20.
+//
+// A launch takes the blocks of up to six runs, as the row selection does: on their own the scales of six runs of a
+// 1100-wide encoder took 10 us each between two weight updates.
 constexpr int kRowLanes = 8;
 
+struct NormuonRun {
+  const float* s;
+  float* variance;
+  const int32_t* index;      // null: every row
+  const float* step_device;  // null: step_host
+  float* denom;
+  float* scale;
+  int parts, rows, k;
+  float inv_count_cols, weight, step_host;
+  bool normalize;
+  unsigned ctas;             // of a cluster that work on a block
+  unsigned first_block;      // blocks of the runs before
+};
+struct NormuonTable {
+  NormuonRun run[kGroupRuns];
+  int n;
+};
+
 __global__ void __launch_bounds__(kReduceThreads)
-normuon_rows_kernel(const float* __restrict__ s, int parts, float* __restrict__ variance,
-                    const int32_t* __restrict__ index, int rows, int k, float inv_count_cols, float weight, float eps,
-                    float step_host, const float* __restrict__ step_device, bool normalize,
-                    float* __restrict__ denom, float* __restrict__ scale) {
+normuon_rows_kernel(const __grid_constant__ NormuonTable tab, float eps) {
   after_previous();
   __shared__ float scratch[kReduceThreads];
   __shared__ float s_totals[2];
-  const uint32_t rank = cluster_rank(), ctas = cluster_size();
-  const long long b = blockIdx.x / ctas;
+  const uint32_t rank = cluster_rank();
+  const unsigned block = blockIdx.x / cluster_size();
+  int at = 0;
+  while (at + 1 < tab.n && block >= tab.run[at + 1].first_block) ++at;
+  const NormuonRun& run = tab.run[at];
+  const float* __restrict__ const s = run.s;
+  float* __restrict__ const variance = run.variance;
+  const int32_t* __restrict__ const index = run.index;
+  float* __restrict__ const denom = run.denom;
+  float* __restrict__ const scale = run.scale;
+  const int parts = run.parts, rows = run.rows, k = run.k;
+  const float inv_count_cols = run.inv_count_cols, weight = run.weight;
+  const uint32_t ctas = run.ctas;
+  const long long b = block - run.first_block;
   const int tid = threadIdx.x;
-  const float step = step_device != nullptr ? *step_device : step_host;
-  if (!normalize) {
+  const float step = run.step_device != nullptr ? *run.step_device : run.step_host;
+  if (rank >= ctas) {   // a wider run of the launch has these CTAs: here they only keep the cluster's barriers
+    if (run.normalize) {
+      cluster_sync();
+      cluster_sync();
+    }
+    return;
+  }
+  if (!run.normalize) {
     for (int r = int(rank) * kReduceThreads + tid; r < k; r += int(ctas) * kReduceThreads) denom[b * k + r] = 1.0f;
     if (rank == 0 && tid == 0) scale[b] = step;
     return;
@@ -108,7 +145,7 @@ normuon_rows_kernel(const float* __restrict__ s, int parts, float* __restrict__ 
     for (int delta = kRowLanes / 2; delta >= 1; delta >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, delta);
     if (r < k && sub == 0) {
       const long long slot = b * rows + (index ? index[b * k + r] : r);
-      const float mean = sr * inv_count_cols;
+      const float mean = __fmul_rn(sr, inv_count_cols);   // rounded by itself: not merged into what follows
       const float old = variance[slot];
       // torch.lerp: start + weight * (end - start) for weight < 0.5, else the mirrored form.
       const float v = weight < 0.5f ? fmaf(weight, mean - old, old) : mean - (mean - old) * (1.0f - weight);
@@ -539,18 +576,38 @@ extern "C" int dionw_row_sumsq_bf16(const void* o, int64_t blocks, int64_t k, in
   return launch_status("row_sumsq_bf16_kernel");
 }
 
+extern "C" int dionw_normuon_rows_group(int n, const float* const* s, const int64_t* parts, float* const* variance,
+                                        const int32_t* const* index, const int64_t* blocks, const int64_t* rows,
+                                        const int64_t* k, const int64_t* cols, const float* weight, float eps,
+                                        const float* step, const float* const* step_device, const int* normalize,
+                                        float* const* denom, float* const* scale, void* stream_ptr) {
+  DIONW_REQUIRE(n >= 1 && n <= kGroupRuns, "normuon_rows_group: takes 1 to %d runs (got %d)", kGroupRuns, n);
+  NormuonTable tab;
+  tab.n = n;
+  long long total = 0;
+  unsigned widest = 1;
+  for (int i = 0; i < n; ++i) {
+    DIONW_REQUIRE(blocks[i] > 0 && rows[i] > 0 && k[i] > 0 && k[i] <= rows[i] && cols[i] > 0 && parts[i] >= 1 && parts[i] <= 4096,
+                  "normuon_rows: bad shape");
+    DIONW_REQUIRE(rows[i] < (1LL << 31), "normuon_rows: too many rows");
+    const unsigned ctas = cluster_for(blocks[i], k[i], kReduceThreads / kRowLanes);
+    tab.run[i] = NormuonRun{s[i], variance[i], index[i], step_device[i], denom[i], scale[i], int(parts[i]), int(rows[i]), int(k[i]),
+                            1.0f / float(cols[i]), weight[i], step[i], normalize[i] != 0, ctas, unsigned(total)};
+    total += blocks[i];
+    widest = ctas > widest ? ctas : widest;
+  }
+  DIONW_REQUIRE(total * widest < (1LL << 31), "normuon_rows: too many blocks");
+  count_launch();
+  return check_cuda(launch_clusters(normuon_rows_kernel, unsigned(total), widest, kReduceThreads, static_cast<cudaStream_t>(stream_ptr), tab, eps),
+                    "normuon_rows_kernel");
+}
+
 extern "C" int dionw_normuon_rows(const float* s, int64_t parts, float* variance, const int32_t* index, int64_t blocks,
                                   int64_t rows, int64_t k, int64_t cols, float weight, float eps, float step,
                                   const float* step_device, int normalize, float* denom, float* scale,
                                   void* stream_ptr) {
-  DIONW_REQUIRE(blocks > 0 && rows > 0 && k > 0 && k <= rows && cols > 0 && parts >= 1 && parts <= 4096,
-                "normuon_rows: bad shape");
-  count_launch();
-  return check_cuda(launch_clusters(normuon_rows_kernel, unsigned(blocks), cluster_for(blocks, k, kReduceThreads / kRowLanes),
-                                    kReduceThreads, static_cast<cudaStream_t>(stream_ptr), s, int(parts), variance, index,
-                                    int(rows), int(k), 1.0f / float(cols), weight, eps, step, step_device, normalize != 0,
-                                    denom, scale),
-                    "normuon_rows_kernel");
+  return dionw_normuon_rows_group(1, &s, &parts, &variance, &index, &blocks, &rows, &k, &cols, &weight, eps, &step, &step_device, &normalize,
+                                  &denom, &scale, stream_ptr);
 }
 
 extern "C" int dionw_apply_round(void* const* weights, const int64_t* rows_per_tensor, const void* const* o,

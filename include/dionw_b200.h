@@ -116,6 +116,13 @@ int dionw_select_rows(const float* scores, const float* sumsq, int64_t blocks,
                       int64_t rows, int64_t k, int32_t* index, int32_t* rowmap,
                       float* frob, void* stream);
 
+/* The same for n (1 to 6) runs in one launch.  The results are those of one call
+ * each. */
+int dionw_select_rows_group(int n, const float* const* scores, const float* const* sumsq,
+                            const int64_t* blocks, const int64_t* rows, const int64_t* k,
+                            int32_t* const* index, int32_t* const* rowmap,
+                            float* const* frob, void* stream);
+
 /* frob[b] = sqrt(sum_r sumsq[b, r]) for blocks that update every row. */
 int dionw_block_norms(const float* sumsq, int64_t blocks, int64_t rows, float* frob,
                       void* stream);
@@ -266,6 +273,16 @@ int dionw_normuon_rows(const float* s, int64_t parts, float* variance, const int
                        int64_t blocks, int64_t rows, int64_t k, int64_t cols,
                        float weight, float eps, float step, const float* step_device,
                        int normalize, float* denom, float* scale, void* stream);
+
+/* The same for n (1 to 6) runs in one launch; index[i] and step_device[i] may be
+ * NULL as there.  The results are those of one call each. */
+int dionw_normuon_rows_group(int n, const float* const* s, const int64_t* parts,
+                             float* const* variance, const int32_t* const* index,
+                             const int64_t* blocks, const int64_t* rows, const int64_t* k,
+                             const int64_t* cols, const float* weight, float eps,
+                             const float* step, const float* const* step_device,
+                             const int* normalize, float* const* denom, float* const* scale,
+                             void* stream);
 
 /* W <- W * decay_factor on every row (when has_decay), then
  * W[row] += (float(o[b, p, :]) / denom[b, p]) * scale[b] for each selected row

@@ -102,3 +102,40 @@ def test_apply(cols: int, selecting: bool, decay: float | None) -> None:
                        [denom[b * k:].data_ptr() for b in first], [scale[b:].data_ptr() for b in first], ldo=ld, rows=rows, k=k,
                        cols=cols, decay_factor=decay or 1.0, has_decay=decay is not None, decay_device=None, cta_warps=0, decay_job=None)
     assert torch.equal(torch.cat(weights).view(blocks, rows, cols), want)
+
+
+def test_selections_and_scales_of_several_runs_in_one_launch() -> None:
+    """Runs of one CTA to a block beside runs of eight: each gets what it gets alone, bit for bit."""
+    gen = _gen(1)
+    shapes = [(3, 300, 75), (1, 9000, 2000), (2, 1025, 1025), (5, 64, 1), (1, 4000, 3999), (2, 2048, 512)]   # blocks, rows, k
+    assert len(shapes) == native.NS_GROUP_MAX
+
+    def selection(scores: torch.Tensor, k: int) -> tuple:
+        index = torch.full((scores.shape[0], k), -7, dtype=torch.int32, device=DEV)
+        rowmap = torch.full(scores.shape, -7, dtype=torch.int32, device=DEV)
+        return scores, scores.square(), k, index, rowmap, torch.full((scores.shape[0],), 7.0, device=DEV)
+
+    scores = [torch.rand(blocks, rows, device=DEV, generator=gen) for blocks, rows, _ in shapes]
+    together = [selection(s, k) for s, (_, _, k) in zip(scores, shapes)]
+    native.select_rows_group(together)
+    for s, (_, _, k), run in zip(scores, shapes, together):
+        alone = selection(s, k)
+        native.select_rows(*alone)
+        assert all(torch.equal(run[i], alone[i]) for i in (3, 4, 5))
+
+    def scales(i: int) -> dict:
+        blocks, rows, k = shapes[i]
+        sums = torch.rand(blocks * k, 4, device=DEV, generator=_gen(i)) + 0.1
+        return {"s": sums, "parts": 4, "variance": torch.rand(blocks, rows, device=DEV, generator=_gen(i + 10)),
+                "index": None if i == 2 else together[i][3], "blocks": blocks, "rows": rows, "k": k, "cols": 500, "weight": 0.05 * (i + 1),
+                "step": -0.01 * (i + 1), "step_device": torch.tensor([0.5], device=DEV) if i == 1 else None, "normalize": i != 4,
+                "denom": torch.zeros(blocks * k, device=DEV), "scale": torch.zeros(blocks, device=DEV)}
+
+    grouped = [scales(i) for i in range(len(shapes))]
+    native.normuon_rows_group(grouped, 1e-8)
+    for i, run in enumerate(grouped):
+        alone = scales(i)
+        native.normuon_rows(**alone, eps=1e-8)
+        assert all(torch.equal(run[key], alone[key]) for key in ("variance", "denom", "scale"))
+    with pytest.raises(ValueError, match="1 to 6"):
+        native.select_rows_group(together + together[:1])
