@@ -438,7 +438,8 @@ int onchip_clusters(int pairs) {
   int value = slot.load(std::memory_order_acquire);
   if (value != 0) return value - 1;
   int clusters = 0;
-  if (cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(onchip::kSmemBytes)) == cudaSuccess) {
+  if (cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(onchip::kSmemBytes)) == cudaSuccess &&
+      cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(unsigned(2 * pairs));
     config.blockDim = dim3(onchip::kThreads);

@@ -1,5 +1,5 @@
 // The Gram iteration of a batch whose shorter side m is at most 256, as one launch in which a matrix never
-// leaves the SMs that work on it: a cluster of 1 to 4 SM pairs per matrix of the batch.  Every pair computes
+// leaves the SMs that work on it: a cluster of 1 to 8 SM pairs per matrix of the batch.  Every pair computes
 // G = X X^T over all of X and the whole chain of m x m products on it; only Q X, whose n columns are split,
 // is shared.  What pairs repeat costs no time (the other SMs have nothing to do) and saves every exchange
 // but one: a cluster barrier between X <- Q X and the next X X^T.
@@ -47,7 +47,9 @@ constexpr int kThreads = 32 * (kProducerWarp + 1);
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kBarrierBytes = 320;
 constexpr uint32_t kNowhereBytes = 32 * 16;
-constexpr int kMaxPairs = 4;
+// (Clusters above 8 CTAs are not portable, and only taken where the device says that all of them run at a time: 1 block of
+// 256 x 2048 82 -> 79 us with up to 8 pairs instead of 4, of 256 x 6000 134 -> 123.)
+constexpr int kMaxPairs = 8;
 constexpr size_t kSmemBytes = 1024 + size_t(kSlots) * kMatrixBytes + kBarrierBytes + kEpilogueWarps * kPieceBytes + kNowhereBytes;
 static_assert(kStages * kStageBytes == 2 * kMatrixBytes, "the ring lies over two slots");
 
