@@ -451,9 +451,13 @@ int onchip_clusters(int pairs) {
     attribute.val.clusterDim.z = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&clusters, onchip::iteration_kernel, &config) != cudaSuccess) clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, onchip::iteration_kernel, &config) != cudaSuccess) {
+      clusters = 0;
+      cudaGetLastError();   // not an error of the call: the plan takes the batch
+    }
+  } else {
+    cudaGetLastError();
   }
-  cudaGetLastError();   // what went wrong here shows at the launch
   slot.store(clusters + 1, std::memory_order_release);
   return clusters;
 }

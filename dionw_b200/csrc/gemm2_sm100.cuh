@@ -7,7 +7,7 @@
 // Roles per CTA: warp 0 = TMA producer for this CTA's operands; warp 1 = in the leader
 // CTA (cluster rank 0) the MMA issuer (idle in the other CTA); warps 2-9 = epilogue of this
 // CTA's 128 accumulator rows (the epilogue code is shared with the one-CTA kernel); warp 10 = in a plan
-// of several products the reporter of stored tiles.  Every
+// of several products the reporter of stored tiles; warp 11 = the scheduler, which hands out tiles.  Every
 // TMA load is a per-CTA load into the CTA's own shared memory (no multicast); both CTAs' loads
 // of a stage complete on ONE barrier, in the leader, which the .cta_group::2 form of the copy
 // permits; only the leader's producer announces the pair's byte count on it.  The other
@@ -36,9 +36,12 @@
 // one's four 8.9 -> 8.0 ms.  A plan's matrices need not lie in L2 for that: running them in cohorts of two
 // waves of tiles, each through all its products, changed nothing.
 //
-// What bounds a plan of small matrices now is the epilogue's chain of latencies: with clocks read inside the
-// kernel, an epilogue warp spent 4000 of 15000 cycles per 768-deep tile waiting for its accumulator.  Sixteen
-// epilogue warps, each with half the columns, were 10 to 25 % slower (96 registers a thread: spills).
+// What bounds it now, with clocks read inside the kernel, in cycles per tile (main loop / whole): K = 3584 29700 / 31800
+// (530 per k-block of 512), K = 1024 8900 / 11000, K = 768 6400 / 9200.  On long main loops that is the tensor cores'
+// rate at the clock the 1 kW cap leaves (1.25 GHz); on short ones the rest is the epilogue of products with a second
+// term (8300 cycles of latencies, eight warps deep) and the way to the next tile's first load.  Even 16 x 1024^2 and
+// 48 x 768^2 run into the cap (1.4 GHz): a cycle saved there is worth about half.  Sixteen epilogue warps, each with half
+// the columns, were 10 to 25 % slower (96 registers a thread: spills); five stages instead of six cost 1 %.
 //
 // Why a plan cannot deadlock, whatever else runs on the GPU: tiles are drawn in order by pairs that are
 // already running, and a tile depends only on tiles before it.  The earliest unfinished tile is therefore

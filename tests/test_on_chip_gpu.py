@@ -37,7 +37,7 @@ def _iterate(x: torch.Tensor, cols: int, kind: int, fill: int = 255) -> tuple[to
 
 
 # m at the edges of a 16-wide step, of 32-wide pieces, 64-wide panels and images, and of the second CTA's rows; n at
-# the edges of 64-wide k-blocks and 256-wide tiles, with one to four pairs to a matrix, tiles for some of them only,
+# the edges of 64-wide k-blocks and 256-wide tiles, with one to eight pairs to a matrix, tiles for some of them only,
 # and more matrices than clusters that run at a time
 @pytest.mark.parametrize("blocks, m, n", [
     (1, 65, 66), (2, 79, 257), (3, 80, 81), (1, 95, 1000), (2, 96, 512), (1, 97, 513), (2, 127, 128), (2, 128, 129),
