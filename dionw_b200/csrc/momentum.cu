@@ -987,8 +987,9 @@ extern "C" int dionw_accumulate_row_l1_run(const void* const* grads, int grad_dt
     if (cols >= kTeamScoreColumns) {
       auto launch = [&](auto g) {
         with_team_rows(cols, [&](auto n) {
-          launch_dependent(team_accumulate_row_l1_kernel<decltype(g), (n < 2 ? 1 : 2)>, unsigned((nrows + n - 1) / n), kTeamThreads, stream, tab, m,
-                           scores + row0, sumsq + row0, cols, nrows, vec);
+          constexpr int kRows = decltype(n)::value < 2 ? 1 : 2;   // of the kernel and of its grid; four need too many sums
+          launch_dependent(team_accumulate_row_l1_kernel<decltype(g), kRows>, unsigned((nrows + kRows - 1) / kRows), kTeamThreads, stream, tab,
+                           m, scores + row0, sumsq + row0, cols, nrows, vec);
         });
       };
       if (grad_dtype == DIONW_F32) launch(float());
