@@ -80,11 +80,11 @@ __device__ __forceinline__ void remote_arrive(uint32_t cluster_address) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 
-// Relaxed arrive that is issued once `loaded`, the result of a load, is there: the arrive is predicated on the
-// value, which is never kNoTile.  (Relaxed, so the memory model does not order the load before it; the
-// dependency does, since an instruction is not issued before its predicate is known.  The comparison is with
-// the largest integer because no branch on the sign of an entry's step decides it.)
-constexpr int kNoTile = 0x7FFFFFFF;   // no step has this number
+// Relaxed arrive that is issued once `loaded`, made of the results of one or more loads, is there: the arrive is
+// predicated on the value, which is never kNoTile.  (Relaxed, so the memory model does not order the loads before
+// it; the dependency does, since an instruction is not issued before its predicate is known.  The comparison is
+// with the largest integer because no branch on the sign of an entry's step decides it.)
+constexpr int kNoTile = 0x7FFFFFFF;   // no step, number of k-blocks or map
 __device__ __forceinline__ void remote_arrive_after(uint32_t cluster_address, int loaded) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %1, %2;\n"
                "@p mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}\n"
@@ -119,7 +119,7 @@ __device__ __forceinline__ void load_entry_word(const Entry* from, int i, Entry&
   asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
                : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(gemm::smem_u32(from) + 16 * i) : "memory");
 }
-// The entry, but for its last word(s) where they are not needed; the word that readers report on is read last.
+// The entry, but for its last word(s) where they are not needed; the tile itself is in the first, which is read last.
 template <int kWords>
 __device__ __forceinline__ Entry load_entry(const Entry* from) {
   Entry e{};
@@ -482,7 +482,10 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
     if (!warp_wait_cluster(&tile_full[slot], phase)) return none;
     const Entry e = load_entry<decltype(words)::value>(&tile_ring[slot]);
     if (kSteps > 1 && when_ready && e.step >= 0 && !warp_wait(&ready[slot], phase)) return none;
-    const int seen = __any_sync(0xffffffffu, e.step == kNoTile) ? kNoTile : 0;   // a value of every lane's load
+    // a value of every load of every lane
+    constexpr int kWords = decltype(words)::value;
+    const bool none_there = e.step == kNoTile || (kWords > 1 && e.k_blocks == kNoTile) || (kWords > 2 && e.map_a == kNoTile);
+    const int seen = __any_sync(0xffffffffu, none_there) ? kNoTile : 0;
     if (lane == 0) remote_arrive_after(leader_tile_empty + slot * uint32_t(sizeof(uint64_t)), seen);
     return e;
   };
