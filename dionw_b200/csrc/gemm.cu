@@ -526,6 +526,10 @@ int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* s
     }
     const Product& result = *list++;
     DIONW_REQUIRE(slot_of(tall ? result.b.base : result.a.base) == 2, "Q is the third slot's");
+    // X is loaded over the other two as soon as the chain's last product has been summed, while its epilogue still runs.
+    const onchip::Op& last = it.ops[part][it.count[part] - 1];
+    DIONW_REQUIRE(last.out == 2 && (last.cin == 2 || last.cin == -1) && (last.out2 == 2 || last.out2 == -1),
+                  "the epilogue of a chain's last product keeps to the third slot");
     it.result[part] = params_of(result);
     it.result_bf16[part] = result.out_dtype == DIONW_BF16;
   }

@@ -302,6 +302,8 @@ iteration_kernel(const __grid_constant__ Iteration it) {
           if (gemm2::elect_one()) commit_pair(&acc_full[op & 1], both);
           __syncwarp();
         }
+        // The ring may lie over slots 0 and 1 from here on: the last product's epilogue, which is still to come, reads
+        // and writes slot 2 only (run_on_chip checks the schedule for that).
         if (ok && gemm2::elect_one()) commit_pair(ring_free, both);
         __syncwarp();
         // Q X (X Q of a tall block)
