@@ -63,6 +63,7 @@ SIGNATURES: dict[str, tuple[object, tuple[object, ...]]] = {
     "dionw_newton_schulz_tall_workspace_bytes": (c_size_t, (c_int64, c_int64, c_int64, c_int)),
     "dionw_newton_schulz_tall": (
         c_int, (c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_size_t, c_void_p, c_void_p)),
+    "dionw_newton_schulz_on_chip_pairs": (c_int, (c_int64, c_int64, c_int64, c_int)),
     "dionw_newton_schulz_group_workspace_bytes": (c_size_t, (c_int, _I64P, _I64P, _I64P, POINTER(c_int))),
     "dionw_newton_schulz_group": (
         c_int, (c_int, _PP, _PP, _I64P, _I64P, _I64P, POINTER(c_int), c_void_p, c_size_t, _PP, c_void_p)),
@@ -310,6 +311,12 @@ def newton_schulz_tall(x: Tensor, out: Tensor, rows: int, cols: int, kind: int, 
     _check(library().dionw_newton_schulz_tall(x.data_ptr(), out.data_ptr(), x.shape[0], rows, cols, x.stride(-2), kind,
                                               workspace.data_ptr(), workspace.numel() * workspace.element_size(),
                                               _ptr(rowsq), _stream(x)))
+
+
+def newton_schulz_on_chip_pairs(blocks: int, rows: int, cols: int, kind: int) -> int:
+    """SM pairs to a matrix with which ``newton_schulz`` or ``newton_schulz_tall`` iterates such a batch on chip
+    on the current device; 0: through global memory."""
+    return int(library().dionw_newton_schulz_on_chip_pairs(blocks, rows, cols, kind))
 
 
 NS_GROUP_MAX = 6   # DIONW_NS_GROUP_MAX

@@ -431,32 +431,29 @@ int run_products(const Product* products, int count, int dtype, void* counters, 
 
 namespace {
 
-// Clusters of `pairs` SM pairs that the current device runs at a time, 0 where it cannot be told.
+// Clusters of `pairs` SM pairs that the current device runs at a time, 0 where it cannot be told (asked again then).
 int onchip_clusters(int pairs) {
-  static std::atomic<int> known[kMaxDevices][onchip::kMaxPairs + 1];   // + 1; zero: not asked yet
+  static std::atomic<int> known[kMaxDevices][onchip::kMaxPairs + 1];   // + 1; zero: not known yet
   std::atomic<int>& slot = known[current_device()][pairs];
   int value = slot.load(std::memory_order_acquire);
   if (value != 0) return value - 1;
   int clusters = 0;
-  if (cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(onchip::kSmemBytes)) == cudaSuccess &&
-      cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(unsigned(2 * pairs));
-    config.blockDim = dim3(onchip::kThreads);
-    config.dynamicSmemBytes = onchip::kSmemBytes;
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeClusterDimension;
-    attribute.val.clusterDim.x = unsigned(2 * pairs);
-    attribute.val.clusterDim.y = 1;
-    attribute.val.clusterDim.z = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&clusters, onchip::iteration_kernel, &config) != cudaSuccess) {
-      clusters = 0;
-      cudaGetLastError();   // not an error of the call: the plan takes the batch
-    }
-  } else {
-    cudaGetLastError();
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(unsigned(2 * pairs));
+  config.blockDim = dim3(onchip::kThreads);
+  config.dynamicSmemBytes = onchip::kSmemBytes;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = unsigned(2 * pairs);
+  attribute.val.clusterDim.y = 1;
+  attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  if (cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(onchip::kSmemBytes)) != cudaSuccess ||
+      cudaFuncSetAttribute(onchip::iteration_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, onchip::iteration_kernel, &config) != cudaSuccess) {
+    cudaGetLastError();   // not an error of the call: the plan takes the batch
+    return 0;
   }
   slot.store(clusters + 1, std::memory_order_release);
   return clusters;
@@ -478,13 +475,15 @@ int pairs_per_matrix(int64_t blocks, int64_t tiles) {
 // of 2048 379 and 412.  m = 96: 1 block of 1024 89 and 43, of 8192 138 and 126; 160 of 1024 196 and 152.
 constexpr int64_t kOnChipColumns = 6144, kOnChipColumnsInWaves = 1024;
 
-bool runs_on_chip(int64_t blocks, int64_t m, int64_t n) {
-  if (!use_cta_pairs() || m > onchip::kSide) return false;
+int on_chip_pairs(int64_t blocks, int64_t m, int64_t n) {
+  if (!use_cta_pairs() || m > onchip::kSide) return 0;
   const int wave = onchip_clusters(1);
-  return wave > 0 && n <= (blocks <= wave ? kOnChipColumns : kOnChipColumnsInWaves);
+  if (wave <= 0 || n > (blocks <= wave ? kOnChipColumns : kOnChipColumnsInWaves)) return 0;
+  return pairs_per_matrix(blocks, (n + onchip::kSide - 1) / onchip::kSide);
 }
 
-int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* slots, int n_slots, bool tall, cudaStream_t stream) {
+int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* slots, int n_slots, bool tall, int pairs,
+                cudaStream_t stream) {
   auto slot_of = [&](const void* base) -> int {
     for (int i = 0; i < n_slots; ++i)
       if (slots[i].base == base) return slots[i].slot;
@@ -533,8 +532,7 @@ int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* s
     it.result[part] = params_of(result);
     it.result_bf16[part] = result.out_dtype == DIONW_BF16;
   }
-  const int64_t tiles = (n + onchip::kSide - 1) / onchip::kSide;
-  it.pairs = pairs_per_matrix(blocks, tiles);
+  it.pairs = pairs;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(unsigned(2 * it.pairs * blocks));
   config.blockDim = dim3(onchip::kThreads);

@@ -230,12 +230,19 @@ size_t group_bytes(const Problem* problems, int n) {
 }
 
 // The list that append_products makes of a Gram iteration, on chip: products 1 to 5 and 8 to 16 are on m x m matrices.
-int iterate_on_chip(const Product* list, int count, bool tall, cudaStream_t stream) {
+int iterate_on_chip(const Product* list, int count, bool tall, int pairs, cudaStream_t stream) {
   const int lengths[2] = {5, 9};
   DIONW_REQUIRE(count == 4 + lengths[0] + lengths[1], "newton_schulz: the Gram schedule has 18 products");
   // G and RZ, Z, both Qs: RZ is written from G and G from RZ, each for the last time
   const ChainSlot slots[] = {{list[0].out.base, 0}, {list[2].out.base, 0}, {list[1].out.base, 1}, {list[1].out2, 2}, {list[5].out.base, 2}};
-  return run_on_chip(list, lengths, slots, 5, tall, stream);
+  return run_on_chip(list, lengths, slots, 5, tall, pairs, stream);
+}
+
+// SM pairs to a matrix with which a batch on its own is iterated on chip; 0: as a plan or product by product.
+int pairs_on_chip(const Problem& p, bool stepwise) {
+  if (stepwise || p.kind != DIONW_NS_GRAM || std::min(p.rows, p.cols) <= kStepwiseSide || plan_counter_bytes(p.blocks) == 0) return 0;
+  const Layout l = layout_of(p.blocks, p.rows, p.cols, p.ldx, p.kind);
+  return l.gram ? on_chip_pairs(p.blocks, l.m, l.n) : 0;
 }
 
 // Up to kMaxChains batches that are iterated in the same dtype, as one launch, or product by product.
@@ -263,11 +270,8 @@ int iterate(const Problem* problems, int n, bool stepwise, void* workspace, size
     first_block += problems[i].blocks;
   }
   const bool gram = problems[0].kind == DIONW_NS_GRAM || problems[0].kind == DIONW_NS_GRAM_FULL;
-  if (n == 1 && counters != nullptr && problems[0].kind == DIONW_NS_GRAM) {
-    const Layout l = layout_of(problems[0].blocks, problems[0].rows, problems[0].cols, problems[0].ldx, problems[0].kind);
-    if (l.gram && runs_on_chip(problems[0].blocks, l.m, l.n))
-      return iterate_on_chip(list, count, problems[0].rows > problems[0].cols, stream);
-  }
+  const int pairs = n == 1 ? pairs_on_chip(problems[0], stepwise) : 0;
+  if (pairs > 0) return iterate_on_chip(list, count, problems[0].rows > problems[0].cols, pairs, stream);
   return run_products(list, count, gram ? DIONW_F16 : DIONW_BF16, counters, stream);
 }
 
@@ -289,6 +293,13 @@ extern "C" size_t dionw_newton_schulz_workspace_bytes(int64_t blocks, int64_t m,
   if (blocks <= 0 || m <= 0 || n <= 0) return 0;
   const Problem problem{nullptr, nullptr, blocks, m, n, round_up(n, 8), kind & ~DIONW_NS_STEPWISE, nullptr};
   return group_bytes(&problem, 1) + 256;
+}
+
+extern "C" int dionw_newton_schulz_on_chip_pairs(int64_t blocks, int64_t rows, int64_t cols, int kind) {
+  using namespace dionw;
+  if (blocks <= 0 || rows <= 0 || cols <= 0) return 0;
+  const Problem problem{nullptr, nullptr, blocks, rows, cols, round_up(cols, 8), kind & ~DIONW_NS_STEPWISE, nullptr};
+  return pairs_on_chip(problem, (kind & DIONW_NS_STEPWISE) != 0);
 }
 
 extern "C" int64_t dionw_newton_schulz_rowsq_parts(int64_t n) { return n <= 0 ? 0 : 2 * ((n + 255) / 256); }

@@ -58,7 +58,9 @@ struct ChainSlot {
   const void* base;
   int slot;
 };
-bool runs_on_chip(int64_t blocks, int64_t m, int64_t n);   // whether that is the faster way
-int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* slots, int n_slots, bool tall, cudaStream_t stream);
+// SM pairs to a matrix on the current device where that is the faster way; 0 where it is not.
+int on_chip_pairs(int64_t blocks, int64_t m, int64_t n);
+int run_on_chip(const Product* list, const int* chain_length, const ChainSlot* slots, int n_slots, bool tall, int pairs,
+                cudaStream_t stream);
 
 }  // namespace dionw

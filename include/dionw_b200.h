@@ -191,6 +191,11 @@ int dionw_newton_schulz_tall(void* x, void* out, int64_t blocks, int64_t rows, i
                              int64_t ldx, int kind, void* workspace, size_t workspace_bytes,
                              float* rowsq, void* stream);
 
+/* SM pairs to a matrix with which dionw_newton_schulz (rows <= cols) or
+ * dionw_newton_schulz_tall iterates such a batch on chip on the current device; 0: as
+ * one launch through global memory, or product by product.  The results are the same. */
+int dionw_newton_schulz_on_chip_pairs(int64_t blocks, int64_t rows, int64_t cols, int kind);
+
 /* The iterations of up to DIONW_NS_GROUP_MAX batches of different shapes (wide, square or tall, ldx =
  * cols rounded up to 8) as one launch: the products of one batch fill the GPU while those of another
  * wait for one another.  All kinds of a group iterate in the same dtype.  rowsq (nullable) holds one

@@ -49,6 +49,11 @@ def test_small_blocks_on_chip_have_the_bits_of_their_products(blocks: int, m: in
     rows, cols = (n, m) if tall else (m, n)
     x = _operand(blocks, rows, cols)
     want, want_sums = _iterate(x, cols, native.NS_GRAM + STEPWISE)
+    # Columns that make a matrix too wide to be the faster on chip: 6144, and 1024 where a wave of pairs is too small.
+    wave = torch.cuda.get_device_properties(DEV).multi_processor_count // 2
+    pairs = native.newton_schulz_on_chip_pairs(blocks, rows, cols, native.NS_GRAM)
+    assert (pairs > 0) == (n <= (6144 if blocks <= wave else 1024))
+    assert pairs <= -(-n // 256) and (pairs > 1 or blocks > 1 or n <= 256 or n > 6144)
     before = native.launch_count()
     got, sums = _iterate(x, cols, native.NS_GRAM)
     assert native.launch_count() - before == 1
@@ -57,6 +62,15 @@ def test_small_blocks_on_chip_have_the_bits_of_their_products(blocks: int, m: in
         again, sums = _iterate(x, cols, native.NS_GRAM)
         assert torch.equal(again, want) and torch.equal(sums, want_sums)
     assert native.device_status() == 0
+
+
+def test_what_is_not_iterated_on_chip() -> None:
+    pairs = native.newton_schulz_on_chip_pairs
+    assert pairs(1, 256, 4096, native.NS_GRAM) == pairs(1, 4096, 256, native.NS_GRAM) == 8
+    for kind in (native.NS_GRAM + STEPWISE, native.NS_GRAM_FULL, native.NS_POLAR_EXPRESS, native.NS_KELLER):
+        assert pairs(1, 256, 4096, kind) == 0
+    for blocks, rows, cols in ((1, 257, 1024), (1, 64, 1024), (1, 256, 256), (20000, 96, 128), (0, 256, 1024)):
+        assert pairs(blocks, rows, cols, native.NS_GRAM) == 0
 
 
 def test_small_blocks_on_chip_in_two_streams() -> None:
