@@ -150,12 +150,15 @@ constexpr int kTeamChunks = 4;
 // and 34, a quarter of 4 x 2048 x 2560 18.4 and 16.4, of 4 x 1024 x 4096 20 and 14; odd rows, a quarter of 8 x 700 x 701
 // 16 and 18, of 6 x 2930 x 1101 22 and 20.
 constexpr int kTeamScoreColumns = 1025, kTeamCopyColumns = 768, kTeamPackColumns = 2560, kTeamOddColumns = 1024;
-inline int team_rows(long long cols) { return cols <= 1024 ? 4 : cols <= 2048 ? 2 : 1; }
+// Four rows at a time only where they go in 16-byte accesses: in shorter ones a thread has four times the addresses and
+// bounds, and copies of fp32 take, warps / four rows / two, us: 4000 x 1001 17.9 / 24.0 / 16.1, 30000 x 770 88 / 110 / 84,
+// 1500 x 1024 off the boundary 8.4 / 11.2 / 7.7; of bf16 30000 x 1001 189 / 157 / 126.
+inline int team_rows(long long cols, bool vec) { return cols <= 1024 && vec ? 4 : cols <= 2048 ? 2 : 1; }
 
 // Calls fn(std::integral_constant<int, rows at a time>).
 template <typename Fn>
-auto with_team_rows(long long cols, Fn&& fn) {
-  switch (team_rows(cols)) {
+auto with_team_rows(long long cols, bool vec, Fn&& fn) {
+  switch (team_rows(cols, vec)) {
     case 4: return fn(std::integral_constant<int, 4>());
     case 2: return fn(std::integral_constant<int, 2>());
     default: return fn(std::integral_constant<int, 1>());
@@ -986,7 +989,7 @@ extern "C" int dionw_accumulate_row_l1_run(const void* const* grads, int grad_dt
     float* m = momentum + row0 * cols;
     if (cols >= kTeamScoreColumns) {
       auto launch = [&](auto g) {
-        with_team_rows(cols, [&](auto n) {
+        with_team_rows(cols, vec, [&](auto n) {
           constexpr int kRows = decltype(n)::value < 2 ? 1 : 2;   // of the kernel and of its grid; four need too many sums
           launch_dependent(team_accumulate_row_l1_kernel<decltype(g), kRows>, unsigned((nrows + kRows - 1) / kRows), kTeamThreads, stream, tab,
                            m, scores + row0, sumsq + row0, cols, nrows, vec);
@@ -1023,7 +1026,7 @@ extern "C" int dionw_accumulate_copy_decay_run(const void* const* grads, int gra
     const bool nest = nesterov != 0;
     if (cols >= kTeamCopyColumns) {
       auto launch = [&](auto g) {
-        with_team_rows(cols, [&](auto n) {
+        with_team_rows(cols, vec, [&](auto n) {
           launch_dependent(team_accumulate_copy_decay_kernel<decltype(g), decltype(n)::value>, unsigned((nrows + n - 1) / n), kTeamThreads, stream, tab,
                            m, out, sumsq + row0, cols, nrows, decay, nest, vec);
         });

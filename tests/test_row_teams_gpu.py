@@ -49,6 +49,24 @@ def test_accumulate(cols: int, dtype: torch.dtype) -> None:
         assert squares_close(sumsq, u[0])
 
 
+@pytest.mark.parametrize("cols", [768, 1000, 1024, 1536, 2048, 4096])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_accumulate_gradients_off_a_boundary(cols: int, dtype: torch.dtype) -> None:
+    """Gradients that start one element behind a 16-byte boundary, in rows that 4 divides: no wide access is allowed."""
+    gen = _gen(cols)
+    rows = [2, 5]
+    grads = [torch.randn(r * cols + 1, device=DEV, generator=gen).to(dtype)[1:].view(r, cols) for r in rows]
+    start = torch.randn(1, sum(rows), cols, device=DEV, generator=gen)
+    total = start[0] + torch.cat(grads).float()
+    momentum, u = start.clone(), torch.empty_like(start)
+    scores, sumsq = (torch.full((1, sum(rows)), 7.0, device=DEV) for _ in range(2))
+    native.accumulate_copy_decay_run(grads, rows, momentum, u, sumsq, cols, 0.95, False)
+    assert torch.equal(momentum[0], total * 0.95) and torch.equal(u[0], total)
+    momentum = start.clone()
+    native.accumulate_row_l1_run(grads, rows, momentum, scores, sumsq, cols)
+    assert torch.equal(momentum[0], total) and torch.equal(scores.cpu(), oracle.row_scores(total.cpu()).view(1, -1))
+
+
 @pytest.mark.parametrize("cols", COLS)
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("selecting", [False, True])
