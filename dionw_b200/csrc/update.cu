@@ -1,5 +1,6 @@
 // NorMuon row statistics, the fused decay + update of the weights, fused
 // AdamW and the EMA passes.  All HBM-bound streaming kernels.
+#include <algorithm>
 #include <type_traits>
 
 #include "cluster.cuh"
@@ -284,6 +285,21 @@ constexpr int kTeamThreads = kWarpsPerBlock * 32;
 // 2304 50 us by warps and 54 so, a quarter of 4 x 2048 x 2560 46 and 38; 4 x 1500 x 257 19.5 and 21.5, 8 x 300 x 302 19.5
 // and 13.4.
 constexpr int kTeamColumns = 2560, kTeamOddColumns = 300;
+// Where most rows are left as they are, or only decayed, a CTA that comes for one row costs more than it does: 1.05 ns of
+// the launch for a row that it does not touch (60000 rows: 64 us), while fewer rows than the GPU holds at a time cost a
+// warp each its latency all the same.  So this is taken where a row's share of what is updated (with a decay, plus an eighth of
+// the rest) is enough for the number of rows.  A warp to a row against this, cold, us, at rows x columns and elements per row;
+// 16-byte accesses, no decay: 14000 x 2560 160 18.5 and 17.1; 20000 x 4096 256 28 and 23; 30000 x 2560 320 35 and 37, 640 55
+// and 48; 60000 x 4096 256 44 and 65, 512 78 and 76.  (With a decay they are faster here: 30000 x 2560, a sixteenth, 107 and 96.)
+// Shorter ones, no decay: 5000 x 302 19 6.0 and 6.9, 8000 x 513 32 even, 14000 x 1022 64 20 and 17, 60000 x 351 88 76 and 78, 302
+// 75 72 and 79; with a decay 5000 x 401 72 12.8 and 11.3, 8000 x 401 72 16.8 and 17.2, 60000 x 401 138 and 802 144 even.
+inline bool team_pays(bool wide, long long launch_rows, int64_t rows, int64_t k, int64_t cols, bool has_decay) {
+  if (cols < (wide ? kTeamColumns : kTeamOddColumns)) return false;
+  if (wide && has_decay) return true;
+  const double n = double(launch_rows), updated = double(cols) * double(k) / double(rows);
+  if (wide) return updated >= std::min(512.0, (n - 16384) / 32);
+  return has_decay ? updated + (double(cols) - updated) / 8 >= std::min(125.0, n / 96) : updated >= std::min(80.0, n / 250);
+}
 template <int kSpan>
 __global__ void __launch_bounds__(kTeamThreads, 5)
 team_apply_run_kernel(const ApplyTable tab, int ldo, int rows, int k, int cols, float decay_host,
@@ -641,7 +657,7 @@ extern "C" int dionw_apply_round(void* const* weights, const int64_t* rows_per_t
       tab.e[i] = ApplyEntry{static_cast<float*>(weights[t]), static_cast<const uint16_t*>(o[t]),
                             rowmap ? rowmap[t] : nullptr, denom[t], scale[t], acc};
     }
-    if (acc > 0 && aligned && cols >= (span == 4 ? kTeamColumns : kTeamOddColumns) && cta_warps == 0 && decay_job == nullptr &&
+    if (acc > 0 && aligned && team_pays(span == 4, acc, rows, k, cols, has_decay != 0) && cta_warps == 0 && decay_job == nullptr &&
         acc <= 0x7FFFFFFFll) {
       auto launch = [&](auto n) {
         launch_dependent(team_apply_run_kernel<decltype(n)::value>, unsigned(acc), kTeamThreads, stream, tab, int(ldo), int(rows), int(k),

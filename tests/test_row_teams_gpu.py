@@ -132,6 +132,26 @@ def test_apply(cols: int, selecting: bool, decay: float | None) -> None:
     assert torch.equal(torch.cat(weights).view(blocks, rows, cols), want)
 
 
+# sparse updates of many rows, on both sides of each line at which the launch changes with their number and share
+@pytest.mark.parametrize("rows, k, cols, decay", [
+    (2000, 40, 302, None), (6000, 400, 302, None), (6000, 500, 302, None), (20000, 5290, 302, None), (20000, 5310, 302, None),
+    (4000, 10, 302, 0.9), (5200, 400, 302, 0.9), (12000, 3950, 302, 0.9), (12000, 3975, 302, 0.9), (16384, 1, 2560, None),
+    (16500, 20, 2560, None), (16500, 50, 2560, None), (32768, 6553, 2560, None), (32768, 6554, 2560, None), (32768, 1, 2560, 0.9)])
+def test_apply_few_of_many_rows(rows: int, k: int, cols: int, decay: float | None) -> None:
+    gen = _gen(cols)
+    weight = torch.randn(rows, cols, device=DEV, generator=gen)
+    update = torch.randn(1, k, (cols + 7) // 8 * 8, device=DEV, generator=gen).bfloat16()
+    denom, scale = torch.rand(k, device=DEV, generator=gen) + 0.5, torch.rand(1, device=DEV, generator=gen)
+    chosen = torch.randperm(rows, device=DEV, generator=gen)[:k].sort().values
+    rowmap = torch.full((1, rows), -1, dtype=torch.int32, device=DEV)
+    rowmap[0, chosen] = torch.arange(k, dtype=torch.int32, device=DEV)
+    want = weight * decay if decay is not None else weight.clone()
+    want[chosen] += update[0, :, :cols].float() / denom[:, None] * scale
+    native.apply_run([weight], [rows], update, rowmap, denom, scale, rows=rows, k=k, cols=cols, decay_factor=decay or 1.0,
+                     has_decay=decay is not None)
+    assert torch.equal(weight, want)
+
+
 def test_selections_and_scales_of_several_runs_in_one_launch() -> None:
     """Runs of one CTA to a block beside runs of eight: each gets what it gets alone, bit for bit."""
     gen = _gen(1)
