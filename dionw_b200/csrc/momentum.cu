@@ -150,11 +150,17 @@ constexpr int kTeamChunks = 4;
 // and 34, a quarter of 4 x 2048 x 2560 18.4 and 16.4, of 4 x 1024 x 4096 20 and 14; odd rows, a quarter of 8 x 700 x 701
 // 16 and 18, of 6 x 2930 x 1101 22 and 20.
 constexpr int kTeamScoreColumns = 1025, kTeamCopyColumns = 768, kTeamPackColumns = 2560, kTeamOddColumns = 1024;
-// Whole blocks in short accesses: a warp takes its row from L2, where the copying pass has left it, in the time that
-// a CTA needs to come and go, so the more rows there are the longer they have to be.  After the copying pass, a warp to a
-// row against a team, us: 2724 x 1101 9.0 and 8.0, 5449 x 1101 12.2 and 13.9, 20435 x 1101 37 and 49; 5002 x 1999 17.7 and
-// 15.5, 11255 x 1999 33 and 33 (bf16 33 and 35), 31265 x 1999 78 and 97; 4164 x 2401 18 and 14; 22305 x 2802 87 and 81.
-inline int team_odd_columns(bool whole, long long rows) { return !whole || rows <= 4096 ? kTeamOddColumns : rows <= 8192 ? 1600 : kTeamPackColumns; }
+// Whole blocks: a warp takes its row from L2, where the copying pass has left it, in the time that a CTA needs to come and
+// go, so the more rows there are the longer they have to be, and longer still for bf16, whose three roundings hold a CTA up.
+// After the copying pass, a warp to a row against a team, us.  16-byte accesses: 5859 x 2560 18.7 and 17.5 (bf16 19.8 and 20.6),
+// 12695 x 2560 34 and 37, 10579 x 3072 36 and 35 (38 and 42), 15258 x 4096 69 and 65 (71 and 76), 36621 x 4096 162 and 163 (165
+// and 184), 24414 x 6144 164 and 151 (167 and 173), 10172 x 6144 (74 and 72).  Shorter ones: 2724 x 1101 9.0 and 8.0, 5449 x 1101 12.2
+// and 13.9, 20435 x 1101 37 and 49; 5002 x 1999 17.7 and 15.5, 11255 x 1999 33 and 33 (33 and 35), 31265 x 1999 78 and 97; 4164 x
+// 2401 18 and 14; 22305 x 2802 87 and 81.
+inline int team_whole_columns(int span, bool bf16, long long rows) {
+  if (span != 4) return rows <= 4096 ? kTeamOddColumns : rows <= 8192 ? 1600 : 2560;
+  return rows <= 8192 ? kTeamPackColumns : rows <= 16384 ? (bf16 ? 4096 : 3072) : bf16 ? 6144 : 4096;
+}
 // Four rows at a time only where they go in 16-byte accesses: in shorter ones a thread has four times the addresses and
 // bounds, and copies of fp32 take, warps / four rows / two, us: 4000 x 1001 17.9 / 24.0 / 16.1, 30000 x 770 88 / 110 / 84,
 // 1500 x 1024 off the boundary 8.4 / 11.2 / 7.7; of bf16 30000 x 1001 189 / 157 / 126.
@@ -1095,7 +1101,8 @@ extern "C" int dionw_pack_rows(float* src, const int32_t* index, const float* fr
   const unsigned grid = unsigned((total + kWarpsPerBlock - 1) / kWarpsPerBlock);
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   const int span = span_of(cols, ldx);
-  if (aligned16(src) && aligned16(x) && cols >= (span == 4 ? kTeamPackColumns : team_odd_columns(index == nullptr, total)) && total <= 0x7FFFFFFFll) {
+  const int team_columns = index == nullptr ? team_whole_columns(span, x_dtype == DIONW_BF16, total) : span == 4 ? kTeamPackColumns : kTeamOddColumns;
+  if (aligned16(src) && aligned16(x) && cols >= team_columns && total <= 0x7FFFFFFFll) {
     auto launch = [&](auto bf16, auto n) {
       launch_dependent(team_pack_rows_kernel<decltype(bf16)::value, decltype(n)::value>, unsigned(total), kTeamThreads, stream, src, index, frob,
                        rows, k, cols, decay, decay_rows != 0, eps, norm_scale, static_cast<uint16_t*>(x), ldx);

@@ -92,14 +92,17 @@ def test_pack(cols: int, dtype: torch.dtype, selecting: bool) -> None:
     assert torch.equal(after, source)
 
 
-# whole blocks of odd rows on both sides of each line at which the launch changes with their number
-@pytest.mark.parametrize("rows, cols", [(4096, 1025), (4097, 1025), (4097, 1602), (8192, 1601), (8193, 1601), (8193, 2561)])
-def test_pack_whole_blocks_of_odd_rows(rows: int, cols: int) -> None:
+# whole blocks on both sides of each line at which the launch changes with the number of rows
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows, cols", [(4096, 1025), (4097, 1025), (4097, 1602), (8192, 1601), (8193, 1601), (8193, 2561), (8192, 2560), (8193, 2560),
+                                        (8193, 3072), (8193, 4096), (16385, 4096), (16385, 6144)])
+def test_pack_many_whole_blocks(rows: int, cols: int, dtype: torch.dtype) -> None:
     source = torch.randn(1, rows, cols, device=DEV, generator=_gen(cols))
     frob = torch.tensor([5.0], device=DEV)
-    x = torch.full((1, rows, (cols + 7) // 8 * 8), 77.0, dtype=torch.float16, device=DEV)
-    native.pack_rows(source, None, frob, rows, x, decay=1.0, decay_rows=False, eps=1e-3)
-    assert torch.equal(x[..., :cols], (source / (frob + 1e-3)).half()) and bool((x[..., cols:] == 0).all())
+    x = torch.full((1, rows, (cols + 7) // 8 * 8), 77.0, dtype=dtype, device=DEV)
+    native.pack_rows(source, None, frob, rows, x, decay=1.0, decay_rows=False, eps=1e-3, norm_scale=1.02)
+    want = (source / (frob + 1e-3)).half() if dtype is torch.float16 else source.bfloat16() / (frob.bfloat16() * 1.02 + 1e-3)
+    assert torch.equal(x[..., :cols], want) and bool((x[..., cols:] == 0).all())
 
 
 @pytest.mark.parametrize("cols", COLS)
