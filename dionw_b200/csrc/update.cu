@@ -290,12 +290,13 @@ constexpr int kTeamColumns = 2560, kTeamOddColumns = 300;
 // warp each its latency all the same.  So this is taken where a row's share of what is updated (with a decay, plus an eighth of
 // the rest) is enough for the number of rows.  A warp to a row against this, cold, us, at rows x columns and elements per row;
 // 16-byte accesses, no decay: 14000 x 2560 160 18.5 and 17.1; 20000 x 4096 256 28 and 23; 30000 x 2560 320 35 and 37, 640 55
-// and 48; 60000 x 4096 256 44 and 65, 512 78 and 76.  (With a decay they are faster here: 30000 x 2560, a sixteenth, 107 and 96.)
+// and 48; 60000 x 4096 256 44 and 65, 512 78 and 76.  (With a decay they are faster here, 30000 x 2560, a sixteenth, 107 and 96, but for the
+// shortest of many rows that are all updated: 14000 x 2560 62 and 66, 2816 68 and 70, 3072 74 and 73; 6000 x 2560 30 and 30.)
 // Shorter ones, no decay: 5000 x 302 19 6.0 and 6.9, 8000 x 513 32 even, 14000 x 1022 64 20 and 17, 60000 x 351 88 76 and 78, 302
 // 75 72 and 79; with a decay 5000 x 401 72 12.8 and 11.3, 8000 x 401 72 16.8 and 17.2, 60000 x 401 138 and 802 144 even.
 inline bool team_pays(bool wide, long long launch_rows, int64_t rows, int64_t k, int64_t cols, bool has_decay) {
   if (cols < (wide ? kTeamColumns : kTeamOddColumns)) return false;
-  if (wide && has_decay) return true;
+  if (wide && has_decay) return k < rows || cols >= 2944 || launch_rows <= 8192;
   const double n = double(launch_rows), updated = double(cols) * double(k) / double(rows);
   if (wide) return updated >= std::min(512.0, (n - 16384) / 32);
   return has_decay ? updated + (double(cols) - updated) / 8 >= std::min(125.0, n / 96) : updated >= std::min(80.0, n / 250);

@@ -139,7 +139,8 @@ def test_apply(cols: int, selecting: bool, decay: float | None) -> None:
 @pytest.mark.parametrize("rows, k, cols, decay", [
     (2000, 40, 302, None), (6000, 400, 302, None), (6000, 500, 302, None), (20000, 5290, 302, None), (20000, 5310, 302, None),
     (4000, 10, 302, 0.9), (5200, 400, 302, 0.9), (12000, 3950, 302, 0.9), (12000, 3975, 302, 0.9), (16384, 1, 2560, None),
-    (16500, 20, 2560, None), (16500, 50, 2560, None), (32768, 6553, 2560, None), (32768, 6554, 2560, None), (32768, 1, 2560, 0.9)])
+    (16500, 20, 2560, None), (16500, 50, 2560, None), (32768, 6553, 2560, None), (32768, 6554, 2560, None), (32768, 1, 2560, 0.9),
+    (8192, 8192, 2560, 0.9), (8193, 8193, 2560, 0.9), (8193, 8193, 2944, 0.9)])
 def test_apply_few_of_many_rows(rows: int, k: int, cols: int, decay: float | None) -> None:
     gen = _gen(cols)
     weight = torch.randn(rows, cols, device=DEV, generator=gen)
