@@ -450,13 +450,15 @@ struct SelectRun {
   unsigned ctas;         // of a cluster that work on a block
   unsigned first_block;  // blocks of the runs before
 };
+template <int kRuns>
 struct SelectTable {
-  SelectRun run[kGroupRuns];
+  SelectRun run[kRuns];
   int n;
 };
 
+template <int kRuns>
 __global__ void __launch_bounds__(kSelectThreads)
-select_rows_kernel(const __grid_constant__ SelectTable tab) {
+select_rows_kernel(const __grid_constant__ SelectTable<kRuns> tab) {
   after_previous();
   __shared__ uint32_t hist[4][256];
   __shared__ uint32_t s_prefix, s_remaining;
@@ -466,11 +468,13 @@ select_rows_kernel(const __grid_constant__ SelectTable tab) {
   const int tid = threadIdx.x;
   const uint32_t rank = cluster_rank();
   const unsigned block = blockIdx.x / cluster_size();
-  int at = 0;
-  while (at + 1 < tab.n && block >= tab.run[at + 1].first_block) ++at;
+  int at = 0;   // a constant, and with it where the run's values lie, for a run on its own
+  if constexpr (kRuns > 1) {
+    while (at + 1 < tab.n && block >= tab.run[at + 1].first_block) ++at;
+  }
   const SelectRun& run = tab.run[at];
   const int rows = run.rows, k = run.k;
-  const uint32_t ctas = run.ctas;
+  const uint32_t ctas = kRuns > 1 ? run.ctas : cluster_size();
   int32_t* __restrict__ const index = run.index;
   int32_t* __restrict__ const rowmap = run.rowmap;
   const long long b = block - run.first_block;
@@ -1061,7 +1065,7 @@ extern "C" int dionw_select_rows_group(int n, const float* const* scores, const 
                                        const int64_t* rows, const int64_t* k, int32_t* const* index, int32_t* const* rowmap,
                                        float* const* frob, void* stream_ptr) {
   DIONW_REQUIRE(n >= 1 && n <= kGroupRuns, "select_rows_group: takes 1 to %d runs (got %d)", kGroupRuns, n);
-  SelectTable tab;
+  SelectTable<kGroupRuns> tab;
   tab.n = n;
   long long total = 0;
   unsigned widest = 1;
@@ -1074,9 +1078,12 @@ extern "C" int dionw_select_rows_group(int n, const float* const* scores, const 
     widest = ctas > widest ? ctas : widest;
   }
   DIONW_REQUIRE(total * widest < (1LL << 31), "select_rows: too many blocks");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   count_launch();
-  return check_cuda(launch_clusters(select_rows_kernel, unsigned(total), widest, kSelectThreads, static_cast<cudaStream_t>(stream_ptr), tab),
-                    "select_rows_kernel");
+  if (n == 1)
+    return check_cuda(launch_clusters(select_rows_kernel<1>, unsigned(total), widest, kSelectThreads, stream, SelectTable<1>{{tab.run[0]}, 1}),
+                      "select_rows_kernel");
+  return check_cuda(launch_clusters(select_rows_kernel<kGroupRuns>, unsigned(total), widest, kSelectThreads, stream, tab), "select_rows_kernel");
 }
 
 extern "C" int dionw_select_rows(const float* scores, const float* sumsq, int64_t blocks, int64_t rows, int64_t k,

@@ -84,20 +84,24 @@ struct NormuonRun {
   unsigned ctas;             // of a cluster that work on a block
   unsigned first_block;      // blocks of the runs before
 };
+template <int kRuns>
 struct NormuonTable {
-  NormuonRun run[kGroupRuns];
+  NormuonRun run[kRuns];
   int n;
 };
 
+template <int kRuns>
 __global__ void __launch_bounds__(kReduceThreads)
-normuon_rows_kernel(const __grid_constant__ NormuonTable tab, float eps) {
+normuon_rows_kernel(const __grid_constant__ NormuonTable<kRuns> tab, float eps) {
   after_previous();
   __shared__ float scratch[kReduceThreads];
   __shared__ float s_totals[2];
   const uint32_t rank = cluster_rank();
   const unsigned block = blockIdx.x / cluster_size();
-  int at = 0;
-  while (at + 1 < tab.n && block >= tab.run[at + 1].first_block) ++at;
+  int at = 0;   // a constant, and with it where the run's values lie, for a run on its own
+  if constexpr (kRuns > 1) {
+    while (at + 1 < tab.n && block >= tab.run[at + 1].first_block) ++at;
+  }
   const NormuonRun& run = tab.run[at];
   const float* __restrict__ const s = run.s;
   float* __restrict__ const variance = run.variance;
@@ -139,13 +143,13 @@ normuon_rows_kernel(const __grid_constant__ NormuonTable tab, float eps) {
           sr += q.x + q.y;
         }
       } else {
-        for (int j = sub; j < parts; j += kRowLanes) sr += partial[j];
+        for (int j = sub; j < parts; j += kRowLanes) sr += __ldg(partial + j);
       }
     }
 #pragma unroll
     for (int delta = kRowLanes / 2; delta >= 1; delta >>= 1) sr += __shfl_xor_sync(0xffffffffu, sr, delta);
     if (r < k && sub == 0) {
-      const long long slot = b * rows + (index ? index[b * k + r] : r);
+      const long long slot = b * rows + (index ? __ldg(index + b * k + r) : r);
       const float mean = __fmul_rn(sr, inv_count_cols);   // rounded by itself: not merged into what follows
       const float old = variance[slot];
       // torch.lerp: start + weight * (end - start) for weight < 0.5, else the mirrored form.
@@ -599,7 +603,7 @@ extern "C" int dionw_normuon_rows_group(int n, const float* const* s, const int6
                                         const float* step, const float* const* step_device, const int* normalize,
                                         float* const* denom, float* const* scale, void* stream_ptr) {
   DIONW_REQUIRE(n >= 1 && n <= kGroupRuns, "normuon_rows_group: takes 1 to %d runs (got %d)", kGroupRuns, n);
-  NormuonTable tab;
+  NormuonTable<kGroupRuns> tab;
   tab.n = n;
   long long total = 0;
   unsigned widest = 1;
@@ -614,8 +618,12 @@ extern "C" int dionw_normuon_rows_group(int n, const float* const* s, const int6
     widest = ctas > widest ? ctas : widest;
   }
   DIONW_REQUIRE(total * widest < (1LL << 31), "normuon_rows: too many blocks");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   count_launch();
-  return check_cuda(launch_clusters(normuon_rows_kernel, unsigned(total), widest, kReduceThreads, static_cast<cudaStream_t>(stream_ptr), tab, eps),
+  if (n == 1)
+    return check_cuda(launch_clusters(normuon_rows_kernel<1>, unsigned(total), widest, kReduceThreads, stream, NormuonTable<1>{{tab.run[0]}, 1}, eps),
+                      "normuon_rows_kernel");
+  return check_cuda(launch_clusters(normuon_rows_kernel<kGroupRuns>, unsigned(total), widest, kReduceThreads, stream, tab, eps),
                     "normuon_rows_kernel");
 }
 
