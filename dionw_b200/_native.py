@@ -235,7 +235,7 @@ def select_rows(scores: Tensor, sumsq: Tensor, k: int, index: Tensor, rowmap: Te
 
 
 def select_rows_group(runs: Sequence[tuple[Tensor, Tensor, int, Tensor, Tensor, Tensor]]) -> None:
-    """``select_rows`` of up to ``NS_GROUP_MAX`` runs in one launch; a run is the arguments of that."""
+    """``select_rows`` of up to ``NS_GROUP_MAX`` runs in one launch or a few; a run is the arguments of that."""
     scores, sumsq, ks, index, rowmap, frob = zip(*runs)
     _check(library().dionw_select_rows_group(
         len(runs), _ptr_array(scores), _ptr_array(sumsq), _i64_array([t.shape[0] for t in sumsq]),
@@ -386,7 +386,7 @@ def normuon_rows(s: Tensor, variance: Tensor, index: Tensor | None, *, blocks: i
 
 
 def normuon_rows_group(runs: Sequence[dict[str, Any]], eps: float) -> None:
-    """``normuon_rows`` of up to ``NS_GROUP_MAX`` runs in one launch; a run is its arguments by name."""
+    """``normuon_rows`` of up to ``NS_GROUP_MAX`` runs in one launch or a few; a run is its arguments by name."""
     def values(key: str) -> list[Any]:
         return [run[key] for run in runs]
 

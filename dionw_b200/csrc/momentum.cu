@@ -11,6 +11,7 @@
 // so the fold below reproduces that order exactly: lanes are combined by
 // halving (512, 256, 128 inside a thread; 64..4 by shuffles; 2, 1 inside
 // thread 0).
+#include <algorithm>
 #include <type_traits>
 
 #include "cluster.cuh"
@@ -435,7 +436,7 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 // clusters they take 141.  A CTA per 1024 rows, because below that a pass is one step and a larger cluster
 // only adds barriers.
 //
-// A launch takes the blocks of up to six runs: the selections of a step are some 10 us of latency each on a few SMs,
+// A launch takes the blocks of up to six runs (launch_together): the selections of a step are some 10 us of latency each on a few SMs,
 // and side by side they take the time of one.  Every run keeps the cluster that its own rows ask for (the first CTAs of
 // the launch's), so that its sums have one order.
 constexpr int kKeep = 4;
@@ -448,6 +449,7 @@ struct SelectRun {
   float* frob;
   int rows, k;
   unsigned ctas;         // of a cluster that work on a block
+  unsigned blocks;
   unsigned first_block;  // blocks of the runs before
 };
 template <int kRuns>
@@ -1065,25 +1067,24 @@ extern "C" int dionw_select_rows_group(int n, const float* const* scores, const 
                                        const int64_t* rows, const int64_t* k, int32_t* const* index, int32_t* const* rowmap,
                                        float* const* frob, void* stream_ptr) {
   DIONW_REQUIRE(n >= 1 && n <= kGroupRuns, "select_rows_group: takes 1 to %d runs (got %d)", kGroupRuns, n);
-  SelectTable<kGroupRuns> tab;
-  tab.n = n;
-  long long total = 0;
-  unsigned widest = 1;
+  SelectRun runs[kGroupRuns];
   for (int i = 0; i < n; ++i) {
     DIONW_REQUIRE(blocks[i] > 0 && rows[i] > 0 && k[i] > 0 && k[i] <= rows[i], "select_rows: need 0 < k <= rows and blocks > 0");
-    DIONW_REQUIRE(rows[i] < (1LL << 30), "select_rows: too many rows");
-    const unsigned ctas = cluster_for(blocks[i], rows[i], kSelectThreads);
-    tab.run[i] = SelectRun{scores[i], sumsq[i], index[i], rowmap[i], frob[i], int(rows[i]), int(k[i]), ctas, unsigned(total)};
-    total += blocks[i];
-    widest = ctas > widest ? ctas : widest;
+    DIONW_REQUIRE(rows[i] < (1LL << 30) && blocks[i] < (1LL << 31), "select_rows: too many rows or blocks");
+    runs[i] = SelectRun{scores[i], sumsq[i], index[i], rowmap[i], frob[i], int(rows[i]), int(k[i]),
+                        cluster_for(blocks[i], rows[i], kSelectThreads), unsigned(blocks[i]), 0};
   }
-  DIONW_REQUIRE(total * widest < (1LL << 31), "select_rows: too many blocks");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  count_launch();
-  if (n == 1)
-    return check_cuda(launch_clusters(select_rows_kernel<1>, unsigned(total), widest, kSelectThreads, stream, SelectTable<1>{{tab.run[0]}, 1}),
-                      "select_rows_kernel");
-  return check_cuda(launch_clusters(select_rows_kernel<kGroupRuns>, unsigned(total), widest, kSelectThreads, stream, tab), "select_rows_kernel");
+  return launch_together(runs, n, [&](const SelectRun* run, int count, unsigned total, unsigned cluster) {
+    count_launch();
+    if (count == 1)
+      return check_cuda(launch_clusters(select_rows_kernel<1>, total, cluster, kSelectThreads, stream, SelectTable<1>{{*run}, 1}),
+                        "select_rows_kernel");
+    SelectTable<kGroupRuns> tab;
+    std::copy(run, run + count, tab.run);
+    tab.n = count;
+    return check_cuda(launch_clusters(select_rows_kernel<kGroupRuns>, total, cluster, kSelectThreads, stream, tab), "select_rows_kernel");
+  });
 }
 
 extern "C" int dionw_select_rows(const float* scores, const float* sumsq, int64_t blocks, int64_t rows, int64_t k,

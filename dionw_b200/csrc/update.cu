@@ -67,7 +67,7 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // Bounded by latency: 2 MB at most.  With one CTA per block and a row per thread, one block of 2048 x 28672
 // took 94 us and two of 7168 x 8192 about as long; on eight CTAs they take 14 and 20.
 //
-// A launch takes the blocks of up to six runs, as the row selection does: on their own the scales of six runs of a
+// A launch takes the blocks of up to six runs (launch_together), as the row selection does: on their own the scales of six runs of a
 // 1100-wide encoder took 10 us each between two weight updates.
 constexpr int kRowLanes = 8;
 
@@ -82,6 +82,7 @@ struct NormuonRun {
   float inv_count_cols, weight, step_host;
   bool normalize;
   unsigned ctas;             // of a cluster that work on a block
+  unsigned blocks;
   unsigned first_block;      // blocks of the runs before
 };
 template <int kRuns>
@@ -603,28 +604,26 @@ extern "C" int dionw_normuon_rows_group(int n, const float* const* s, const int6
                                         const float* step, const float* const* step_device, const int* normalize,
                                         float* const* denom, float* const* scale, void* stream_ptr) {
   DIONW_REQUIRE(n >= 1 && n <= kGroupRuns, "normuon_rows_group: takes 1 to %d runs (got %d)", kGroupRuns, n);
-  NormuonTable<kGroupRuns> tab;
-  tab.n = n;
-  long long total = 0;
-  unsigned widest = 1;
+  NormuonRun runs[kGroupRuns];
   for (int i = 0; i < n; ++i) {
     DIONW_REQUIRE(blocks[i] > 0 && rows[i] > 0 && k[i] > 0 && k[i] <= rows[i] && cols[i] > 0 && parts[i] >= 1 && parts[i] <= 4096,
                   "normuon_rows: bad shape");
-    DIONW_REQUIRE(rows[i] < (1LL << 31), "normuon_rows: too many rows");
-    const unsigned ctas = cluster_for(blocks[i], k[i], kReduceThreads / kRowLanes);
-    tab.run[i] = NormuonRun{s[i], variance[i], index[i], step_device[i], denom[i], scale[i], int(parts[i]), int(rows[i]), int(k[i]),
-                            1.0f / float(cols[i]), weight[i], step[i], normalize[i] != 0, ctas, unsigned(total)};
-    total += blocks[i];
-    widest = ctas > widest ? ctas : widest;
+    DIONW_REQUIRE(rows[i] < (1LL << 31) && blocks[i] < (1LL << 31), "normuon_rows: too many rows or blocks");
+    runs[i] = NormuonRun{s[i], variance[i], index[i], step_device[i], denom[i], scale[i], int(parts[i]), int(rows[i]), int(k[i]),
+                         1.0f / float(cols[i]), weight[i], step[i], normalize[i] != 0,
+                         cluster_for(blocks[i], k[i], kReduceThreads / kRowLanes), unsigned(blocks[i]), 0};
   }
-  DIONW_REQUIRE(total * widest < (1LL << 31), "normuon_rows: too many blocks");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  count_launch();
-  if (n == 1)
-    return check_cuda(launch_clusters(normuon_rows_kernel<1>, unsigned(total), widest, kReduceThreads, stream, NormuonTable<1>{{tab.run[0]}, 1}, eps),
-                      "normuon_rows_kernel");
-  return check_cuda(launch_clusters(normuon_rows_kernel<kGroupRuns>, unsigned(total), widest, kReduceThreads, stream, tab, eps),
-                    "normuon_rows_kernel");
+  return launch_together(runs, n, [&](const NormuonRun* run, int count, unsigned total, unsigned cluster) {
+    count_launch();
+    if (count == 1)
+      return check_cuda(launch_clusters(normuon_rows_kernel<1>, total, cluster, kReduceThreads, stream, NormuonTable<1>{{*run}, 1}, eps),
+                        "normuon_rows_kernel");
+    NormuonTable<kGroupRuns> tab;
+    std::copy(run, run + count, tab.run);
+    tab.n = count;
+    return check_cuda(launch_clusters(normuon_rows_kernel<kGroupRuns>, total, cluster, kReduceThreads, stream, tab, eps), "normuon_rows_kernel");
+  });
 }
 
 extern "C" int dionw_normuon_rows(const float* s, int64_t parts, float* variance, const int32_t* index, int64_t blocks,

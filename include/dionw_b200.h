@@ -116,8 +116,8 @@ int dionw_select_rows(const float* scores, const float* sumsq, int64_t blocks,
                       int64_t rows, int64_t k, int32_t* index, int32_t* rowmap,
                       float* frob, void* stream);
 
-/* The same for n (1 to 6) runs in one launch.  The results are those of one call
- * each. */
+/* The same for n (1 to 6) runs, in one launch where their blocks are few enough to be
+ * worked on at the same time.  The results are those of one call each. */
 int dionw_select_rows_group(int n, const float* const* scores, const float* const* sumsq,
                             const int64_t* blocks, const int64_t* rows, const int64_t* k,
                             int32_t* const* index, int32_t* const* rowmap,
@@ -279,7 +279,7 @@ int dionw_normuon_rows(const float* s, int64_t parts, float* variance, const int
                        float weight, float eps, float step, const float* step_device,
                        int normalize, float* denom, float* scale, void* stream);
 
-/* The same for n (1 to 6) runs in one launch; index[i] and step_device[i] may be
+/* The same for n (1 to 6) runs, in as few launches; index[i] and step_device[i] may be
  * NULL as there.  The results are those of one call each. */
 int dionw_normuon_rows_group(int n, const float* const* s, const int64_t* parts,
                              float* const* variance, const int32_t* const* index,

@@ -191,3 +191,36 @@ def test_selections_and_scales_of_several_runs_in_one_launch() -> None:
         assert all(torch.equal(run[key], alone[key]) for key in ("variance", "denom", "scale"))
     with pytest.raises(ValueError, match="1 to 6"):
         native.select_rows_group(together + together[:1])
+
+
+def test_many_narrow_blocks_beside_a_wide_one_have_their_own_launch() -> None:
+    """Blocks of one CTA would otherwise each take the eight of the widest run; same values either way."""
+    gen = _gen(2)
+    shapes = [(300, 128, 32), (1, 9000, 2000), (2, 4000, 1024), (500, 100, 100)]   # blocks, rows, k
+
+    def runs() -> tuple[list, list]:
+        selections, scales = [], []
+        for i, (blocks, rows, k) in enumerate(shapes):
+            scores = torch.rand(blocks, rows, device=DEV, generator=_gen(i))
+            index = torch.full((blocks, k), -7, dtype=torch.int32, device=DEV)
+            selections.append((scores, scores.square(), k, index, torch.full((blocks, rows), -7, dtype=torch.int32, device=DEV),
+                               torch.full((blocks,), 7.0, device=DEV)))
+            scales.append({"s": torch.rand(blocks * k, 2, device=DEV, generator=_gen(i)) + 0.1, "parts": 2,
+                           "variance": torch.rand(blocks, rows, device=DEV, generator=_gen(i)), "index": index, "blocks": blocks, "rows": rows,
+                           "k": k, "cols": 500, "weight": 0.05, "step": -0.01, "step_device": None, "normalize": True,
+                           "denom": torch.zeros(blocks * k, device=DEV), "scale": torch.zeros(blocks, device=DEV)})
+        return selections, scales
+
+    (together, grouped), (alone, single) = runs(), runs()
+    before = native.launch_count()
+    native.select_rows_group(together)
+    native.normuon_rows_group(grouped, 1e-8)
+    assert native.launch_count() - before == 2 + 2   # the two wide runs, the two narrow ones
+    for run, own, group, lone in zip(together, alone, grouped, single):
+        native.select_rows(*own)
+        native.normuon_rows(**lone, eps=1e-8)
+        assert all(torch.equal(run[i], own[i]) for i in (3, 4, 5))
+        assert all(torch.equal(group[key], lone[key]) for key in ("variance", "denom", "scale"))
+    before = native.launch_count()
+    native.select_rows_group(together[1:3])
+    assert native.launch_count() - before == 1
