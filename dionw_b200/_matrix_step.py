@@ -361,8 +361,8 @@ def step_runs(runs: Sequence[tuple[Bucket, Sequence[int]]], param_groups: Sequen
     """One Dion step for several runs (one entry of ``groups_of_runs``; their parameter groups may differ),
     stage by stage.
 
-    Their row selections, their Newton-Schulz iterations and their NorMuon scales run as one launch each: the
-    first and the last are a few blocks that wait for memory, 5 to 15 us each on their own.  An iteration is a chain of 15 to 18 products;
+    Their row selections and their NorMuon scales share launches: a few blocks that wait for memory, 5 to 15 us
+    each on their own.  Their Newton-Schulz iterations run as one launch: an iteration is a chain of 15 to 18 products;
     on small blocks each is one part-filled wave and most of its time is the way from one product to
     the next, which the products of the other runs fill.  Same kernels on the same values: the
     results are those of ``step_run`` on each."""
