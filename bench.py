@@ -150,15 +150,17 @@ def flops_newton_schulz(m: int, n: int) -> float:
     return 2.0 * (3.0 * m * m * n + 11.5 * m**3)
 
 
-# DRAM bytes the products of one Gram Newton-Schulz move for an m x n operand: the operand census
-# 2 B x (6 m n + 40 m^2) (every product reads its operands and writes its result once) times 1.06,
-# the ratio an ncu capture of the 18 products of four 3584 x 4096 blocks measured against it
-# (1.278 GB per block; dram__bytes_read.sum + dram__bytes_write.sum).
-NS_TRAFFIC_CALIBRATION = 1.06
-
-
-def traffic_newton_schulz(m: int, n: int) -> float:
-    return NS_TRAFFIC_CALIBRATION * 2.0 * (6.0 * m * n + 40.0 * m * m)
+def traffic_newton_schulz(m: int, n: int, on_chip: bool = False) -> float:
+    """DRAM bytes of one orthogonalization of an m x n operand (m <= n): every product reads each matrix
+    it takes and writes its results once, and a symmetric matrix consists of its 256 x 256 blocks up to the
+    diagonal.  An ncu capture of four 3584 x 4096 operands (dram__bytes_read.sum + dram__bytes_write.sum)
+    has 0.763 GB each, this 0.768.  On chip only the operand moves."""
+    symmetric = sum(min(256, m - first) * min(m, first + 256) for first in range(0, m, 256))
+    if on_chip:
+        return 2.0 * 6.0 * m * n
+    if m == n:
+        return 2.0 * (15.0 * m * n + 20.0 * symmetric)
+    return 2.0 * (6.0 * m * n + 43.0 * symmetric)
 
 
 def flops_newton_schulz_executed(m: int, n: int) -> float:
@@ -303,6 +305,17 @@ def split_ns_shapes(stages: dict[str, float], blocks: dict[str, int], steps: int
                      "algorithmic_TFLOP/s": count * flops_newton_schulz(m, n) / ms / 1e9 if ms else None})
     blocks.clear()
     return rows
+
+
+def iterated_on_chip(by_operand: list[dict]) -> bool:
+    """Whether a step's Newton-Schulz iterations ran on chip: one run whose blocks are small enough (several
+    runs are one plan of products)."""
+    from dionw_b200 import _native
+
+    if len(by_operand) != 1:
+        return False
+    m, n = by_operand[0]["operand"]
+    return _native.newton_schulz_on_chip_pairs(round(by_operand[0]["blocks"]), m, n, _native.NS_GRAM) > 0
 
 
 def measured_peaks() -> tuple[dict, str]:
@@ -1106,6 +1119,10 @@ def run_gpu_arm(args) -> None:
 
     peaks, peaks_kind = measured_peaks()
     share = 1.0 / world  # matrix blocks and the AdamW space are sharded evenly by cost
+    on_chip = not distributed and iterated_on_chip(ns_by_shape)
+    ns_traffic = work["ns_traffic"] * share
+    if on_chip:
+        ns_traffic = ns_by_shape[0]["blocks"] * traffic_newton_schulz(*ns_by_shape[0]["operand"], on_chip=True)
     ns_ms = stages.get("newton_schulz", 0.0)
     ns_tflops = work["ns_flops"] * share / ns_ms / 1e9 if ns_ms else None
     ns_exec_tflops = work["ns_flops_executed"] * share / ns_ms / 1e9 if ns_ms else None
@@ -1192,14 +1209,16 @@ def run_gpu_arm(args) -> None:
                    "gradients": ("one tensor per shape shared by all layers (weights + gradients would not fit "
                                  "beside the state)" if shared_grads else "one tensor per parameter")},
         "roofline": {
-            "kernel": "gemm2_kernel (all Newton-Schulz products of a step)",
+            "kernel": ("onchip::iteration_kernel (the Newton-Schulz iteration of the step's one run)" if on_chip
+                       else "gemm2_kernel (all Newton-Schulz products of a step)"),
             "bound": "tensor", "achieved": ns_exec_tflops, "peak": peak_tf, "unit": "TFLOP/s",
-            "frac": ns_exec_tflops / peak_tf if ns_exec_tflops else None, "traffic": work["ns_traffic"] * share,
+            "frac": ns_exec_tflops / peak_tf if ns_exec_tflops else None, "traffic": ns_traffic,
             "achieved_kind": ("FLOPs the kernels execute, 2(3m^2n + 7m^3) per m x n operand (the products Q Z, G Z and "
                               "Z RZ run on the lower-triangle schedule), / the summed CUDA-event time of the stage"),
-            "traffic_kind": ("DRAM bytes of all gemm2_kernel launches of one step on this rank: the operand census "
-                             "of the products, calibrated x1.06 on an ncu capture of the 18 products of four "
-                             "3584x4096 blocks and scaled by blocks (traffic grows with the blocks processed)"),
+            "traffic_kind": ("DRAM bytes of the Newton-Schulz kernels of one step on this rank: every matrix a product "
+                             "takes read once and every result written once, symmetric ones up to their diagonal "
+                             "blocks (0.994 of it measured in an ncu capture of four 3584x4096 operands), "
+                             "summed over the blocks"),
             "peak_kind": f"{peaks_kind} bf16 cuBLAS, sustained (the kernel is timed inside the step)",
             "flops_per_step": work["ns_flops_executed"] * share,
             "algorithmic": {"TFLOP/s": ns_tflops, "flops_per_step": work["ns_flops"] * share,

@@ -33,6 +33,15 @@ def test_llama3_8b_census() -> None:
     assert total == pytest.approx(160.5e9, rel=2e-3)           # 20 E + 12 Es
 
 
+def test_newton_schulz_traffic_counts_symmetric_matrices_up_to_the_diagonal() -> None:
+    # the bytes an ncu capture of the plan counted for one gate/up operand
+    assert bench.traffic_newton_schulz(3584, 4096) == pytest.approx(0.763e9, rel=0.02)
+    # one 256-row block: nothing lies past the diagonal
+    assert bench.traffic_newton_schulz(200, 1000) == 2 * (6 * 200 * 1000 + 43 * 200 * 200)
+    assert bench.traffic_newton_schulz(512, 512) == 2 * (15 * 512**2 + 20 * (256 * 256 + 256 * 512))
+    assert bench.traffic_newton_schulz(256, 1024, on_chip=True) == 12 * 256 * 1024
+
+
 def test_gpt2_small_census_takes_the_full_row_path() -> None:
     work = bench.census(_groups("gpt2-small"))
     assert work["matrix_elements"] == work["selected_elements"] == 12 * (768 * 2304 + 768 * 768 + 2 * 768 * 3072)
