@@ -468,11 +468,12 @@ int pairs_per_matrix(int64_t blocks, int64_t tiles) {
 
 }  // namespace
 
-// On chip a chain of products takes 14 x 2.4 us whatever the rest of the GPU does, but every pair sums the whole Gram
-// matrix (0.26 us per 64 columns of n) and a batch takes whole waves of clusters.  Iteration as a plan against on
-// chip, us, m = 256: 1 block of n = 1024 107 and 69, 4096 129 and 109, 8192 157 and 162; 37 blocks 130 and 84, 192 and
-// 162, 285 and 296; 74 blocks (one wave) 182 and 89, 318 and 220, 463 and 388; 160 (two and a bit) of 1024 282 and 261,
-// of 2048 379 and 412.  m = 96: 1 block of 1024 89 and 43, of 8192 138 and 126; 160 of 1024 196 and 152.
+// On chip a chain of products takes 14 x 2.8 us (m = 256) whatever the rest of the GPU does, but every pair sums the whole
+// Gram matrix (0.27 us per 64 columns of n, twice) and a batch takes whole waves of clusters.  Iteration as a plan against on
+// chip, us, m = 256: 1 block of n = 1024 105 and 69, 4096 126 and 102, 6144 140 and 125; 37 blocks of 1024 129 and 83, 4096
+// 189 and 162; 74 blocks (one wave) 178 and 91, 310 and 223; 160 (two and a bit) of 1024 303 and 257.  m = 96: 1 block of 1024
+// 82 and 42; 160 of 1024 190 and 155.  The lines were drawn where, with four pairs to a matrix, the two met; with eight it is
+// still ahead behind them: 1 block of 8192 154 and 147, 74 of 8192 529 and 425, 160 of 2048 418 and 340.
 constexpr int64_t kOnChipColumns = 6144, kOnChipColumnsInWaves = 1024;
 
 int on_chip_pairs(int64_t blocks, int64_t m, int64_t n) {

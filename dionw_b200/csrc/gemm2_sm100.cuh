@@ -30,10 +30,10 @@
 // that run out of tiles of one product go on with the next one's, so only the last product of a plan ends in a
 // part-filled wave; the start of a product (launch, descriptor fetch, first loads) and the end of the one
 // before (last epilogue, teardown) overlap across matrices; and the host makes one launch where it made 15 to 18.
-// Measured, an iteration as one launch per product against one plan: 16 blocks of 1024^2 453 -> 380 us,
-// 16 of 1024 x 4096 805 -> 720 us, 1 of 256 x 1024 146 -> 143 us; the four batches of a 12-layer 768-wide
-// language model 1259 -> 900 us, the six of a 1100-wide image encoder 3.3 -> 1.9 ms, a 4-layer 4096-wide
-// one's four 8.9 -> 8.0 ms.  A plan's matrices need not lie in L2 for that: running them in cohorts of two
+// Measured, an iteration as one launch per product against one plan, replayed from a graph: 16 blocks of 1024^2
+// 443 -> 325 us, 16 of 1024 x 4096 810 -> 700 us, 1 of 256 x 1024 137 -> 108 us; the four batches of a 12-layer 768-wide
+// language model 1108 -> 893 us, the six of a 1100-wide image encoder 964 -> 271 us, a 4-layer 4096-wide
+// one's four 7.5 -> 7.1 ms.  A plan's matrices need not lie in L2 for that: running them in cohorts of two
 // waves of tiles, each through all its products, changed nothing.
 //
 // What bounds it now, with clocks read inside the kernel, in cycles per tile (main loop / whole): K = 3584 29700 / 31800
@@ -92,7 +92,7 @@ __device__ __forceinline__ void remote_arrive_after(uint32_t cluster_address, in
 }
 
 // An entry of the tile ring: the product of the plan (negative: no more tiles), the tile of it, and what the
-// loads and the main loop need to know about the two (see Ranges), so that neither waits for the parameters of a
+// loads and the main loop need to know about the two (see entry_of), so that neither waits for the parameters of a
 // product it has not met yet: read from the kernel's arguments they took 700 cycles between tile and first load.
 struct alignas(16) Entry {
   int step, batch, tm, tn;
@@ -330,8 +330,8 @@ __device__ __forceinline__ bool elect_one() {
   return one != 0;
 }
 
-// Orders this thread's accesses through the generic proxy (ordinary loads and stores) with those of the
-// async proxy (TMA) on both sides.
+// Orders this thread's accesses to global memory through the generic proxy (ordinary loads and stores) with those of
+// the async proxy (TMA) on both sides.
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 // Bounded wait until the progress of a matrix has reached `need`.
@@ -367,7 +367,7 @@ __device__ __forceinline__ bool progress_wait(const unsigned* progress, unsigned
 // index, finds the product and the tile that it stands for, and publishes them to every consumer of the pair
 // through a ring of kTileSlots entries kept in BOTH CTAs' shared memory: it writes its own copy and arrives on
 // the slot's `tile_full` barrier, and sends the peer's, where the bytes themselves complete the phase that the
-// peer's scheduler has armed.  Consumers -- the leader's MMA thread, the producer thread and the epilogue warps
+// peer's scheduler has armed.  Consumers -- the leader's MMA issuer, the producer and the epilogue warps
 // of each CTA, the peer's scheduler -- wait on their own
 // CTA's `tile_full` (acquire at cluster scope), read the entry and arrive on the LEADER's `tile_empty`
 // barrier of the slot; the scheduler reuses a slot after all of them have done so.  A negative step ends the pair's work.
@@ -496,62 +496,60 @@ gemm2_kernel(const __grid_constant__ Plan<kMaps, kSteps> plan) {
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     // A whole warp of which one elected lane issues, as in the MMA issuer.
-    {
-      int s = 0;                 // stage of the ring, and the parity that its slot's next release has
-      uint32_t released = 1;
-      bool ok = true;
-      const uint32_t ring = smem_u32(smem), leader_full = peer_address(full_bar, 0);
-      for (uint32_t n = 0; ok; ++n) {
-        const Entry tile = take_tile(n, true, kWholeEntry);
-        if (tile.step < 0) break;
-        const bool shared = (tile.flags & kSharedFlag) != 0;
-        const int tile_n = (tile.flags & kWideFlag) != 0 ? kBN : kBN / 2, half_n = tile_n / 2;
-        const int m0 = tile.tm * kPairM + int(rank) * kBM;
-        const int n0 = tile.tn * tile_n + int(rank) * half_n;
-        // the k-block after whose loads this pair's next tile may be drawn
-        const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? tile.k_blocks - 1 : max(0, tile.k_blocks - kDrawAhead);
-        const uint32_t pair_bytes = 2 * (kABytes + (shared ? 0u : uint32_t(half_n) * kBK * 2));
-        // The layout of the operands is a constant inside the loop.
-        auto load_loop = [&](int begin, int end, auto a_major_mn, auto b_major_mn) {
-          constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
-          if (!ok || begin >= end) return;
-          const CUtensorMap* map_a = &plan.maps[kAMN ? tile.map_a_mn : tile.map_a];
-          const CUtensorMap* map_b = &plan.maps[kBMN ? tile.map_b_mn : tile.map_b];
-          for (int kb = begin; kb < end; ++kb) {
-            if (!warp_wait(&empty_bar[s], released)) { ok = false; break; }
-            const uint32_t a_dst = ring + uint32_t(s) * kStageBytes, b_dst = a_dst + kABytes;
-            const uint32_t landed = leader_full + uint32_t(s) * uint32_t(sizeof(uint64_t));
-            const int k0 = kb * kBK;
-            if (elect_one()) {
-              // The peer's bytes may land before the leader has announced them: the phase still
-              // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
-              // because its empty barrier is released by the MMAs that consumed this one.
-              if (rank == 0) mbar_expect_tx(&full_bar[s], pair_bytes);
-              if constexpr (kAMN) {
+    int s = 0;                 // stage of the ring, and the parity that its slot's next release has
+    uint32_t released = 1;
+    bool ok = true;
+    const uint32_t ring = smem_u32(smem), leader_full = peer_address(full_bar, 0);
+    for (uint32_t n = 0; ok; ++n) {
+      const Entry tile = take_tile(n, true, kWholeEntry);
+      if (tile.step < 0) break;
+      const bool shared = (tile.flags & kSharedFlag) != 0;
+      const int tile_n = (tile.flags & kWideFlag) != 0 ? kBN : kBN / 2, half_n = tile_n / 2;
+      const int m0 = tile.tm * kPairM + int(rank) * kBM;
+      const int n0 = tile.tn * tile_n + int(rank) * half_n;
+      // the k-block after whose loads this pair's next tile may be drawn
+      const int draw_at = !dynamic || rank != 0 ? -1 : n == 0 ? tile.k_blocks - 1 : max(0, tile.k_blocks - kDrawAhead);
+      const uint32_t pair_bytes = 2 * (kABytes + (shared ? 0u : uint32_t(half_n) * kBK * 2));
+      // The layout of the operands is a constant inside the loop.
+      auto load_loop = [&](int begin, int end, auto a_major_mn, auto b_major_mn) {
+        constexpr bool kAMN = decltype(a_major_mn)::value, kBMN = decltype(b_major_mn)::value;
+        if (!ok || begin >= end) return;
+        const CUtensorMap* map_a = &plan.maps[kAMN ? tile.map_a_mn : tile.map_a];
+        const CUtensorMap* map_b = &plan.maps[kBMN ? tile.map_b_mn : tile.map_b];
+        for (int kb = begin; kb < end; ++kb) {
+          if (!warp_wait(&empty_bar[s], released)) { ok = false; break; }
+          const uint32_t a_dst = ring + uint32_t(s) * kStageBytes, b_dst = a_dst + kABytes;
+          const uint32_t landed = leader_full + uint32_t(s) * uint32_t(sizeof(uint64_t));
+          const int k0 = kb * kBK;
+          if (elect_one()) {
+            // The peer's bytes may land before the leader has announced them: the phase still
+            // cannot complete before the leader's arrive, and the peer cannot run a phase ahead
+            // because its empty barrier is released by the MMAs that consumed this one.
+            if (rank == 0) mbar_expect_tx(&full_bar[s], pair_bytes);
+            if constexpr (kAMN) {
 #pragma unroll
-                for (int panel = 0; panel < kBM / 64; ++panel)
-                  tma_load_3d_pair(a_dst + panel * kPanelBytes, map_a, landed, m0 + panel * 64, k0, tile.batch);
-              } else {
-                tma_load_3d_pair(a_dst, map_a, landed, k0, m0, tile.batch);
-              }
-              if (!shared) {
-                if constexpr (kBMN) {
-                  tma_load_3d_pair(b_dst, map_b, landed, n0, k0, tile.batch);
-                  if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, landed, n0 + 64, k0, tile.batch);
-                } else {
-                  tma_load_3d_pair(b_dst, map_b, landed, k0, n0, tile.batch);
-                }
-              }
-              if (kb == draw_at) mbar_arrive(may_draw);
+              for (int panel = 0; panel < kBM / 64; ++panel)
+                tma_load_3d_pair(a_dst + panel * kPanelBytes, map_a, landed, m0 + panel * 64, k0, tile.batch);
+            } else {
+              tma_load_3d_pair(a_dst, map_a, landed, k0, m0, tile.batch);
             }
-            __syncwarp();
-            if (++s == kStages) s = 0, released ^= 1u;
+            if (!shared) {
+              if constexpr (kBMN) {
+                tma_load_3d_pair(b_dst, map_b, landed, n0, k0, tile.batch);
+                if (half_n > 64) tma_load_3d_pair(b_dst + kPanelBytes, map_b, landed, n0 + 64, k0, tile.batch);
+              } else {
+                tma_load_3d_pair(b_dst, map_b, landed, k0, n0, tile.batch);
+              }
+            }
+            if (kb == draw_at) mbar_arrive(may_draw);
           }
-        };
-        load_loop(0, tile.b_end, std::false_type(), std::false_type());
-        load_loop(tile.b_end, tile.a_end, std::false_type(), std::true_type());
-        load_loop(tile.a_end, tile.k_blocks, std::true_type(), std::true_type());
-      }
+          __syncwarp();
+          if (++s == kStages) s = 0, released ^= 1u;
+        }
+      };
+      load_loop(0, tile.b_end, std::false_type(), std::false_type());
+      load_loop(tile.b_end, tile.a_end, std::false_type(), std::true_type());
+      load_loop(tile.a_end, tile.k_blocks, std::true_type(), std::true_type());
     }
   } else if (warp == 1) {
     if (rank == 0) {   // the second CTA's MMA warp has nothing to issue

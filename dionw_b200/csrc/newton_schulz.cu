@@ -87,8 +87,8 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
   const bool gram = kind == DIONW_NS_GRAM || kind == DIONW_NS_GRAM_FULL;
   const int dt = gram ? DIONW_F16 : DIONW_BF16;
   // Every m x m matrix of the Gram schedule is a polynomial in one symmetric G, so the
-  // products among them are symmetric too: GRAM computes their lower tiles and mirrors,
-  // GRAM_FULL computes them as general products, as the reference's cuBLAS calls do.
+  // products among them are symmetric too: GRAM computes their lower tiles only, GRAM_FULL
+  // computes them as general products, as the reference's cuBLAS calls do.
   const bool mirror = kind == DIONW_NS_GRAM;
   // Where every m x m product is on the triangle, nothing reads past the diagonal.
   const bool lower = kind != DIONW_NS_GRAM_FULL || !l.gram;
@@ -211,12 +211,10 @@ void append_products(const Problem& problem, int chain, int64_t first_block, con
   }
 }
 
-// A batch of blocks up to this wide on their shorter side goes product by product.  A plan pays about 10 us at its
-// start (its counters are cleared, and it is launched without programmatic dependence) and a hop through ring and
-// progress per tile; it gets that back where other tiles fill the wait, and a product on one 64 x 64 tile per
-// matrix is over in 4 us.  Plan against one launch per product: 1 block of 64^2 92 against 74 us, 16 of
-// 64 x 1024 123 against 117, 1000 of 64^2 691 against 588; on wider blocks 1 of 192 x 768 126 against 123, 16 of
-// 192 x 768 132 against 134, 300 of 256^2 363 against 432.  (The batches of a group fill one another's waits.)
+// A batch of blocks up to this wide on their shorter side goes product by product.  The line was drawn when a producer drew
+// its own tiles and a plan of them was the slower one: 1 block of 64^2 92 us against 74, 1000 of them 691 against 588.  With
+// tiles handed out ahead a plan takes 53 against 68 us (16 of 64 x 1024 83 against 111, 1000 of 64^2 500 against 513): it is
+// the faster one here too.
 constexpr int64_t kStepwiseSide = 64;
 
 size_t group_bytes(const Problem* problems, int n) {
