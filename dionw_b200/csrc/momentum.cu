@@ -167,6 +167,14 @@ inline int team_whole_columns(int span, bool bf16, long long rows) {
 // 1500 x 1024 off the boundary 8.4 / 11.2 / 7.7; of bf16 30000 x 1001 189 / 157 / 126.
 inline int team_rows(long long cols, bool vec) { return cols <= 1024 && vec ? 4 : cols <= 2048 ? 2 : 1; }
 
+// Runs of six to eight rows an SM: one even wave of warps, eight to an SM, but the beginning of a second wave of teams.
+// fp32, a warp to a row against a team, us: copies of 1024 x 1024 4.5 and 5.1, 1184 x 1022 5.5 and 7.3, 1100 x 1999 9.9
+// and 10.8, scores of 1100 x 1202 6.1 and 7.0; 860 x 1022 5.2 and 4.7, 1200 x 1022 8.6 and 7.4; 1024 x 1280 (16-byte accesses) 6.0 and
+// 5.9.  (16-bit gradients 1000 x 1001 8.6 and 7.7.)
+inline bool one_wave_of_warps(int grad_dtype, bool vec, long long cols, long long rows) {
+  return grad_dtype == DIONW_F32 && rows > 6 * sm_count() && rows <= 8 * sm_count() && cols <= (vec ? 1024 : 2048);
+}
+
 // Calls fn(std::integral_constant<int, rows at a time>).
 template <typename Fn>
 auto with_team_rows(long long cols, bool vec, Fn&& fn) {
@@ -1004,7 +1012,7 @@ extern "C" int dionw_accumulate_row_l1_run(const void* const* grads, int grad_dt
     if (nrows == 0) return DIONW_OK;
     const unsigned grid = unsigned((nrows + kWarpsPerBlock - 1) / kWarpsPerBlock);
     float* m = momentum + row0 * cols;
-    if (cols >= kTeamScoreColumns) {
+    if (cols >= kTeamScoreColumns && !one_wave_of_warps(grad_dtype, vec, cols, nrows)) {
       auto launch = [&](auto g) {
         with_team_rows(cols, vec, [&](auto n) {
           constexpr int kRows = decltype(n)::value < 2 ? 1 : 2;   // of the kernel and of its grid; four need too many sums
@@ -1041,7 +1049,7 @@ extern "C" int dionw_accumulate_copy_decay_run(const void* const* grads, int gra
     float* m = momentum + row0 * cols;
     float* out = u + row0 * cols;
     const bool nest = nesterov != 0;
-    if (cols >= kTeamCopyColumns) {
+    if (cols >= kTeamCopyColumns && !one_wave_of_warps(grad_dtype, vec, cols, nrows)) {
       auto launch = [&](auto g) {
         with_team_rows(cols, vec, [&](auto n) {
           launch_dependent(team_accumulate_copy_decay_kernel<decltype(g), decltype(n)::value>, unsigned((nrows + n - 1) / n), kTeamThreads, stream, tab,

@@ -92,6 +92,23 @@ def test_pack(cols: int, dtype: torch.dtype, selecting: bool) -> None:
     assert torch.equal(after, source)
 
 
+@pytest.mark.parametrize("per_sm", [6, 7, 8, 9])
+@pytest.mark.parametrize("cols", [1001, 1024, 1026, 2048])
+def test_accumulate_a_wave_of_rows(per_sm: int, cols: int) -> None:
+    """About as many rows as a wave of warps takes, where the launch changes with their number."""
+    rows = per_sm * torch.cuda.get_device_properties(DEV).multi_processor_count + 1 - (per_sm == 8)
+    gen = _gen(cols)
+    grad, start = torch.randn(rows, cols, device=DEV, generator=gen), torch.randn(1, rows, cols, device=DEV, generator=gen)
+    total = start[0] + grad
+    scores, sumsq = (torch.full((1, rows), 7.0, device=DEV) for _ in range(2))
+    momentum, u = start.clone(), torch.empty_like(start)
+    native.accumulate_copy_decay_run([grad], [rows], momentum, u, sumsq, cols, 0.95, False)
+    assert torch.equal(momentum[0], total * 0.95) and torch.equal(u[0], total)
+    momentum = start.clone()
+    native.accumulate_row_l1_run([grad], [rows], momentum, scores, sumsq, cols)
+    assert torch.equal(momentum[0], total) and torch.equal(scores.cpu(), oracle.row_scores(total.cpu()).view(1, -1))
+
+
 # whole blocks on both sides of each line at which the launch changes with the number of rows
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("rows, cols", [(4096, 1025), (4097, 1025), (4097, 1602), (8192, 1601), (8193, 1601), (8193, 2561), (8192, 2560), (8193, 2560),
