@@ -1083,7 +1083,7 @@ extern "C" int dionw_select_rows_group(int n, const float* const* scores, const 
                         cluster_for(blocks[i], rows[i], kSelectThreads), unsigned(blocks[i]), 0};
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  return launch_together(runs, n, [&](const SelectRun* run, int count, unsigned total, unsigned cluster) {
+  return launch_together(runs, n, 3 * sm_count() / 2, [&](const SelectRun* run, int count, unsigned total, unsigned cluster) {
     count_launch();
     if (count == 1)
       return check_cuda(launch_clusters(select_rows_kernel<1>, total, cluster, kSelectThreads, stream, SelectTable<1>{{*run}, 1}),
