@@ -1,8 +1,8 @@
 // Kernel launches: clusters (rank, barrier, the other CTAs' shared memory) and programmatic dependence.
 #pragma once
 
-#include <algorithm>
 #include <cstdint>
+#include <utility>
 
 #include <cuda_runtime.h>
 
@@ -105,14 +105,16 @@ cudaError_t launch_clusters(void (*kernel)(Params...), unsigned blocks, unsigned
 // Calls launch(first run, runs, blocks, cluster) for launches that take all n runs of `runs`, which it puts in the order
 // of their clusters (Run::ctas, the CTAs that a block's sums are made by) and whose Run::first_block it fills in.  Every
 // block of a launch gets the widest cluster of its runs, whose other CTAs only keep the barriers: narrower runs go along up to
-// `limit` CTAs.  A launch against one per run, us, beside 1 x 4096 rows with 1024 selected: selections (an SM holds one CTA) of
+// `per_two_sms` CTAs to two SMs.  A launch against one per run, us, beside 1 x 4096 rows with 1024 selected: selections (an SM holds one CTA) of
 // 16 x 128 16 and 26, 228 CTAs 24 and 26, beside 8 x 4096 256 CTAs 28 and 27, 288 36 and 27, beside one 1000 x 128 365 and 85;
 // scales (it holds two) 256 CTAs 6.9 and 9.3, 312 9.9 and 9.3, 368 10.4 and 9.2, 520 11.6 and 9.1, 1000 x 128 147 and 25.  (Alone; in a
 // step a launch more is one more of some 3 us, so that the scales' line lies past where the two meet: 1100-wide encoder, 304 CTAs, a
 // step 736 us with one launch, 739 with two.)
 template <typename Run, typename Launch>
-int launch_together(Run* runs, int n, long long limit, Launch&& launch) {
-  std::stable_sort(runs, runs + n, [](const Run& a, const Run& b) { return a.ctas > b.ctas; });
+int launch_together(Run* runs, int n, int per_two_sms, Launch&& launch) {
+  for (int i = 1; i < n; ++i)   // six at most
+    for (int j = i; j > 0 && runs[j].ctas > runs[j - 1].ctas; --j) std::swap(runs[j], runs[j - 1]);
+  const long long limit = n > 1 ? per_two_sms * sm_count() / 2 : 0;
   for (int first = 0, last = 0; first < n; first = last) {
     const long long widest = runs[first].ctas;
     long long blocks = 0;

@@ -172,7 +172,7 @@ inline int team_rows(long long cols, bool vec) { return cols <= 1024 && vec ? 4 
 // and 10.8, scores of 1100 x 1202 6.1 and 7.0; 860 x 1022 5.2 and 4.7, 1200 x 1022 8.6 and 7.4; 1024 x 1280 (16-byte accesses) 6.0 and
 // 5.9.  (16-bit gradients 1000 x 1001 8.6 and 7.7.)
 inline bool one_wave_of_warps(int grad_dtype, bool vec, long long cols, long long rows) {
-  return grad_dtype == DIONW_F32 && rows > 6 * sm_count() && rows <= 8 * sm_count() && cols <= (vec ? 1024 : 2048);
+  return cols <= (vec ? 1024 : 2048) && grad_dtype == DIONW_F32 && rows > 6 * sm_count() && rows <= 8 * sm_count();
 }
 
 // Calls fn(std::integral_constant<int, rows at a time>).
@@ -1083,7 +1083,7 @@ extern "C" int dionw_select_rows_group(int n, const float* const* scores, const 
                         cluster_for(blocks[i], rows[i], kSelectThreads), unsigned(blocks[i]), 0};
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  return launch_together(runs, n, 3 * sm_count() / 2, [&](const SelectRun* run, int count, unsigned total, unsigned cluster) {
+  return launch_together(runs, n, 3, [&](const SelectRun* run, int count, unsigned total, unsigned cluster) {
     count_launch();
     if (count == 1)
       return check_cuda(launch_clusters(select_rows_kernel<1>, total, cluster, kSelectThreads, stream, SelectTable<1>{{*run}, 1}),

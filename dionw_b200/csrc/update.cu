@@ -614,7 +614,7 @@ extern "C" int dionw_normuon_rows_group(int n, const float* const* s, const int6
                          cluster_for(blocks[i], k[i], kReduceThreads / kRowLanes), unsigned(blocks[i]), 0};
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  return launch_together(runs, n, 5 * sm_count() / 2, [&](const NormuonRun* run, int count, unsigned total, unsigned cluster) {
+  return launch_together(runs, n, 5, [&](const NormuonRun* run, int count, unsigned total, unsigned cluster) {
     count_launch();
     if (count == 1)
       return check_cuda(launch_clusters(normuon_rows_kernel<1>, total, cluster, kReduceThreads, stream, NormuonTable<1>{{*run}, 1}, eps),
